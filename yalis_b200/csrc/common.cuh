@@ -60,6 +60,8 @@ inline int yalis_sm_count() {
 // its last tile: blocks of the next kernels that start earlier fill their rings with bandwidth that
 // this kernel's own tiles still wait for, and hold registers and shared memory that its later
 // blocks need (measured: 9 % of a batch-64 decode step).
+// Kernels that hold few blocks for long (a recurrence's walk over a prompt) are launched without the attribute
+// (yalis_launch_after): let in early, their blocks would all land on the SMs that come free first.
 bool yalis_pdl_enabled();   // defined in elementwise.cu; switched by yalis_set_pdl()
 
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
@@ -78,6 +80,17 @@ inline int yalis_launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t 
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = yalis_pdl_enabled() ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...) == cudaSuccess ? YALIS_OK : YALIS_ERR_LAUNCH;
+}
+
+// The same without the attribute: the grid starts when the kernel in front has ended, on an empty GPU.
+template <typename... KArgs, typename... Args>
+inline int yalis_launch_after(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...) == cudaSuccess ? YALIS_OK : YALIS_ERR_LAUNCH;
 }
 

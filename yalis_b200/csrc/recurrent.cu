@@ -21,7 +21,7 @@
 // state and the convolution's tail live in the per-request slot memory of the cache manager.
 //
 // The columns of S are independent of one another (column j only ever meets v_j), so a thread
-// owns 8 (or 16) rows of one column in registers, the lanes that share a column sit in one warp, and
+// owns 8 or 16 rows of one or two columns in registers, the lanes that share a column sit in one warp, and
 // a block walks the tokens of one request in order: a portion of a prompt and a single
 // decoded token are the same loop, and the result for a token does not depend on how the
 // request was cut into steps or on what else is in the batch.
@@ -212,7 +212,6 @@ __global__ void short_conv_tail_kernel(const T* __restrict__ x, int x_stride, fl
 
 // ---- the recurrence ------------------------------------------------------------------------------
 constexpr int kScanThreads = 128;
-constexpr int kMaxTile = 16;         // tokens staged in shared memory at a time
 
 struct ScanParams {
   const float* q; int q_stride;      // [N, kv_heads * dim]
@@ -226,7 +225,7 @@ struct ScanParams {
   float* state; size_t slot_stride;  // per slot: [heads][vdim][dim_padded]
   float* out; int out_stride;        // [N, heads * vdim]
   const int32_t* q_start; const int32_t* slots;
-  int heads, kv_heads, dim, dim_padded, vdim, lanes, tile;
+  int heads, kv_heads, dim, dim_padded, vdim;
   int wide;                          // 1: rows of q, k and the decay may be copied 16 bytes at a time
 };
 
@@ -240,234 +239,318 @@ __device__ __forceinline__ void copy_async_commit() { asm volatile("cp.async.com
 template <int N>
 __device__ __forceinline__ void copy_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N)); }
 
+// Two float32 operations in one instruction, each half rounded as the single operation is.
+__device__ __forceinline__ uint64_t bits2(float2 v) { return *reinterpret_cast<uint64_t*>(&v); }
+__device__ __forceinline__ float2 pair2(uint64_t v) { return *reinterpret_cast<float2*>(&v); }
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  uint64_t d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(bits2(a)), "l"(bits2(b)), "l"(bits2(c)));
+  return pair2(d);
+}
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+  uint64_t d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(bits2(a)), "l"(bits2(b)));
+  return pair2(d);
+}
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+  uint64_t d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(bits2(a)), "l"(bits2(b)));
+  return pair2(d);
+}
+__device__ __forceinline__ float2 lo2(const float4& v) { return make_float2(v.x, v.y); }
+__device__ __forceinline__ float2 hi2(const float4& v) { return make_float2(v.z, v.w); }
+
+// Floats of one staging buffer (see the kernel), a multiple of four.
+constexpr int scan_buffer_floats(int vec_cols, int tile, int width, int cols) {
+  return (vec_cols * tile * width + tile * cols + 2 * tile + 3) & ~3;
+}
+
+// What a lane needs of one token, in registers.
+template <int ROWS, int COLS, int RULE, int DECAY>
+struct ScanToken {
+  float4 q[ROWS / 4], k[ROWS / 4];
+  float4 g[DECAY == 2 ? ROWS / 4 : 1];                                 // decay vector
+  float4 u[RULE == 2 ? ROWS / 4 : 1], a[RULE == 2 ? ROWS / 4 : 1];     // unit key, removal vector
+  float v[COLS], beta, decay;
+};
+
+// A lane's share of the dot product of a column of the state with a vector: four partial sums, a fixed tree.
+template <int Q>
+__device__ __forceinline__ float share_dot(const float2 (&S)[2 * Q], const float4 (&x)[Q]) {
+  float2 a = mul2(S[0], lo2(x[0])), b = mul2(S[1], hi2(x[0]));
+#pragma unroll
+  for (int i = 1; i < Q; ++i) {
+    a = fma2(S[2 * i], lo2(x[i]), a);
+    b = fma2(S[2 * i + 1], hi2(x[i]), b);
+  }
+  a = add2(a, b);
+  return a.x + a.y;
+}
+
+// The dot products of a thread's columns: a butterfly over the L lanes (the same order of additions for every token).
+template <int Q, int L, int C>
+__device__ __forceinline__ void lane_dots(const float2 (&S)[C][2 * Q], const float4 (&x)[Q], float (&dot)[C]) {
+#pragma unroll
+  for (int cc = 0; cc < C; ++cc) dot[cc] = share_dot<Q>(S[cc], x);
+#pragma unroll
+  for (int o = 1; o < L; o <<= 1)
+#pragma unroll
+    for (int cc = 0; cc < C; ++cc) dot[cc] += __shfl_xor_sync(0xffffffffu, dot[cc], o);
+}
+
+// Sums over the L lanes of a column of N values a lane holds (one per token and column): halves are exchanged while there
+// are several, so N values cost about N shuffles and not N log L.  Afterwards lane l holds the sums of values l N / L ...
+// (N >= L), or of value l / (L / N).  Every sum adds the lanes in the same tree, which is also that of one value alone.
+template <int N, int L>
+__device__ __forceinline__ void lane_sums(float (&r)[N], int l) {
+  int n = N;
+#pragma unroll
+  for (int o = L / 2; o >= 1; o >>= 1) {
+    if (n > 1) {
+      const bool upper = (l & o) != 0;
+#pragma unroll
+      for (int i = 0; i < N / 2; ++i) {
+        if (i < n / 2) {
+          const float send = upper ? r[i] : r[i + n / 2], keep = upper ? r[i + n / 2] : r[i];
+          r[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+        }
+      }
+      n >>= 1;
+    } else {
+      r[0] += __shfl_xor_sync(0xffffffffu, r[0], o);
+    }
+  }
+}
+
 // RULE: 0 plain outer-product write, 1 delta rule, 2 generalized delta rule (needs DECAY 2), 3 plain write of beta v
 // with skip_h v beside the read-out.
 // DECAY: 0 constant per head, 1 scalar per token and head, 2 vector per token, head and key channel.
-// ROWS: rows of a column that a thread keeps (8: twice the warps, which hide each other's waits; 16: dim up to 512).
-// The tokens of a request are staged through two buffers in shared memory: while one tile is walked, the
-// asynchronous copies of the next are in flight.
-// LANES: lanes that share a column (a power of two up to 32; ROWS * LANES >= dim).
-template <int ROWS, int LANES, int RULE, int DECAY>
+// ROWS x COLS: rows and neighbouring columns of the state that a thread keeps.  LANES: lanes that share a column (a power
+// of two; ROWS * LANES >= dim).  TILE: tokens staged in shared memory at a time, through two buffers: while one tile is
+// walked, the asynchronous copies of the next are in flight.  TILE 1 is the form for single tokens: small blocks, many of
+// them per SM.
+//
+// What bounds a prompt is one warp's stream of instructions (a single request has only heads * vdim * dim / (32 * 16) warps,
+// under one per scheduler; a warp issues an instruction every two to three cycles) and, for several requests, the loads from
+// shared memory (16 bytes a lane are four passes whatever lanes share).  Hence tokens in groups of four without a run-time
+// address or a move between them, a token's vectors loaded while the one before is computed, two float32 operations per
+// instruction, and read-outs summed over the lanes four tokens at a time instead of one by one through shared memory.
+// Measured for 16 heads of 128 x 128, us for 1 x 2,048 / 4 x 2,048 tokens (8 x 1 rows by columns a thread, a token at a time,
+// before): delta rule 473 / 1156 -> 380 / 800, decay per channel 516 -> 430, generalized rule 582 -> 449, plain write
+// 300 -> 250, selective 328 / 860 -> 260 / 518; 64 single tokens 37 to 41 -> 29 (134 MB: 4.6 TB/s).
+// Why this split: the delta rules' chain (dot product over the lanes, write, next token) is shortest with 16 rows and 8
+// lanes (two columns of 8 rows: 488 us); the others read each q and k once for two columns of 8 rows (16 rows: 262 us, and
+// 717 for four selective prompts).
+template <int ROWS, int LANES, int COLS, int RULE, int DECAY, int TILE>
 __global__ void __launch_bounds__(kScanThreads) state_scan_kernel(const ScanParams p) {
   extern __shared__ __align__(16) float sm[];
   constexpr int Q = ROWS / 4;          // 16-byte pieces of a column per thread
+  constexpr int L = LANES, C = COLS, cols = kScanThreads / L * C, width = ROWS * L;
+  // one buffer: q [TILE][width], k [TILE][width], decay vectors [TILE][width] (DECAY 2), unit keys and removal vectors
+  // [TILE][width] each (RULE 2), v [TILE][cols], beta [TILE], decay [TILE]; behind the two buffers the read-outs [TILE][cols]
+  constexpr int vec_cols = RULE == 2 ? 5 : (DECAY == 2 ? 3 : 2);
+  constexpr int array = TILE * width, buf_floats = scan_buffer_floats(vec_cols, TILE, width, cols);
   pdl_launch_dependents();
   pdl_wait();
   const int req = blockIdx.z, h = blockIdx.y;
   const int t_begin = p.q_start[req], q_len = p.q_start[req + 1] - t_begin;
   if (q_len <= 0) return;
-  constexpr int L = LANES, cols = kScanThreads / L, width = ROWS * L;
   const int tid = threadIdx.x, l = tid % L, c = tid / L;
-  const int j = blockIdx.x * cols + c;
-  const bool live = j < p.vdim;
+  const int j = blockIdx.x * cols + c * C;               // the thread's first column
   const int kvh = h / (p.heads / p.kv_heads);
-  const int D = p.dim, Dp = p.dim_padded, V = p.vdim, TT = p.tile;
-  constexpr bool DELTA = RULE == 1;
-  // one buffer: q [TT][width], k [TT][width], decay vectors [TT][width] (DECAY 2), unit keys and removal vectors
-  // [TT][width] each (RULE 2), v [TT][cols], beta [TT], decay [TT]
-  constexpr int vec_cols = RULE == 2 ? 5 : (DECAY == 2 ? 3 : 2);
-  const size_t buf_floats = ((size_t)vec_cols * TT * width + (size_t)TT * cols + 2 * TT + 3) & ~(size_t)3;
-  // behind the two buffers: every lane's share of a read-out, [TT][cols][L + 1]; the shares are added after the
-  // tile is walked, off the chain from one token's state to the next
-  float* shares = sm + 2 * buf_floats;
+  const int D = p.dim, Dp = p.dim_padded, V = p.vdim;
+  float* sp = p.state + (size_t)p.slots[req] * p.slot_stride + ((size_t)h * V + j) * Dp;
+  float2 S[C][ROWS / 2];
+#pragma unroll
+  for (int cc = 0; cc < C; ++cc)
+#pragma unroll
+    for (int i = 0; i < Q; ++i) {
+      const int d = (i * L + l) * 4;
+      float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (j + cc < V && d < Dp) x = *reinterpret_cast<const float4*>(sp + (size_t)cc * Dp + d);
+      S[cc][2 * i] = lo2(x); S[cc][2 * i + 1] = hi2(x);
+    }
+  float* outs = sm + 2 * buf_floats;
 
   // what no copy ever writes: the rows past dim (zeros; ones for the decay)
   const int pad = width - D;
-  for (int e = tid; e < 2 * vec_cols * TT * pad; e += kScanThreads) {
+  for (int e = tid; e < 2 * vec_cols * TILE * pad; e += kScanThreads) {
     const int row = e / pad, d = D + (e - row * pad);          // row: (buffer, array, token)
-    const int b = row / (vec_cols * TT), r = row - b * (vec_cols * TT);
-    sm[(size_t)b * buf_floats + (size_t)r * width + d] = (r / TT) == 2 ? 1.f : 0.f;
+    const int b = row / (vec_cols * TILE), r = row - b * (vec_cols * TILE);
+    sm[b * buf_floats + r * width + d] = (r / TILE) == 2 ? 1.f : 0.f;
   }
 
   auto issue = [&](int t0, int b) {
-    float* qs = sm + (size_t)b * buf_floats;
-    float* ks = qs + (size_t)TT * width;
-    float* gv = ks + (size_t)TT * width;
-    float* uv = gv + (size_t)TT * width;
-    float* av = uv + (size_t)TT * width;
-    float* vs = qs + (size_t)vec_cols * TT * width;
-    float* bs = vs + (size_t)TT * cols;
-    float* gs = bs + TT;
-    const int tt = min(TT, q_len - t0);
-    if (p.wide) {
+    float* qs = sm + b * buf_floats;
+    float* vs = qs + vec_cols * array;
+    float* bs = vs + TILE * cols;
+    float* gs = bs + TILE;
+    const int tt = min(TILE, q_len - t0);
+    auto copy_row = [&](auto copy, int t, int d) {
+      const size_t n = (size_t)(t_begin + t0 + t);
+      float* to = qs + t * width + d;
+      copy(to, p.q + n * p.q_stride + (size_t)kvh * D + d);
+      copy(to + array, p.k + n * p.k_stride + (size_t)kvh * D + d);
+      if (DECAY == 2) copy(to + 2 * array, p.decay + (n * p.heads + h) * D + d);
+      if (RULE == 2) {
+        copy(to + 3 * array, p.unit + (n * p.heads + h) * D + d);
+        copy(to + 4 * array, p.removal + (n * p.heads + h) * D + d);
+      }
+    };
+    if (p.wide && pad == 0) {                      // a row of a power of two: no division
+      for (int e = tid; e < tt * (width / 4); e += kScanThreads) copy_row(copy_async16, e / (width / 4), e % (width / 4) * 4);
+    } else if (p.wide) {
       const int quads = D >> 2;
-      for (int e = tid; e < tt * quads; e += kScanThreads) {
-        const int t = e / quads, d = (e - t * quads) << 2;
-        const size_t n = (size_t)(t_begin + t0 + t);
-        copy_async16(qs + t * width + d, p.q + n * p.q_stride + (size_t)kvh * D + d);
-        copy_async16(ks + t * width + d, p.k + n * p.k_stride + (size_t)kvh * D + d);
-        if (DECAY == 2) copy_async16(gv + t * width + d, p.decay + (n * p.heads + h) * D + d);
-        if (RULE == 2) {
-          copy_async16(uv + t * width + d, p.unit + (n * p.heads + h) * D + d);
-          copy_async16(av + t * width + d, p.removal + (n * p.heads + h) * D + d);
-        }
-      }
+      for (int e = tid; e < tt * quads; e += kScanThreads) copy_row(copy_async16, e / quads, e % quads * 4);
     } else {
-      for (int e = tid; e < tt * D; e += kScanThreads) {
-        const int t = e / D, d = e - t * D;
-        const size_t n = (size_t)(t_begin + t0 + t);
-        copy_async4(qs + t * width + d, p.q + n * p.q_stride + (size_t)kvh * D + d);
-        copy_async4(ks + t * width + d, p.k + n * p.k_stride + (size_t)kvh * D + d);
-        if (DECAY == 2) copy_async4(gv + t * width + d, p.decay + (n * p.heads + h) * D + d);
-        if (RULE == 2) {
-          copy_async4(uv + t * width + d, p.unit + (n * p.heads + h) * D + d);
-          copy_async4(av + t * width + d, p.removal + (n * p.heads + h) * D + d);
-        }
-      }
+      for (int e = tid; e < tt * D; e += kScanThreads) copy_row(copy_async4, e / D, e % D);
     }
     for (int e = tid; e < tt * cols; e += kScanThreads) {
-      const int t = e / cols, cc = e - t * cols;
-      const int jj = blockIdx.x * cols + cc;
+      const int t = e / cols, jj = blockIdx.x * cols + e % cols;
       if (jj < V) copy_async4(vs + e, p.v + (size_t)(t_begin + t0 + t) * p.v_stride + (size_t)h * V + jj);
       else vs[e] = 0.f;
     }
     if (tid < tt) {
       const size_t n = (size_t)(t_begin + t0 + tid);
-      if (DELTA || RULE == 3) copy_async4(bs + tid, p.beta + n * p.heads + h);
+      if (RULE == 1 || RULE == 3) copy_async4(bs + tid, p.beta + n * p.heads + h);
       if (DECAY == 1) copy_async4(gs + tid, p.decay + n * p.heads + h);
     }
     copy_async_commit();
   };
 
-  float* sp = p.state + (size_t)p.slots[req] * p.slot_stride + ((size_t)h * V + (live ? j : 0)) * Dp;
-  float S[ROWS];
-#pragma unroll
-  for (int i = 0; i < Q; ++i) {
-    const int d = (i * L + l) * 4;
-    float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (live && d < Dp) x = *reinterpret_cast<const float4*>(sp + d);
-    S[4 * i] = x.x; S[4 * i + 1] = x.y; S[4 * i + 2] = x.z; S[4 * i + 3] = x.w;
-  }
   const float g_const = DECAY == 0 ? p.decay[h] : 1.f;
   const float skip = (RULE == 3 && p.skip) ? p.skip[h] : 0.f;
 
   issue(0, 0);
   int b = 0;
-  for (int t0 = 0; t0 < q_len; t0 += TT, b ^= 1) {
-    const int tt = min(TT, q_len - t0);
-    if (t0 + TT < q_len) {
-      issue(t0 + TT, b ^ 1);
+  for (int t0 = 0; t0 < q_len; t0 += TILE, b ^= 1) {
+    const int tt = min(TILE, q_len - t0);
+    if (t0 + TILE < q_len) {
+      issue(t0 + TILE, b ^ 1);
       copy_async_wait<1>();
     } else {
       copy_async_wait<0>();
     }
     __syncthreads();
-    const float* qs = sm + (size_t)b * buf_floats;
-    const float* vs = qs + (size_t)vec_cols * TT * width;
-    const float* bs = vs + (size_t)TT * cols;
-    const float* gs = bs + TT;
-    const float* qp = qs + l * 4;                          // this lane's first piece of q; k and the decay follow
-    const float* kp = qp + (size_t)TT * width;
-    const float* gp = kp + (size_t)TT * width;
-    for (int t = 0; t < tt; ++t, qp += width, kp += width, gp += width) {
-      float kr[ROWS], qr[ROWS];
+    const float* qp = sm + b * buf_floats + l * 4;         // this lane's first piece of q; the other vectors follow
+    const float* vp = sm + b * buf_floats + vec_cols * array + c * C;
+    const float* bp = sm + b * buf_floats + vec_cols * array + TILE * cols;
+    using Token = ScanToken<ROWS, C, RULE, DECAY>;
+    auto load = [&](Token& x, int t) {
+      const float* r = qp + t * width;
 #pragma unroll
       for (int i = 0; i < Q; ++i) {
-        const float4 a = *reinterpret_cast<const float4*>(kp + i * L * 4);
-        const float4 bq = *reinterpret_cast<const float4*>(qp + i * L * 4);
-        kr[4 * i] = a.x; kr[4 * i + 1] = a.y; kr[4 * i + 2] = a.z; kr[4 * i + 3] = a.w;
-        qr[4 * i] = bq.x; qr[4 * i + 1] = bq.y; qr[4 * i + 2] = bq.z; qr[4 * i + 3] = bq.w;
-      }
-      if (RULE == 2) {
-        // both the decay and the removal read the old state: the dot product u . S first (pairs, then a fixed tree
-        // and a butterfly over the lanes), then every row in one expression, then the read-out as in the other rules
-        const float* up = gp + (size_t)TT * width;
-        const float* ap = up + (size_t)TT * width;
-        float ur[ROWS], ar[ROWS], gr[ROWS];
-#pragma unroll
-        for (int i = 0; i < Q; ++i) {
-          const float4 a = *reinterpret_cast<const float4*>(up + i * L * 4);
-          const float4 b2 = *reinterpret_cast<const float4*>(ap + i * L * 4);
-          const float4 g = *reinterpret_cast<const float4*>(gp + i * L * 4);
-          ur[4 * i] = a.x; ur[4 * i + 1] = a.y; ur[4 * i + 2] = a.z; ur[4 * i + 3] = a.w;
-          ar[4 * i] = b2.x; ar[4 * i + 1] = b2.y; ar[4 * i + 2] = b2.z; ar[4 * i + 3] = b2.w;
-          gr[4 * i] = g.x; gr[4 * i + 1] = g.y; gr[4 * i + 2] = g.z; gr[4 * i + 3] = g.w;
+        x.q[i] = *reinterpret_cast<const float4*>(r + i * L * 4);
+        x.k[i] = *reinterpret_cast<const float4*>(r + array + i * L * 4);
+        if constexpr (DECAY == 2) x.g[i] = *reinterpret_cast<const float4*>(r + 2 * array + i * L * 4);
+        if constexpr (RULE == 2) {
+          x.u[i] = *reinterpret_cast<const float4*>(r + 3 * array + i * L * 4);
+          x.a[i] = *reinterpret_cast<const float4*>(r + 4 * array + i * L * 4);
         }
-        float part[ROWS / 2];
-#pragma unroll
-        for (int i = 0; i < ROWS / 2; ++i) part[i] = __fmaf_rn(S[2 * i + 1], ur[2 * i + 1], S[2 * i] * ur[2 * i]);
-#pragma unroll
-        for (int w = ROWS / 4; w >= 1; w >>= 1)
-#pragma unroll
-          for (int i = 0; i < w; ++i) part[i] += part[i + w];
-        float dot = part[0];
-#pragma unroll
-        for (int o = 1; o < L; o <<= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
-        const float vj = vs[t * cols + c];
-#pragma unroll
-        for (int i = 0; i < ROWS / 2; ++i) {
-          S[2 * i] = __fmaf_rn(kr[2 * i], vj, __fmaf_rn(-ar[2 * i], dot, S[2 * i] * gr[2 * i]));
-          S[2 * i + 1] = __fmaf_rn(kr[2 * i + 1], vj, __fmaf_rn(-ar[2 * i + 1], dot, S[2 * i + 1] * gr[2 * i + 1]));
-          part[i] = __fmaf_rn(S[2 * i + 1], qr[2 * i + 1], S[2 * i] * qr[2 * i]);
-        }
-#pragma unroll
-        for (int w = ROWS / 4; w >= 1; w >>= 1)
-#pragma unroll
-          for (int i = 0; i < w; ++i) part[i] += part[i + w];
-        shares[(t * cols + c) * (L + 1) + l] = part[0];
-        continue;
       }
-      if (DECAY == 2) {
 #pragma unroll
-        for (int i = 0; i < Q; ++i) {
-          const float4 g = *reinterpret_cast<const float4*>(gp + i * L * 4);
-          S[4 * i] *= g.x; S[4 * i + 1] *= g.y; S[4 * i + 2] *= g.z; S[4 * i + 3] *= g.w;
+      for (int cc = 0; cc < C; ++cc) x.v[cc] = vp[t * cols + cc];
+      if constexpr (RULE == 1 || RULE == 3) x.beta = bp[t];
+      if constexpr (DECAY == 1) x.decay = bp[TILE + t];
+    };
+    // one token: the state moves on; this lane's shares of the read-outs
+    auto step = [&](const Token& x, float* share) {
+      float dot[C];
+      if constexpr (RULE == 2) {
+        // both the decay and the removal read the old state: the dot products u . S first, then every row in one
+        // expression, then the read-out as in the other rules
+        lane_dots<Q, L, C>(S, x.u, dot);
+#pragma unroll
+        for (int cc = 0; cc < C; ++cc) {
+          const float2 md = make_float2(-dot[cc], -dot[cc]), vv = make_float2(x.v[cc], x.v[cc]);
+#pragma unroll
+          for (int i = 0; i < Q; ++i) {
+            S[cc][2 * i] = fma2(lo2(x.k[i]), vv, fma2(lo2(x.a[i]), md, mul2(S[cc][2 * i], lo2(x.g[i]))));
+            S[cc][2 * i + 1] = fma2(hi2(x.k[i]), vv, fma2(hi2(x.a[i]), md, mul2(S[cc][2 * i + 1], hi2(x.g[i]))));
+          }
         }
       } else {
-        const float g = DECAY == 1 ? gs[t] : g_const;
+        const float g = DECAY == 1 ? x.decay : g_const;
+        const float2 gg = make_float2(g, g);
 #pragma unroll
-        for (int r = 0; r < ROWS; ++r) S[r] *= g;
-      }
-      float u = vs[t * cols + c];
-      if (DELTA) {
-        // sums of pairs, then a fixed tree: short chains, and the same order of additions for every token
-        float part[ROWS / 2];
+        for (int cc = 0; cc < C; ++cc)
 #pragma unroll
-        for (int i = 0; i < ROWS / 2; ++i) part[i] = __fmaf_rn(S[2 * i + 1], kr[2 * i + 1], S[2 * i] * kr[2 * i]);
+          for (int i = 0; i < Q; ++i) {
+            S[cc][2 * i] = mul2(S[cc][2 * i], DECAY == 2 ? lo2(x.g[i]) : gg);
+            S[cc][2 * i + 1] = mul2(S[cc][2 * i + 1], DECAY == 2 ? hi2(x.g[i]) : gg);
+          }
+        if constexpr (RULE == 1) lane_dots<Q, L, C>(S, x.k, dot);
 #pragma unroll
-        for (int w = ROWS / 4; w >= 1; w >>= 1)
+        for (int cc = 0; cc < C; ++cc) {
+          float u = x.v[cc];
+          if constexpr (RULE == 1) u = x.beta * (u - dot[cc]);
+          if constexpr (RULE == 3) u *= x.beta;
+          const float2 uu = make_float2(u, u);
 #pragma unroll
-          for (int i = 0; i < w; ++i) part[i] += part[i + w];
-        float dot = part[0];
-#pragma unroll
-        for (int o = 1; o < L; o <<= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
-        u = bs[t] * (u - dot);
-      }
-      if (RULE == 3) u *= bs[t];
-      float part[ROWS / 2];
-#pragma unroll
-      for (int i = 0; i < ROWS / 2; ++i) {
-        S[2 * i] = __fmaf_rn(kr[2 * i], u, S[2 * i]);
-        S[2 * i + 1] = __fmaf_rn(kr[2 * i + 1], u, S[2 * i + 1]);
-        part[i] = __fmaf_rn(S[2 * i + 1], qr[2 * i + 1], S[2 * i] * qr[2 * i]);
+          for (int i = 0; i < Q; ++i) {
+            S[cc][2 * i] = fma2(lo2(x.k[i]), uu, S[cc][2 * i]);
+            S[cc][2 * i + 1] = fma2(hi2(x.k[i]), uu, S[cc][2 * i + 1]);
+          }
+        }
       }
 #pragma unroll
-      for (int w = ROWS / 4; w >= 1; w >>= 1)
+      for (int cc = 0; cc < C; ++cc) {
+        share[cc] = share_dot<Q>(S[cc], x.q);
+        if (RULE == 3 && l == 0) share[cc] = __fmaf_rn(skip, x.v[cc], share[cc]);   // the token's own value joins the first lane's share
+      }
+    };
+    int t = 0;
+    if constexpr (TILE >= 4) {
+      if (tt >= 4) {
+        Token x[2];
+        load(x[0], 0);
+#pragma unroll 1
+        for (; t + 4 <= tt; t += 4) {
+          float r[4 * C];
+          load(x[1], t + 1);
+          step(x[0], r);
+          load(x[0], t + 2);
+          step(x[1], r + C);
+          load(x[1], t + 3);
+          step(x[0], r + 2 * C);
+          load(x[0], min(t + 4, TILE - 1));       // (the row past the tile's last token is not used)
+          step(x[1], r + 3 * C);
+          lane_sums<4 * C, L>(r, l);
+          constexpr int per = L >= 4 * C ? 1 : 4 * C / L, share = L >= 4 * C ? L / (4 * C) : 1;
+          if (l % share == 0)
 #pragma unroll
-        for (int i = 0; i < w; ++i) part[i] += part[i + w];
-      // (the token's own value joins the first lane's share here: the copies of the next tile may already be
-      // overwriting this one while the shares are added)
-      if (RULE == 3 && l == 0) part[0] = __fmaf_rn(skip, vs[t * cols + c], part[0]);
-      shares[(t * cols + c) * (L + 1) + l] = part[0];
+            for (int i = 0; i < per; ++i) {
+              const int at = l / share * per + i;                     // (token, column) of the sum
+              outs[(t + at / C) * cols + c * C + at % C] = r[i];
+            }
+        }
+      }
+    }
+    for (; t < tt; ++t) {
+      Token x;
+      load(x, t);
+      float r[C];
+      step(x, r);
+      lane_sums<C, L>(r, l);
+      constexpr int per = L >= C ? 1 : C / L, share = L >= C ? L / C : 1;
+      if (l % share == 0)
+#pragma unroll
+        for (int i = 0; i < per; ++i) outs[t * cols + c * C + l / share * per + i] = r[i];
     }
     __syncthreads();                // the next round's copies overwrite the other buffer, which the round after reads
     for (int e = tid; e < tt * cols; e += kScanThreads) {
-      const int t = e / cols, cc = e - t * cols;
-      const int jj = blockIdx.x * cols + cc;
-      const float* sh = shares + (size_t)e * (L + 1);
-      float o_acc = sh[0];
-#pragma unroll
-      for (int i = 1; i < L; ++i) o_acc += sh[i];          // lane order: the same sum for every token
-      if (jj < V) p.out[(size_t)(t_begin + t0 + t) * p.out_stride + (size_t)h * V + jj] = o_acc;
+      const int jj = blockIdx.x * cols + e % cols;
+      if (jj < V) p.out[(size_t)(t_begin + t0 + e / cols) * p.out_stride + (size_t)h * V + jj] = outs[e];
     }
   }
-  if (live) {
+#pragma unroll
+  for (int cc = 0; cc < C; ++cc)
 #pragma unroll
     for (int i = 0; i < Q; ++i) {
       const int d = (i * L + l) * 4;
-      if (d < Dp) *reinterpret_cast<float4*>(sp + d) = make_float4(S[4 * i], S[4 * i + 1], S[4 * i + 2], S[4 * i + 3]);
+      if (j + cc < V && d < Dp)
+        *reinterpret_cast<float4*>(sp + (size_t)cc * Dp + d) = make_float4(S[cc][2 * i].x, S[cc][2 * i].y, S[cc][2 * i + 1].x, S[cc][2 * i + 1].y);
     }
-  }
 }
 
 // ---- per-head norm, weight and gate of a mixer's read-out ---------------------------------------------
@@ -660,45 +743,50 @@ YALIS_API int yalis_delta_prepare(const void* x, int dtype, int x_stride, const 
   return YALIS_OK;
 }
 
-// Rows of a column that a thread keeps: 8 up to dim 256, 16 beyond (up to 512).
-static int scan_rows(int dim) { return dim <= 256 ? 8 : 16; }
-
-// Lanes that share a column of the state: the smallest power of two with rows * lanes >= dim.
-YALIS_API int yalis_state_scan_lanes(int dim) {
-  int lanes = 1;
-  while (lanes * scan_rows(dim) < dim) lanes <<= 1;
-  return lanes;
+template <int ROWS, int LANES, int COLS, int RULE, int DECAY, int TILE>
+static int launch_scan_tile(const ScanParams& p, int n_requests, cudaStream_t stream) {
+  constexpr int cols = kScanThreads / LANES * COLS, vec_cols = RULE == 2 ? 5 : (DECAY == 2 ? 3 : 2);
+  constexpr size_t smem = (2 * (size_t)scan_buffer_floats(vec_cols, TILE, ROWS * LANES, cols) + TILE * cols) * sizeof(float);
+  static_assert(smem <= 200 * 1024, "two buffers and the read-outs fit a block");
+  auto kernel = state_scan_kernel<ROWS, LANES, COLS, RULE, DECAY, TILE>;
+  if (smem > 48 * 1024 && cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+    return YALIS_ERR_LAUNCH;
+  const dim3 grid((p.vdim + cols - 1) / cols, p.heads, n_requests);
+  if (TILE > 1) return yalis_launch_after(kernel, grid, dim3(kScanThreads), smem, stream, p);
+  return yalis_launch(kernel, grid, dim3(kScanThreads), smem, stream, p);
 }
 
-template <int ROWS, int LANES, int RULE, int DECAY>
-static int launch_scan(const ScanParams& p, dim3 grid, size_t smem, cudaStream_t stream) {
-  static size_t allowed = 48 * 1024;
-  if (smem > allowed) {
-    if (cudaFuncSetAttribute(state_scan_kernel<ROWS, LANES, RULE, DECAY>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             200 * 1024) != cudaSuccess)
-      return YALIS_ERR_LAUNCH;
-    allowed = 200 * 1024;
+template <int ROWS, int LANES, int COLS, int RULE, int DECAY>
+static int launch_scan(const ScanParams& p, int n_requests, int single, cudaStream_t stream) {
+  if (single) return launch_scan_tile<ROWS, LANES, COLS, RULE, DECAY, 1>(p, n_requests, stream);
+  return launch_scan_tile<ROWS, LANES, COLS, RULE, DECAY, (ROWS * LANES > 256 ? 8 : 16)>(p, n_requests, stream);
+}
+
+// The smallest power of two of lanes that covers dim.  Delta rules: 16 rows of one column a thread; the others 8 rows of two
+// neighbouring columns (beyond 256 rows 16 of one).  Sums over a column have one order per rule and dim, whatever the step.
+template <int RULE, int DECAY>
+static int launch_scan_dim(const ScanParams& p, int n_requests, int single, cudaStream_t stream) {
+  if constexpr (RULE == 1) {
+    if (p.dim <= 16) return launch_scan<16, 1, 1, RULE, DECAY>(p, n_requests, single, stream);
+    if (p.dim <= 32) return launch_scan<16, 2, 1, RULE, DECAY>(p, n_requests, single, stream);
+    if (p.dim <= 64) return launch_scan<16, 4, 1, RULE, DECAY>(p, n_requests, single, stream);
+    if (p.dim <= 128) return launch_scan<16, 8, 1, RULE, DECAY>(p, n_requests, single, stream);
+    if (p.dim <= 256) return launch_scan<16, 16, 1, RULE, DECAY>(p, n_requests, single, stream);
+  } else {
+    if (p.dim <= 8) return launch_scan<8, 1, 2, RULE, DECAY>(p, n_requests, single, stream);
+    if (p.dim <= 16) return launch_scan<8, 2, 2, RULE, DECAY>(p, n_requests, single, stream);
+    if (p.dim <= 32) return launch_scan<8, 4, 2, RULE, DECAY>(p, n_requests, single, stream);
+    if (p.dim <= 64) return launch_scan<8, 8, 2, RULE, DECAY>(p, n_requests, single, stream);
+    if (p.dim <= 128) return launch_scan<8, 16, 2, RULE, DECAY>(p, n_requests, single, stream);
+    if (p.dim <= 256) return launch_scan<8, 32, 2, RULE, DECAY>(p, n_requests, single, stream);
   }
-  return yalis_launch(state_scan_kernel<ROWS, LANES, RULE, DECAY>, grid, dim3(kScanThreads), smem, stream, p);
+  return launch_scan<16, 32, 1, RULE, DECAY>(p, n_requests, single, stream);
 }
-
-template <int ROWS, int LANES>
-static int launch_scan_kind(const ScanParams& p, dim3 grid, size_t smem, int delta, int decay_kind, cudaStream_t stream) {
-  if (delta == 2) return launch_scan<ROWS, LANES, 2, 2>(p, grid, smem, stream);
-  if (delta == 3) return launch_scan<ROWS, LANES, 3, 1>(p, grid, smem, stream);
-  if (delta && decay_kind == 1) return launch_scan<ROWS, LANES, 1, 1>(p, grid, smem, stream);
-  if (delta && decay_kind == 2) return launch_scan<ROWS, LANES, 1, 2>(p, grid, smem, stream);
-  if (delta) return launch_scan<ROWS, LANES, 1, 0>(p, grid, smem, stream);
-  if (decay_kind == 0) return launch_scan<ROWS, LANES, 0, 0>(p, grid, smem, stream);
-  if (decay_kind == 1) return launch_scan<ROWS, LANES, 0, 1>(p, grid, smem, stream);
-  return launch_scan<ROWS, LANES, 0, 2>(p, grid, smem, stream);
-}
-
 // decay_kind 0: decay [heads]; 1: decay [N, heads]; 2: decay [N, heads * dim].  delta 1: the delta rule with beta
 // [N, heads]; delta 2: the generalized delta rule with unit keys and removal vectors [N, heads * dim] (contiguous,
 // kv_heads = heads, decay_kind 2); delta 3: the selective form, beta [N, heads] the step sizes and skip [heads] (or null)
 // the token's own value in the read-out (decay_kind 1).
-// max_q_len: the longest portion of the step if the caller knows it (0: not known); it only bounds the staging tile.
+// max_q_len: the longest portion of the step if the caller knows it (0: not known); it only chooses the staging tile.
 YALIS_API int yalis_state_scan(const float* q, int q_stride, const float* k, int k_stride, const float* v, int v_stride,
                                const float* decay, int decay_kind, const float* beta, const float* skip, const float* unit,
                                const float* removal, float* state, int64_t slot_stride,
@@ -707,38 +795,29 @@ YALIS_API int yalis_state_scan(const float* q, int q_stride, const float* k, int
   if (n_requests <= 0) return YALIS_OK;
   if (dim <= 0 || vdim <= 0 || heads <= 0 || kv_heads <= 0 || heads % kv_heads || heads > 65535 || n_requests > 65535)
     return YALIS_ERR_SHAPE;
-  const int lanes = yalis_state_scan_lanes(dim);
-  if (lanes > 32) return YALIS_ERR_SHAPE;           // dim <= 512
+  if (dim > 512) return YALIS_ERR_SHAPE;
   if (decay_kind < 0 || decay_kind > 2 || !decay || delta < 0 || delta > 3 || (delta == 1 && !beta)) return YALIS_ERR_SHAPE;
   if (delta == 3 && (decay_kind != 1 || !beta)) return YALIS_ERR_SHAPE;
   if (delta == 2 && (decay_kind != 2 || !unit || !removal || kv_heads != heads)) return YALIS_ERR_SHAPE;
   const int dim_padded = (dim + 3) & ~3;
   if ((slot_stride & 3) || ((uintptr_t)state & 15)) return YALIS_ERR_ALIGN;
-  const int rows = scan_rows(dim);
-  const int cols = kScanThreads / lanes, width = rows * lanes;
-  const size_t per_token = ((delta == 2 ? 5 : (decay_kind == 2 ? 3 : 2)) * (size_t)width + cols + 2) * sizeof(float);
-  int tile = (int)((180 * 1024) / (2 * per_token));
-  tile = tile > kMaxTile ? kMaxTile : (tile < 1 ? 1 : tile);
-  if (max_q_len > 0 && tile > max_q_len) tile = max_q_len;      // single tokens: small blocks, many of them per SM
   ScanParams p;
   p.q = q; p.q_stride = q_stride; p.k = k; p.k_stride = k_stride; p.v = v; p.v_stride = v_stride;
   p.decay = decay; p.beta = beta; p.skip = skip; p.unit = unit; p.removal = removal; p.state = state; p.slot_stride = (size_t)slot_stride; p.out = out;
   p.out_stride = out_stride; p.q_start = q_start; p.slots = slots; p.heads = heads; p.kv_heads = kv_heads;
-  p.dim = dim; p.dim_padded = dim_padded; p.vdim = vdim; p.lanes = lanes; p.tile = tile;
+  p.dim = dim; p.dim_padded = dim_padded; p.vdim = vdim;
   p.wide = (dim % 4 == 0 && q_stride % 4 == 0 && k_stride % 4 == 0 && !((uintptr_t)q & 15) && !((uintptr_t)k & 15) &&
             (decay_kind != 2 || !((uintptr_t)decay & 15)) &&
             (delta != 2 || (!((uintptr_t)unit & 15) && !((uintptr_t)removal & 15)))) ? 1 : 0;
-  const dim3 grid((vdim + cols - 1) / cols, heads, n_requests);
-  const size_t smem = 2 * ((per_token * tile + 15) & ~(size_t)15) + (size_t)tile * cols * (lanes + 1) * sizeof(float);
-  if (rows == 16) return launch_scan_kind<16, 32>(p, grid, smem, delta, decay_kind, stream);
-  switch (lanes) {
-    case 1: return launch_scan_kind<8, 1>(p, grid, smem, delta, decay_kind, stream);
-    case 2: return launch_scan_kind<8, 2>(p, grid, smem, delta, decay_kind, stream);
-    case 4: return launch_scan_kind<8, 4>(p, grid, smem, delta, decay_kind, stream);
-    case 8: return launch_scan_kind<8, 8>(p, grid, smem, delta, decay_kind, stream);
-    case 16: return launch_scan_kind<8, 16>(p, grid, smem, delta, decay_kind, stream);
-    default: return launch_scan_kind<8, 32>(p, grid, smem, delta, decay_kind, stream);
-  }
+  const int single = max_q_len == 1;
+  if (delta == 2) return launch_scan_dim<2, 2>(p, n_requests, single, stream);
+  if (delta == 3) return launch_scan_dim<3, 1>(p, n_requests, single, stream);
+  if (delta && decay_kind == 1) return launch_scan_dim<1, 1>(p, n_requests, single, stream);
+  if (delta && decay_kind == 2) return launch_scan_dim<1, 2>(p, n_requests, single, stream);
+  if (delta) return launch_scan_dim<1, 0>(p, n_requests, single, stream);
+  if (decay_kind == 0) return launch_scan_dim<0, 0>(p, n_requests, single, stream);
+  if (decay_kind == 1) return launch_scan_dim<0, 1>(p, n_requests, single, stream);
+  return launch_scan_dim<0, 2>(p, n_requests, single, stream);
 }
 
 YALIS_API int yalis_head_norm_gate(const float* o, int o_stride, const float* weight, const void* gate, int gate_stride,
