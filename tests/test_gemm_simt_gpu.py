@@ -1,0 +1,27 @@
+"""The float32 product at the edges of its tiles, aligned and not, against float64; a row's result is the same bits whatever
+tile it falls into."""
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+@pytest.mark.parametrize("k", [1, 15, 16, 63, 200])
+@pytest.mark.parametrize("n", [1, 33, 130, 4100])
+def test_tiles(n, k):
+    from yalis_b200.ops.linear import gemm_simt
+    g = torch.Generator().manual_seed(n + k)
+    # rows of a wider matrix: strides that are not the width, and starts off a 16-byte boundary
+    for pad, off in ((0, 0), (4, 4), (3, 1)):
+        x = torch.randn(300, k + pad + off, generator=g).to(DEV)[:, off:off + k]
+        w = torch.randn(n, k + pad + off, generator=g).to(DEV)[:, off:off + k]
+        whole = gemm_simt(x, w)
+        want = x.double() @ w.double().t()
+        # a sum of k products in one chain: k 2^-24 of the sum of magnitudes at most
+        assert bool(((whole.double() - want).abs() <= (k + 1) * 2.0 ** -24 * (x.double().abs() @ w.double().abs().t())).all())
+        for m in (1, 31, 32, 33, 64, 65, 128, 129):
+            assert torch.equal(gemm_simt(x[:m], w), whole[:m])
+        assert torch.equal(gemm_simt(x[:70].to(torch.bfloat16), w, out_dtype=torch.float32),
+                           gemm_simt(x[:70].to(torch.bfloat16).float(), w))

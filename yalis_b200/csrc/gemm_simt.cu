@@ -14,19 +14,27 @@
 
 namespace {
 
-constexpr int BM = 64, BN = 64, BK = 16;
-constexpr int TM = 4, TN = 4;  // per-thread tile; 16 x 16 threads
-
-template <typename TA, typename TW, typename TO>
-__global__ void __launch_bounds__(256)
-gemm_tn_simt_kernel(const TA* __restrict__ A, long long lda, const TW* __restrict__ W, long long ldw,
-                    TO* __restrict__ O, long long ldo, int M, int N, int K) {
-  __shared__ float As[BK][BM + 4];
-  __shared__ float Ws[BK][BN + 4];
+// A tile of BM x BN outputs per block, BK values of k at a time through two buffers in shared memory; a thread keeps
+// TM x TN outputs (TM rows apart by one, TN columns in groups of four).  Values of the next tile are loaded to registers
+// while the current one is multiplied, 16 bytes at a time where rows are aligned.
+//
+// What bounds it: float32 FMAs (128 a cycle and SM).  8 x 8 outputs a thread read 16 values from shared memory for 64 FMAs,
+// which the two units then spend equally long on; 4 x 4 outputs (the tile this kernel had before) read 8 for 16 and waited
+// for shared memory, and its loads from global memory, one value at a time, stood between two barriers.
+// Tiles are chosen by how many blocks a launch gets: see launch().
+template <typename TA, typename TW, typename TO, int BM, int BN, int TM, int TN, bool VEC>
+__global__ void __launch_bounds__((BM / TM) * (BN / TN))
+gemm_tn_simt_kernel(const TA* A, long long lda, const TW* W, long long ldw, TO* O, long long ldo, int M, int N, int K) {
+  // (No __restrict__: a load the compiler takes for one of constant data may be moved above the wait for the kernel before.)
+  constexpr int BK = 16, THREADS = (BM / TM) * (BN / TN), TX = BN / TN;
+  constexpr int LA = BM + 4, LW = BN + 4;                  // padded rows: the transposed stores spread over the banks
+  constexpr int NA = BM * BK / 4 / THREADS, NW = BN * BK / 4 / THREADS;      // groups of four k values a thread loads
+  static_assert(NA >= 1 && NW >= 1 && TM % 4 == 0 && TN % 4 == 0, "whole groups");
+  __shared__ __align__(16) float As[2][BK][LA];
+  __shared__ __align__(16) float Ws[2][BK][LW];
   pdl_launch_dependents();
   pdl_wait();
-  const int tid = threadIdx.x;
-  const int tx = tid & 15, ty = tid >> 4;
+  const int tid = threadIdx.x, tx = tid % TX, ty = tid / TX;
   const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
   float acc[TM][TN];
 #pragma unroll
@@ -34,50 +42,110 @@ gemm_tn_simt_kernel(const TA* __restrict__ A, long long lda, const TW* __restric
 #pragma unroll
     for (int j = 0; j < TN; ++j) acc[i][j] = 0.f;
 
-  const int lr = tid >> 2;        // 0..63: row of the tile this thread loads
-  const int lk = (tid & 3) * 4;   // 0,4,8,12: first k of its four elements
-  for (int k0 = 0; k0 < K; k0 += BK) {
+  float4 ra[NA], rw[NW];
+  // four values of row `row` from k on; zeros outside the matrix
+  auto fetch4 = [&](const auto* p, long long ld, int row, int rows, int k) -> float4 {
+    if (row >= rows || k >= K) return make_float4(0.f, 0.f, 0.f, 0.f);
+    const auto* q = p + (size_t)row * ld + k;
+    if constexpr (VEC) return load4_f32(q);                // K is a multiple of four
+    float v[4];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int k = k0 + lk + u;
-      const int am = m0 + lr, wn = n0 + lr;
-      As[lk + u][lr] = (am < M && k < K) ? to_f32<TA>(A[(size_t)am * lda + k]) : 0.f;
-      Ws[lk + u][lr] = (wn < N && k < K) ? to_f32<TW>(W[(size_t)wn * ldw + k]) : 0.f;
+    for (int u = 0; u < 4; ++u) v[u] = k + u < K ? to_f32(q[u]) : 0.f;
+    return make_float4(v[0], v[1], v[2], v[3]);
+  };
+  // a group g of four k values: rows run fastest over threads within a group of k, so that the stores below spread
+  auto fetch = [&](int k0) {
+#pragma unroll
+    for (int i = 0; i < NA; ++i) {
+      const int e = tid + i * THREADS;
+      ra[i] = fetch4(A, lda, m0 + e / (BK / 4), M, k0 + (e % (BK / 4)) * 4);
     }
-    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < NW; ++i) {
+      const int e = tid + i * THREADS;
+      rw[i] = fetch4(W, ldw, n0 + e / (BK / 4), N, k0 + (e % (BK / 4)) * 4);
+    }
+  };
+  auto put = [&](int b) {
+#pragma unroll
+    for (int i = 0; i < NA; ++i) {
+      const int e = tid + i * THREADS, r = e / (BK / 4), k = (e % (BK / 4)) * 4;
+      As[b][k][r] = ra[i].x; As[b][k + 1][r] = ra[i].y; As[b][k + 2][r] = ra[i].z; As[b][k + 3][r] = ra[i].w;
+    }
+#pragma unroll
+    for (int i = 0; i < NW; ++i) {
+      const int e = tid + i * THREADS, r = e / (BK / 4), k = (e % (BK / 4)) * 4;
+      Ws[b][k][r] = rw[i].x; Ws[b][k + 1][r] = rw[i].y; Ws[b][k + 2][r] = rw[i].z; Ws[b][k + 3][r] = rw[i].w;
+    }
+  };
+
+  fetch(0);
+  put(0);
+  __syncthreads();
+  int b = 0;
+  for (int k0 = 0; k0 < K; k0 += BK, b ^= 1) {
+    const bool more = k0 + BK < K;
+    if (more) fetch(k0 + BK);
 #pragma unroll
     for (int kk = 0; kk < BK; ++kk) {
       float a[TM], w[TN];
 #pragma unroll
-      for (int i = 0; i < TM; ++i) a[i] = As[kk][ty * TM + i];
+      for (int i = 0; i < TM; i += 4) {
+        const float4 v = *reinterpret_cast<const float4*>(&As[b][kk][(i / 4) * (BM * 4 / TM) + ty * 4]);
+        a[i] = v.x; a[i + 1] = v.y; a[i + 2] = v.z; a[i + 3] = v.w;
+      }
 #pragma unroll
-      for (int j = 0; j < TN; ++j) w[j] = Ws[kk][tx * TN + j];
+      for (int j = 0; j < TN; j += 4) {
+        const float4 v = *reinterpret_cast<const float4*>(&Ws[b][kk][(j / 4) * (BN * 4 / TN) + tx * 4]);
+        w[j] = v.x; w[j + 1] = v.y; w[j + 2] = v.z; w[j + 3] = v.w;
+      }
 #pragma unroll
       for (int i = 0; i < TM; ++i)
 #pragma unroll
         for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a[i], w[j], acc[i][j]);
     }
+    if (more) put(b ^ 1);             // the buffer that the round before read: everyone passed the barrier behind it
     __syncthreads();
   }
 #pragma unroll
   for (int i = 0; i < TM; ++i) {
-    const int m = m0 + ty * TM + i;
+    const int m = m0 + (i / 4) * (BM * 4 / TM) + ty * 4 + i % 4;
     if (m >= M) continue;
 #pragma unroll
     for (int j = 0; j < TN; ++j) {
-      const int n = n0 + tx * TN + j;
+      const int n = n0 + (j / 4) * (BN * 4 / TN) + tx * 4 + j % 4;
       if (n < N) O[(size_t)m * ldo + n] = from_f32<TO>(acc[i][j]);
     }
   }
 }
 
+template <typename TA, typename TW, typename TO, int BM, int BN, int TM, int TN>
+int launch_tile(const void* A, long long lda, const void* W, long long ldw, void* O, long long ldo, int M, int N, int K,
+                cudaStream_t stream) {
+  const dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM), block((BM / TM) * (BN / TN));
+  if (grid.y > 65535) return YALIS_ERR_SHAPE;
+  const bool vec = K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 && (uintptr_t)A % (4 * sizeof(TA)) == 0 &&
+                   (uintptr_t)W % (4 * sizeof(TW)) == 0;
+  if (vec)
+    return yalis_launch(gemm_tn_simt_kernel<TA, TW, TO, BM, BN, TM, TN, true>, grid, block, 0, stream, (const TA*)A, lda,
+                        (const TW*)W, ldw, (TO*)O, ldo, M, N, K);
+  return yalis_launch(gemm_tn_simt_kernel<TA, TW, TO, BM, BN, TM, TN, false>, grid, block, 0, stream, (const TA*)A, lda,
+                      (const TW*)W, ldw, (TO*)O, ldo, M, N, K);
+}
+
+// Which tile: a large one only where it leaves two blocks to an SM (250 rows by 16,384 columns, K = 2,048: 128 x 128 would be
+// 256 blocks).  Measured (us, float32; before, 64 x 64 with 4 x 4 outputs a thread -> now), columns x K:
+//   250 rows   3,072 x 2,048  227 -> 141    2,048 x 2,048  158 -> 100    16,384 x 2,048  699 -> 418    2,048 x 8,192  610 -> 390
+//   1,024 rows 3,072 x 2,048  602 -> 359    2,048 x 2,048  411 -> 248    16,384 x 2,048  2,704 -> 1,918  2,048 x 8,192  1,614 -> 956
+//   8 rows     3,072 x 2,048  159 -> 126    16,384 x 2,048  221 -> 141   2,048 x 8,192  633 -> 497  (32 x 32 tiles: more blocks)
 template <typename TA, typename TW, typename TO>
 int launch(const void* A, long long lda, const void* W, long long ldw, void* O, long long ldo, int M, int N, int K,
            cudaStream_t stream) {
-  dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
-  if (grid.y > 65535) return YALIS_ERR_SHAPE;
-  return yalis_launch(gemm_tn_simt_kernel<TA, TW, TO>, grid, dim3(256), 0, stream, (const TA*)A, lda, (const TW*)W, ldw,
-                      (TO*)O, ldo, M, N, K);
+  const long long sms = yalis_sm_count();
+  auto blocks = [&](int bm, int bn) { return (long long)((N + bn - 1) / bn) * ((M + bm - 1) / bm); };
+  if (M > 64 && blocks(128, 128) >= 2 * sms) return launch_tile<TA, TW, TO, 128, 128, 8, 8>(A, lda, W, ldw, O, ldo, M, N, K, stream);
+  if (M > 32 && blocks(64, 64) >= sms / 2) return launch_tile<TA, TW, TO, 64, 64, 8, 4>(A, lda, W, ldw, O, ldo, M, N, K, stream);
+  return launch_tile<TA, TW, TO, 32, 32, 4, 4>(A, lda, W, ldw, O, ldo, M, N, K, stream);
 }
 
 }  // namespace
