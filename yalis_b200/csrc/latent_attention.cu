@@ -15,6 +15,14 @@
 #include "common.cuh"
 
 
+// latent_attention_tcgen05.cu
+YALIS_API int yalis_latent_attention_tcgen05_supports(int r, int p, int page_size);
+int yalis_latent_tc_launch(const void* q_lat, long ql_n, long ql_h, const float* q_rot, long qr_n, long qr_h, void* out,
+                           int out_bf16, long o_n, long o_h, const void* pool, const int32_t* positions,
+                           const int32_t* q_start, const int32_t* block_table, int table_width, int page_size, int num_pages,
+                           int n_requests, int n_tokens, int max_q_len, int heads, int r, int p, float scale, int window,
+                           const float* sink, int n_splits, float* part_o, float* part_ml, int32_t* error, cudaStream_t stream);
+
 namespace {
 
 // ---- prepare -----------------------------------------------------------------------------------------------
@@ -558,11 +566,14 @@ __global__ void __launch_bounds__(128 * WR) latent_attention_mma_kernel(const La
     }
 }
 
-// out = sum_z o_z exp(m_z - M) / sum_z l_z exp(m_z - M) in the order of z (at most 32 shares).  One warp per
-// (token, head): lane z weighs share z, then every column adds its shares in the order of z.
-__global__ void latent_merge_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml, int n_splits,
-                                    int n_tokens, int heads, int r, const int32_t* __restrict__ req_of_token, void* out,
-                                    int out_bf16, long o_n, long o_h, const float* __restrict__ sink) {
+// out = sum_z o_z exp(m_z - M) / sum_z l_z exp(m_z - M) in the order of z (at most 32 shares).  A warp per (token, head) and
+// 128 columns: lane z weighs share z, then every lane adds the shares of its four columns in the order of z, all of them
+// requested before the first is added (what bounds the kernel is that trip to the L2: a warp per row and a column at a time
+// took 22 us for 128 rows of 16 shares).
+// (No __restrict__: a load the compiler takes for one of constant data may be moved above the wait for the kernel before.)
+__global__ void latent_merge_kernel(const float* part_o, const float* part_ml, int n_splits, int n_tokens, int heads, int r,
+                                    const int32_t* req_of_token, void* out, int out_bf16, long o_n, long o_h,
+                                    const float* sink) {
   pdl_launch_dependents();
   pdl_wait();
   const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
@@ -570,6 +581,7 @@ __global__ void latent_merge_kernel(const float* __restrict__ part_o, const floa
   const int tok = row / heads, h = row - tok * heads;
   if (req_of_token[tok] < 0) return;
   const size_t rows = (size_t)n_tokens * heads;
+  const int c = (int)blockIdx.y * 128 + lane * 4;
   const float m = lane < n_splits ? part_ml[((size_t)lane * rows + row) * 2] : -INFINITY;
   const float lz = lane < n_splits ? part_ml[((size_t)lane * rows + row) * 2 + 1] : 0.f;
   float M = warp_max(m);
@@ -578,18 +590,31 @@ __global__ void latent_merge_kernel(const float* __restrict__ part_o, const floa
   float l = warp_sum(lz * wz);
   if (sink != nullptr) l += expf(sink[h] - M);
   const float inv = l > 0.f ? 1.0f / l : 0.f;
-  for (int c = lane; c < r; c += 32) {
-    float acc = 0.f;
-#pragma unroll 8
-    for (int z = 0; z < n_splits; ++z) {
+  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int z0 = 0; z0 < n_splits; z0 += 16) {
+    float4 v[16];
+#pragma unroll
+    for (int z = 0; z < 16; ++z) {
       // loaded whether it counts or not (a share without rows holds no numbers), so that the loads go out together
-      const float v = part_o[((size_t)z * rows + row) * r + c];
-      const float w = __shfl_sync(0xffffffffu, wz, z);
-      acc = __fmaf_rn(w > 0.f ? v : 0.f, w, acc);
+      const bool in = z0 + z < n_splits && c < r;
+      v[z] = in ? load4_f32(part_o + ((size_t)(z0 + z) * rows + row) * r + c) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
-    const size_t at = (size_t)tok * o_n + (size_t)h * o_h + c;
-    if (out_bf16) reinterpret_cast<__nv_bfloat16*>(out)[at] = __float2bfloat16_rn(acc * inv);
-    else reinterpret_cast<float*>(out)[at] = acc * inv;
+#pragma unroll
+    for (int z = 0; z < 16; ++z) {
+      const float w = __shfl_sync(0xffffffffu, wz, (z0 + z) & 31);
+      if (z0 + z < n_splits && w > 0.f) {
+        acc.x = __fmaf_rn(v[z].x, w, acc.x); acc.y = __fmaf_rn(v[z].y, w, acc.y);
+        acc.z = __fmaf_rn(v[z].z, w, acc.z); acc.w = __fmaf_rn(v[z].w, w, acc.w);
+      }
+    }
+  }
+  if (c >= r) return;
+  const float o[4] = {acc.x * inv, acc.y * inv, acc.z * inv, acc.w * inv};
+  const size_t at = (size_t)tok * o_n + (size_t)h * o_h + c;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    if (out_bf16) reinterpret_cast<__nv_bfloat16*>(out)[at + i] = __float2bfloat16_rn(o[i]);
+    else reinterpret_cast<float*>(out)[at + i] = o[i];
   }
 }
 
@@ -617,6 +642,17 @@ template <int R>
 int launch_latent_mma_any(const LatentMma& a, int max_rows, int n_requests, cudaStream_t stream) {
   if (max_rows > 32 && latent_mma_smem<R, 2>(a.p) <= 227 * 1024) return launch_latent_mma<R, 2>(a, max_rows, n_requests, stream);
   return launch_latent_mma<R, 1>(a, max_rows, n_requests, stream);
+}
+
+// Whether the tcgen05 form takes the call: its sizes, a pool that is one matrix of rows for TMA, and operands it reads and
+// writes 16 bytes at a time.
+bool latent_tc_applies(const LatentMma& a, int r, int num_pages) {
+  const auto aligned = [](const void* ptr, long n, long h, int size) {
+    return !((uintptr_t)ptr & 15) && (n * size) % 16 == 0 && (h * size) % 16 == 0;
+  };
+  return yalis_latent_attention_tcgen05_supports(r, a.p, a.page_size) && a.q_lat_bf16 && a.scale > 0.f &&
+         aligned(a.q_lat, a.ql_n, a.ql_h, 2) && aligned(a.q_rot, a.qr_n, a.qr_h, 4) &&
+         aligned(a.out, a.o_n, a.o_h, a.out_bf16 ? 2 : 4) && (long long)num_pages * a.page_size < 0x7fffffffLL;
 }
 
 }  // namespace
@@ -721,7 +757,7 @@ YALIS_API int yalis_latent_attention_mma(const void* q_lat, int q_lat_bf16, long
                                          const int32_t* block_table, int table_width, int page_size, int num_pages,
                                          int n_requests, int n_tokens, int max_q_len, int heads, int r, int p, float scale,
                                          int window, const float* sink, int n_splits, float* part_o, float* part_ml,
-                                         cudaStream_t stream) {
+                                         int32_t* error, cudaStream_t stream) {
   if (n_requests <= 0 || max_q_len <= 0) return YALIS_OK;
   if (!yalis_latent_attention_mma_supports(r, p) || heads <= 0 || n_requests > 65535 || n_splits < 1 || n_splits > 32)
     return YALIS_ERR_SHAPE;
@@ -735,7 +771,11 @@ YALIS_API int yalis_latent_attention_mma(const void* q_lat, int q_lat_bf16, long
   a.n_splits = n_splits; a.part_o = part_o; a.part_ml = part_ml; a.n_tokens = n_tokens;
   const int max_rows = max_q_len * heads;
   int status = YALIS_ERR_SHAPE;
-  switch (r) {
+  if (latent_tc_applies(a, r, num_pages)) {
+    status = yalis_latent_tc_launch(q_lat, ql_n, ql_h, q_rot, qr_n, qr_h, out, out_bf16, o_n, o_h, pool, positions, q_start,
+                                    block_table, table_width, page_size, num_pages, n_requests, n_tokens, max_q_len, heads, r, p,
+                                    scale, window, sink, n_splits, part_o, part_ml, error, stream);
+  } else switch (r) {
     case 64: status = launch_latent_mma_any<64>(a, max_rows, n_requests, stream); break;
     case 96: status = launch_latent_mma_any<96>(a, max_rows, n_requests, stream); break;
     case 128: status = launch_latent_mma_any<128>(a, max_rows, n_requests, stream); break;
@@ -745,6 +785,6 @@ YALIS_API int yalis_latent_attention_mma(const void* q_lat, int q_lat_bf16, long
   }
   if (status != YALIS_OK || n_splits == 1) return status;
   const int rows = n_tokens * heads, warps = 4;
-  return yalis_launch(latent_merge_kernel, dim3((rows + warps - 1) / warps), dim3(32 * warps), 0, stream, (const float*)part_o,
+  return yalis_launch(latent_merge_kernel, dim3((rows + warps - 1) / warps, (r + 127) / 128), dim3(32 * warps), 0, stream, (const float*)part_o,
                       (const float*)part_ml, n_splits, n_tokens, heads, r, req_of_token, out, out_bf16, o_n, o_h, sink);
 }

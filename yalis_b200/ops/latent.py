@@ -7,7 +7,7 @@ from typing import Optional
 
 import torch
 
-from ._lib import check, dtype_code, f32, i32, i64, lib, need, need_cuda, ptr, stream
+from ._lib import check, dtype_code, error_word, f32, i32, i64, lib, need, need_cuda, ptr, stream
 
 
 def latent_prepare(src: torch.Tensor, q_off: int, kv_off: Optional[int], heads: int, d: int, r: int, p: int,
@@ -174,5 +174,5 @@ def latent_attention_mma(q_lat: torch.Tensor, q_rot: torch.Tensor, out: torch.Te
         i64(q_rot.stride(0)), i64(q_rot.stride(1)), ptr(out), i32(out.dtype == torch.bfloat16), i64(out.stride(0)),
         i64(out.stride(1)), ptr(pool), ptr(positions), ptr(q_start), ptr(req_of_token), ptr(block_table), i32(block_table.shape[1]),
         i32(pool.shape[2]), i32(pool.shape[0]), i32(n_requests), i32(n), i32(max_q_len), i32(h), i32(r), i32(p), f32(scale),
-        i32(window or 0), ptr(sink), i32(n_splits), ptr(part_o), ptr(part_ml), stream()), name)
+        i32(window or 0), ptr(sink), i32(n_splits), ptr(part_o), ptr(part_ml), ptr(error_word(q_lat.device)), stream()), name)
     return out
