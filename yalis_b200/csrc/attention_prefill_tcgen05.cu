@@ -27,10 +27,10 @@
 // free, so that a wait for one never holds up the other.  The grid is (tiles of queries of the step x KV heads, 1,
 // shares of the keys); a block finds the request of its tile from the requests' token ranges.
 // Same semantics as paged_attention_generic (mask by absolute position,
-// yalis/attention/backend_impl/sdpa_and_flex.py:15-19, 301-307) without a window.
+// yalis/attention/backend_impl/sdpa_and_flex.py:15-19, 301-307), in the plain form without a window.
 //
 // Limits (else the caller uses the mma.sync kernel): bfloat16, head_dim 64 or 128, page_size 8,
-// 16, 32, 64 or 128, at most 128 heads per KV head, no window.
+// 16, 32, 64 or 128, at most 128 heads per KV head; a window, chunks and the like in the general form.
 // Rows of V past a tile's last visible key may hold anything; they are zeroed in shared memory
 // before they are multiplied.  All mbarrier waits are bounded (error word, tensor memory freed).
 #include <cuda.h>
@@ -76,6 +76,14 @@ struct PrefillParams {
   float* part_o;               // [N, nh, n_splits, HS]
   float* part_ml;              // [N, nh, n_splits, 2]
   int32_t* error;
+  // the general form (see attention_mma.cu, whose arithmetic of scores, sinks and gates this is)
+  int window, chunk;           // 0: none
+  float cap_log2, scale_over_cap, out_scale;
+  int sink;                    // 1: a score without key and value in every denominator
+  const float* sink_logits;    // [nh] (null: 0)
+  const float* slopes;         // [nh] or null
+  const __nv_bfloat16* gate;   // [N, gate_stride] or null
+  int gate_stride, gate_per_head;
 #ifdef YALIS_TRACE_CLOCKS
   long long* trace;            // [blocks][64 tiles][32 stamps] of clock64(), for timeline probes (compiled out by default)
 #endif
@@ -111,10 +119,24 @@ struct ItemDesc {
   int n_rows;       // rows of the tile in use: tokens * heads_per_group
   int pos_first;    // absolute position of the first query token
   int hi_key;       // absolute position of the last one = the last visible key
+  int lo_last;      // general form: the first key that the last token sees
   int trace_row;
 };
 
-template <int HS>
+// The first key a row at position `pos` sees.
+__device__ __forceinline__ int first_visible(const PrefillParams& p, int pos) {
+  int lo = p.window > 0 ? max(0, pos - p.window + 1) : 0;
+  if (p.chunk > 0) lo = max(lo, pos / p.chunk * p.chunk);
+  return lo;
+}
+
+// GEN: the general form.  Rows see a window or a chunk, scores may be capped or fall off with the distance, a sink joins the
+// denominator, a gate and a factor multiply the result, and the weights meet V as two bfloat16 halves (16 bits of mantissa),
+// which fill the scores' 64 columns of tensor memory: half as many products again.  Tiles of keys that no row of an item sees
+// are left out at both ends.  Shares of an item's keys are for the plain form only.
+// Measured: the layer of 16 heads of 128 over 8 KV heads with chunks, sinks and a gate, 2,048 tokens: 346 us with the mma.sync
+// form (237 us of it that kernel), 172 us with this one.
+template <int HS, bool GEN>
 __global__ void __launch_bounds__(kThreads, 2)
 prefill_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                                  const __grid_constant__ CUtensorMap map_v, const PrefillParams p) {
@@ -246,7 +268,7 @@ prefill_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
       // The loads below are issued back to back: two round trips to memory (token range and first pages; then
       // positions) stand between the draw of an item and its first copy, not four.
       int early_page = -2;                                    // this lane's page of tile 0 (known before the positions are)
-      if (slots == 1) {
+      if (slots == 1 && !GEN) {
         const int pi = (my_box << box_shift) >> page_shift;
         early_page = (my_box < boxes_per_tile && pi < p.table_width) ? bt[pi] : -1;
       }
@@ -265,7 +287,8 @@ prefill_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
       const int pos_first = p.positions[tok0 + t0];
       const int hi_key = p.positions[tok0 + t0 + n_tok - 1];
       // This item's share of the key tiles (all of them without splits).
-      const int all_tiles = hi_key / BN + 1;
+      const int lo_key = GEN ? first_visible(p, pos_first) : 0, tile_lo = lo_key / BN;
+      const int all_tiles = hi_key / BN + 1 - tile_lo;
       const int wanted = slots > 1 ? min(slots, (all_tiles + p.tiles_per_split - 1) / p.tiles_per_split) : 1;
       const int per_split = (all_tiles + wanted - 1) / wanted;
       const int n_splits = (all_tiles + per_split - 1) / per_split;   // shares that get a tile (7 tiles in 5 shares: 4 of 2)
@@ -278,8 +301,8 @@ prefill_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
           }
         continue;
       }
-      const int tile_base = split * per_split;
-      const int n_tiles = min(all_tiles, tile_base + per_split) - tile_base;     // >= 1
+      const int tile_base = tile_lo + split * per_split;
+      const int n_tiles = min(all_tiles, (split + 1) * per_split) - split * per_split;     // >= 1
 #ifdef YALIS_TRACE_CLOCKS
       const int trace_row = in_share;
 #endif
@@ -291,6 +314,7 @@ prefill_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
         ItemDesc& it = descs[d];
         it.n_tiles = n_tiles; it.tile_base = tile_base; it.n_splits = n_splits; it.split = split; it.kvh = kvh;
         it.tok_first = tok0 + t0; it.n_rows = n_rows; it.pos_first = pos_first; it.hi_key = hi_key;
+        if (GEN) it.lo_last = first_visible(p, hi_key);
         it.trace_row = in_share;
         mbar_arrive(&desc_full[d]);
         // Q, once the products of the item before, which read it, are done.
@@ -309,9 +333,13 @@ prefill_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
       auto box_row = [&](int j) -> int {
         const int key = ((tile_base + j) << 6) + (my_box << box_shift);
         if (j >= n_tiles || my_box >= boxes_per_tile || key > hi_key) return -1;
+        // general form: rows no query sees (their page may be gone) and rows without a page are zeros (past the pool)
+        const int none = (p.num_pages * p.g) << page_shift;
+        if (GEN && key + box_rows <= lo_key) return none;
         const int pi = key >> page_shift;
         int page = (j == 0 && early_page != -2) ? early_page : (pi < p.table_width ? bt[pi] : -1);
         if (page < 0 || page >= p.num_pages) {
+          if (GEN) return none;
           if (p.error) atomicOr(p.error, YALIS_FLAG_BAD_PAGE);
           page = 0;
         }
@@ -426,6 +454,11 @@ prefill_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
           umma_ts(elected, tmem + COL_O, tmem + COL_S + b * BN + ks * 8, v_desc + ((ks * 2048) >> 4), idesc_pv,
                   (j > 0 || ks > 0) ? 1u : 0u);
         }
+        if constexpr (GEN) {
+#pragma unroll
+          for (int ks = 0; ks < BN / 16; ++ks)               // the weights' lower halves
+            umma_ts(elected, tmem + COL_O, tmem + COL_S + b * BN + BN / 2 + ks * 8, v_desc + ((ks * 2048) >> 4), idesc_pv, 1u);
+        }
         umma_commit(elected, o_full);
         umma_commit(elected, &v_empty[b]);
         if (lane == 0) STAMP(j, 10);
@@ -458,6 +491,12 @@ prefill_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
       const bool valid = r < n_rows;
       const int t_in = r / p.per, head = r - t_in * p.per;
       const int pos_row = valid ? p.positions[tok_first + t_in] : -1;
+      const int lo_row = GEN ? first_visible(p, max(pos_row, 0)) : 0, lo_last = GEN ? descs[d].lo_last : 0;
+      const int head_all = kvh * p.per + head;
+      const float slope2 = GEN && p.slopes ? p.slopes[head_all] * 1.4426950408889634f : 0.f;
+      // scores that are capped or fall off with the distance are brought to the exp2 domain one by one, others on the way
+      const bool one_by_one = GEN && (p.cap_log2 > 0.f || p.slopes != nullptr);
+      const float to_log2 = one_by_one ? 1.0f : p.scale_log2;
       float m_run = -INFINITY, l_run = 0.f;
       for (int j = 0; j < n_tiles && ok; ++j) {
         const int b = (T + j) & 1;
@@ -476,10 +515,22 @@ prefill_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
         }
         // S is in registers now; its buffer is written again only after P(j), which takes its place, has been used.
         if (lane == 0) STAMP(j, 2 + (warp ? 6 + warp * 6 : 0));
-        if (key0 + BN - 1 > pos_first || !valid) {           // some key of the tile is hidden from this row
+        if (GEN && one_by_one) {
+#pragma unroll
+          for (int c = 0; c < BN; ++c) {
+            const float off = slope2 * (float)(pos_row - (key0 + c));
+            if (p.cap_log2 > 0.f) {                            // c tanh(x / c), saturated where exp would overflow
+              const float x = fminf(sv[c] * p.scale_over_cap - off / p.cap_log2, 15.f);
+              sv[c] = p.cap_log2 * (1.0f - __fdividef(2.0f, __expf(2.0f * x) + 1.0f));
+            } else {
+              sv[c] = sv[c] * p.scale_log2 - off;
+            }
+          }
+        }
+        if (key0 + BN - 1 > pos_first || (GEN && key0 < lo_last) || !valid) {      // some key of the tile is hidden from some row
 #pragma unroll
           for (int c = 0; c < BN; ++c)
-            if (!valid || key0 + c > pos_row) sv[c] = -INFINITY;
+            if (!valid || key0 + c > pos_row || (GEN && key0 + c < lo_row)) sv[c] = -INFINITY;
         }
         float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
@@ -487,7 +538,7 @@ prefill_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
           mx[0] = max3(mx[0], sv[c], sv[c + 1]); mx[1] = max3(mx[1], sv[c + 2], sv[c + 3]);
           mx[2] = max3(mx[2], sv[c + 4], sv[c + 5]); mx[3] = max3(mx[3], sv[c + 6], sv[c + 7]);
         }
-        const float m_tile = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * p.scale_log2;
+        const float m_tile = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * to_log2;
         const float m_new = fmaxf(m_run, m_tile);
         if (lane == 0) STAMP(j, 3 + (warp ? 6 + warp * 6 : 0));
         // Keep the older maximum unless the new one is more than 2^8 larger: exp2 of at most 8 is
@@ -497,11 +548,11 @@ prefill_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
         const float mb = (m_use == -INFINITY) ? 0.f : m_use;
         const float corr = grow ? ((m_run == -INFINITY) ? 0.f : ex2(m_run - mb)) : 1.f;
         uint64_t ls2[2] = {pack2(0.f, 0.f), pack2(0.f, 0.f)};
-        const uint64_t scale2 = pack2(p.scale_log2, p.scale_log2), nmb2 = pack2(-mb, -mb);
+        const uint64_t scale2 = pack2(to_log2, to_log2), nmb2 = pack2(-mb, -mb);
         const uint32_t p_addr = lane_base + COL_S + b * BN;          // over the first half of S(j)
 #pragma unroll
         for (int c0 = 0; c0 < BN; c0 += 32) {
-          uint32_t pk[16];
+          uint32_t pk[16], lw[GEN ? 16 : 1];
 #pragma unroll
           for (int c = 0; c < 32; c += 4) {
             // scale and shift, and the row sums, two values to an instruction
@@ -513,8 +564,14 @@ prefill_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
             ls2[1] = add2(ls2[1], pack2(p2, p3));
             pk[c >> 1] = pack_bf16(p0, p1);
             pk[(c >> 1) + 1] = pack_bf16(p2, p3);
+            if constexpr (GEN) {
+              const uint32_t h0 = pk[c >> 1], h1 = pk[(c >> 1) + 1];
+              lw[c >> 1] = pack_bf16(p0 - __uint_as_float(h0 << 16), p1 - __uint_as_float(h0 & 0xffff0000u));
+              lw[(c >> 1) + 1] = pack_bf16(p2 - __uint_as_float(h1 << 16), p3 - __uint_as_float(h1 & 0xffff0000u));
+            }
           }
           tmem_st16(p_addr + (c0 >> 1), pk);
+          if constexpr (GEN) tmem_st16(p_addr + BN / 2 + (c0 >> 1), lw);
         }
         float ls[4];
         unpack2(ls2[0], ls[0], ls[1]);
@@ -581,7 +638,20 @@ prefill_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
           const size_t slot = ((size_t)(tok_first + t_in) * p.nh + kvh * p.per + head) * slots;
           *reinterpret_cast<float2*>(p.part_ml + slot * 2) = make_float2(INFINITY, 0.f);
         }
-        const float inv = l_run > 0.f ? 1.0f / l_run : 0.f;
+        float inv = l_run > 0.f ? 1.0f / l_run : 0.f;
+        const __nv_bfloat16* gate = nullptr;
+        if constexpr (GEN) {
+          if (p.sink) {                                         // the sums stand relative to m_run: the sink joins there
+            const float z = p.sink_logits ? p.sink_logits[head_all] * 1.4426950408889634f : 0.f, mf = fmaxf(m_run, z);
+            const float c = exp2f(m_run - mf);
+            inv = c / (l_run * c + exp2f(z - mf));
+          }
+          inv *= p.out_scale;
+          if (p.gate != nullptr && valid) {
+            gate = p.gate + (size_t)(tok_first + t_in) * p.gate_stride + (p.gate_per_head ? head_all : head_all * HS);
+            if (p.gate_per_head) inv *= 1.0f / (1.0f + __expf(-__bfloat162float(*gate)));
+          }
+        }
         __nv_bfloat16* dst = p.out + (size_t)(tok_first + (valid ? t_in : 0)) * p.out_stride +
                              (size_t)(kvh * p.per + (valid ? head : 0)) * HS;
 #pragma unroll 1
@@ -589,6 +659,18 @@ prefill_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
           uint32_t o[16];
           tmem_ld16(lane_base + COL_O + c0, o);
           asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+          if constexpr (GEN) {
+            if (gate != nullptr && !p.gate_per_head) {
+              const uint4 ga = *reinterpret_cast<const uint4*>(gate + c0), gb = *reinterpret_cast<const uint4*>(gate + c0 + 8);
+              const uint32_t gw[8] = {ga.x, ga.y, ga.z, ga.w, gb.x, gb.y, gb.z, gb.w};
+#pragma unroll
+              for (int c = 0; c < 8; ++c) {
+                o[2 * c] = __float_as_uint(__uint_as_float(o[2 * c]) * (1.0f / (1.0f + __expf(-__uint_as_float(gw[c] << 16)))));
+                o[2 * c + 1] = __float_as_uint(__uint_as_float(o[2 * c + 1]) *
+                                               (1.0f / (1.0f + __expf(-__uint_as_float(gw[c] & 0xffff0000u)))));
+              }
+            }
+          }
           if (valid) {
             uint4 v0, v1;
             v0.x = pack_bf16(__uint_as_float(o[0]) * inv, __uint_as_float(o[1]) * inv);
@@ -714,23 +796,48 @@ __global__ void prefill_merge_splits_kernel(const float* __restrict__ part_o, co
   }
 }
 
-template <int HS>
+template <int HS, bool GEN>
 int launch(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const PrefillParams& p, int n_splits,
            int n_tokens, cudaStream_t stream) {
   const size_t smem = 1024 + (size_t)BM * HS * 2 + (size_t)4 * BN * HS * 2 + kBarriers * 8 + 8 + 2 * sizeof(ItemDesc);
   static bool configured = false;
   if (!configured) {
-    if (cudaFuncSetAttribute(prefill_attention_tcgen05_kernel<HS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    if (cudaFuncSetAttribute(prefill_attention_tcgen05_kernel<HS, GEN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)smem) != cudaSuccess)
       return YALIS_ERR_LAUNCH;
     configured = true;
   }
   // Two blocks to an SM for the whole launch (fewer if the step has fewer items).
   dim3 grid((unsigned)std::min<long long>(p.n_items, 2LL * yalis_sm_count()), 1, 1);
-  int st = yalis_launch(prefill_attention_tcgen05_kernel<HS>, grid, dim3(kThreads), smem, stream, mq, mk, mv, p);
+  int st = yalis_launch(prefill_attention_tcgen05_kernel<HS, GEN>, grid, dim3(kThreads), smem, stream, mq, mk, mv, p);
   if (st != YALIS_OK || n_splits == 1) return st;
   return yalis_launch(prefill_merge_splits_kernel, dim3(n_tokens), dim3(256), 0, stream, (const float*)p.part_o,
                       (const float*)p.part_ml, p.out, p.out_stride, p.nh, HS, n_splits);
+}
+
+// Tiles of queries in the step: sum of ceil(q / tokens_per_tile) over the requests, bounded from their number, the step's
+// tokens and the longest request.
+bool count_items(PrefillParams& p, int n_tokens, int max_q_len, int n_splits) {
+  const long long tpt = p.tokens_per_tile;
+  const long long tiles = std::min(((long long)n_tokens + (long long)p.n_requests * (tpt - 1)) / tpt,
+                                   (long long)p.n_requests * ((max_q_len + tpt - 1) / tpt));
+  if (tiles * p.g * n_splits > 0x7fffffffLL) return false;
+  p.items_per_share = (int)(tiles * p.g);
+  p.n_z = n_splits;
+  p.n_items = p.items_per_share * n_splits;
+  return true;
+}
+
+template <bool GEN>
+int launch_prefill(const PrefillParams& p, const void* q, int q_stride, const void* k_pool, const void* v_pool, int n_tokens,
+                   int hs, int n_splits, cudaStream_t stream) {
+  CUtensorMap mq, mk, mv;
+  const long long rows = (long long)p.num_pages * p.g * p.page_size;
+  if (!make_q_map(&mq, q, n_tokens, q_stride, p.nh, hs, p.per, p.tokens_per_tile) ||
+      !make_pool_map(&mk, k_pool, rows, hs, p.page_size) || !make_pool_map(&mv, v_pool, rows, hs, p.page_size))
+    return YALIS_ERR_LAUNCH;
+  return hs == 64 ? launch<64, GEN>(mq, mk, mv, p, n_splits, n_tokens, stream)
+                  : launch<128, GEN>(mq, mk, mv, p, n_splits, n_tokens, stream);
 }
 
 }  // namespace
@@ -777,24 +884,14 @@ YALIS_API int yalis_prefill_attention_tcgen05(const void* q, int q_stride, void*
   if (!yalis_prefill_attention_tcgen05_supports(hs, page_size, nh / g)) return YALIS_ERR_SHAPE;
   if (((uintptr_t)q | (uintptr_t)k_pool | (uintptr_t)v_pool | (uintptr_t)out) & 15) return YALIS_ERR_ALIGN;
   if ((q_stride % 8) || (out_stride % 8)) return YALIS_ERR_ALIGN;
-  PrefillParams p;
+  PrefillParams p = {};
   p.out = (__nv_bfloat16*)out; p.out_stride = out_stride;
   p.positions = positions; p.q_start = q_start; p.block_table = block_table;
   p.table_width = table_width; p.page_size = page_size; p.num_pages = num_pages;
   p.nh = nh; p.g = g; p.per = nh / g;
   p.n_requests = n_requests;
   p.tokens_per_tile = BM / p.per;
-  {
-    // Tiles of queries in the step: sum of ceil(q / tokens_per_tile) over the requests, bounded from their
-    // number, the step's tokens and the longest request.
-    const long long tpt = p.tokens_per_tile;
-    const long long tiles = std::min(((long long)n_tokens + (long long)n_requests * (tpt - 1)) / tpt,
-                                     (long long)n_requests * ((max_q_len + tpt - 1) / tpt));
-    if (tiles * g * n_splits > 0x7fffffffLL) return YALIS_ERR_SHAPE;
-    p.items_per_share = (int)(tiles * g);
-    p.n_z = n_splits;
-    p.n_items = p.items_per_share * n_splits;
-  }
+  if (!count_items(p, n_tokens, max_q_len, n_splits)) return YALIS_ERR_SHAPE;
   p.work = work;
   p.scale_log2 = scale * 1.4426950408889634f;
   p.tiles_per_split = tiles_per_split > 0 ? tiles_per_split : 1;
@@ -805,11 +902,41 @@ YALIS_API int yalis_prefill_attention_tcgen05(const void* q, int q_stride, void*
 #ifdef YALIS_TRACE_CLOCKS
   p.trace = trace;
 #endif
-  CUtensorMap mq, mk, mv;
-  const long long rows = (long long)num_pages * g * page_size;
-  if (!make_q_map(&mq, q, n_tokens, q_stride, nh, hs, p.per, p.tokens_per_tile) ||
-      !make_pool_map(&mk, k_pool, rows, hs, page_size) || !make_pool_map(&mv, v_pool, rows, hs, page_size))
-    return YALIS_ERR_LAUNCH;
-  return hs == 64 ? launch<64>(mq, mk, mv, p, n_splits, n_tokens, stream)
-                  : launch<128>(mq, mk, mv, p, n_splits, n_tokens, stream);
+  return launch_prefill<false>(p, q, q_stride, k_pool, v_pool, n_tokens, hs, n_splits, stream);
+}
+
+// The general form: `out` may be a column block of a wider matrix; window / chunk 0: none; softcap 0: none; sink 1 with
+// sink_logits [nh] (or null: 0); slopes [nh] or null; gate [N, gate_stride] bfloat16 on 16-byte boundaries (per head: any) or
+// null.  Otherwise as above, without shares of the keys.
+YALIS_API int yalis_prefill_attention_tcgen05_general(
+    const void* q, int q_stride, void* out, int out_stride, const void* k_pool, const void* v_pool, const int32_t* positions,
+    const int32_t* q_start, const int32_t* block_table, int table_width, int page_size, int num_pages, int n_tokens,
+    int n_requests, int max_q_len, int nh, int g, int hs, float scale, int window, int chunk, float softcap, int sink,
+    const float* sink_logits, const float* slopes, const void* gate, int gate_stride, int gate_per_head, float out_scale,
+    int32_t* work, int32_t* error, cudaStream_t stream) {
+  if (n_tokens <= 0 || n_requests <= 0) return YALIS_OK;
+  if (g <= 0 || nh % g != 0 || max_q_len < 1 || softcap < 0.f || !(scale > 0.f)) return YALIS_ERR_SHAPE;
+  if (work == nullptr) return YALIS_ERR_ALIGN;
+  if (!yalis_prefill_attention_tcgen05_supports(hs, page_size, nh / g)) return YALIS_ERR_SHAPE;
+  if (((uintptr_t)q | (uintptr_t)k_pool | (uintptr_t)v_pool | (uintptr_t)out) & 15) return YALIS_ERR_ALIGN;
+  if ((q_stride % 8) || (out_stride % 8)) return YALIS_ERR_ALIGN;
+  if (gate && !gate_per_head && ((gate_stride % 8) || ((uintptr_t)gate & 15))) return YALIS_ERR_ALIGN;
+  PrefillParams p = {};
+  p.out = (__nv_bfloat16*)out; p.out_stride = out_stride;
+  p.positions = positions; p.q_start = q_start; p.block_table = block_table;
+  p.table_width = table_width; p.page_size = page_size; p.num_pages = num_pages;
+  p.nh = nh; p.g = g; p.per = nh / g;
+  p.n_requests = n_requests;
+  p.tokens_per_tile = BM / p.per;
+  if (!count_items(p, n_tokens, max_q_len, 1)) return YALIS_ERR_SHAPE;
+  p.work = work;
+  p.scale_log2 = scale * 1.4426950408889634f;
+  p.tiles_per_split = 1;
+  p.error = error;
+  p.window = window; p.chunk = chunk;
+  p.cap_log2 = softcap * 1.4426950408889634f; p.scale_over_cap = softcap > 0.f ? scale / softcap : 0.f;
+  p.out_scale = out_scale;
+  p.sink = sink; p.sink_logits = sink ? sink_logits : nullptr; p.slopes = slopes;
+  p.gate = (const __nv_bfloat16*)gate; p.gate_stride = gate_stride; p.gate_per_head = gate_per_head;
+  return launch_prefill<true>(p, q, q_stride, k_pool, v_pool, n_tokens, hs, 1, stream);
 }

@@ -317,7 +317,7 @@ class GeneralAttention(Mixer, Projected):
         return {"tokens": tokens, "blocks": PagedKV(self.g, self.hs, None, v_head_dim=vd, pool=self.pool)}
 
     def _tensor_core_form(self, dtype: torch.dtype) -> bool:
-        """bfloat16 steps with head sizes the kernel is built for go to the tensor cores (scores and the sum of weights
+        """bfloat16 steps with head sizes the kernels are built for go to the tensor cores (scores and the sum of weights
         in float32, the weights against V in two bfloat16 halves); float32 steps and other shapes go to the exact
         kernel."""
         if dtype != torch.bfloat16:
@@ -335,7 +335,8 @@ class GeneralAttention(Mixer, Projected):
         return host.max_q_len, (attn_ops.decode_splits(len(host.slots), blocks) if rows <= 16 else 1)
 
     def capture_key(self, host):
-        # the exact kernel launches the same for every step; the tensor-core one by the longest portion
+        # the exact kernel launches the same for every step; the choice among the tensor-core ones and their launch go by the
+        # longest portion
         return ("general_attention",) + self._launch_shape(host)
 
     def keys_seen(self, position: int) -> int:
@@ -388,6 +389,14 @@ class GeneralAttention(Mixer, Projected):
         scale_out = self.out_scale if self.difference is None else 1.0 - self.difference[0]
         if self._tensor_core_form(z.dtype):
             longest, splits = self._launch_shape(ctx.host)
+            if (longest * (self.nh // self.g) > 16 and self.difference is None and self.rel is None and blocks is None
+                    and attn_ops.prefill_general_applies(q, y, gate, cache.k.shape[2], self.nh, self.g, self.hs, self.vd, self.scale)):
+                # portions with more rows than a decode tile holds (single tokens of the same step ride along)
+                attn_ops.prefill_attention_general(q, cache.k, cache.v, ctx.positions, ctx.q_start, table, longest, self.nh, self.g,
+                                                   self.hs, self.scale, y, window=self.window, chunk=self.chunk,
+                                                   softcap=self.softcap, sink=self.sink, sink_logits=self.sink_logits,
+                                                   slopes=self.slopes, gate=gate, out_scale=scale_out, error_flag=ctx.error_flag)
+                return
             direct = y.data_ptr() % 16 == 0 and y.stride(0) % 2 == 0
             out = attn_ops.paged_attention_mma(q, cache.k, cache.v, ctx.positions, ctx.q_start, ctx.req_of_token, table, longest,
                                                self.nh, self.g, self.hs, scale=self.scale, window=self.window, n_splits=splits,
