@@ -636,11 +636,36 @@ __global__ void residual_add_kernel(float* __restrict__ x, const TD* __restrict_
   x[i] = h;
 }
 
+// The same, four values a thread (x, the partial sums and their stride on the boundaries of four values): bound by memory.
+// 2,048 x 2,048 rows with one bfloat16 delta, 42 MB: 19 us a value a thread, 9 us this way (ncu, cold).
+// (No __restrict__: a load the compiler takes for one of constant data may be moved above the wait for the kernel before.)
+template <typename TD>
+__global__ void residual_add_x4_kernel(float* x, const TD* delta, int n_delta, size_t delta_stride, size_t quads) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= quads) return;
+  float4 h = load4_f32(x + 4 * i);
+#pragma unroll 4
+  for (int s = 0; s < n_delta; ++s) {
+    const float4 d = load4_f32(delta + (size_t)s * delta_stride + 4 * i);
+    h.x += d.x; h.y += d.y; h.z += d.z; h.w += d.w;
+  }
+  store4(x + 4 * i, h);
+}
+
 YALIS_API int yalis_residual_add(float* x, const void* delta, int delta_dtype, int n_delta, long long delta_stride,
                                  long long n, cudaStream_t stream) {
   if (n <= 0) return YALIS_OK;
   const int threads = 256;
   const unsigned blocks = (unsigned)((n + threads - 1) / threads);
+  const uintptr_t narrow = delta_dtype == YALIS_BF16 ? 7 : 15;
+  if (n % 4 == 0 && (n_delta <= 1 || delta_stride % 4 == 0) && !((uintptr_t)x & 15) && !((uintptr_t)delta & narrow)) {
+    const size_t quads = (size_t)n / 4;
+    const dim3 grid((unsigned)((quads + threads - 1) / threads));
+    YALIS_DISPATCH_DTYPE(delta_dtype, TD, return yalis_launch(residual_add_x4_kernel<TD>, grid, dim3(threads), 0, stream, x,
+                                                              (const TD*)delta, n_delta, (size_t)delta_stride, quads));
+  }
   if (delta_dtype == YALIS_F32)
     return yalis_launch(residual_add_kernel<float>, dim3(blocks), dim3(threads), 0, stream, x, (const float*)delta,
                         n_delta, (size_t)delta_stride, (size_t)n);

@@ -153,6 +153,23 @@ __global__ void head_project_kernel(const TX* __restrict__ x, long xs_n, long xs
   }
 }
 
+// y[n, h * e + c] = x[n, h, c] * sigmoid(g[n, h * e + c]), four neighbouring values a thread (e a multiple of four, all rows
+// on the boundaries of four values).  Bound by memory: 2,048 tokens of 16 x 128 values, 25 MB: 22 us a value a thread with
+// two divisions each, 10.5 us this way (ncu, cold).
+template <typename T, typename TX>
+__global__ void sigmoid_gate_x4_kernel(const TX* x, long xs_n, long xs_h, int e, const T* g, long gs, T* y, long ys, int cols) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const int n = blockIdx.y, c = (blockIdx.x * blockDim.x + threadIdx.x) * 4;
+  if (c >= cols) return;
+  const int h = c / e;
+  float4 v = load4_f32(x + (size_t)n * xs_n + (size_t)h * xs_h + (c - h * e));
+  const float4 z = load4_f32(g + (size_t)n * gs + c);
+  v.x /= 1.0f + expf(-z.x); v.y /= 1.0f + expf(-z.y);
+  v.z /= 1.0f + expf(-z.z); v.w /= 1.0f + expf(-z.w);
+  store4(y + (size_t)n * ys + c, v);
+}
+
 // y[n, h * e + c] = x[n, h, c] * sigmoid(g[n, h * e + c])  (x float32 or model dtype with strides over n and h,
 // y and g model dtype)
 template <typename T, typename TX>
@@ -714,6 +731,20 @@ YALIS_API int yalis_sigmoid_gate(const void* x, int x_dtype, long xs_n, long xs_
   if (e <= 0 || cols % e) return YALIS_ERR_SHAPE;
   const size_t total = (size_t)rows * cols;
   const int blocks = (int)((total + 255) / 256 < 148 * 16 ? (total + 255) / 256 : 148 * 16);
+  const auto on4 = [](const void* p, int size) { return ((uintptr_t)p & (4 * size - 1)) == 0; };
+  if (e % 4 == 0 && ((xs_n | xs_h | gs | ys) & 3) == 0 && rows <= 65535 && on4(x, x_dtype == YALIS_F32 ? 4 : 2) &&
+      on4(g, dtype == YALIS_F32 ? 4 : 2) && on4(y, dtype == YALIS_F32 ? 4 : 2)) {
+    const dim3 grid((cols / 4 + 127) / 128, rows), block(128);
+    if (dtype == YALIS_F32 && x_dtype == YALIS_F32)
+      return yalis_launch(sigmoid_gate_x4_kernel<float, float>, grid, block, 0, stream, (const float*)x, xs_n, xs_h, e,
+                          (const float*)g, gs, (float*)y, ys, cols);
+    if (dtype == YALIS_BF16 && x_dtype == YALIS_F32)
+      return yalis_launch(sigmoid_gate_x4_kernel<__nv_bfloat16, float>, grid, block, 0, stream, (const float*)x, xs_n, xs_h, e,
+                          (const __nv_bfloat16*)g, gs, (__nv_bfloat16*)y, ys, cols);
+    if (dtype == YALIS_BF16 && x_dtype == YALIS_BF16)
+      return yalis_launch(sigmoid_gate_x4_kernel<__nv_bfloat16, __nv_bfloat16>, grid, block, 0, stream, (const __nv_bfloat16*)x,
+                          xs_n, xs_h, e, (const __nv_bfloat16*)g, gs, (__nv_bfloat16*)y, ys, cols);
+  }
   if (dtype == YALIS_F32 && x_dtype == YALIS_F32)
     return yalis_launch(sigmoid_gate_kernel<float, float>, dim3(blocks), dim3(256), 0, stream, (const float*)x, xs_n, xs_h, e,
                         (const float*)g, gs, (float*)y, ys, rows, cols);

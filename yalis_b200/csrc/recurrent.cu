@@ -582,6 +582,52 @@ __global__ void head_norm_gate_kernel(const float* __restrict__ o, int o_stride,
   }
 }
 
+// The same for heads of up to 512 values, a multiple of four, on the boundaries of four values: a head stays in registers
+// between the sum and the result, everything is read and written once, four values at a time.  Bound by memory: 2,048 tokens
+// of 16 heads of 128, 34 MB: 19 us a value at a time, 15 us this way (ncu, cold).
+template <typename T>
+__global__ void head_norm_gate_x4_kernel(const float* o, int o_stride, const float* weight, const T* gate, int gate_stride,
+                                         int gate_kind, T* y, int y_stride, const int32_t* req_of_token, int heads, int vdim,
+                                         float eps, float out_scale, int weight_stride) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const int n = blockIdx.x, h = blockIdx.y * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (h >= heads || req_of_token[n] < 0) return;
+  const float* op = o + (size_t)n * o_stride + (size_t)h * vdim;
+  const T* gp = gate_kind ? gate + (size_t)n * gate_stride + (size_t)h * vdim : nullptr;
+  float4 v[4], g[4];
+  float ss = 0.f;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int d = i * 128 + lane * 4;
+    if (i * 128 >= vdim) break;                    // (uniform)
+    v[i] = g[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (d < vdim) {
+      v[i] = load4_f32(op + d);
+      if (gate_kind) g[i] = load4_f32(gp + d);
+    }
+    ss += (v[i].x * v[i].x + v[i].y * v[i].y) + (v[i].z * v[i].z + v[i].w * v[i].w);
+  }
+  ss = warp_sum(ss);
+  const float r = 1.0f / sqrtf(ss / (float)vdim + eps);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int d = i * 128 + lane * 4;
+    if (d >= vdim) break;
+    float4 x = make_float4(v[i].x * r, v[i].y * r, v[i].z * r, v[i].w * r);
+    if (weight) {
+      const float4 w = load4_f32(weight + (size_t)h * weight_stride + d);
+      x.x *= w.x; x.y *= w.y; x.z *= w.z; x.w *= w.w;
+    }
+    if (gate_kind == 1) {
+      x.x *= silu_exact(g[i].x); x.y *= silu_exact(g[i].y); x.z *= silu_exact(g[i].z); x.w *= silu_exact(g[i].w);
+    } else if (gate_kind) {
+      x.x *= sigmoid_f(g[i].x); x.y *= sigmoid_f(g[i].y); x.z *= sigmoid_f(g[i].z); x.w *= sigmoid_f(g[i].w);
+    }
+    store4(y + (size_t)n * y_stride + (size_t)h * vdim + d, make_float4(x.x * out_scale, x.y * out_scale, x.z * out_scale, x.w * out_scale));
+  }
+}
+
 // ---- gate and norm in equal parts -------------------------------------------------------------------------------
 //   y = o * act(z);   y[part] <- y / sqrt(mean(y^2 over the part) + eps) * weight * out_scale           (after = 0)
 //   y = o / sqrt(mean(o^2 over the part) + eps) * weight * act(z) * out_scale                            (after = 1)
@@ -827,6 +873,14 @@ YALIS_API int yalis_head_norm_gate(const float* o, int o_stride, const float* we
   if (n_tokens <= 0) return YALIS_OK;
   if (heads <= 0 || heads > 65535 || vdim <= 0 || gate_kind < 0 || gate_kind > 2 || (gate_kind && !gate)) return YALIS_ERR_SHAPE;
   const int warps = heads < 4 ? heads : 4;
+  const uintptr_t narrow = dtype == YALIS_BF16 ? 7 : 15;
+  if (vdim <= 512 && ((vdim | o_stride | y_stride | (gate_kind ? gate_stride : 0)) & 3) == 0 &&
+      !(((uintptr_t)o | (uintptr_t)weight) & 15) && !(((uintptr_t)y | (uintptr_t)(gate_kind ? gate : nullptr)) & narrow))
+    YALIS_DISPATCH_DTYPE(dtype, T,
+                         return yalis_launch(head_norm_gate_x4_kernel<T>, dim3(n_tokens, (heads + warps - 1) / warps),
+                                             dim3(32 * warps), 0, stream, o, o_stride, weight, (const T*)gate, gate_stride,
+                                             gate_kind, (T*)y, y_stride, req_of_token, heads, vdim, eps, out_scale,
+                                             weight_per_head ? vdim : 0));
   YALIS_DISPATCH_DTYPE(dtype, T,
                        return yalis_launch(head_norm_gate_kernel<T>, dim3(n_tokens, (heads + warps - 1) / warps),
                                            dim3(32 * warps), 0, stream, o, o_stride, weight, (const T*)gate, gate_stride,
