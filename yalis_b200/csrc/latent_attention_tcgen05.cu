@@ -14,14 +14,15 @@
 //   O += (P_hi + P_lo) V    tcgen05.mma with A from tensor memory and the tile's rows as an MN-major operand; O [128][R]
 //                   stays in tensor memory and is rescaled only when a row's maximum has grown by more than 2^8.
 //
-// One warp looks up pages and issues the copies (a ring of two or three tiles), one issues the products: the scores of tile
-// j + 1 run while the softmax of tile j is computed.  Blocks are numbered so that the heaviest tiles of queries start first.
+// One warp looks up pages and issues the copies (a ring of two or three tiles), one issues the products, whichever are ready:
+// the scores of tile j + 1 run while the softmax of tile j is computed.  Blocks are numbered so that the heaviest tiles of queries start first.
 //
 // What bounds it: the tensor pipe.  A tile of 64 rows costs R + p over 16 products of 128 x 64 x 16 (limited by their
 // operands' way out of shared memory: 48 instead of 32 cycles) and 2 * 64 / 16 of 128 x R x 16.  R = 256, p = 64: 1,984
 // cycles a tile beside about 1,100 of the softmax warps.  The tile is 64 rows wide because O (R columns) and two S fill the
 // tensor memory at R = 384, and because three tiles of 320 columns beside Q are what shared memory holds.
-// Measured: a layer with r = 256, p = 64, 16 heads and 2,048 tokens (products, preparation and gate included) 582 -> 245 us;
+// Measured: a layer with r = 256, p = 64, 16 heads and 2,048 tokens (products, preparation and gate included) 582 -> 194 us,
+// 523 -> 93 us for this kernel (140 with Q loaded piece by piece and products in a fixed order);
 // 8 single tokens of 16 heads behind 1,024 rows in 16 shares: 37 -> 17 us for this kernel, 22 -> 8 us for the merge.
 //
 // With n_splits > 1 the tiles of a request are dealt to that many blocks in contiguous shares, which leave unnormalised sums
@@ -126,22 +127,51 @@ latent_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map, const L
   // The queries, as bfloat16, into the swizzled K-major layout: 16-byte piece c of row r lies at piece c ^ (r & 7) of its
   // 128 bytes.  Rows past the last one are zeros.  (The copy warp leaves this to the others and starts on the tiles.)
   if (warp != 4) {
+    // Loads in batches before their stores: the compiler cannot tell that a store to shared memory leaves the next load
+    // alone, and a trip to memory per 16 bytes made this a third of a block's time.
     const int first = warp == 5 ? 128 + lane : tid;        // 160 threads
-#pragma unroll 8
-    for (int e = first; e < LM * subs * 8; e += 160) {
-      const int r = e / (subs * 8), piece = e - r * (subs * 8), c = piece * 8;
-      uint4 v = make_uint4(0u, 0u, 0u, 0u);
-      if (r < rows_here) {
-        const int tok = q0 + (row0 + r) / a.heads, h = (row0 + r) % a.heads;
-        if (c < R) {
-          v = *reinterpret_cast<const uint4*>(a.q_lat + (size_t)tok * a.ql_n + (size_t)h * a.ql_h + c);
-        } else {
-          const float* src = a.q_rot + (size_t)tok * a.qr_n + (size_t)h * a.qr_h + (c - R);
-          const float4 x = *reinterpret_cast<const float4*>(src), y = *reinterpret_cast<const float4*>(src + 4);
-          v = make_uint4(pack_bf16(x.x, x.y), pack_bf16(x.z, x.w), pack_bf16(y.x, y.y), pack_bf16(y.z, y.w));
+    constexpr int RP = R / 8, BATCH = 8;                   // 16-byte pieces of a row's first part
+    auto place = [&](int r, int piece) -> uint4* {
+      return reinterpret_cast<uint4*>(q_s + (piece >> 3) * (LM * 128) + r * 128 + (((piece & 7) ^ (r & 7)) << 4));
+    };
+    for (int e0 = first; e0 < LM * RP; e0 += 160 * BATCH) {
+      uint4 v[BATCH];
+#pragma unroll
+      for (int i = 0; i < BATCH; ++i) {
+        const int e = e0 + i * 160, r = e / RP;
+        v[i] = make_uint4(0u, 0u, 0u, 0u);
+        if (e < LM * RP && r < rows_here) {
+          const int t = (row0 + r) / a.heads, h = row0 + r - t * a.heads;
+          v[i] = *reinterpret_cast<const uint4*>(a.q_lat + (size_t)(q0 + t) * a.ql_n + (size_t)h * a.ql_h + (e - r * RP) * 8);
         }
       }
-      *reinterpret_cast<uint4*>(q_s + (piece >> 3) * (LM * 128) + r * 128 + (((piece & 7) ^ (r & 7)) << 4)) = v;
+#pragma unroll
+      for (int i = 0; i < BATCH; ++i) {
+        const int e = e0 + i * 160, r = e / RP;
+        if (e < LM * RP) *place(r, e - r * RP) = v[i];
+      }
+    }
+    const int pp = a.p / 8;
+    for (int e0 = first; e0 < LM * pp; e0 += 160 * (BATCH / 2)) {
+      float4 x[BATCH / 2], y[BATCH / 2];
+#pragma unroll
+      for (int i = 0; i < BATCH / 2; ++i) {
+        const int e = e0 + i * 160, r = e / pp;
+        x[i] = y[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (e < LM * pp && r < rows_here) {
+          const int t = (row0 + r) / a.heads, h = row0 + r - t * a.heads;
+          const float* src = a.q_rot + (size_t)(q0 + t) * a.qr_n + (size_t)h * a.qr_h + (e - r * pp) * 8;
+          x[i] = load4_f32(src);
+          y[i] = load4_f32(src + 4);
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < BATCH / 2; ++i) {
+        const int e = e0 + i * 160, r = e / pp;
+        if (e < LM * pp)
+          *place(r, RP + e - r * pp) = make_uint4(pack_bf16(x[i].x, x[i].y), pack_bf16(x[i].z, x[i].w), pack_bf16(y[i].x, y[i].y),
+                                                  pack_bf16(y[i].z, y[i].w));
+      }
     }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
@@ -191,10 +221,9 @@ latent_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map, const L
     const uint32_t idesc_qk = idesc_f16(LM, LN, false);
     const uint64_t q_desc = desc_kmajor(smem_u32(q_s)), k_desc0 = desc_kmajor(smem_u32(k_s));
     const uint64_t v_desc0 = desc_mnmajor(smem_u32(k_s), LN * 128);
-    auto issue_qk = [&](int j) -> bool {
+    auto issue_qk = [&](int j) {
       const int b = j % a.stages;
-      // the S buffer is free: P(j - 2), which lay in it, has been waited for and its product issued before this one
-      if (!mbar_wait(&full[b], (j / a.stages) & 1, abort_flag)) return false;
+      // the S buffer is free: P(j - 2), which lay in it, was read by a product issued before this one
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint64_t k_desc = k_desc0 + (uint64_t)((b * tile_bytes) >> 4);
       for (int ks = 0; ks < W / 16; ++ks) {
@@ -202,13 +231,9 @@ latent_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map, const L
         umma_ss(elected, tmem + COL_S + (j & 1) * LN, q_desc + (q_off >> 4), k_desc + (k_off >> 4), idesc_qk, ks > 0);
       }
       umma_commit(elected, &s_full[j & 1]);
-      return true;
     };
-    bool ok = issue_qk(0);
-    for (int j = 0; j < n_tiles && ok; ++j) {
+    auto issue_pv = [&](int j) {
       const int b = j % a.stages;
-      if (j + 1 < n_tiles) ok = issue_qk(j + 1);
-      if (!ok || !mbar_wait(&p_full[j & 1], (j >> 1) & 1, abort_flag)) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint64_t v_desc = v_desc0 + (uint64_t)((b * tile_bytes) >> 4);
       const uint32_t p_at = tmem + COL_S + (j & 1) * LN;
@@ -227,6 +252,22 @@ latent_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map, const L
       umma_commit(elected, o_full);
       umma_commit(elected, &empty[b]);
       if (j + 1 == n_tiles) umma_commit(elected, o_done);
+    };
+    // Whatever is ready goes out: P V of a tile whose weights are there before the scores of the tile after the next, whose
+    // rows may still be on their way (waiting for those first held P V back, and with it the buffer they wait for).
+    int next_s = 0, next_o = 0;
+    for (uint32_t idle = 0; next_o < n_tiles;) {
+      if (next_o < next_s && __all_sync(0xffffffffu, mbar_test(&p_full[next_o & 1], (next_o >> 1) & 1))) {
+        issue_pv(next_o++);
+        idle = 0;
+      } else if (next_s < n_tiles && next_s < next_o + 2 &&
+                 __all_sync(0xffffffffu, mbar_test(&full[next_s % a.stages], (next_s / a.stages) & 1))) {
+        issue_qk(next_s++);
+        idle = 0;
+      } else if (++idle > kSpinLimit * 4 || ((idle & 1023u) == 1023u && __any_sync(0xffffffffu, *abort_flag))) {
+        if (lane == 0) *abort_flag = 1;
+        break;
+      }
     }
     __syncwarp();
   } else {
@@ -290,7 +331,7 @@ latent_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map, const L
       l_run = l_run * corr + ((ls[0] + ls[1]) + (ls[2] + ls[3]));
       m_run = m_use;
       if (j > 0 && __any_sync(0xffffffffu, grow)) {                  // rescale O (never for the first tile)
-        // (the scores of tile j are there, so P V of tile j - 2 is done: the phase waited for is the current one)
+        // (the scores of tile j are there, and P V of tile j - 2 was issued before them: the phase waited for is the current one)
         if (!warp_wait(o_full, (j - 1) & 1, abort_flag, lane)) { ok = false; break; }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll 1
