@@ -4,9 +4,9 @@
 // is stored).  Products and sums are float32 FMAs; there is no tensor-core
 // instruction and no reduced-precision mode anywhere in this file, so with
 // float32 operands the result is a true 32-bit product.  Each output element
-// is accumulated over k = 0..K-1 in ascending order by one thread, so it does
-// not depend on M, N or the tile a row falls into: a token's result is the
-// same bits whatever batch it is computed in.
+// is accumulated in chains over fixed values of k that are added in a fixed
+// order, so it does not depend on M, N or the tile a row falls into: a token's
+// result is the same bits whatever batch it is computed in.
 //
 // Operand and output types are independent (float or bfloat16), which lets the
 // same kernel serve as the twin of the tensor-core kernels in tests.
@@ -14,27 +14,33 @@
 
 namespace {
 
-// A tile of BM x BN outputs per block, BK values of k at a time through two buffers in shared memory; a thread keeps
-// TM x TN outputs (TM rows apart by one, TN columns in groups of four).  Values of the next tile are loaded to registers
-// while the current one is multiplied, 16 bytes at a time where rows are aligned.
+// A tile of BM x BN outputs per block, BK values of k at a time through two buffers in shared memory.  The block's threads
+// are kGroups groups that each take every output of the tile over their own quarter of every BK values, TM x TN outputs a
+// thread; at the end the groups' sums are added in order.  An output is therefore four chains of FMAs over fixed values of
+// k, added in a fixed order: the same bits whatever M, N and the tile.  Values of the next tile are loaded to registers while
+// the current one is multiplied, 16 bytes at a time where rows are aligned.
 //
 // What bounds it: float32 FMAs (128 a cycle and SM).  8 x 8 outputs a thread read 16 values from shared memory for 64 FMAs,
-// which the two units then spend equally long on; 4 x 4 outputs (the tile this kernel had before) read 8 for 16 and waited
-// for shared memory, and its loads from global memory, one value at a time, stood between two barriers.
-// Tiles are chosen by how many blocks a launch gets: see launch().
+// which the two units then spend equally long on.  A warp alone on its scheduler issues an instruction every four cycles
+// whatever their independence, and a step of a few hundred rows has about as many tiles as there are SMs: hence four groups,
+// two warps per scheduler from one block.
+constexpr int kGroups = 4;
+
 template <typename TA, typename TW, typename TO, int BM, int BN, int TM, int TN, bool VEC>
-__global__ void __launch_bounds__((BM / TM) * (BN / TN))
+__global__ void __launch_bounds__(kGroups * (BM / TM) * (BN / TN), 2)
 gemm_tn_simt_kernel(const TA* A, long long lda, const TW* W, long long ldw, TO* O, long long ldo, int M, int N, int K) {
   // (No __restrict__: a load the compiler takes for one of constant data may be moved above the wait for the kernel before.)
-  constexpr int BK = 16, THREADS = (BM / TM) * (BN / TN), TX = BN / TN;
+  constexpr int BK = 32, KG = BK / kGroups, PER = (BM / TM) * (BN / TN), THREADS = kGroups * PER, TX = BN / TN;
   constexpr int LA = BM + 4, LW = BN + 4;                  // padded rows: the transposed stores spread over the banks
   constexpr int NA = BM * BK / 4 / THREADS, NW = BN * BK / 4 / THREADS;      // groups of four k values a thread loads
   static_assert(NA >= 1 && NW >= 1 && TM % 4 == 0 && TN % 4 == 0, "whole groups");
-  __shared__ __align__(16) float As[2][BK][LA];
-  __shared__ __align__(16) float Ws[2][BK][LW];
+  static_assert(BM * BN <= 2 * BK * (LA + LW), "a group's sums fit the buffers");
+  __shared__ __align__(16) float buffers[2 * BK * (LA + LW)];
+  auto As = [&](int b, int k) { return buffers + (size_t)(b * BK + k) * LA; };
+  auto Ws = [&](int b, int k) { return buffers + 2 * BK * LA + (size_t)(b * BK + k) * LW; };
   pdl_launch_dependents();
   pdl_wait();
-  const int tid = threadIdx.x, tx = tid % TX, ty = tid / TX;
+  const int tid = threadIdx.x, group = tid / PER, tx = tid % PER % TX, ty = tid % PER / TX;
   const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
   float acc[TM][TN];
 #pragma unroll
@@ -53,7 +59,6 @@ gemm_tn_simt_kernel(const TA* A, long long lda, const TW* W, long long ldw, TO* 
     for (int u = 0; u < 4; ++u) v[u] = k + u < K ? to_f32(q[u]) : 0.f;
     return make_float4(v[0], v[1], v[2], v[3]);
   };
-  // a group g of four k values: rows run fastest over threads within a group of k, so that the stores below spread
   auto fetch = [&](int k0) {
 #pragma unroll
     for (int i = 0; i < NA; ++i) {
@@ -70,12 +75,14 @@ gemm_tn_simt_kernel(const TA* A, long long lda, const TW* W, long long ldw, TO* 
 #pragma unroll
     for (int i = 0; i < NA; ++i) {
       const int e = tid + i * THREADS, r = e / (BK / 4), k = (e % (BK / 4)) * 4;
-      As[b][k][r] = ra[i].x; As[b][k + 1][r] = ra[i].y; As[b][k + 2][r] = ra[i].z; As[b][k + 3][r] = ra[i].w;
+      float* to = As(b, k) + r;
+      to[0] = ra[i].x; to[LA] = ra[i].y; to[2 * LA] = ra[i].z; to[3 * LA] = ra[i].w;
     }
 #pragma unroll
     for (int i = 0; i < NW; ++i) {
       const int e = tid + i * THREADS, r = e / (BK / 4), k = (e % (BK / 4)) * 4;
-      Ws[b][k][r] = rw[i].x; Ws[b][k + 1][r] = rw[i].y; Ws[b][k + 2][r] = rw[i].z; Ws[b][k + 3][r] = rw[i].w;
+      float* to = Ws(b, k) + r;
+      to[0] = rw[i].x; to[LW] = rw[i].y; to[2 * LW] = rw[i].z; to[3 * LW] = rw[i].w;
     }
   };
 
@@ -86,17 +93,19 @@ gemm_tn_simt_kernel(const TA* A, long long lda, const TW* W, long long ldw, TO* 
   for (int k0 = 0; k0 < K; k0 += BK, b ^= 1) {
     const bool more = k0 + BK < K;
     if (more) fetch(k0 + BK);
+    const float* ap = As(b, group * KG) + ty * 4;
+    const float* wp = Ws(b, group * KG) + tx * 4;
 #pragma unroll
-    for (int kk = 0; kk < BK; ++kk) {
+    for (int kk = 0; kk < KG; ++kk) {
       float a[TM], w[TN];
 #pragma unroll
       for (int i = 0; i < TM; i += 4) {
-        const float4 v = *reinterpret_cast<const float4*>(&As[b][kk][(i / 4) * (BM * 4 / TM) + ty * 4]);
+        const float4 v = *reinterpret_cast<const float4*>(ap + kk * LA + (i / 4) * (BM * 4 / TM));
         a[i] = v.x; a[i + 1] = v.y; a[i + 2] = v.z; a[i + 3] = v.w;
       }
 #pragma unroll
       for (int j = 0; j < TN; j += 4) {
-        const float4 v = *reinterpret_cast<const float4*>(&Ws[b][kk][(j / 4) * (BN * 4 / TN) + tx * 4]);
+        const float4 v = *reinterpret_cast<const float4*>(wp + kk * LW + (j / 4) * (BN * 4 / TN));
         w[j] = v.x; w[j + 1] = v.y; w[j + 2] = v.z; w[j + 3] = v.w;
       }
 #pragma unroll
@@ -107,6 +116,24 @@ gemm_tn_simt_kernel(const TA* A, long long lda, const TW* W, long long ldw, TO* 
     if (more) put(b ^ 1);             // the buffer that the round before read: everyone passed the barrier behind it
     __syncthreads();
   }
+  // the groups' sums, in order, through the buffers
+  for (int g = 1; g < kGroups; ++g) {
+    if (group == g) {
+#pragma unroll
+      for (int i = 0; i < TM; ++i)
+#pragma unroll
+        for (int j = 0; j < TN; ++j) buffers[(i * TN + j) * PER + tid % PER] = acc[i][j];
+    }
+    __syncthreads();
+    if (group == 0) {
+#pragma unroll
+      for (int i = 0; i < TM; ++i)
+#pragma unroll
+        for (int j = 0; j < TN; ++j) acc[i][j] += buffers[(i * TN + j) * PER + tid % PER];
+    }
+    __syncthreads();
+  }
+  if (group != 0) return;
 #pragma unroll
   for (int i = 0; i < TM; ++i) {
     const int m = m0 + (i / 4) * (BM * 4 / TM) + ty * 4 + i % 4;
@@ -122,7 +149,7 @@ gemm_tn_simt_kernel(const TA* A, long long lda, const TW* W, long long ldw, TO* 
 template <typename TA, typename TW, typename TO, int BM, int BN, int TM, int TN>
 int launch_tile(const void* A, long long lda, const void* W, long long ldw, void* O, long long ldo, int M, int N, int K,
                 cudaStream_t stream) {
-  const dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM), block((BM / TM) * (BN / TN));
+  const dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM), block(kGroups * (BM / TM) * (BN / TN));
   if (grid.y > 65535) return YALIS_ERR_SHAPE;
   const bool vec = K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 && (uintptr_t)A % (4 * sizeof(TA)) == 0 &&
                    (uintptr_t)W % (4 * sizeof(TW)) == 0;
@@ -133,18 +160,18 @@ int launch_tile(const void* A, long long lda, const void* W, long long ldw, void
                       (const TW*)W, ldw, (TO*)O, ldo, M, N, K);
 }
 
-// Which tile: a large one only where it leaves two blocks to an SM (250 rows by 16,384 columns, K = 2,048: 128 x 128 would be
-// 256 blocks).  Measured (us, float32; before, 64 x 64 with 4 x 4 outputs a thread -> now), columns x K:
-//   250 rows   3,072 x 2,048  227 -> 141    2,048 x 2,048  158 -> 100    16,384 x 2,048  699 -> 418    2,048 x 8,192  610 -> 390
-//   1,024 rows 3,072 x 2,048  602 -> 359    2,048 x 2,048  411 -> 248    16,384 x 2,048  2,704 -> 1,918  2,048 x 8,192  1,614 -> 956
-//   8 rows     3,072 x 2,048  159 -> 126    16,384 x 2,048  221 -> 141   2,048 x 8,192  633 -> 497  (32 x 32 tiles: more blocks)
+// Which tile: 32 x 128 with 8 x 8 outputs a thread (a warp's lanes lie 2 x 16, which loads from shared memory in fewer passes
+// than 4 x 8) where that makes a block for every other SM at least, else 32 x 32 with 4 x 4: more blocks.
+// Measured (us, float32; 64 x 64 tiles with 4 x 4 outputs a thread, as it was -> now), columns x K:
+//   250 rows   3,072 x 2,048  227 -> 147    2,048 x 2,048  158 -> 90     16,384 x 2,048  699 -> 494    2,048 x 8,192  610 -> 331
+//   1,024 rows 3,072 x 2,048  602 -> 424    2,048 x 2,048  411 -> 287    16,384 x 2,048  2,704 -> 1,907  2,048 x 8,192  1,614 -> 1,104
+//   8 rows     3,072 x 2,048  159 -> 71     16,384 x 2,048  221 -> 90    2,048 x 8,192  633 -> 262
 template <typename TA, typename TW, typename TO>
 int launch(const void* A, long long lda, const void* W, long long ldw, void* O, long long ldo, int M, int N, int K,
            cudaStream_t stream) {
   const long long sms = yalis_sm_count();
-  auto blocks = [&](int bm, int bn) { return (long long)((N + bn - 1) / bn) * ((M + bm - 1) / bm); };
-  if (M > 64 && blocks(128, 128) >= 2 * sms) return launch_tile<TA, TW, TO, 128, 128, 8, 8>(A, lda, W, ldw, O, ldo, M, N, K, stream);
-  if (M > 32 && blocks(64, 64) >= sms / 2) return launch_tile<TA, TW, TO, 64, 64, 8, 4>(A, lda, W, ldw, O, ldo, M, N, K, stream);
+  const long long blocks = (long long)((N + 127) / 128) * ((M + 31) / 32);
+  if (blocks >= sms / 2) return launch_tile<TA, TW, TO, 32, 128, 8, 8>(A, lda, W, ldw, O, ldo, M, N, K, stream);
   return launch_tile<TA, TW, TO, 32, 32, 4, 4>(A, lda, W, ldw, O, ldo, M, N, K, stream);
 }
 
