@@ -125,7 +125,7 @@ latent_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map, const L
     return;
   }
   // The queries, as bfloat16, into the swizzled K-major layout: 16-byte piece c of row r lies at piece c ^ (r & 7) of its
-  // 128 bytes.  Rows past the last one are zeros.  (The copy warp leaves this to the others and starts on the tiles.)
+  // 128 bytes.  Rows past the last one hold anything: nothing of theirs is stored.  (The copy warp leaves this to the others and starts on the tiles.)
   if (warp != 4) {
     // Loads in batches before their stores: the compiler cannot tell that a store to shared memory leaves the next load
     // alone, and a trip to memory per 16 bytes made this a third of a block's time.
@@ -134,13 +134,13 @@ latent_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map, const L
     auto place = [&](int r, int piece) -> uint4* {
       return reinterpret_cast<uint4*>(q_s + (piece >> 3) * (LM * 128) + r * 128 + (((piece & 7) ^ (r & 7)) << 4));
     };
-    for (int e0 = first; e0 < LM * RP; e0 += 160 * BATCH) {
+    const int lat_end = rows_here * RP;
+    for (int e0 = first; e0 < lat_end; e0 += 160 * BATCH) {
       uint4 v[BATCH];
 #pragma unroll
       for (int i = 0; i < BATCH; ++i) {
         const int e = e0 + i * 160, r = e / RP;
-        v[i] = make_uint4(0u, 0u, 0u, 0u);
-        if (e < LM * RP && r < rows_here) {
+        if (e < lat_end) {
           const int t = (row0 + r) / a.heads, h = row0 + r - t * a.heads;
           v[i] = *reinterpret_cast<const uint4*>(a.q_lat + (size_t)(q0 + t) * a.ql_n + (size_t)h * a.ql_h + (e - r * RP) * 8);
         }
@@ -148,17 +148,16 @@ latent_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map, const L
 #pragma unroll
       for (int i = 0; i < BATCH; ++i) {
         const int e = e0 + i * 160, r = e / RP;
-        if (e < LM * RP) *place(r, e - r * RP) = v[i];
+        if (e < lat_end) *place(r, e - r * RP) = v[i];
       }
     }
-    const int pp = a.p / 8;
-    for (int e0 = first; e0 < LM * pp; e0 += 160 * (BATCH / 2)) {
+    const int pp = a.p / 8, rot_end = rows_here * pp;
+    for (int e0 = first; e0 < rot_end; e0 += 160 * (BATCH / 2)) {
       float4 x[BATCH / 2], y[BATCH / 2];
 #pragma unroll
       for (int i = 0; i < BATCH / 2; ++i) {
         const int e = e0 + i * 160, r = e / pp;
-        x[i] = y[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (e < LM * pp && r < rows_here) {
+        if (e < rot_end) {
           const int t = (row0 + r) / a.heads, h = row0 + r - t * a.heads;
           const float* src = a.q_rot + (size_t)(q0 + t) * a.qr_n + (size_t)h * a.qr_h + (e - r * pp) * 8;
           x[i] = load4_f32(src);
@@ -168,7 +167,7 @@ latent_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map, const L
 #pragma unroll
       for (int i = 0; i < BATCH / 2; ++i) {
         const int e = e0 + i * 160, r = e / pp;
-        if (e < LM * pp)
+        if (e < rot_end)
           *place(r, RP + e - r * pp) = make_uint4(pack_bf16(x[i].x, x[i].y), pack_bf16(x[i].z, x[i].w), pack_bf16(y[i].x, y[i].y),
                                                   pack_bf16(y[i].z, y[i].w));
       }

@@ -168,7 +168,7 @@ def latent_attention_mma(q_lat: torch.Tensor, q_rot: torch.Tensor, out: torch.Te
     part_o = part_ml = None
     if n_splits > 1:
         part_o = torch.empty((n_splits, n * h, r), dtype=torch.float32, device=q_lat.device)
-        part_ml = torch.full((n_splits, n * h, 2), float("-inf"), dtype=torch.float32, device=q_lat.device)
+        part_ml = torch.empty((n_splits, n * h, 2), dtype=torch.float32, device=q_lat.device)   # every share of a request's rows is written
     check(lib().yalis_latent_attention_mma(
         ptr(q_lat), i32(q_lat.dtype == torch.bfloat16), i64(q_lat.stride(0)), i64(q_lat.stride(1)), ptr(q_rot),
         i64(q_rot.stride(0)), i64(q_rot.stride(1)), ptr(out), i32(out.dtype == torch.bfloat16), i64(out.stride(0)),
