@@ -1,5 +1,5 @@
-"""The general form of the tcgen05 prompt attention at the edges of its tiles (128 query rows, 64 keys) against plain
-attention in float64, option by option."""
+"""The general forms of the tcgen05 prompt attention (tiles of 128 query rows and 64 keys) and of the decode attention that
+deals tiles of 64 keys to a fixed grid, at the edges of their tiles, against plain attention in float64, option by option."""
 
 import pytest
 import torch
@@ -42,10 +42,23 @@ CASES = [
 ]
 
 
-@pytest.mark.parametrize("d,heads,kv,page,new,before,options", CASES)
+# steps of single tokens
+DECODE = [
+    (128, 16, 8, 64, [0, 63, 64, 130, 2000], dict(window=100)),
+    (128, 6, 2, 16, [21, 64, 300], dict(window=1, sink="learned")),
+    (64, 4, 4, 8, [64, 250, 1], dict(chunk=70, gate="element")),
+    (64, 16, 1, 32, [300, 7], dict(chunk=64, sink="learned", gate="element", out_scale=0.7)),
+    (192, 8, 4, 64, [63, 200], dict(softcap=5.0, sink="one")),
+    (256, 3, 3, 64, [57, 900, 3], dict(slopes=True, window=90, gate="head")),
+    (128, 8, 2, 16, [100, 500] * 40, dict(slopes=True, softcap=3.0)),
+    (128, 2, 2, 64, [4000], dict()),
+]
+
+
+@pytest.mark.parametrize("d,heads,kv,page,new,before,options", CASES + [(a, b, c, p, [1] * len(n), n, o) for a, b, c, p, n, o in DECODE])
 def test_against_plain_attention(d, heads, kv, page, new, before, options):
     from yalis_b200.ops._lib import error_word
-    from yalis_b200.ops.attention import prefill_attention_general
+    from yalis_b200.ops.attention import decode_attention_general, prefill_attention_general
     g = torch.Generator().manual_seed(d + heads + page)
     window, chunk, scale = options.get("window"), options.get("chunk"), 0.9 / d ** 0.5
     sink = {"learned": torch.randn(heads, generator=g) * 2, "one": torch.zeros(heads)}.get(options.get("sink"))
@@ -80,12 +93,15 @@ def test_against_plain_attention(d, heads, kv, page, new, before, options):
     gate = None
     if options.get("gate"):
         gate = torch.randn(total, heads * d if options["gate"] == "element" else heads, generator=g).to(torch.bfloat16)
-    prefill_attention_general(torch.cat(queries).flatten(1).contiguous().to(DEV), pools[0].to(DEV), pools[1].to(DEV), ints(pos),
-                              ints(starts), table.to(DEV), max(new), heads, kv, d, scale, out, window=window, chunk=chunk,
-                              softcap=options.get("softcap"), sink=sink is not None,
-                              sink_logits=sink.to(DEV) if options.get("sink") == "learned" else None,
-                              slopes=None if slopes is None else slopes.to(DEV), gate=None if gate is None else gate.to(DEV),
-                              out_scale=options.get("out_scale", 1.0))
+    args = [torch.cat(queries).flatten(1).contiguous().to(DEV), pools[0].to(DEV), pools[1].to(DEV), ints(pos), ints(starts), table.to(DEV),
+            max(new), heads, kv, d, scale, out]
+    call = prefill_attention_general
+    if max(new) == 1:
+        call = decode_attention_general
+        del args[6]
+    call(*args, window=window, chunk=chunk, softcap=options.get("softcap"), sink=sink is not None,
+         sink_logits=sink.to(DEV) if options.get("sink") == "learned" else None, slopes=None if slopes is None else slopes.to(DEV),
+         gate=None if gate is None else gate.to(DEV), out_scale=options.get("out_scale", 1.0))
     assert int(error_word(DEV)) == 0
     want = torch.cat(want) * options.get("out_scale", 1.0)
     if gate is not None:

@@ -52,7 +52,48 @@ struct LeanParams {
   float* part_ml;              // [blocks, 2, 16, 2]
   int32_t* tickets;            // [R * g], zero before and after
   int32_t* error;
+  // the general form (see attention_mma.cu, whose arithmetic of scores, sinks and gates this is)
+  int window, chunk;           // 0: none
+  float cap_log2, scale_over_cap, out_scale;
+  int sink;                    // 1: a score without key and value in every denominator
+  const float* sink_logits;    // [nh] (null: 0)
+  const float* slopes;         // [nh] or null
+  const __nv_bfloat16* gate;   // [N, gate_stride] or null
+  int gate_stride, gate_per_head;
 };
+
+// The first key that the query at position `pos` sees.
+__device__ __forceinline__ int first_visible(const LeanParams& p, int pos) {
+  int lo = p.window > 0 ? max(0, pos - p.window + 1) : 0;
+  if (p.chunk > 0) lo = max(lo, pos / p.chunk * p.chunk);
+  return lo;
+}
+
+// Four finished values of a head: divided by the sum of weights (general form: the sink's share with it), times factor and
+// gate, rounded and stored.
+template <int HS, bool GEN>
+__device__ __forceinline__ void finish(const LeanParams& p, int tok, int head, int d, float4 acc, float m, float l) {
+  float inv = l > 0.f ? 1.0f / l : 0.f;
+  if constexpr (GEN) {
+    if (p.sink) {                                 // the sums stand relative to m: the sink joins there
+      const float z = p.sink_logits ? p.sink_logits[head] * 1.4426950408889634f : 0.f, mf = fmaxf(m, z);
+      const float c = exp2f(m - mf);
+      inv = c / (l * c + exp2f(z - mf));
+    }
+    inv *= p.out_scale;
+    if (p.gate != nullptr) {
+      const __nv_bfloat16* g = p.gate + (size_t)tok * p.gate_stride;
+      if (p.gate_per_head) {
+        inv *= 1.0f / (1.0f + __expf(-__bfloat162float(g[head])));
+      } else {
+        const float4 z = load4_f32(g + (size_t)head * HS + d);
+        acc.x *= 1.0f / (1.0f + __expf(-z.x)); acc.y *= 1.0f / (1.0f + __expf(-z.y));
+        acc.z *= 1.0f / (1.0f + __expf(-z.z)); acc.w *= 1.0f / (1.0f + __expf(-z.w));
+      }
+    }
+  }
+  store_bf16x4(p.out + (size_t)tok * p.out_stride + (size_t)head * HS + d, acc, inv);
+}
 
 // First tile of block b when `total` tiles are dealt to `blocks` blocks.
 __device__ __forceinline__ long long first_tile_of(int b, long long total, int blocks) { return (long long)b * total / blocks; }
@@ -103,7 +144,13 @@ struct Walker {
 
 // Registers: two blocks of five warps share an SM only up to 168 a thread (the register file is dealt out
 // to warps in groups), which head sizes up to 128 keep to; larger ones run one block per SM.
-template <int HS, int NST>
+// GEN: the general form.  A request's tiles start at the first key its query sees (window, chunk), scores may be capped or
+// fall off with the distance, a sink joins the denominator, a gate and a factor multiply the result, and the weights meet V as
+// two bfloat16 halves (16 bits of mantissa).  Rows of V that no query sees or that have no page arrive as zeros.
+// Measured (layers of 16 heads of 128 over 8 KV heads, this kernel / the mma.sync kernel with its key splits, us, L2 flushed, launches
+// included): 1 request of 30 tokens 33 / 43, 1 of 1,900 41 / 45, 8 of 1,000 47 / 47, 32 of 1,000 72 / 78 (window 1,024);
+// 64 of 1,900 131 / 180 (chunk 2,048).  It is no slower anywhere in that range, so it takes every step of single tokens.
+template <int HS, int NST, bool GEN>
 __global__ void __maxnreg__(HS <= 128 ? 168 : 255)
 decode_attention_lean_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
                              const LeanParams p) {
@@ -149,7 +196,9 @@ decode_attention_lean_kernel(const __grid_constant__ CUtensorMap map_k, const __
   for (int r = threadIdx.x; r < p.n_requests; r += kThreads) {
     const int tok = p.q_start[r];
     const int n_tok = p.q_start[r + 1] - tok;
-    cum[r + 1] = (p.only_single ? n_tok == 1 : n_tok > 0) ? p.positions[tok] / BN + 1 : 0;
+    const bool counts = p.only_single ? n_tok == 1 : n_tok > 0;
+    const int pos = counts ? p.positions[tok] : 0;
+    cum[r + 1] = counts ? pos / BN + 1 - (GEN ? first_visible(p, pos) / BN : 0) : 0;
   }
   if (threadIdx.x == 0) cum[0] = 0;
   __syncthreads();
@@ -185,6 +234,7 @@ decode_attention_lean_kernel(const __grid_constant__ CUtensorMap map_k, const __
     bool waited = !p.early_fetch;              // whether this warp has waited for the preceding kernel
     while (alive && w.next(&sg)) {
       const int hi_key = p.positions[p.q_start[sg.req]];
+      const int lo_key = GEN ? first_visible(p, hi_key) : 0, tile0 = GEN ? lo_key / BN : 0;
       const int32_t* bt = p.block_table + (size_t)sg.req * p.table_width;
       for (int tile = sg.tile_lo; tile < sg.tile_hi; ++tile) {
         if (!waited && (tile == sg.tiles - 1 || armed >= NST)) {
@@ -194,7 +244,7 @@ decode_attention_lean_kernel(const __grid_constant__ CUtensorMap map_k, const __
         }
         const int s = armed % NST;
         const uint32_t ph = (armed / NST) & 1;
-        const int key0 = tile * BN;
+        const int key0 = (tile0 + tile) * BN;
         const int n_pages = min(pages_per_tile, (hi_key - key0) / p.page_size + 1);
         int ok = 1;
         if (lane == 0) {
@@ -207,11 +257,17 @@ decode_attention_lean_kernel(const __grid_constant__ CUtensorMap map_k, const __
           const int i = c / (2 * H2), kv = (c / H2) & 1, h = c % H2;
           const int pi = key0 / p.page_size + i;
           int page = pi < p.table_width ? bt[pi] : -1;
-          if (page < 0 || page >= p.num_pages) {   // a visible key without a page: a caller's bug
-            if (p.error) atomicOr(p.error, YALIS_FLAG_BAD_PAGE);
-            page = 0;
+          int y;
+          if constexpr (GEN) {
+            const bool none = page < 0 || page >= p.num_pages || key0 + (i + 1) * p.page_size <= lo_key;
+            y = (none ? p.num_pages * p.g : page * p.g + sg.kvh) * p.page_size;      // past the pool: zeros
+          } else {
+            if (page < 0 || page >= p.num_pages) { // a visible key without a page: a caller's bug
+              if (p.error) atomicOr(p.error, YALIS_FLAG_BAD_PAGE);
+              page = 0;
+            }
+            y = (page * p.g + sg.kvh) * p.page_size;
           }
-          const int y = (page * p.g + sg.kvh) * p.page_size;
           const int off = h * (BN * 128) + i * p.page_size * 128;
           tma_load_2d((kv ? v_s : k_s) + s * TILE_BYTES + off, kv ? &map_v : &map_k, h * 64, y, &full[s]);
         }
@@ -253,6 +309,7 @@ decode_attention_lean_kernel(const __grid_constant__ CUtensorMap map_k, const __
       sg = nx;
       const int tok = tok_next;
       const int hi_key = hi_next;
+      const int lo_key = GEN ? first_visible(p, hi_key) : 0, tile0 = GEN ? lo_key / BN : 0;
       consumer_sync();                         // the previous segment's merge has been read, its queries are in registers
 #pragma unroll
       for (int j = 0; j < QLOADS; ++j) {
@@ -274,6 +331,12 @@ decode_attention_lean_kernel(const __grid_constant__ CUtensorMap map_k, const __
 #pragma unroll
       for (int d = 0; d < DT; ++d) o[d][0] = o[d][1] = o[d][2] = o[d][3] = 0.f;
       float m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.f, 0.f};
+      float slope[2] = {0.f, 0.f};               // in the exp2 domain
+      if (GEN && p.slopes) {
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+          if (row_ok[i]) slope[i] = p.slopes[sg.kvh * p.per + gid + i * 8] * 1.4426950408889634f;
+      }
 
       for (int tile = sg.tile_lo; tile < sg.tile_hi; ++tile, ++armed) {
         const int s = armed % NST;
@@ -282,7 +345,7 @@ decode_attention_lean_kernel(const __grid_constant__ CUtensorMap map_k, const __
         if (lane == 0) ok = mbar_wait(&full[s], ph, abort_flag) ? 1 : 0;
         ok = __shfl_sync(0xffffffffu, ok, 0);
         if (!ok) break;                        // timed out: the block stops after this segment
-        const int key0 = tile * BN;
+        const int key0 = (tile0 + tile) * BN;
         const uint32_t kt = smem_u32(k_s + s * TILE_BYTES), vt = smem_u32(v_s + s * TILE_BYTES);
         const bool last = key0 + BN - 1 > hi_key;
         if (last) {
@@ -314,7 +377,19 @@ decode_attention_lean_kernel(const __grid_constant__ CUtensorMap map_k, const __
           for (int e = 0; e < 4; ++e) {
             const int i = e >> 1;
             const int key = key0 + wkey + j * 8 + tig * 2 + (e & 1);
-            const float v = (row_ok[i] && (!last || key <= hi_key)) ? sc[j][e] * p.scale_log2 : -INFINITY;
+            float v;
+            if constexpr (GEN) {
+              const float off = slope[i] * (float)(hi_key - key);
+              if (p.cap_log2 > 0.f) {              // c tanh(x / c), saturated where exp would overflow
+                const float x = fminf(sc[j][e] * p.scale_over_cap - off / p.cap_log2, 15.f);
+                v = p.cap_log2 * (1.0f - __fdividef(2.0f, __expf(2.0f * x) + 1.0f));
+              } else {
+                v = sc[j][e] * p.scale_log2 - off;
+              }
+              if (!row_ok[i] || (last && key > hi_key) || key < lo_key) v = -INFINITY;
+            } else {
+              v = (row_ok[i] && (!last || key <= hi_key)) ? sc[j][e] * p.scale_log2 : -INFINITY;
+            }
             sc[j][e] = v;
             m_new[i] = fmaxf(m_new[i], v);
           }
@@ -331,7 +406,7 @@ decode_attention_lean_kernel(const __grid_constant__ CUtensorMap map_k, const __
           corr[i] = exp2f(m_run[i] - bs[i]);
           m_run[i] = m_new[i];
         }
-        unsigned pf[4];
+        unsigned pf[4], pl[GEN ? 4 : 1];
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
           const float p0 = exp2f(sc[j][0] - bs[0]), p1 = exp2f(sc[j][1] - bs[0]);
@@ -340,6 +415,11 @@ decode_attention_lean_kernel(const __grid_constant__ CUtensorMap map_k, const __
           l_add[1] += p2 + p3;
           pf[j * 2 + 0] = pack_bf16(p0, p1);
           pf[j * 2 + 1] = pack_bf16(p2, p3);
+          if constexpr (GEN) {
+            const unsigned a = pf[j * 2], c = pf[j * 2 + 1];
+            pl[j * 2 + 0] = pack_bf16(p0 - __uint_as_float(a << 16), p1 - __uint_as_float(a & 0xffff0000u));
+            pl[j * 2 + 1] = pack_bf16(p2 - __uint_as_float(c << 16), p3 - __uint_as_float(c & 0xffff0000u));
+          }
         }
 #pragma unroll
         for (int i = 0; i < 2; ++i) l_run[i] = l_run[i] * corr[i] + l_add[i];
@@ -357,6 +437,10 @@ decode_attention_lean_kernel(const __grid_constant__ CUtensorMap map_k, const __
           ldmatrix_x4_trans(vb, vt + tile_off(key, dim));
           mma_bf16(o[d], pf, vb[0], vb[1]);
           mma_bf16(o[d + 1], pf, vb[2], vb[3]);
+          if constexpr (GEN) {
+            mma_bf16(o[d], pl, vb[0], vb[1]);
+            mma_bf16(o[d + 1], pl, vb[2], vb[3]);
+          }
         }
         __syncwarp();
         if (lane == 0) mbar_arrive(&empty[s]);
@@ -404,7 +488,7 @@ decode_attention_lean_kernel(const __grid_constant__ CUtensorMap map_k, const __
           acc.x += v.x * f; acc.y += v.y * f; acc.z += v.z * f; acc.w += v.w * f;
         }
         if (whole) {
-          store_bf16x4(p.out + (size_t)tok * p.out_stride + (size_t)(sg.kvh * p.per + r) * HS + d, acc, ll > 0.f ? 1.0f / ll : 0.f);
+          finish<HS, GEN>(p, tok, sg.kvh * p.per + r, d, acc, mm, ll);
         } else {
           *reinterpret_cast<float4*>(p.part_o + ((size_t)slot * 16 + r) * HS + d) = acc;
           if (d == 0) *reinterpret_cast<float2*>(p.part_ml + ((size_t)slot * 16 + r) * 2) = make_float2(mm, ll);
@@ -456,7 +540,7 @@ decode_attention_lean_kernel(const __grid_constant__ CUtensorMap map_k, const __
                 acc.x += v[j].x * f; acc.y += v[j].y * f; acc.z += v[j].z * f; acc.w += v[j].w * f;
               }
             }
-            store_bf16x4(p.out + (size_t)tok * p.out_stride + (size_t)(sg.kvh * p.per + r) * HS + d, acc, ll > 0.f ? 1.0f / ll : 0.f);
+            finish<HS, GEN>(p, tok, sg.kvh * p.per + r, d, acc, mm, ll);
           }
           if (threadIdx.x == 0) p.tickets[pair] = 0;
         }
@@ -483,28 +567,48 @@ size_t lean_smem_bytes(int hs, int stages, int per, int n_requests) {
          2 * stages * 8 + 16 + (size_t)(n_requests + 1) * 4 + 16;
 }
 
-template <int HS, int NST>
+template <int HS, int NST, bool GEN>
 int launch_lean_stages(const CUtensorMap& mk, const CUtensorMap& mv, const LeanParams& p, int n_blocks, cudaStream_t stream) {
   const size_t smem = lean_smem_bytes(HS, NST, p.per, p.n_requests);
   static size_t configured = 0;
   if (smem > configured) {
-    if (cudaFuncSetAttribute(decode_attention_lean_kernel<HS, NST>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
+    if (cudaFuncSetAttribute(decode_attention_lean_kernel<HS, NST, GEN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
         cudaSuccess)
       return YALIS_ERR_LAUNCH;
     configured = smem;
   }
-  return yalis_launch(decode_attention_lean_kernel<HS, NST>, dim3(n_blocks), dim3(kThreads), smem, stream, mk, mv, p);
+  return yalis_launch(decode_attention_lean_kernel<HS, NST, GEN>, dim3(n_blocks), dim3(kThreads), smem, stream, mk, mv, p);
 }
 
 // Three ring stages where two blocks of them still share an SM (or one block holds them at all), else two.
-template <int HS>
+template <int HS, bool GEN>
 int launch_lean(const CUtensorMap& mk, const CUtensorMap& mv, const LeanParams& p, int n_blocks, cudaStream_t stream) {
   const size_t three = lean_smem_bytes(HS, 3, p.per, p.n_requests), two = lean_smem_bytes(HS, 2, p.per, p.n_requests);
   const size_t half_sm = 113 * 1024, whole_sm = 226 * 1024;
   const bool use_three = three <= half_sm || (two > half_sm && three <= whole_sm);
-  if (use_three) return launch_lean_stages<HS, 3>(mk, mv, p, n_blocks, stream);
+  if (use_three) return launch_lean_stages<HS, 3, GEN>(mk, mv, p, n_blocks, stream);
   if (two > whole_sm) return YALIS_ERR_SHAPE;
-  return launch_lean_stages<HS, 2>(mk, mv, p, n_blocks, stream);
+  return launch_lean_stages<HS, 2, GEN>(mk, mv, p, n_blocks, stream);
+}
+
+template <bool GEN>
+int launch_lean_any(const LeanParams& p, const void* k_pool, const void* v_pool, int hs, int n_blocks, cudaStream_t stream) {
+  CUtensorMap mk, mv;
+  const long long rows = (long long)p.num_pages * p.g * p.page_size;
+  if (!make_pool_map(&mk, k_pool, rows, hs, p.page_size) || !make_pool_map(&mv, v_pool, rows, hs, p.page_size))
+    return YALIS_ERR_LAUNCH;
+  switch (hs) {
+    case 64: return launch_lean<64, GEN>(mk, mv, p, n_blocks, stream);
+    case 128: return launch_lean<128, GEN>(mk, mv, p, n_blocks, stream);
+    case 192: return launch_lean<192, GEN>(mk, mv, p, n_blocks, stream);
+    default: return launch_lean<256, GEN>(mk, mv, p, n_blocks, stream);
+  }
+}
+
+bool lean_sizes_ok(int g, int nh, int hs, int page_size, int n_blocks, int n_requests) {
+  const bool hs_ok = hs == 64 || hs == 128 || hs == 192 || hs == 256;
+  const bool page_ok = page_size == 8 || page_size == 16 || page_size == 32 || page_size == 64;
+  return g > 0 && nh % g == 0 && n_blocks >= 1 && n_requests <= kMaxRequests && hs_ok && page_ok && nh / g <= 16;
 }
 
 }  // namespace
@@ -528,18 +632,11 @@ YALIS_API int yalis_decode_attention_lean(const void* q, int q_stride, void* out
                                           int n_tokens, int n_requests, int nh, int g, int hs, float scale, int n_blocks,
                                           int early_fetch, int only_single, float* scratch, int32_t* tickets, int32_t* error, cudaStream_t stream) {
   if (n_tokens <= 0 || n_requests <= 0) return YALIS_OK;
-  if (g <= 0 || nh % g != 0 || n_blocks < 1 || n_requests > kMaxRequests) return YALIS_ERR_SHAPE;
-  const bool hs_ok = hs == 64 || hs == 128 || hs == 192 || hs == 256;
-  const bool page_ok = page_size == 8 || page_size == 16 || page_size == 32 || page_size == 64;
-  if (!hs_ok || !page_ok || nh / g > 16) return YALIS_ERR_SHAPE;
+  if (!lean_sizes_ok(g, nh, hs, page_size, n_blocks, n_requests)) return YALIS_ERR_SHAPE;
   if (scratch == nullptr || tickets == nullptr) return YALIS_ERR_SHAPE;
   if (((uintptr_t)q | (uintptr_t)k_pool | (uintptr_t)v_pool | (uintptr_t)out | (uintptr_t)scratch) & 15) return YALIS_ERR_ALIGN;
   if ((q_stride % 8) || (out_stride % 4)) return YALIS_ERR_ALIGN;
-  CUtensorMap mk, mv;
-  const long long rows = (long long)num_pages * g * page_size;
-  if (!make_pool_map(&mk, k_pool, rows, hs, page_size) || !make_pool_map(&mv, v_pool, rows, hs, page_size))
-    return YALIS_ERR_LAUNCH;
-  LeanParams p;
+  LeanParams p = {};
   p.q = (const __nv_bfloat16*)q; p.q_stride = q_stride;
   p.out = (__nv_bfloat16*)out; p.out_stride = out_stride;
   p.positions = positions; p.q_start = q_start; p.block_table = block_table;
@@ -552,10 +649,39 @@ YALIS_API int yalis_decode_attention_lean(const void* q, int q_stride, void* out
   p.part_ml = scratch + (size_t)n_blocks * 2 * 16 * hs;
   p.tickets = tickets;
   p.error = error;
-  switch (hs) {
-    case 64: return launch_lean<64>(mk, mv, p, n_blocks, stream);
-    case 128: return launch_lean<128>(mk, mv, p, n_blocks, stream);
-    case 192: return launch_lean<192>(mk, mv, p, n_blocks, stream);
-    default: return launch_lean<256>(mk, mv, p, n_blocks, stream);
-  }
+  return launch_lean_any<false>(p, k_pool, v_pool, hs, n_blocks, stream);
+}
+
+// The general form: `out` may be a column block of a wider matrix (rows on the boundaries of four values); window / chunk 0:
+// none; softcap 0: none; sink 1 with sink_logits [nh] (or null: 0); slopes [nh] or null; gate [N, gate_stride] bfloat16 (per
+// element: on the boundaries of four values) or null.  One query token per request.
+YALIS_API int yalis_decode_attention_lean_general(
+    const void* q, int q_stride, void* out, int out_stride, const void* k_pool, const void* v_pool, const int32_t* positions,
+    const int32_t* q_start, const int32_t* block_table, int table_width, int page_size, int num_pages, int n_tokens,
+    int n_requests, int nh, int g, int hs, float scale, int window, int chunk, float softcap, int sink, const float* sink_logits,
+    const float* slopes, const void* gate, int gate_stride, int gate_per_head, float out_scale, int n_blocks, float* scratch,
+    int32_t* tickets, int32_t* error, cudaStream_t stream) {
+  if (n_tokens <= 0 || n_requests <= 0) return YALIS_OK;
+  if (!lean_sizes_ok(g, nh, hs, page_size, n_blocks, n_requests) || softcap < 0.f || !(scale > 0.f)) return YALIS_ERR_SHAPE;
+  if (scratch == nullptr || tickets == nullptr) return YALIS_ERR_SHAPE;
+  if (((uintptr_t)q | (uintptr_t)k_pool | (uintptr_t)v_pool | (uintptr_t)scratch) & 15) return YALIS_ERR_ALIGN;
+  if ((q_stride % 8) || (out_stride % 4) || ((uintptr_t)out & 7)) return YALIS_ERR_ALIGN;
+  if (gate && !gate_per_head && ((gate_stride % 4) || ((uintptr_t)gate & 7))) return YALIS_ERR_ALIGN;
+  LeanParams p = {};
+  p.q = (const __nv_bfloat16*)q; p.q_stride = q_stride;
+  p.out = (__nv_bfloat16*)out; p.out_stride = out_stride;
+  p.positions = positions; p.q_start = q_start; p.block_table = block_table;
+  p.table_width = table_width; p.page_size = page_size; p.num_pages = num_pages;
+  p.n_requests = n_requests; p.nh = nh; p.g = g; p.per = nh / g;
+  p.scale_log2 = scale * 1.4426950408889634f;
+  p.part_o = scratch;
+  p.part_ml = scratch + (size_t)n_blocks * 2 * 16 * hs;
+  p.tickets = tickets;
+  p.error = error;
+  p.window = window; p.chunk = chunk;
+  p.cap_log2 = softcap * 1.4426950408889634f; p.scale_over_cap = softcap > 0.f ? scale / softcap : 0.f;
+  p.out_scale = out_scale;
+  p.sink = sink; p.sink_logits = sink ? sink_logits : nullptr; p.slopes = slopes;
+  p.gate = (const __nv_bfloat16*)gate; p.gate_stride = gate_stride; p.gate_per_head = gate_per_head;
+  return launch_lean_any<true>(p, k_pool, v_pool, hs, n_blocks, stream);
 }

@@ -607,6 +607,50 @@ def prefill_attention_general(q: torch.Tensor, k_pool: torch.Tensor, v_pool: tor
     return out
 
 
+def decode_general_applies(q: torch.Tensor, out: torch.Tensor, gate: Optional[torch.Tensor], n_requests: int, page_size: int,
+                           num_heads: int, num_kv_heads: int, head_dim: int, v_head_dim: int, scale: float) -> bool:
+    """Whether ``decode_attention_general`` takes a step of single tokens: its head and page sizes, and rows on the boundaries
+    that its loads and stores need."""
+    return (USE_DECODE_LEAN and q.dtype == torch.bfloat16 and v_head_dim == head_dim and scale > 0 and n_requests <= 4096
+            and decode_tma_supports(head_dim, page_size, num_heads // num_kv_heads) and q.data_ptr() % 16 == 0 and q.stride(0) % 8 == 0
+            and out.data_ptr() % 8 == 0 and out.stride(0) % 4 == 0
+            and (gate is None or gate.shape[1] == num_heads or (gate.data_ptr() % 8 == 0 and gate.stride(0) % 4 == 0)))
+
+
+def decode_attention_general(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, positions: torch.Tensor,
+                             q_start: torch.Tensor, block_table: torch.Tensor, num_heads: int, num_kv_heads: int, head_dim: int,
+                             scale: float, out: torch.Tensor, window: Optional[int] = None, chunk: Optional[int] = None,
+                             softcap: Optional[float] = None, sink: bool = False, sink_logits: Optional[torch.Tensor] = None,
+                             slopes: Optional[torch.Tensor] = None, gate: Optional[torch.Tensor] = None, out_scale: float = 1.0,
+                             error_flag: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """``paged_attention_mma`` with ``exact_weights`` for steps of one token per request, by the kernel that deals the key tiles
+    of all requests evenly to a fixed grid (``decode_attention_lean``): the same arguments.  ``out`` may be a column block of a
+    wider matrix (see ``decode_general_applies``)."""
+    name = "decode_attention_general"
+    LAUNCHED["decode_lean"] += 1
+    n, r = q.shape[0], q_start.numel() - 1
+    _check_common(name, q, k_pool, v_pool, positions, positions, block_table, num_heads, num_kv_heads, head_dim)
+    need(q_start.dtype == torch.int32 and q_start.is_contiguous() and q_start.is_cuda, name, "q_start must be int32 [R+1]")
+    need(block_table.shape[0] >= r, name, "block_table has fewer rows than requests")
+    need(out.shape == (n, num_heads * head_dim) and out.dtype == q.dtype and out.stride(1) == 1, name, "bad out tensor")
+    need(softcap is None or softcap > 0, name, "the soft cap must be positive")
+    _check_extras(name, q, num_heads, head_dim, chunk, sink, sink_logits, slopes, gate, None)
+    need(decode_general_applies(q, out, gate, r, k_pool.shape[2], num_heads, num_kv_heads, head_dim, head_dim, scale), name,
+         "head_dim 64/128/192/256, page_size 8..64, at most 16 heads per KV head, at most 4096 requests, aligned rows")
+    blocks = decode_lean_blocks(head_dim)
+    floats = lib().yalis_decode_attention_lean_scratch_floats
+    floats.restype = ctypes.c_longlong
+    scratch = torch.empty(int(floats(i32(blocks), i32(head_dim))), dtype=torch.float32, device=q.device)
+    check(lib().yalis_decode_attention_lean_general(
+        ptr(q), i32(q.stride(0)), ptr(out), i32(out.stride(0)), ptr(k_pool), ptr(v_pool), ptr(positions), ptr(q_start),
+        ptr(block_table), i32(block_table.shape[1]), i32(k_pool.shape[2]), i32(k_pool.shape[0]), i32(n), i32(r),
+        i32(num_heads), i32(num_kv_heads), i32(head_dim), f32(scale), i32(window or 0), i32(chunk or 0), f32(softcap or 0.0),
+        i32(int(sink)), ptr(sink_logits), ptr(slopes), ptr(gate), i32(gate.stride(0) if gate is not None else 0),
+        i32(_per_head(gate, num_heads, head_dim)), f32(out_scale), i32(blocks), ptr(scratch),
+        ptr(_tickets(q.device, r * num_kv_heads)), ptr(error_flag), stream()), name)
+    return out
+
+
 PREFILL_SPLIT_MIN_TILES = 16     # a share of a divided tile of queries is at least this many key tiles long
 PREFILL_SPLIT_START_UP = 20.0    # what one more block costs (fill and drain, its share's outputs), in key tiles
 PREFILL_SPLIT_UNSHARED = 1.4     # pace of a block whose keys no other block reads at the time (they come from HBM)

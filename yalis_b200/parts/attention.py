@@ -397,6 +397,14 @@ class GeneralAttention(Mixer, Projected):
                                                    softcap=self.softcap, sink=self.sink, sink_logits=self.sink_logits,
                                                    slopes=self.slopes, gate=gate, out_scale=scale_out, error_flag=ctx.error_flag)
                 return
+            if (longest == 1 and self.difference is None and self.rel is None and blocks is None
+                    and attn_ops.decode_general_applies(q, y, gate, ctx.n_requests, cache.k.shape[2], self.nh, self.g, self.hs, self.vd,
+                                                        self.scale)):
+                attn_ops.decode_attention_general(q, cache.k, cache.v, ctx.positions, ctx.q_start, table, self.nh, self.g, self.hs,
+                                                  self.scale, y, window=self.window, chunk=self.chunk, softcap=self.softcap,
+                                                  sink=self.sink, sink_logits=self.sink_logits, slopes=self.slopes, gate=gate,
+                                                  out_scale=scale_out, error_flag=ctx.error_flag)
+                return
             direct = y.data_ptr() % 16 == 0 and y.stride(0) % 2 == 0
             out = attn_ops.paged_attention_mma(q, cache.k, cache.v, ctx.positions, ctx.q_start, ctx.req_of_token, table, longest,
                                                self.nh, self.g, self.hs, scale=self.scale, window=self.window, n_splits=splits,
