@@ -310,33 +310,8 @@ __global__ void __launch_bounds__(512) route_kernel(const T* __restrict__ x, lon
   const bool vec = (K & 3) == 0 && ((uintptr_t)w & 15) == 0 && ((uintptr_t)side & 15) == 0;
   // `side` [K]: one more row beside the router's, whose sigmoid goes to side_out[n] (a gate per token that reads
   // the same rows; same order of sums as an expert's logit)
-  for (int e = warp; e < E + (side ? 1 : 0); e += warps) {
-    const float* wr = e < E ? w + (size_t)e * K : side;
-    float acc[TOK];
-#pragma unroll
-    for (int t = 0; t < TOK; ++t) acc[t] = 0.f;
-    if (vec) {
-#pragma unroll (TOK == 1 ? 8 : 2)
-      for (int k = 4 * lane; k < K; k += 128) {
-        const float4 wv = *reinterpret_cast<const float4*>(wr + k);
-#pragma unroll
-        for (int t = 0; t < TOK; ++t) {
-          float x0, x1, x2, x3;
-          load4(xs + (size_t)t * K + k, x0, x1, x2, x3);
-          acc[t] = __fmaf_rn(wv.x, x0, acc[t]);
-          acc[t] = __fmaf_rn(wv.y, x1, acc[t]);
-          acc[t] = __fmaf_rn(wv.z, x2, acc[t]);
-          acc[t] = __fmaf_rn(wv.w, x3, acc[t]);
-        }
-      }
-    } else {
-#pragma unroll 4
-      for (int k = lane; k < K; k += 32) {
-        const float wv = wr[k];
-#pragma unroll
-        for (int t = 0; t < TOK; ++t) acc[t] = __fmaf_rn(wv, to_f32<T>(xs[t * K + k]), acc[t]);
-      }
-    }
+  const int rows = E + (side ? 1 : 0);
+  auto finish = [&](int e, float (&acc)[TOK]) {
 #pragma unroll
     for (int t = 0; t < TOK; ++t) {
       const float v = warp_sum(acc[t]);
@@ -345,6 +320,56 @@ __global__ void __launch_bounds__(512) route_kernel(const T* __restrict__ x, lon
         else if (t < here) side_out[n0 + t] = 1.0f / (1.0f + expf(-v));
       }
     }
+  };
+  // Where a block has several tokens, a warp takes two rows of the router at a time: the tokens' values are read from shared
+  // memory once for both, and twice as many loads are under way.  K = 2,048, 16 experts: 2,048 tokens 21.3 -> 18.3 us, 4,096 tokens 40.8 -> 35.1;
+  // 64 experts 55.9 -> 41.1; 128 experts of K = 2,880 136 -> 93.
+  constexpr int ROWS = TOK > 1 ? 2 : 1;
+  for (int e = warp; e < rows; e += ROWS * warps) {
+    const float* wr[ROWS];
+#pragma unroll
+    for (int i = 0; i < ROWS; ++i) {
+      const int at = e + i * warps < rows ? e + i * warps : e;
+      wr[i] = at < E ? w + (size_t)at * K : side;
+    }
+    float acc[ROWS][TOK];
+#pragma unroll
+    for (int i = 0; i < ROWS; ++i)
+#pragma unroll
+      for (int t = 0; t < TOK; ++t) acc[i][t] = 0.f;
+    if (vec) {
+#pragma unroll (TOK == 1 ? 8 : 4)
+      for (int k = 4 * lane; k < K; k += 128) {
+        float4 wv[ROWS];
+#pragma unroll
+        for (int i = 0; i < ROWS; ++i) wv[i] = *reinterpret_cast<const float4*>(wr[i] + k);
+#pragma unroll
+        for (int t = 0; t < TOK; ++t) {
+          float x0, x1, x2, x3;
+          load4(xs + (size_t)t * K + k, x0, x1, x2, x3);
+#pragma unroll
+          for (int i = 0; i < ROWS; ++i) {
+            acc[i][t] = __fmaf_rn(wv[i].x, x0, acc[i][t]);
+            acc[i][t] = __fmaf_rn(wv[i].y, x1, acc[i][t]);
+            acc[i][t] = __fmaf_rn(wv[i].z, x2, acc[i][t]);
+            acc[i][t] = __fmaf_rn(wv[i].w, x3, acc[i][t]);
+          }
+        }
+      }
+    } else {
+#pragma unroll 4
+      for (int k = lane; k < K; k += 32) {
+#pragma unroll
+        for (int i = 0; i < ROWS; ++i) {
+          const float wv = wr[i][k];
+#pragma unroll
+          for (int t = 0; t < TOK; ++t) acc[i][t] = __fmaf_rn(wv, to_f32<T>(xs[t * K + k]), acc[i][t]);
+        }
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < ROWS; ++i)
+      if (e + i * warps < rows) finish(e + i * warps, acc[i]);
   }
   __syncthreads();
   for (int t = warp; t < here; t += warps) {
