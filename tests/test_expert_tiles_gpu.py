@@ -1,4 +1,4 @@
-"""Experts' products over tiles whose last slots are few, and the router's rows taken two at a time, against float64."""
+"""Experts' products over tiles that end anywhere, and the router's rows taken two at a time, against float64."""
 
 import pytest
 import torch
@@ -9,10 +9,12 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("bm", [64, 128, 256])
 @pytest.mark.parametrize("act", [0, 1])
 @pytest.mark.parametrize("width,inner", [(200, 72), (128, 520), (384, 1024)])
-def test_tiles_end_anywhere_in_their_boxes(bm, act, width, inner):
-    """Experts with every number of slots around a box's 64 and a tile's ``bm``; one with none; the last ends the tensor."""
+@pytest.mark.parametrize("most", [0, 5000])
+def test_tiles_end_anywhere(bm, act, width, inner, most):
+    """Experts with every number of slots around a tile's ``bm``, one with none; with ``most`` the average is large enough for
+    two row blocks a tile, whose second one ends inside the expert's rows, past them, or past the tensor."""
     from yalis_b200.ops import experts as X
-    counts = [1, 63, 64, 65, 0, 127, 129, 191, 192, 193, 255, 256, 257, 320, 5]
+    counts = [1, 63, 64, 65, 0, 127, 129, 191, 192, 193, 255, 256, 257, 320, most, 5]
     g = torch.Generator().manual_seed(bm + width)
     ids = torch.repeat_interleave(torch.arange(len(counts)), torch.tensor(counts))
     ids = ids[torch.randperm(ids.numel(), generator=g)].to(torch.int32)[:, None].cuda()

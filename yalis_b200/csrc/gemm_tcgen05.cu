@@ -384,7 +384,7 @@ gemm_wstream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
 
 // ---- the same product over the experts of a routed feed-forward ---------------------------------------
 // C[slot, :] = act(A[slot, :] . W[expert(slot)]^T) for rows sorted by expert (A holds one row per slot).  A block owns
-// 128 rows of one expert's matrix and one tile of up to NTOK slots of that expert, both named by a plan that an earlier
+// WT x 128 rows of one expert's matrix and one tile of up to NTOK slots of that expert, both named by a plan that an earlier
 // kernel of the step wrote (row tiles as (expert, first slot), their number, the experts' offsets): nothing about the
 // routing is known on the host, so the grid has room for the most tiles the shapes allow and blocks past the last tile
 // leave.  W is one tensor map over all experts' rows [E * N, K]; a box that runs over the end of an expert's rows or
@@ -398,16 +398,33 @@ struct GroupedParams {
   int32_t* error;
 };
 
-template <int NTOK>
+// WT: row blocks of 128 of the expert's matrix in a tile, each with its own accumulator; the slots' rows are fetched once for
+// both, 48 KB from the L2 for 2 x 128 x 128 x 64 products instead of 64.  Two stages of 48 KB and 256 columns of tensor
+// memory still leave room for two blocks on an SM, which hide each other's start and epilogue.
+// Rows (128 slots, WT 1 / 128 slots, WT 2 / 256 slots, WT 1; us) of 16 experts of 4096 x 1024:
+//   slots an expert   64: 29 / 28 / 41   128: 37 / 44 / 47   256: 59 / 58 / 74   384: 77 / 68 / 94   512: 102 / 90 / 129   1024: 192 / 168 / 238
+// of 32 experts of 2880 x 2880:
+//   64: 97 / 113 / 122   128: 126 / 121 / 135   256: 189 / 226 / 226   384: 271 / 271 / 290   512: 349 / 310 / 382   1024: 658 / 583 / 697
+// of 128 experts of 768 x 2048:
+//   64: 79 / 99 / 106   128: 105 / 101 / 126   256: 160 / 158 / 171   384: 212 / 203 / 243   512: 270 / 249 / 295   1024: 495 / 459 / 523
+// so two row blocks from kWideSlots slots an expert on, where they never lose (below, fewer and larger tiles fill the last
+// wave worse).  256 slots, one block on an SM, pay for the empty part of an expert's last tile and for an epilogue that nothing
+// covers; only a plan that asks for them gets them.
+constexpr int kWideSlots = 384;
+
+template <int NTOK, int WT>
+__host__ __device__ constexpr int grouped_stages() { return WT > 1 ? 2 : stages_for<NTOK>(); }
+
+template <int NTOK, int WT>
 __global__ void __launch_bounds__(kThreads, NTOK > 128 ? 1 : 2)
 gemm_grouped_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
                     const GroupedParams p) {
-  constexpr int STAGES = stages_for<NTOK>();
+  constexpr int STAGES = grouped_stages<NTOK, WT>();
   constexpr int KB = kblocks_for<NTOK>();
-  constexpr int A_SUB = TILE_N * TILE_K * 2, B_SUB = NTOK * TILE_K * 2;
+  constexpr int A_SUB = WT * TILE_N * TILE_K * 2, B_SUB = NTOK * TILE_K * 2;
   constexpr int A_BYTES = KB * A_SUB;
   constexpr int B_BYTES = KB * B_SUB;
-  constexpr int TMEM_COLS = NTOK < 32 ? 32 : NTOK;
+  constexpr int TMEM_COLS = NTOK < 32 ? 32 : WT * NTOK;
   extern __shared__ __align__(1024) unsigned char smem[];
   unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem) + 1023) & ~uintptr_t(1023));
   unsigned char* a_s = base;
@@ -446,7 +463,7 @@ gemm_grouped_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
     slot0 = p.tile_slot[blockIdx.y];
     m_rows = min(NTOK, p.offsets[expert + 1] - slot0);
   }
-  const int n0 = blockIdx.x * TILE_N;
+  const int n0 = blockIdx.x * (WT * TILE_N);
   const int n_kt = active ? (p.K + KB * TILE_K - 1) / (KB * TILE_K) : 0;
 
   int armed = 0;
@@ -462,7 +479,9 @@ gemm_grouped_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
 #pragma unroll
         for (int kb = 0; kb < KB; ++kb) {
           const int k = (kt * KB + kb) * TILE_K;
-          tma_load_2d_hint(a_s + s * A_BYTES + kb * A_SUB, &map_w, k, expert * p.N + n0, &full[s], pol_w);
+#pragma unroll
+          for (int h = 0; h < WT; ++h)
+            tma_load_2d_hint(a_s + s * A_BYTES + kb * A_SUB + h * (TILE_N * TILE_K * 2), &map_w, k, expert * p.N + n0 + h * TILE_N, &full[s], pol_w);
           tma_load_2d_hint(b_s + s * B_BYTES + kb * B_SUB, &map_x, k, slot0, &full[s], pol_x);
         }
         armed = kt + 1;
@@ -485,11 +504,14 @@ gemm_grouped_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
         for (int kb = 0; kb < KB; ++kb) {
-          const uint64_t da = umma_desc_sw128(a_s + s * A_BYTES + kb * A_SUB);
           const uint64_t db = umma_desc_sw128(b_s + s * B_BYTES + kb * B_SUB);
 #pragma unroll
-          for (int j = 0; j < TILE_K / UMMA_K; ++j)
-            umma(tmem_d, da + 2 * j, db + 2 * j, idesc, (kt > 0 || kb > 0 || j > 0) ? 1u : 0u);
+          for (int h = 0; h < WT; ++h) {
+            const uint64_t da = umma_desc_sw128(a_s + s * A_BYTES + kb * A_SUB + h * (TILE_N * TILE_K * 2));
+#pragma unroll
+            for (int j = 0; j < TILE_K / UMMA_K; ++j)
+              umma(tmem_d + (uint32_t)(h * NTOK), da + 2 * j, db + 2 * j, idesc, (kt > 0 || kb > 0 || j > 0) ? 1u : 0u);
+          }
         }
         umma_commit(&empty[s]);
       }
@@ -503,24 +525,27 @@ gemm_grouped_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
     ok = __shfl_sync(0xffffffffu, ok, 0);
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     if (ok && n_kt > 0) {
-      const int n = n0 + q * 32 + lane;
 #pragma unroll
-      for (int c0 = 0; c0 < NTOK; c0 += 16) {
-        if (c0 >= m_rows) break;                       // the same for the whole warp
-        uint32_t r[16];
-        tmem_ld16(tmem_d + ((uint32_t)(q * 32) << 16) + (uint32_t)c0, r);
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        if (n < p.N) {
+      for (int h = 0; h < WT; ++h) {
+        const int n = n0 + h * TILE_N + q * 32 + lane;
 #pragma unroll
-          for (int i = 0; i < 16; ++i) {
-            const int m = c0 + i;
-            if (m < m_rows) {
-              float v = __uint_as_float(r[i]);
-              if (p.act == 1) {
-                v = fmaxf(v, 0.f);
-                v = v * v;
+        for (int c0 = 0; c0 < NTOK; c0 += 16) {
+          if (c0 >= m_rows) break;                     // the same for the whole warp
+          uint32_t r[16];
+          tmem_ld16(tmem_d + ((uint32_t)(q * 32) << 16) + (uint32_t)(h * NTOK + c0), r);
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+          if (n < p.N) {
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {
+              const int m = c0 + i;
+              if (m < m_rows) {
+                float v = __uint_as_float(r[i]);
+                if (p.act == 1) {
+                  v = fmaxf(v, 0.f);
+                  v = v * v;
+                }
+                p.out[(size_t)(slot0 + m) * p.ldo + n] = __float2bfloat16_rn(v);
               }
-              p.out[(size_t)(slot0 + m) * p.ldo + n] = __float2bfloat16_rn(v);
             }
           }
         }
@@ -639,20 +664,20 @@ int launch(const CUtensorMap& mw, const CUtensorMap& mx, const GemmParams& p, cu
   return p.silu_inter ? launch_cfg<NTOK, true>(mw, mx, p, stream) : launch_cfg<NTOK, false>(mw, mx, p, stream);
 }
 
-template <int NTOK>
+template <int NTOK, int WT>
 int launch_grouped(const CUtensorMap& mw, const CUtensorMap& mx, const GroupedParams& p, int max_tiles, cudaStream_t stream) {
-  constexpr int STAGES = stages_for<NTOK>();
-  const size_t smem = 1024 + (size_t)STAGES * kblocks_for<NTOK>() * (TILE_N * TILE_K * 2 + NTOK * TILE_K * 2) +
+  constexpr int STAGES = grouped_stages<NTOK, WT>();
+  const size_t smem = 1024 + (size_t)STAGES * kblocks_for<NTOK>() * (WT * TILE_N * TILE_K * 2 + NTOK * TILE_K * 2) +
                       (2 * STAGES + 1) * 8 + 16;
   static bool configured = false;
   if (!configured) {
-    if (cudaFuncSetAttribute(gemm_grouped_kernel<NTOK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+    if (cudaFuncSetAttribute(gemm_grouped_kernel<NTOK, WT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
       return YALIS_ERR_LAUNCH;
     configured = true;
   }
-  dim3 grid((p.N + TILE_N - 1) / TILE_N, max_tiles);
+  dim3 grid((p.N + WT * TILE_N - 1) / (WT * TILE_N), max_tiles);
   if (grid.y > 65535) return YALIS_ERR_SHAPE;
-  return yalis_launch(gemm_grouped_kernel<NTOK>, grid, dim3(kThreads), smem, stream, mw, mx, p);
+  return yalis_launch(gemm_grouped_kernel<NTOK, WT>, grid, dim3(kThreads), smem, stream, mw, mx, p);
 }
 
 }  // namespace
@@ -673,11 +698,13 @@ YALIS_API int yalis_grouped_gemm_wstream(const void* a, long long lda, int rows_
   p.out = (__nv_bfloat16*)out; p.ldo = ldo; p.N = N; p.K = K; p.act = act; p.offsets = offsets; p.tile_expert = tile_expert;
   p.tile_slot = tile_slot; p.n_tiles = n_tiles; p.error = error;
   switch (bm) {
-    case 16: return launch_grouped<16>(mw, mx, p, max_tiles, stream);
-    case 32: return launch_grouped<32>(mw, mx, p, max_tiles, stream);
-    case 64: return launch_grouped<64>(mw, mx, p, max_tiles, stream);
-    case 128: return launch_grouped<128>(mw, mx, p, max_tiles, stream);
-    case 256: return launch_grouped<256>(mw, mx, p, max_tiles, stream);
+    case 16: return launch_grouped<16, 1>(mw, mx, p, max_tiles, stream);
+    case 32: return launch_grouped<32, 1>(mw, mx, p, max_tiles, stream);
+    case 64: return launch_grouped<64, 1>(mw, mx, p, max_tiles, stream);
+    case 128:
+      if (rows_a / n_experts >= kWideSlots) return launch_grouped<128, 2>(mw, mx, p, max_tiles, stream);
+      return launch_grouped<128, 1>(mw, mx, p, max_tiles, stream);
+    case 256: return launch_grouped<256, 1>(mw, mx, p, max_tiles, stream);
   }
   return YALIS_ERR_SHAPE;
 }

@@ -144,16 +144,17 @@ class RoutedExperts(FeedForward):
                 and x.data_ptr() % 16 == 0)
 
     def row_tile(self, x: torch.Tensor, wstream: bool) -> int:
-        """Rows of a tile of the experts' products, from the step's shape alone.  tcgen05 form: the smallest of 16 ... 256
+        """Rows of a tile of the experts' products, from the step's shape alone.  tcgen05 form: the smallest of 16 ... 128
         that holds twice the rows an expert gets on average (a tile is the N side of the MMA: a half-empty one costs
-        nothing where the weights set the pace, and few experts then need a second tile).  mma form: 128 when an
-        expert gets about that many, 16 when at most 8, else 32.  The float32 form has tiles of 32."""
+        nothing where the weights set the pace, and few experts then need a second tile), and 128 for more: the kernel's
+        comment has the times of 256.  mma form: 128 when an expert gets about that many, 16 when at most 8, else 32.
+        The float32 form has tiles of 32."""
         entries = x.shape[0] * self.top
         if wstream:
-            for tile in ops.WSTREAM_TILES:
+            for tile in (16, 32, 64):
                 if 2 * entries <= tile * self.n_experts:
                     return tile
-            return ops.WSTREAM_TILES[-1]
+            return 128 if entries // 128 + self.n_experts <= 65535 else 256      # the tiles a grid can have
         if not self._aligned(x):
             return 32
         return 128 if entries >= 96 * self.n_experts else (16 if entries <= 8 * self.n_experts else 32)
