@@ -384,6 +384,160 @@ int launch_qkv_plain(const PrepParams& p, int n_tokens, cudaStream_t stream) {
   return go(qkv_plain_kernel<T, TO, 32, 2>, 32);
 }
 
+// The same where heads turn and are normed one by one or not at all, nothing averaged: L lanes take a head, eight values
+// each, which stay in registers from load to store: two groups of four that turn with one another (half-split pairs: d and
+// d + half) or eight neighbours (interleaved pairs, and sizes that do not turn).  A lane turns the same sizes in all heads of
+// its token, so it fetches its sines and cosines once from the block's table.  Every group loads two heads before it needs
+// the first.  The lanes, and so the order of a norm's sum, depend on the sizes alone, never on the step.
+// What bounds it: the latency of a token's chain (row, table, loads, norm, store); a row's values through shared memory and
+// one head at a time cost more of it.
+// Measured (16 + 2 x 8 heads of 128 that turn whole, norms, pages; us at 64 / 512 / 2,048 tokens): through shared memory
+// 3.8 / 10.9 / 26.6, here 3.7 / 7.6 / 17.8; 32 + 2 x 8 heads of 64: 4.4 / 15.5 / 38.1 -> 3.7 / 4.6 / 13.8; 16 + 2 x 8 of 256:
+// 4.4 / 13.7 / 37.6 -> 4.1 / 10.3 / 30.8.  Fetching the rows before the request is known costs registers and gains nothing.
+template <typename T, typename TO, int L, bool INTER>
+__global__ void __launch_bounds__(256) qkv_turn_kernel(const PrepParams p) {
+  extern __shared__ __align__(16) float table_s[];  // cosines, then sines
+  pdl_launch_dependents();
+  pdl_wait();
+  const int n = blockIdx.x, l = threadIdx.x % L, groups = blockDim.x / L;
+  const int req = p.req_of_token[n], pos = p.positions[n];
+  if (req < 0) return;
+  const int half = p.inv_freq ? p.rot_dims >> 1 : 0, keys = p.nk * p.maps, heads = p.nq + keys + p.nk;
+  const T* row = reinterpret_cast<const T*>(p.src) + (size_t)n * p.src_stride;
+  // a lane's two groups of four sizes in a query or key
+  const bool turns = INTER ? 8 * l < 2 * half : 4 * l < half;
+  const int d0 = INTER ? 8 * l : (turns ? 4 * l : 2 * half + 8 * (l - half / 4));
+  const int d1 = INTER ? 8 * l + 4 : (turns ? 4 * l + half : d0 + 4);
+  float* cos_s = table_s;
+  float* sin_s = table_s + ((half + 3) & ~3);
+  const long long row0 = p.k_pool != nullptr ? paged_row(p.block_table + (size_t)req * p.table_width, p.table_width, p.page_size,
+                                                         p.num_pages, p.nk, 0, pos)
+                                             : 0;
+  const int first = blockIdx.y * groups + threadIdx.x / L, step = gridDim.y * groups;
+  float4 xa[2], xb[2];
+  auto load = [&](int head, float4& a, float4& b) {
+    const bool is_q = head < p.nq, is_v = head >= p.nq + keys;
+    const int hh = is_q ? head : (is_v ? head - p.nq - keys : head - p.nq), width = is_v ? p.vdim : p.dim;
+    const int at = is_v ? 8 * l : d0, at1 = is_v ? 8 * l + 4 : d1;
+    a = b = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (head >= heads || 8 * l >= width) return;
+    const T* src = row + (is_q ? p.q_off : (is_v ? p.v_off : p.k_off)) + (size_t)hh * width;
+    a = load4_f32(src + at);
+    b = load4_f32(src + at1);
+    const T* bias = reinterpret_cast<const T*>(is_q ? p.q_bias : (is_v ? p.v_bias : p.k_bias));
+    if (bias) {
+      const float4 u = load4_f32(bias + (size_t)hh * width + at), v = load4_f32(bias + (size_t)hh * width + at1);
+      a.x += u.x; a.y += u.y; a.z += u.z; a.w += u.w;
+      b.x += v.x; b.y += v.y; b.z += v.z; b.w += v.w;
+    }
+  };
+#pragma unroll
+  for (int i = 0; i < 2; ++i) load(first + i * step, xa[i], xb[i]);
+  for (int i = threadIdx.x; i < half; i += blockDim.x) {
+    float sn, cs;
+    sincosf((float)pos * p.inv_freq[i], &sn, &cs);
+    cos_s[i] = cs * p.rot_scale;
+    sin_s[i] = sn * p.rot_scale;
+  }
+  __syncthreads();
+  float4 cs = make_float4(1.f, 1.f, 1.f, 1.f), sn = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (turns) {
+    if (INTER && 8 * l + 8 > 2 * half) {           // the last four sizes that turn are half of a lane's eight
+      cs.x = cos_s[4 * l]; cs.y = cos_s[4 * l + 1];
+      sn.x = sin_s[4 * l]; sn.y = sin_s[4 * l + 1];
+    } else {
+      cs = *reinterpret_cast<const float4*>(cos_s + 4 * l);
+      sn = *reinterpret_cast<const float4*>(sin_s + 4 * l);
+    }
+  }
+  const bool turns_b = INTER ? 8 * l + 4 < 2 * half : turns;
+  const float q_factor = p.q_temp_every > 0 ? p.q_scale * (1.0f + p.q_temp_coef * logf((float)((pos + 1) / p.q_temp_every + 1)))
+                                            : p.q_scale;
+  // (the bound is the same for a warp's groups: all lanes take part in the sums)
+  for (int base = first - (int)(threadIdx.x % 32) / L; base < heads; base += 2 * step) {
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int head = base + (int)(threadIdx.x % 32) / L + i * step;
+      const bool is_q = head < p.nq, is_v = head >= p.nq + keys;
+      const int hh = is_q ? head : (is_v ? head - p.nq - keys : head - p.nq), width = is_v ? p.vdim : p.dim;
+      float4 a = xa[i], b = xb[i];
+      const float* nw = head >= heads || is_v ? nullptr : (is_q ? p.q_norm : p.k_norm);
+      float ss = ((a.x * a.x + a.y * a.y) + (a.z * a.z + a.w * a.w)) + ((b.x * b.x + b.y * b.y) + (b.z * b.z + b.w * b.w));
+#pragma unroll
+      for (int o = L / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+      load(head + 2 * step, xa[i], xb[i]);
+      if (head >= heads || 8 * l >= width) continue;
+      TO* dst;
+      if (is_q) {
+        dst = reinterpret_cast<TO*>(p.q_out) + (size_t)n * p.q_out_stride + (size_t)hh * width;
+      } else if (p.k_pool != nullptr) {
+        if (row0 < 0) {
+          if (l == 0 && p.bad_page) atomicOr(p.bad_page, YALIS_FLAG_BAD_PAGE);
+          continue;
+        }
+        if (is_v) dst = reinterpret_cast<TO*>(p.v_pool) + (row0 + (long long)hh * p.page_size) * width;
+        else dst = reinterpret_cast<TO*>(p.k_pool) + (row0 + (long long)(hh / p.maps) * p.page_size) * (p.maps * width) + hh % p.maps * width;
+      } else {
+        if (p.k_out == nullptr) continue;            // nothing keeps this layer's keys and values: queries only
+        dst = is_v ? reinterpret_cast<TO*>(p.v_out) + (size_t)n * p.v_out_stride + (size_t)hh * width
+                   : reinterpret_cast<TO*>(p.k_out) + (size_t)n * p.k_out_stride + (size_t)hh * width;
+      }
+      if (is_v) {
+        store4(dst + 8 * l, a);
+        store4(dst + 8 * l + 4, b);
+        continue;
+      }
+      if (nw) {
+        const float r = 1.0f / sqrtf(ss / (float)width + p.norm_eps);
+        const float4 u = load4_f32(nw + d0), v = load4_f32(nw + d1);
+        a.x = a.x * r * u.x; a.y = a.y * r * u.y; a.z = a.z * r * u.z; a.w = a.w * r * u.w;
+        b.x = b.x * r * v.x; b.y = b.y * r * v.y; b.z = b.z * r * v.z; b.w = b.w * r * v.w;
+      }
+      float4 oa = a, ob = b;
+      if constexpr (INTER) {
+        if (turns) {
+          rotate_pair(a.x, a.y, cs.x, sn.x, oa.x, oa.y);
+          rotate_pair(a.z, a.w, cs.y, sn.y, oa.z, oa.w);
+        }
+        if (turns_b) {
+          rotate_pair(b.x, b.y, cs.z, sn.z, ob.x, ob.y);
+          rotate_pair(b.z, b.w, cs.w, sn.w, ob.z, ob.w);
+        }
+      } else if (turns) {
+        rotate_pair(a.x, b.x, cs.x, sn.x, oa.x, ob.x);
+        rotate_pair(a.y, b.y, cs.y, sn.y, oa.y, ob.y);
+        rotate_pair(a.z, b.z, cs.z, sn.z, oa.z, ob.z);
+        rotate_pair(a.w, b.w, cs.w, sn.w, oa.w, ob.w);
+      }
+      const float factor = is_q ? q_factor : p.k_scale;
+      store4(dst + d0, make_float4(oa.x * factor, oa.y * factor, oa.z * factor, oa.w * factor));
+      store4(dst + d1, make_float4(ob.x * factor, ob.y * factor, ob.z * factor, ob.w * factor));
+    }
+  }
+}
+
+template <typename T, typename TO>
+int launch_qkv_turn(const PrepParams& p, int n_tokens, cudaStream_t stream) {
+  const int widest = p.dim < p.vdim ? p.vdim : p.dim, heads = p.nq + (p.maps + 1) * p.nk;
+  const int half = p.inv_freq ? p.rot_dims / 2 : 0;
+  const size_t smem = 2 * (size_t)((half + 3) & ~3) * sizeof(float);
+  // steps of many tokens: blocks that hold a token's heads in one pass, as far as 256 threads do; few tokens: four warps
+  auto go = [&](auto kernel, int lanes) {
+    const int needed = ((heads + 1) / 2 * lanes + 31) / 32 * 32;
+    const bool many = n_tokens >= 2 * yalis_sm_count();
+    const int threads = many ? (needed < 256 ? needed : 256) : 128, pass = 2 * (threads / lanes);
+    return yalis_launch(kernel, dim3(n_tokens, many ? 1 : (heads + pass - 1) / pass), dim3(threads), smem, stream, p);
+  };
+  if (p.rot_interleaved) {
+    if (widest <= 64) return go(qkv_turn_kernel<T, TO, 8, true>, 8);
+    if (widest <= 128) return go(qkv_turn_kernel<T, TO, 16, true>, 16);
+    return go(qkv_turn_kernel<T, TO, 32, true>, 32);
+  }
+  if (widest <= 64) return go(qkv_turn_kernel<T, TO, 8, false>, 8);
+  if (widest <= 128) return go(qkv_turn_kernel<T, TO, 16, false>, 16);
+  return go(qkv_turn_kernel<T, TO, 32, false>, 32);
+}
+
 template <typename T, typename TO>
 int launch_qkv_prepare(const PrepParams& p, dim3 grid, int warps, bool table, bool vec, cudaStream_t stream) {
   const int row_floats = ((p.dim > p.vdim ? p.dim : p.vdim) + 3) & ~3;
@@ -600,6 +754,13 @@ YALIS_API int yalis_qkv_prepare(const void* src, int dtype, int src_stride, int 
   if (plain && dtype == YALIS_BF16 && out_dtype == YALIS_BF16)
     return launch_qkv_plain<__nv_bfloat16, __nv_bfloat16>(p, n_tokens, stream);
   if (plain && dtype == YALIS_BF16 && out_dtype == YALIS_F32) return launch_qkv_plain<__nv_bfloat16, float>(p, n_tokens, stream);
+  // heads in registers: eight values a lane, four of which turn with four others where pairs are half-split
+  // (at 64 tokens the general form is level, from there on it is slower; below, both are the latency of a launch)
+  const bool turn = vec && ((dim | vdim) & 7) == 0 && dim <= 256 && vdim <= 256 && !norm_all && pool == 0 &&
+                    (rot_interleaved || !inv_freq || (rot_dims & 7) == 0);
+  if (turn && dtype == YALIS_F32 && out_dtype == YALIS_F32) return launch_qkv_turn<float, float>(p, n_tokens, stream);
+  if (turn && dtype == YALIS_BF16 && out_dtype == YALIS_BF16) return launch_qkv_turn<__nv_bfloat16, __nv_bfloat16>(p, n_tokens, stream);
+  if (turn && dtype == YALIS_BF16 && out_dtype == YALIS_F32) return launch_qkv_turn<__nv_bfloat16, float>(p, n_tokens, stream);
   if (dtype == YALIS_F32 && out_dtype == YALIS_F32) st = launch_qkv_prepare<float, float>(p, grid, warps, table, vec, stream);
   else if (dtype == YALIS_BF16 && out_dtype == YALIS_BF16)
     st = launch_qkv_prepare<__nv_bfloat16, __nv_bfloat16>(p, grid, warps, table, vec, stream);
