@@ -755,7 +755,8 @@ YALIS_API int yalis_qkv_prepare(const void* src, int dtype, int src_stride, int 
     return launch_qkv_plain<__nv_bfloat16, __nv_bfloat16>(p, n_tokens, stream);
   if (plain && dtype == YALIS_BF16 && out_dtype == YALIS_F32) return launch_qkv_plain<__nv_bfloat16, float>(p, n_tokens, stream);
   // heads in registers: eight values a lane, four of which turn with four others where pairs are half-split
-  // (at 64 tokens the general form is level, from there on it is slower; below, both are the latency of a launch)
+  // (one form whatever the number of tokens, so that a row's bits do not depend on the step: from 64 tokens on it is the
+  // faster one, for up to 8 it takes 3.5 us where the general form takes 3.3)
   const bool turn = vec && ((dim | vdim) & 7) == 0 && dim <= 256 && vdim <= 256 && !norm_all && pool == 0 &&
                     (rot_interleaved || !inv_freq || (rot_dims & 7) == 0);
   if (turn && dtype == YALIS_F32 && out_dtype == YALIS_F32) return launch_qkv_turn<float, float>(p, n_tokens, stream);
