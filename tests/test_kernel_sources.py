@@ -1,0 +1,49 @@
+"""Rules that hold for every kernel and whose breach shows on a GPU only now and then, if at all: read from the sources."""
+
+import glob
+import os
+import re
+
+import pytest
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "yalis_b200", "csrc")
+
+
+def _block(text, start):
+    """The text between the brace at or after ``start`` and its partner."""
+    begin = text.index("{", start)
+    depth = 0
+    for i in range(begin, len(text)):
+        depth += {"{": 1, "}": -1}.get(text[i], 0)
+        if depth == 0:
+            return text[begin + 1:i]
+    raise ValueError("unbalanced braces")
+
+
+def _kernels():
+    """(name, parameters, body) of every kernel, without comments."""
+    found = []
+    for path in sorted(glob.glob(os.path.join(CSRC, "*.cu")) + glob.glob(os.path.join(CSRC, "*.cuh"))):
+        text = re.sub(r"//[^\n]*", "", open(path).read())
+        for m in re.finditer(r"__global__", text):
+            head = text[m.start():text.index("{", m.start())]
+            name = re.findall(r"(\w+)\s*\((?=[^()]*$|[^()]*\))", head)[-1]
+            found.append((name, head[head.index(name):], _block(text, m.start())))
+    return found
+
+
+KERNELS = _kernels()
+ids = lambda kernels: [k[0] for k in kernels]
+WITH_TENSOR_MEMORY = [k for k in KERNELS if "tcgen05.alloc" in k[2]]
+
+
+def test_kernels_are_found():
+    assert len(KERNELS) > 50 and len(WITH_TENSOR_MEMORY) >= 4
+
+
+@pytest.mark.parametrize("name,parameters,body", WITH_TENSOR_MEMORY, ids=ids(WITH_TENSOR_MEMORY))
+def test_tensor_memory_is_taken_before_the_next_kernel_is_let_in(name, parameters, body):
+    """One thread that lets the next kernel in does so for its block.  A block that has let it in and still waits for tensor
+    memory may see a block of that kernel take the columns, which then waits for this kernel: neither ever ends."""
+    alloc, let_in = body.index("tcgen05.alloc"), body.index("pdl_launch_dependents")
+    assert alloc < let_in and "__syncthreads()" in body[alloc:let_in]

@@ -205,11 +205,13 @@ prefill_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(TMEM_COLS));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::);
   }
-  pdl_launch_dependents();
-  pdl_wait();             // the counter is read only after this: the launch before this one has left it at zero
+  // Tensor memory is taken before the next kernel's blocks are let in: one thread of a block lets them in for all of it, and
+  // a block of theirs that took these columns first would hold them while it waits for this kernel.
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  pdl_launch_dependents();
+  pdl_wait();             // the counter is read only after this: the launch before this one has left it at zero
   const uint32_t tmem = *tmem_slot;
   const int slots = p.n_z;                                  // shares that the scratch memory has room for
 
