@@ -47,3 +47,24 @@ def test_tensor_memory_is_taken_before_the_next_kernel_is_let_in(name, parameter
     memory may see a block of that kernel take the columns, which then waits for this kernel: neither ever ends."""
     alloc, let_in = body.index("tcgen05.alloc"), body.index("pdl_launch_dependents")
     assert alloc < let_in and "__syncthreads()" in body[alloc:let_in]
+
+
+def _inner_loops(body):
+    """The bodies of loops with braces that hold no such loop themselves."""
+    for m in re.finditer(r"\bfor \(", body):
+        depth, i = 1, m.end()
+        while depth:
+            depth += {"(": 1, ")": -1}.get(body[i], 0)
+            i += 1
+        if body[i:].lstrip().startswith("{"):
+            inside = _block(body, i)
+            if not re.search(r"\bfor \([^;]*;[^;]*;[^)]*\) \{[^}]*tmem_ld", inside):
+                yield inside
+
+
+@pytest.mark.parametrize("name,parameters,body", WITH_TENSOR_MEMORY, ids=ids(WITH_TENSOR_MEMORY))
+def test_a_warp_is_whole_when_it_loads_tensor_memory(name, parameters, body):
+    """The instruction asks for a converged warp: a loop whose lanes part after the load brings them together before the next."""
+    for loop in _inner_loops(body):
+        if "tmem_ld" in loop and re.search(r"\bif \(", loop[loop.index("tmem_ld"):]):
+            assert "__syncwarp()" in loop[:loop.index("tmem_ld")], loop[:300]

@@ -627,6 +627,7 @@ prefill_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
 #pragma unroll 1
         for (int c0 = 0; c0 < HS; c0 += 16) {
           uint32_t o[16];
+          __syncwarp();                                       // rows without a token and rows with one part below
           tmem_ld16(lane_base + COL_O + c0, o);
           asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
           if (valid) {
@@ -659,6 +660,7 @@ prefill_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
 #pragma unroll 1
         for (int c0 = 0; c0 < HS; c0 += 16) {
           uint32_t o[16];
+          __syncwarp();                                       // rows without a token and rows with one part below
           tmem_ld16(lane_base + COL_O + c0, o);
           asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
           if constexpr (GEN) {

@@ -307,6 +307,7 @@ gemm_wstream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
 #pragma unroll
       for (int c0 = 0; c0 < NTOK; c0 += 16) {
         uint32_t r[16];
+        __syncwarp();                                 // lanes past the last row part from the others below
         tmem_ld16(tmem_d + ((uint32_t)(q * 32) << 16) + (uint32_t)c0, r);
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
         float* buf = ex + ((c0 >> 4) & 1) * (16 * 64);
@@ -334,6 +335,7 @@ gemm_wstream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
 #pragma unroll
       for (int c0 = 0; c0 < NTOK; c0 += 16) {
         uint32_t r[16];
+        __syncwarp();                                 // lanes past the last row part from the others below
         if (n_kt > 0) {
           tmem_ld16(tmem_d + ((uint32_t)(q * 32) << 16) + (uint32_t)c0, r);
           asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
@@ -532,6 +534,7 @@ gemm_grouped_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
         for (int c0 = 0; c0 < NTOK; c0 += 16) {
           if (c0 >= m_rows) break;                     // the same for the whole warp
           uint32_t r[16];
+          __syncwarp();                                 // lanes past the last row part from the others below
           tmem_ld16(tmem_d + ((uint32_t)(q * 32) << 16) + (uint32_t)(h * NTOK + c0), r);
           asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
           if (n < p.N) {

@@ -380,6 +380,7 @@ latent_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map, const L
 #pragma unroll 1
       for (int c0 = 0; c0 < R; c0 += 32) {
         uint32_t o[32];
+        __syncwarp();                                                // rows past the last one and the others part below
         tmem_ld32(lane_base + COL_O + c0, o);
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
         if (!valid) continue;
