@@ -68,3 +68,16 @@ def test_a_warp_is_whole_when_it_loads_tensor_memory(name, parameters, body):
     for loop in _inner_loops(body):
         if "tmem_ld" in loop and re.search(r"\bif \(", loop[loop.index("tmem_ld"):]):
             assert "__syncwarp()" in loop[:loop.index("tmem_ld")], loop[:300]
+
+
+# weights and other constants of a model, which no kernel of a step writes
+CONSTANTS = {"w", "weight", "norm_w", "d_w", "bias", "inv_freq", "a_bias", "w_bias", "side", "table", "sink"}
+
+
+@pytest.mark.parametrize("path", sorted(glob.glob(os.path.join(CSRC, "*.cu")) + glob.glob(os.path.join(CSRC, "*.cuh"))), ids=os.path.basename)
+def test_what_another_kernel_writes_is_not_read_through_restrict(path):
+    """A load through a restrict pointer may be moved above the wait for the kernel that writes what it reads."""
+    text = re.sub(r"//[^\n]*", "", open(path).read())
+    assert "__ldg" not in text
+    for kind, name in re.findall(r"([\w ]+)\*\s*__restrict__\s+(\w+)", text):
+        assert "const " in kind and name in CONSTANTS, (kind, name)

@@ -770,8 +770,8 @@ bool make_q_map(CUtensorMap* map, const void* q, long long n_tokens, int q_strid
 }
 
 // Adds the shares of every (token, head) that was divided: one block per token, a thread per four output columns.
-__global__ void prefill_merge_splits_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml,
-                                            __nv_bfloat16* __restrict__ out, int out_stride, int nh, int hs, int n_splits) {
+__global__ void prefill_merge_splits_kernel(const float* part_o, const float* part_ml,
+                                            __nv_bfloat16* out, int out_stride, int nh, int hs, int n_splits) {
   pdl_launch_dependents();
   pdl_wait();
   const int tok = blockIdx.x, vec = hs / 4;

@@ -62,6 +62,9 @@ inline int yalis_sm_count() {
 // blocks need (measured: 9 % of a batch-64 decode step).
 // Kernels that hold few blocks for long (a recurrence's walk over a prompt) are launched without the attribute
 // (yalis_launch_after): let in early, their blocks would all land on the SMs that come free first.
+// What the kernel in front writes is read through pointers without __restrict__: the compiler takes a load through a restrict
+// pointer for one that nothing else in the kernel can affect and may move it above the wait (a float32 product read its
+// predecessor's rows before they were written).  Weights, which no kernel of a step writes, may keep it.
 bool yalis_pdl_enabled();   // defined in elementwise.cu; switched by yalis_set_pdl()
 
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
@@ -154,7 +157,7 @@ __device__ __forceinline__ void store2(__nv_bfloat16* p, float2 v) {
 // Sum of the n partial values p[s * stride], added in index order but loaded eight at a time
 // (a load per addition would cost a trip to the L2 for each).
 template <typename TS>
-__device__ __forceinline__ float sum_parts(const TS* __restrict__ p, int n, size_t stride) {
+__device__ __forceinline__ float sum_parts(const TS* p, int n, size_t stride) {
   float acc = 0.f;
   for (int s0 = 0; s0 < n; s0 += 8) {
     float v[8];

@@ -21,9 +21,9 @@ YALIS_API void yalis_set_pdl(int enabled) { g_pdl_enabled = enabled != 0; }
 // With `norm_w` the row enters the stream normed: v / sqrt(mean(v^2) + norm_eps) * norm_w (float32, after `scale`).
 // --------------------------------------------------------------------------
 template <typename T>
-__global__ void embedding_kernel(const T* __restrict__ table, const int32_t* __restrict__ ids,
-                                 const int32_t* __restrict__ from_slot, const int32_t* __restrict__ chosen,
-                                 float* __restrict__ out, int width, int vocab, float scale, int32_t* bad_id,
+__global__ void embedding_kernel(const T* __restrict__ table, const int32_t* ids,
+                                 const int32_t* from_slot, const int32_t* chosen,
+                                 float* out, int width, int vocab, float scale, int32_t* bad_id,
                                  const float* __restrict__ norm_w, float norm_eps) {
   __shared__ float scratch[32];
   pdl_launch_dependents();
@@ -62,7 +62,7 @@ __global__ void embedding_kernel(const T* __restrict__ table, const int32_t* __r
 // --------------------------------------------------------------------------
 // Soft cap of float32 logits in place: v <- cap * tanh(v / cap).
 // --------------------------------------------------------------------------
-__global__ void softcap_kernel(float* __restrict__ v, size_t n, float cap) {
+__global__ void softcap_kernel(float* v, size_t n, float cap) {
   pdl_launch_dependents();
   pdl_wait();
   const float inv = 1.0f / cap;
@@ -91,9 +91,9 @@ YALIS_API int yalis_softcap_f32(float* v, long long n, float cap, cudaStream_t s
 // --------------------------------------------------------------------------
 // MAXV: values a thread keeps in registers (the row is read once); 0 = re-read variant for wide rows.
 template <typename T, typename TD, int MAXV>
-__global__ void __launch_bounds__(1024) add_rmsnorm_kernel(float* __restrict__ x, const TD* __restrict__ delta, int n_delta,
-                                   size_t delta_stride, const float* __restrict__ w, T* __restrict__ y,
-                                   const int32_t* __restrict__ rows, int width, float eps, int write_back) {
+__global__ void __launch_bounds__(1024) add_rmsnorm_kernel(float* x, const TD* delta, int n_delta,
+                                   size_t delta_stride, const float* __restrict__ w, T* y,
+                                   const int32_t* rows, int width, float eps, int write_back) {
   __shared__ float scratch[32];
   pdl_launch_dependents();
   pdl_wait();
@@ -171,9 +171,9 @@ __global__ void __launch_bounds__(1024) add_rmsnorm_kernel(float* __restrict__ x
 // The normed embedding for rows whose width is a multiple of four and at most 4096: a thread keeps up to four groups
 // of four values in registers between the sum of squares and the store, so the table row is read once.
 template <typename T>
-__global__ void embedding_norm_vec_kernel(const T* __restrict__ table, const int32_t* __restrict__ ids,
-                                          const int32_t* __restrict__ from_slot, const int32_t* __restrict__ chosen,
-                                          float* __restrict__ out, int width, int vocab, float scale, int32_t* bad_id,
+__global__ void embedding_norm_vec_kernel(const T* __restrict__ table, const int32_t* ids,
+                                          const int32_t* from_slot, const int32_t* chosen,
+                                          float* out, int width, int vocab, float scale, int32_t* bad_id,
                                           const float* __restrict__ norm_w, float norm_eps) {
   __shared__ float scratch[32];
   pdl_launch_dependents();
@@ -230,10 +230,10 @@ YALIS_API int yalis_embedding(const void* table, int dtype, const int32_t* ids, 
 // every thread keeps NV groups of four columns, all loads of a row are in flight at once, and the
 // norm's weight is fetched before the wait for the preceding kernel.
 template <typename T, typename TD, int NV>
-__global__ void __launch_bounds__(1024) add_rmsnorm_vec_kernel(float* __restrict__ x, const TD* __restrict__ delta,
+__global__ void __launch_bounds__(1024) add_rmsnorm_vec_kernel(float* x, const TD* delta,
                                                                int n_delta, size_t delta_stride,
-                                                               const float* __restrict__ w, T* __restrict__ y,
-                                                               const int32_t* __restrict__ rows, int width, float eps,
+                                                               const float* __restrict__ w, T* y,
+                                                               const int32_t* rows, int width, float eps,
                                                                int write_back) {
   __shared__ float scratch[32];
   pdl_launch_dependents();
@@ -387,11 +387,11 @@ __device__ __forceinline__ float4 tail_value4(const SumTail& t, size_t row_off) 
 }
 
 template <typename T, typename TD>
-__global__ void __launch_bounds__(1024) add_normed_rmsnorm_kernel(float* __restrict__ x, const TD* __restrict__ delta, int n_delta,
+__global__ void __launch_bounds__(1024) add_normed_rmsnorm_kernel(float* x, const TD* delta, int n_delta,
                                                                   size_t delta_stride, const float* __restrict__ bias,
                                                                   const float* __restrict__ d_w, float d_eps,
-                                                                  const float* __restrict__ w, T* __restrict__ y,
-                                                                  const int32_t* __restrict__ rows, int width, float eps,
+                                                                  const float* __restrict__ w, T* y,
+                                                                  const int32_t* rows, int width, float eps,
                                                                   int write_back, const SumTail tail) {
   extern __shared__ float row_s[];        // [width], with a second result [2 * width]
   __shared__ float scratch[32];
@@ -444,12 +444,12 @@ __global__ void __launch_bounds__(1024) add_normed_rmsnorm_kernel(float* __restr
 // except inside the two means, which are fixed-order block reductions in both.
 // TAIL: a second result, a factor or a vector on the sum may follow (their loads are left where they are used).
 template <typename T, typename TD, int NV, bool TAIL>
-__global__ void __launch_bounds__(NV == 1 ? 1024 : 256, NV == 2 ? 3 : 1) add_normed_rmsnorm_vec_kernel(float* __restrict__ x, const TD* __restrict__ delta,
+__global__ void __launch_bounds__(NV == 1 ? 1024 : 256, NV == 2 ? 3 : 1) add_normed_rmsnorm_vec_kernel(float* x, const TD* delta,
                                                                       int n_delta, size_t delta_stride,
                                                                       const float* __restrict__ bias,
                                                                       const float* __restrict__ d_w, float d_eps,
-                                                                      const float* __restrict__ w, T* __restrict__ y,
-                                                                      const int32_t* __restrict__ rows, int width, float eps,
+                                                                      const float* __restrict__ w, T* y,
+                                                                      const int32_t* rows, int width, float eps,
                                                                       int write_back, const SumTail tail) {
   __shared__ float scratch[32];
   pdl_launch_dependents();
@@ -625,7 +625,7 @@ YALIS_API int yalis_add_normed_rmsnorm(float* x, const void* delta, int delta_dt
 // Plain residual add without a norm: x[r] += sum_s delta[s][r]. Used to flush a
 // pending delta when a caller wants the residual stream itself.
 template <typename TD>
-__global__ void residual_add_kernel(float* __restrict__ x, const TD* __restrict__ delta, int n_delta,
+__global__ void residual_add_kernel(float* x, const TD* delta, int n_delta,
                                     size_t delta_stride, size_t n) {
   pdl_launch_dependents();
   pdl_wait();
@@ -638,7 +638,6 @@ __global__ void residual_add_kernel(float* __restrict__ x, const TD* __restrict_
 
 // The same, four values a thread (x, the partial sums and their stride on the boundaries of four values): bound by memory.
 // 2,048 x 2,048 rows with one bfloat16 delta, 42 MB: 19 us a value a thread, 9 us this way (ncu, cold).
-// (No __restrict__: a load the compiler takes for one of constant data may be moved above the wait for the kernel before.)
 template <typename TD>
 __global__ void residual_add_x4_kernel(float* x, const TD* delta, int n_delta, size_t delta_stride, size_t quads) {
   pdl_launch_dependents();
@@ -694,11 +693,11 @@ YALIS_API int yalis_residual_add(float* x, const void* delta, int delta_dtype, i
 // One block per (token, head of the fused row).
 // --------------------------------------------------------------------------
 template <typename T, typename TS>
-__global__ void rope_kv_write_kernel(const TS* __restrict__ src, int src_stride, int n_parts, size_t part_stride,
-                                     T* __restrict__ q_out, const int32_t* __restrict__ positions,
-                                     const int32_t* __restrict__ req_of_token, const float* __restrict__ inv_freq,
-                                     T* __restrict__ k_pool, T* __restrict__ v_pool,
-                                     const int32_t* __restrict__ block_table, int table_width, int page_size,
+__global__ void rope_kv_write_kernel(const TS* src, int src_stride, int n_parts, size_t part_stride,
+                                     T* q_out, const int32_t* positions,
+                                     const int32_t* req_of_token, const float* __restrict__ inv_freq,
+                                     T* k_pool, T* v_pool,
+                                     const int32_t* block_table, int table_width, int page_size,
                                      int num_pages, int nh, int g, int hs, int32_t* bad_page) {
   pdl_launch_dependents();
   pdl_wait();
@@ -740,11 +739,11 @@ __global__ void rope_kv_write_kernel(const TS* __restrict__ src, int src_stride,
 // The same for steps with many tokens: one block per token walks all heads, with the token's
 // cosines and sines computed once in shared memory.
 template <typename T, typename TS>
-__global__ void rope_kv_write_token_kernel(const TS* __restrict__ src, int src_stride, int n_parts, size_t part_stride,
-                                           T* __restrict__ q_out, const int32_t* __restrict__ positions,
-                                           const int32_t* __restrict__ req_of_token,
-                                           const float* __restrict__ inv_freq, T* __restrict__ k_pool,
-                                           T* __restrict__ v_pool, const int32_t* __restrict__ block_table,
+__global__ void rope_kv_write_token_kernel(const TS* src, int src_stride, int n_parts, size_t part_stride,
+                                           T* q_out, const int32_t* positions,
+                                           const int32_t* req_of_token,
+                                           const float* __restrict__ inv_freq, T* k_pool,
+                                           T* v_pool, const int32_t* block_table,
                                            int table_width, int page_size, int num_pages, int nh, int g, int hs,
                                            int32_t* bad_page) {
   extern __shared__ float cs[];   // cos[hs/2], sin[hs/2]
@@ -803,11 +802,11 @@ __global__ void rope_kv_write_token_kernel(const TS* __restrict__ src, int src_s
 // The per-token kernel for head sizes that are multiples of 8 and 16-byte aligned rows: a thread
 // rotates four pairs at once (8- or 16-byte loads and stores).
 template <typename T, typename TS>
-__global__ void rope_kv_write_token_vec_kernel(const TS* __restrict__ src, int src_stride, int n_parts, size_t part_stride,
-                                               T* __restrict__ q_out, const int32_t* __restrict__ positions,
-                                               const int32_t* __restrict__ req_of_token,
-                                               const float* __restrict__ inv_freq, T* __restrict__ k_pool,
-                                               T* __restrict__ v_pool, const int32_t* __restrict__ block_table,
+__global__ void rope_kv_write_token_vec_kernel(const TS* src, int src_stride, int n_parts, size_t part_stride,
+                                               T* q_out, const int32_t* positions,
+                                               const int32_t* req_of_token,
+                                               const float* __restrict__ inv_freq, T* k_pool,
+                                               T* v_pool, const int32_t* block_table,
                                                int table_width, int page_size, int num_pages, int nh, int g, int hs,
                                                int32_t* bad_page) {
   extern __shared__ __align__(16) float cs[];   // cos[hs/2], sin[hs/2]
@@ -923,7 +922,7 @@ YALIS_API int yalis_rope_kv_write(const void* src, int src_dtype, int src_stride
 // gate0, up0, gate1, up1, ... when interleaved == 1 (the reference's layout).
 // --------------------------------------------------------------------------
 template <typename T>
-__global__ void silu_mul_kernel(const T* __restrict__ in, T* __restrict__ out, int inter, int interleaved,
+__global__ void silu_mul_kernel(const T* in, T* out, int inter, int interleaved,
                                 size_t total) {
   pdl_launch_dependents();
   pdl_wait();
@@ -954,7 +953,7 @@ __device__ __forceinline__ uint4 silu_mul_8(const uint4 g4, const uint4 u4) {
   return o4;
 }
 
-__global__ void silu_mul_bf16x8_kernel(const __nv_bfloat16* __restrict__ in, __nv_bfloat16* __restrict__ out,
+__global__ void silu_mul_bf16x8_kernel(const __nv_bfloat16* in, __nv_bfloat16* out,
                                        int inter, size_t total_vec) {
   pdl_launch_dependents();
   pdl_wait();
@@ -999,8 +998,8 @@ YALIS_API int yalis_silu_mul(const void* in, void* out, int dtype, int n_tokens,
 }
 
 // Gather rows of a float32 matrix: out[i, :] = x[rows[i], :].
-__global__ void gather_rows_kernel(const float* __restrict__ x, const int32_t* __restrict__ rows,
-                                   float* __restrict__ out, int width) {
+__global__ void gather_rows_kernel(const float* x, const int32_t* rows,
+                                   float* out, int width) {
   pdl_launch_dependents();
   pdl_wait();
   const int r = rows[blockIdx.x];

@@ -26,7 +26,7 @@ constexpr int kMaxTop = 32;
 // weights are the chosen scores, divided by their sum + eps unless eps < 0, times `factor`.
 template <typename F>
 __device__ __forceinline__ void choose_experts_sigmoid(F logit, int E, int top, float eps, float factor, int lane,
-                                                       int32_t* __restrict__ ids, float* __restrict__ weights) {
+                                                       int32_t* ids, float* weights) {
   constexpr int kPer = kMaxExperts / 32;
   float s[kPer];
 #pragma unroll
@@ -72,7 +72,7 @@ __device__ __forceinline__ void choose_experts_sigmoid(F logit, int E, int top, 
 // The choice of one token by one warp: softmax over `logit(e)`, the `top` largest, renormalised.
 template <typename F>
 __device__ __forceinline__ void choose_experts(F logit, int E, int top, float eps, float factor, int lane,
-                                               int32_t* __restrict__ ids, float* __restrict__ weights, int sigmoid = 0) {
+                                               int32_t* ids, float* weights, int sigmoid = 0) {
   if (sigmoid) {
     choose_experts_sigmoid(logit, E, top, eps, factor, lane, ids, weights);
     return;
@@ -149,8 +149,8 @@ struct ChoiceRules {
 // sigmoid of each; ties go to the smaller index, among groups too.  kPer: outputs a lane holds (32 kPer >= E).
 template <int kPer>
 __device__ __forceinline__ void choose_experts_by_rules(float* z, float* gs, const ChoiceRules& rules, int E, int top, float eps,
-                                                        float factor, int lane, int32_t* __restrict__ ids,
-                                                        float* __restrict__ weights, float* __restrict__ identity, int sigmoid) {
+                                                        float factor, int lane, int32_t* ids,
+                                                        float* weights, float* identity, int sigmoid) {
   float s[kPer], c[kPer];                // scores and choice scores
   if (sigmoid) {
 #pragma unroll
@@ -243,9 +243,9 @@ __device__ __forceinline__ void choose_experts_by_rules(float* z, float* gs, con
 }
 
 // From given logits: one warp per token.
-__global__ void route_topk_kernel(const float* __restrict__ logits, int E, int top, float eps, float factor,
-                                  const int32_t* __restrict__ req_of_token, int32_t* __restrict__ ids,
-                                  float* __restrict__ weights, int n_tokens, int sigmoid) {
+__global__ void route_topk_kernel(const float* logits, int E, int top, float eps, float factor,
+                                  const int32_t* req_of_token, int32_t* ids,
+                                  float* weights, int n_tokens, int sigmoid) {
   pdl_launch_dependents();
   pdl_wait();
   const int n = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
@@ -278,10 +278,10 @@ __device__ __forceinline__ void load4(const __nv_bfloat16* p, float& a, float& b
 // the experts, and a row of the router read once serves all TOK tokens (each token's sum has the same order whatever
 // TOK is); then warp t chooses for token t.
 template <typename T, int TOK, bool RULES>
-__global__ void __launch_bounds__(512) route_kernel(const T* __restrict__ x, long x_stride, const float* __restrict__ w, int E, int K, int top,
-                             float eps, float factor, const int32_t* __restrict__ req_of_token, int32_t* __restrict__ ids,
-                             float* __restrict__ weights, int n_tokens, int sigmoid, const float* __restrict__ side,
-                             float* __restrict__ side_out, const ChoiceRules rules) {
+__global__ void __launch_bounds__(512) route_kernel(const T* x, long x_stride, const float* __restrict__ w, int E, int K, int top,
+                             float eps, float factor, const int32_t* req_of_token, int32_t* ids,
+                             float* weights, int n_tokens, int sigmoid, const float* __restrict__ side,
+                             float* side_out, const ChoiceRules rules) {
   // [TOK][K] rows (T), then [TOK][E] logits and [TOK][groups] group scores (float)
   extern __shared__ __align__(16) unsigned char route_smem[];
   T* xs = reinterpret_cast<T*>(route_smem);
@@ -416,9 +416,9 @@ int launch_route(const void* x, long x_stride, const float* w, int n_tokens, int
 }
 
 // One block.  entries = n_tokens * top.  tiles: (expert, first slot) per row tile of `bm` slots, ended by n_tiles.
-__global__ void expert_plan_kernel(const int32_t* __restrict__ ids, int entries, int E, int bm, int32_t* __restrict__ offsets,
-                                   int32_t* __restrict__ perm, int32_t* __restrict__ inv, int32_t* __restrict__ tile_expert,
-                                   int32_t* __restrict__ tile_slot, int32_t* __restrict__ n_tiles) {
+__global__ void expert_plan_kernel(const int32_t* ids, int entries, int E, int bm, int32_t* offsets,
+                                   int32_t* perm, int32_t* inv, int32_t* tile_expert,
+                                   int32_t* tile_slot, int32_t* n_tiles) {
   __shared__ int count[kMaxExperts], start[kMaxExperts + 1], tile0[kMaxExperts + 1];
   pdl_launch_dependents();
   pdl_wait();
@@ -466,8 +466,8 @@ __global__ void expert_plan_kernel(const int32_t* __restrict__ ids, int entries,
 
 // xg[slot, :] = x[perm[slot] / top, :] for the slots in use (16-byte pieces): the rows of every expert side by side,
 // as a product that reads its rows as one box needs them.
-__global__ void gather_rows_kernel(const uint4* __restrict__ x, long x_stride16, const int32_t* __restrict__ perm, int top,
-                                   const int32_t* __restrict__ offsets, int E, uint4* __restrict__ out, int cols16) {
+__global__ void gather_rows_kernel(const uint4* x, long x_stride16, const int32_t* perm, int top,
+                                   const int32_t* offsets, int E, uint4* out, int cols16) {
   pdl_launch_dependents();
   pdl_wait();
   const int slot = blockIdx.x;
@@ -479,9 +479,9 @@ __global__ void gather_rows_kernel(const uint4* __restrict__ x, long x_stride16,
 // xg[slot, :] = x[perm[slot] / top, :] * weights[perm[slot]] in any dtype: the rows of every expert side by side,
 // each times the weight of its (token, choice) entry (weights null: 1), float32 product, one rounding.
 template <typename T>
-__global__ void gather_scale_rows_kernel(const T* __restrict__ x, long x_stride, const int32_t* __restrict__ perm, int top,
-                                         const float* __restrict__ weights, const int32_t* __restrict__ offsets, int E,
-                                         T* __restrict__ out, int cols) {
+__global__ void gather_scale_rows_kernel(const T* x, long x_stride, const int32_t* perm, int top,
+                                         const float* weights, const int32_t* offsets, int E,
+                                         T* out, int cols) {
   pdl_launch_dependents();
   pdl_wait();
   const int slot = blockIdx.x;
@@ -493,9 +493,9 @@ __global__ void gather_scale_rows_kernel(const T* __restrict__ x, long x_stride,
 }
 
 // The same for bfloat16 rows on 16-byte boundaries, eight columns a thread (same product and rounding per element).
-__global__ void gather_scale_rows_bf16x8_kernel(const uint4* __restrict__ x, long x_stride16, const int32_t* __restrict__ perm,
-                                                int top, const float* __restrict__ weights, const int32_t* __restrict__ offsets,
-                                                int E, uint4* __restrict__ out, int cols16) {
+__global__ void gather_scale_rows_bf16x8_kernel(const uint4* x, long x_stride16, const int32_t* perm,
+                                                int top, const float* weights, const int32_t* offsets,
+                                                int E, uint4* out, int cols16) {
   pdl_launch_dependents();
   pdl_wait();
   const int slot = blockIdx.x;
@@ -711,10 +711,10 @@ int launch_grouped_mma(const GroupedArgs& g, int max_tiles, cudaStream_t stream)
 
 // out[n, :] = sum_j weights[n, j] * y[inv[n * top + j], :] + shared[n, :]
 template <typename T>
-__global__ void expert_combine_kernel(const T* __restrict__ y, long y_stride, const int32_t* __restrict__ inv,
-                                      const float* __restrict__ weights, int top, const T* __restrict__ shared,
-                                      long shared_stride, T* __restrict__ out, long out_stride, int cols,
-                                      const float* __restrict__ shared_scale) {
+__global__ void expert_combine_kernel(const T* y, long y_stride, const int32_t* inv,
+                                      const float* weights, int top, const T* shared,
+                                      long shared_stride, T* out, long out_stride, int cols,
+                                      const float* shared_scale) {
   pdl_launch_dependents();
   pdl_wait();
   const int n = blockIdx.x;
@@ -730,10 +730,10 @@ __global__ void expert_combine_kernel(const T* __restrict__ y, long y_stride, co
 }
 
 // The same for bfloat16 rows on 16-byte boundaries: 8 columns a thread, the same order of sums per column.
-__global__ void expert_combine_bf16x8_kernel(const __nv_bfloat16* __restrict__ y, long y_stride, const int32_t* __restrict__ inv,
-                                             const float* __restrict__ weights, int top, const __nv_bfloat16* __restrict__ shared,
-                                             long shared_stride, __nv_bfloat16* __restrict__ out, long out_stride, int cols,
-                                             const float* __restrict__ shared_scale) {
+__global__ void expert_combine_bf16x8_kernel(const __nv_bfloat16* y, long y_stride, const int32_t* inv,
+                                             const float* weights, int top, const __nv_bfloat16* shared,
+                                             long shared_stride, __nv_bfloat16* out, long out_stride, int cols,
+                                             const float* shared_scale) {
   pdl_launch_dependents();
   pdl_wait();
   const int n = blockIdx.x, c = (blockIdx.y * blockDim.x + threadIdx.x) * 8;

@@ -29,7 +29,6 @@ constexpr int kGroups = 4;
 template <typename TA, typename TW, typename TO, int BM, int BN, int TM, int TN, bool VEC>
 __global__ void __launch_bounds__(kGroups * (BM / TM) * (BN / TN), 2)
 gemm_tn_simt_kernel(const TA* A, long long lda, const TW* W, long long ldw, TO* O, long long ldo, int M, int N, int K) {
-  // (No __restrict__: a load the compiler takes for one of constant data may be moved above the wait for the kernel before.)
   constexpr int BK = 32, KG = BK / kGroups, PER = (BM / TM) * (BN / TN), THREADS = kGroups * PER, TX = BN / TN;
   constexpr int LA = BM + 4, LW = BN + 4;                  // padded rows: the transposed stores spread over the banks
   constexpr int NA = BM * BK / 4 / THREADS, NW = BN * BK / 4 / THREADS;      // groups of four k values a thread loads

@@ -12,6 +12,8 @@
 // sigmoid gate on the result; large bfloat16 steps use the library's batched product and `sigmoid_gate` instead),
 // and the attention itself in two forms: an exact one (float32 path, twin of the other) and a tensor-core one
 // (bfloat16 pages).  Scores, weights and sums are float32 in every form.
+#include <type_traits>
+
 #include "common.cuh"
 
 
@@ -43,7 +45,7 @@ struct LatentPrep {
 // The first rot_dims of src[0..p) turned by position * inv_freq (pairs (2i, 2i+1) or (i, i + rot_dims / 2)),
 // the rest copied.  One warp.
 template <typename T, typename TO>
-__device__ __forceinline__ void rotate_part(const T* __restrict__ src, TO* __restrict__ dst, int p, int pos,
+__device__ __forceinline__ void rotate_part(const T* src, TO* dst, int p, int pos,
                                             const LatentPrep& a, int lane) {
   const int half = a.inv_freq ? a.rot_dims >> 1 : 0;
   for (int i = lane; i < half; i += 32) {
@@ -98,14 +100,17 @@ __global__ void latent_prepare_kernel(const LatentPrep a) {
 
 // y[n, :] = x[n, :] / sqrt(mean(x[n, :]^2) + eps) * w for a column block x [N, width] of a wider matrix (the normed
 // latent that queries pass through).  A warp per row; float32 arithmetic, one rounding.
+// (Results up to sixteen at a time, fetched before the first is stored: a load behind each store took 12 us for 2,048 columns
+// instead of 5.)
 template <typename T>
-__global__ void norm_rows_kernel(const T* __restrict__ x, long x_stride, const float* __restrict__ w, float eps, int width,
-                                 T* __restrict__ y, long y_stride, int n_rows) {
+__global__ void norm_rows_kernel(const T* x, long x_stride, const float* __restrict__ w, float eps, int width,
+                                 T* y, long y_stride, int n_rows) {
   pdl_launch_dependents();
   pdl_wait();
   const int n = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (n >= n_rows) return;
   const T* s = x + (size_t)n * x_stride;
+  T* out = y + (size_t)n * y_stride;
   float ss = 0.f;
   for (int i = lane; i < width; i += 32) {
     const float v = to_f32<T>(s[i]);
@@ -113,16 +118,28 @@ __global__ void norm_rows_kernel(const T* __restrict__ x, long x_stride, const f
   }
   ss = warp_sum(ss);
   const float inv = 1.0f / sqrtf(ss / (float)width + eps);
-  for (int i = lane; i < width; i += 32) y[(size_t)n * y_stride + i] = from_f32<T>(to_f32<T>(s[i]) * inv * w[i]);
+  auto columns = [&](auto batch, int i) {         // columns i, i + 32, ...
+    constexpr int B = decltype(batch)::value;
+    T v[B];
+#pragma unroll
+    for (int j = 0; j < B; ++j) v[j] = s[i + 32 * j];
+#pragma unroll
+    for (int j = 0; j < B; ++j) out[i + 32 * j] = from_f32<T>(to_f32<T>(v[j]) * inv * w[i + 32 * j]);
+  };
+  int i = lane;
+  for (; i + 32 * 15 < width; i += 32 * 16) columns(std::integral_constant<int, 16>{}, i);
+  for (; i + 32 * 7 < width; i += 32 * 8) columns(std::integral_constant<int, 8>{}, i);
+  for (; i + 32 * 3 < width; i += 32 * 4) columns(std::integral_constant<int, 4>{}, i);
+  for (; i < width; i += 32) columns(std::integral_constant<int, 1>{}, i);
 }
 
 // ---- per-head linear maps -------------------------------------------------------------------------------------
 // out[n, h, o] = sum_k w[h, o, k] x[n, h, k]   (optionally times sigmoid(gate[n, h * O + o])), float32 sums in k
 // order per lane and a fixed butterfly across lanes.  Block (n, h); a warp per output.
 template <typename T, typename TX, typename TO>
-__global__ void head_project_kernel(const TX* __restrict__ x, long xs_n, long xs_h, const T* __restrict__ w, int O, int K,
-                                    TO* __restrict__ out, long os_n, long os_h, const T* __restrict__ gate, long gs_n,
-                                    const int32_t* __restrict__ req_of_token) {
+__global__ void head_project_kernel(const TX* x, long xs_n, long xs_h, const T* __restrict__ w, int O, int K,
+                                    TO* out, long os_n, long os_h, const T* gate, long gs_n,
+                                    const int32_t* req_of_token) {
   extern __shared__ float xs[];
   pdl_launch_dependents();
   pdl_wait();
@@ -173,8 +190,8 @@ __global__ void sigmoid_gate_x4_kernel(const TX* x, long xs_n, long xs_h, int e,
 // y[n, h * e + c] = x[n, h, c] * sigmoid(g[n, h * e + c])  (x float32 or model dtype with strides over n and h,
 // y and g model dtype)
 template <typename T, typename TX>
-__global__ void sigmoid_gate_kernel(const TX* __restrict__ x, long xs_n, long xs_h, int e, const T* __restrict__ g, long gs,
-                                    T* __restrict__ y, long ys, int rows, int cols) {
+__global__ void sigmoid_gate_kernel(const TX* x, long xs_n, long xs_h, int e, const T* g, long gs,
+                                    T* y, long ys, int rows, int cols) {
   pdl_launch_dependents();
   pdl_wait();
   const size_t total = (size_t)rows * cols;
@@ -192,10 +209,10 @@ constexpr int kMaxPerLane = 20;   // r + p <= 640
 // Block (token, head).  Each warp walks every fourth visible row in ascending order with an online softmax; the
 // four partial results are merged in warp order, so a (position, head) has one order of sums whatever the step.
 template <typename T>
-__global__ void latent_attention_exact_kernel(const float* __restrict__ qc, float* __restrict__ out,
-                                              const T* __restrict__ pool, const int32_t* __restrict__ positions,
-                                              const int32_t* __restrict__ req_of_token,
-                                              const int32_t* __restrict__ block_table, int table_width, int page_size,
+__global__ void latent_attention_exact_kernel(const float* qc, float* out,
+                                              const T* pool, const int32_t* positions,
+                                              const int32_t* req_of_token,
+                                              const int32_t* block_table, int table_width, int page_size,
                                               int num_pages, int heads, int r, int p, float scale, int window,
                                               const float* __restrict__ sink) {
   extern __shared__ float smem[];   // [kWarps][r] sums, then m[kWarps], l[kWarps]
@@ -587,7 +604,6 @@ __global__ void __launch_bounds__(128 * WR) latent_attention_mma_kernel(const La
 // 128 columns: lane z weighs share z, then every lane adds the shares of its four columns in the order of z, all of them
 // requested before the first is added (what bounds the kernel is that trip to the L2: a warp per row and a column at a time
 // took 22 us for 128 rows of 16 shares).
-// (No __restrict__: a load the compiler takes for one of constant data may be moved above the wait for the kernel before.)
 __global__ void latent_merge_kernel(const float* part_o, const float* part_ml, int n_splits, int n_tokens, int heads, int r,
                                     const int32_t* req_of_token, void* out, int out_bf16, long o_n, long o_h,
                                     const float* sink) {

@@ -554,7 +554,7 @@ int launch_qkv_prepare(const PrepParams& p, dim3 grid, int warps, bool table, bo
 // ACT: 0 gelu with erf, 1 gelu with tanh, 2 silu, 3 the square of relu, 4 tanh.
 // With `bias` (float32, one per column) it is added to x first.  TO: the result's type (T, or float32).
 template <typename T, typename TO>
-__global__ void activation_kernel(const T* __restrict__ x, int x_stride, TO* __restrict__ y, int y_stride, int rows,
+__global__ void activation_kernel(const T* x, int x_stride, TO* y, int y_stride, int rows,
                                   int cols, int act, const float* __restrict__ bias) {
   pdl_launch_dependents();
   pdl_wait();
@@ -583,7 +583,7 @@ __device__ __forceinline__ float act_value(float z, int act) {
   return silu_exact(z);
 }
 
-__global__ void activation_bf16x8_kernel(const __nv_bfloat16* __restrict__ x, int x_stride, __nv_bfloat16* __restrict__ y,
+__global__ void activation_bf16x8_kernel(const __nv_bfloat16* x, int x_stride, __nv_bfloat16* y,
                                          int y_stride, int cols, int act, const float* __restrict__ bias) {
   pdl_launch_dependents();
   pdl_wait();
@@ -609,7 +609,7 @@ __global__ void activation_bf16x8_kernel(const __nv_bfloat16* __restrict__ x, in
 // reader may be a kernel of few, long blocks (a recurrence over the rows it makes): those are let in only once this one
 // has begun, so that they do not crowd onto the SMs that come free first.
 template <typename T>
-__global__ void activation_f32x4_kernel(const T* __restrict__ x, int x_stride, float* __restrict__ y, int y_stride, int rows,
+__global__ void activation_f32x4_kernel(const T* x, int x_stride, float* y, int y_stride, int rows,
                                         int cols, int act, const float* __restrict__ bias) {
   pdl_wait();
   pdl_launch_dependents();
@@ -632,7 +632,7 @@ __global__ void activation_f32x4_kernel(const T* __restrict__ x, int x_stride, f
 //   kind 1:  g <- min(g, limit), u <- clamp(u, -limit, limit);  y = g * sigmoid(alpha * g) * (u + shift)
 // float32 arithmetic, one rounding.
 template <typename T>
-__global__ void gated_activation_kernel(const T* __restrict__ x, long x_stride, int gate_off, int up_off, T* __restrict__ y,
+__global__ void gated_activation_kernel(const T* x, long x_stride, int gate_off, int up_off, T* y,
                                         long y_stride, int rows, int cols, int kind, float limit, float alpha, float shift) {
   pdl_launch_dependents();
   pdl_wait();
@@ -655,8 +655,8 @@ __global__ void gated_activation_kernel(const T* __restrict__ x, long x_stride, 
 // The same, eight elements a thread, for bfloat16 rows whose two parts and whose results start on 16-byte boundaries
 // (width and both offsets multiples of 8).  The result is rounded to 8 bits of mantissa at once, so the fast
 // exponential and division do not show.  grid: (ceil(cols / 8 / 128), rows).
-__global__ void gated_activation_bf16x8_kernel(const __nv_bfloat16* __restrict__ x, long x_stride, int gate_off, int up_off,
-                                               __nv_bfloat16* __restrict__ y, long y_stride, int cols, int kind, float limit,
+__global__ void gated_activation_bf16x8_kernel(const __nv_bfloat16* x, long x_stride, int gate_off, int up_off,
+                                               __nv_bfloat16* y, long y_stride, int cols, int kind, float limit,
                                                float alpha, float shift) {
   pdl_launch_dependents();
   pdl_wait();
@@ -684,8 +684,8 @@ __global__ void gated_activation_bf16x8_kernel(const __nv_bfloat16* __restrict__
 }
 
 // x[n, :] += other[n, :] + vec[:]   (either may be absent)
-__global__ void add_rows_vector_kernel(float* __restrict__ x, const float* __restrict__ other,
-                                       const float* __restrict__ vec, int rows, int cols) {
+__global__ void add_rows_vector_kernel(float* x, const float* other,
+                                       const float* vec, int rows, int cols) {
   pdl_launch_dependents();
   pdl_wait();
   const size_t total = (size_t)rows * cols;

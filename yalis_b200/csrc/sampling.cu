@@ -56,11 +56,11 @@ __device__ __forceinline__ float uniform_open(uint32_t x) { return ((float)(x >>
 // flight at once: one block walking a wide row is bound by load latency otherwise.  Which thread
 // sees which entry is unspecified; every entry is seen exactly once by the block.
 template <class F>
-__device__ __forceinline__ void for_each_entry(const float* __restrict__ row, int n, F f) {
+__device__ __forceinline__ void for_each_entry(const float* row, int n, F f) {
   const int step = blockDim.x;
   int done = 0;
   if ((reinterpret_cast<uintptr_t>(row) & 15u) == 0) {
-    const float4* __restrict__ row4 = reinterpret_cast<const float4*>(row);
+    const float4* row4 = reinterpret_cast<const float4*>(row);
     const int n4 = n >> 2;
     constexpr int U = 4;
     int i = threadIdx.x;
@@ -131,8 +131,8 @@ __device__ ArgMax block_argmax(ArgMax a, ArgMax* scratch) {
 // A chosen token goes to out[row] and, when `scatter_index` is given and not negative for the row, also to
 // scatter[scatter_index[row]]: the engine keeps each request's last chosen token in a per-slot array on the
 // device, from which the next step can take its input without the host in between.
-__device__ __forceinline__ void put_choice(int row, int token, int32_t* __restrict__ out,
-                                           const int32_t* __restrict__ scatter_index, int32_t* __restrict__ scatter) {
+__device__ __forceinline__ void put_choice(int row, int token, int32_t* out,
+                                           const int32_t* scatter_index, int32_t* scatter) {
   out[row] = token;
   if (scatter_index != nullptr) {
     const int where = scatter_index[row];
@@ -140,10 +140,10 @@ __device__ __forceinline__ void put_choice(int row, int token, int32_t* __restri
   }
 }
 
-__global__ void __launch_bounds__(kThreads) argmax_kernel(const float* __restrict__ logits, long long row_stride,
-                                                          int vocab, int32_t* __restrict__ out,
-                                                          const int32_t* __restrict__ scatter_index,
-                                                          int32_t* __restrict__ scatter) {
+__global__ void __launch_bounds__(kThreads) argmax_kernel(const float* logits, long long row_stride,
+                                                          int vocab, int32_t* out,
+                                                          const int32_t* scatter_index,
+                                                          int32_t* scatter) {
   __shared__ ArgMax scratch[32];
   pdl_launch_dependents();
   pdl_wait();
@@ -279,9 +279,9 @@ struct Found {
 // normaliser is summed block by block in rank order.
 template <int CL>
 __global__ void __launch_bounds__(kThreads)
-sample_cut_kernel(const float* __restrict__ logits, long long row_stride, int vocab,
-                  const float* __restrict__ temperature, const int32_t* __restrict__ top_k,
-                  const float* __restrict__ top_p, Cut* __restrict__ cuts) {
+sample_cut_kernel(const float* logits, long long row_stride, int vocab,
+                  const float* temperature, const int32_t* top_k,
+                  const float* top_p, Cut* cuts) {
   extern __shared__ unsigned long long hist[];          // [kBins] 64-bit bins (leading block), then [3][kBins] 32-bit pieces
   __shared__ float fscratch[32];
   __shared__ unsigned long long warp_totals[32];
@@ -489,11 +489,11 @@ sample_cut_kernel(const float* __restrict__ logits, long long row_stride, int vo
 constexpr int kDrawChunks = 32;
 
 __global__ void __launch_bounds__(kThreads)
-sample_draw_partial_kernel(const float* __restrict__ logits, long long row_stride, int vocab,
-                           const float* __restrict__ temperature, const float* __restrict__ top_p,
-                           const unsigned long long* __restrict__ seed,
-                           const unsigned long long* __restrict__ draw_index, const Cut* __restrict__ cuts,
-                           float* __restrict__ part_v, int32_t* __restrict__ part_i) {
+sample_draw_partial_kernel(const float* logits, long long row_stride, int vocab,
+                           const float* temperature, const float* top_p,
+                           const unsigned long long* seed,
+                           const unsigned long long* draw_index, const Cut* cuts,
+                           float* part_v, int32_t* part_i) {
   __shared__ ArgMax scratch[32];
   pdl_launch_dependents();
   pdl_wait();
@@ -540,9 +540,9 @@ constexpr int kCutBlocks = 8;       // most blocks per row of the cut search (on
 constexpr int kCutClusterVocab = 16384;
 
 // Phase 1 of the wide argmax: block (row, chunk) finds the best entry of its slice.
-__global__ void __launch_bounds__(kThreads) argmax_partial_kernel(const float* __restrict__ logits, long long row_stride,
-                                                                  int vocab, float* __restrict__ part_v,
-                                                                  int32_t* __restrict__ part_i) {
+__global__ void __launch_bounds__(kThreads) argmax_partial_kernel(const float* logits, long long row_stride,
+                                                                  int vocab, float* part_v,
+                                                                  int32_t* part_i) {
   __shared__ ArgMax scratch[32];
   pdl_launch_dependents();
   pdl_wait();
@@ -566,9 +566,9 @@ __global__ void __launch_bounds__(kThreads) argmax_partial_kernel(const float* _
 }
 
 // Phase 2: one warp per row merges the slices (ties still go to the lowest index).
-__global__ void argmax_merge_kernel(const float* __restrict__ part_v, const int32_t* __restrict__ part_i,
-                                    int32_t* __restrict__ out, const int32_t* __restrict__ scatter_index,
-                                    int32_t* __restrict__ scatter) {
+__global__ void argmax_merge_kernel(const float* part_v, const int32_t* part_i,
+                                    int32_t* out, const int32_t* scatter_index,
+                                    int32_t* scatter) {
   pdl_launch_dependents();
   pdl_wait();
   ArgMax a;

@@ -267,12 +267,12 @@ int launch_rms(const StreamStep& a, int count, cudaStream_t stream) {
 
 // x[n, :] += table[row(n), :] for every token of a request (float32 stream of one copy).
 template <typename T>
-__global__ void pair_rows_add_kernel(float* __restrict__ x, int width, const T* __restrict__ table, int buckets,
-                                     long long mul_prev, long long mul_cur, const int32_t* __restrict__ ids,
-                                     const int32_t* __restrict__ from_slot, const int32_t* __restrict__ chosen,
-                                     const int32_t* __restrict__ positions, const int32_t* __restrict__ req_of_token,
-                                     const int32_t* __restrict__ q_start, const int32_t* __restrict__ slots,
-                                     const int32_t* __restrict__ last_token, int vocab) {
+__global__ void pair_rows_add_kernel(float* x, int width, const T* __restrict__ table, int buckets,
+                                     long long mul_prev, long long mul_cur, const int32_t* ids,
+                                     const int32_t* from_slot, const int32_t* chosen,
+                                     const int32_t* positions, const int32_t* req_of_token,
+                                     const int32_t* q_start, const int32_t* slots,
+                                     const int32_t* last_token, int vocab) {
   pdl_launch_dependents();
   pdl_wait();
   const int n = blockIdx.x;
@@ -297,9 +297,9 @@ __global__ void pair_rows_add_kernel(float* __restrict__ x, int width, const T* 
 }
 
 // last_token[slot of request] = the last token the request brought in this step.
-__global__ void remember_last_tokens_kernel(const int32_t* __restrict__ ids, const int32_t* __restrict__ from_slot,
-                                            const int32_t* __restrict__ chosen, const int32_t* __restrict__ q_start,
-                                            const int32_t* __restrict__ slots, int n_requests, int32_t* __restrict__ last_token) {
+__global__ void remember_last_tokens_kernel(const int32_t* ids, const int32_t* from_slot,
+                                            const int32_t* chosen, const int32_t* q_start,
+                                            const int32_t* slots, int n_requests, int32_t* last_token) {
   pdl_launch_dependents();
   pdl_wait();
   const int r = blockIdx.x * blockDim.x + threadIdx.x;
