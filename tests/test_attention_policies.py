@@ -3,6 +3,8 @@ get a kernel of their own, and how the keys of prompt tiles are divided among bl
 step's lengths; the times quoted are measurements on a B200 (profiles/), the assertions say which of the
 measured options the choice must be."""
 
+import gc
+import weakref
 from types import SimpleNamespace
 
 import pytest
@@ -100,3 +102,18 @@ def test_model_of_the_prompt_kernels_launch():
     halves = attn._prefill_step_length(items + [(100, 1.0)], 37, 2, 50)
     assert one_round < halves < 2 * one_round                                                     # 76 halves: three short rounds
     assert attn._prefill_step_length([(300, 1.4)] + [(10, 1.0)] * 30, 37, 1, 1) == 300 * 1.4 + attn.PREFILL_SPLIT_START_UP
+
+
+def test_counters_that_a_recording_may_use_stay_when_a_larger_step_comes(monkeypatch):
+    """A recorded step points to the buffer of its time: it has to outlive the buffer that replaces it."""
+    monkeypatch.setattr(attn, "_ticket_cache", {})
+    monkeypatch.setattr(attn, "_replaced_tickets", [])
+    first = attn._tickets("cpu", 600)
+    recorded, size = weakref.ref(first), first.numel()
+    del first
+    for n in (size + 1, 3 * size, 5 * size):
+        assert attn._tickets("cpu", n).numel() >= n
+    gc.collect()
+    assert recorded() is not None and attn._tickets("cpu", 1).data_ptr() != recorded().data_ptr()
+    # what is kept stays below the size of the buffer in use
+    assert sum(t.numel() for t in attn._replaced_tickets) < attn._tickets("cpu", 1).numel()

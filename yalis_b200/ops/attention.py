@@ -234,15 +234,19 @@ def decode_tma_splits(n_requests: int, num_kv_heads: int, long_context: bool) ->
 
 
 _ticket_cache = {}
+_replaced_tickets = []     # smaller buffers of before: recordings point to them, so they stay for as long as the process
 
 
 def _tickets(device, n: int) -> torch.Tensor:
     """Zeroed int32 counters, one per (request, KV head): every split launch leaves them zero,
-    so one buffer per device is allocated once (outside any graph capture) and shared."""
+    so one buffer per device is allocated once (outside any graph capture) and shared.  A step that needs more gets a
+    buffer at least twice as large; the one before is kept, because a recorded step goes on counting in it."""
     key = torch.device(device)
     t = _ticket_cache.get(key)
     if t is None or t.numel() < n:
-        t = _ticket_cache[key] = torch.zeros(max(n, 4096), dtype=torch.int32, device=key)
+        if t is not None:
+            _replaced_tickets.append(t)
+        t = _ticket_cache[key] = torch.zeros(max(n, 4096 if t is None else 2 * t.numel()), dtype=torch.int32, device=key)
     return t
 
 
