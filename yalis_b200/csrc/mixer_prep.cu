@@ -32,10 +32,18 @@ struct PrepParams {
   int nq, nk, dim, vdim;
   int maps;                                  // keys per key/value head, side by side in its cached row [maps * dim] (1: the usual)
   int32_t* bad_page;
+  int32_t* zeroed; int n_zeroed;             // counters of a kernel behind this one, set to zero
   int pool;                                  // P > 0: the warp that stores the last row of a block of P positions stores their mean
   void* pk_pool; void* pv_pool;              // [pages, nk, pool_page_size, dim] and [..., vdim], an entry per block
   const int32_t* pool_table; int pool_table_width, pool_page_size, pool_num_pages;
 };
+
+// Counters for the kernel behind this one: its blocks meet in them, and what they hold before is of no matter.
+__device__ __forceinline__ void zero_counters(const PrepParams& p) {
+  const size_t threads = (size_t)gridDim.x * gridDim.y * blockDim.x;
+  for (size_t i = ((size_t)blockIdx.y * gridDim.x + blockIdx.x) * blockDim.x + threadIdx.x; i < (size_t)p.n_zeroed; i += threads)
+    p.zeroed[i] = 0;
+}
 
 // Where a request's cached row `at` lies in pages of `page_size` rows: its index among the rows of one head, or -1.
 __device__ __forceinline__ long long paged_row(const int32_t* table, int width, int page_size, int num_pages, int nk, int head,
@@ -160,6 +168,7 @@ __global__ void __launch_bounds__(256, 5) qkv_prepare_kernel(const PrepParams p)
   __shared__ float scratch[32];
   pdl_launch_dependents();
   pdl_wait();
+  zero_counters(p);
   const int n = blockIdx.x, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
   const int row_floats = ((p.dim > p.vdim ? p.dim : p.vdim) + 3) & ~3;
   float* xs = xs_all + (size_t)(threadIdx.x >> 5) * row_floats;
@@ -320,6 +329,7 @@ template <typename T, typename TO, int L, int NV>
 __global__ void __launch_bounds__(256) qkv_plain_kernel(const PrepParams p, int n_tokens) {
   pdl_launch_dependents();
   pdl_wait();
+  zero_counters(p);
   const int keys = p.nk * p.maps, heads = p.nq + keys + p.nk;
   const unsigned at = blockIdx.x * (256u / L) + threadIdx.x / L;
   const int n = (int)(at / (unsigned)heads), head = (int)(at - (unsigned)n * heads), sl = threadIdx.x % L;
@@ -399,6 +409,7 @@ __global__ void __launch_bounds__(256) qkv_turn_kernel(const PrepParams p) {
   extern __shared__ __align__(16) float table_s[];  // cosines, then sines
   pdl_launch_dependents();
   pdl_wait();
+  zero_counters(p);
   const int n = blockIdx.x, l = threadIdx.x % L, groups = blockDim.x / L;
   const int req = p.req_of_token[n], pos = p.positions[n];
   if (req < 0) return;
@@ -704,6 +715,7 @@ __global__ void add_rows_vector_kernel(float* x, const float* other,
 // the step are stored.
 // maps > 1 (without pooled blocks): every key/value head has `maps` keys of size dim, which lie side by side in src and in a
 // cached row; nk counts the key/value heads.
+// zeroed: n_zeroed counters that a kernel behind this one on the stream starts from (none: null, 0).
 // out_dtype: the dtype of q_out and of the plain k_out / v_out (pools always have the model dtype `dtype`).
 YALIS_API int yalis_qkv_prepare(const void* src, int dtype, int src_stride, int q_off, int k_off, int v_off,
                                 const void* q_bias, const void* k_bias, const void* v_bias, const float* q_norm,
@@ -715,8 +727,9 @@ YALIS_API int yalis_qkv_prepare(const void* src, int dtype, int src_stride, int 
                                 const int32_t* positions, const int32_t* req_of_token, int n_tokens, int nq, int nk,
                                 int dim, int vdim, int32_t* bad_page, int pool, void* pk_pool, void* pv_pool,
                                 const int32_t* pool_table, int pool_table_width, int pool_page_size, int pool_num_pages,
-                                int single_tokens, int maps, cudaStream_t stream) {
+                                int single_tokens, int maps, int32_t* zeroed, int n_zeroed, cudaStream_t stream) {
   if (n_tokens <= 0) return YALIS_OK;
+  if (n_zeroed < 0 || (n_zeroed > 0 && !zeroed)) return YALIS_ERR_SHAPE;
   if (pool < 0 || (pool > 0 && (!k_pool || !pk_pool || !pv_pool || !pool_table || pool_page_size < 1))) return YALIS_ERR_SHAPE;
   if (dim <= 0 || dim > kMaxHeadDim || vdim <= 0 || vdim > kMaxHeadDim || nq <= 0 || nk <= 0 || maps < 1 ||
       nq + (maps + 1) * nk > 65535 || (maps > 1 && pool > 0))
@@ -733,6 +746,7 @@ YALIS_API int yalis_qkv_prepare(const void* src, int dtype, int src_stride, int 
   p.v_out = v_out; p.v_out_stride = v_out_stride; p.k_pool = k_pool; p.v_pool = v_pool; p.block_table = block_table;
   p.table_width = table_width; p.page_size = page_size; p.num_pages = num_pages; p.positions = positions;
   p.req_of_token = req_of_token; p.nq = nq; p.nk = nk; p.dim = dim; p.vdim = vdim; p.maps = maps; p.bad_page = bad_page;
+  p.zeroed = zeroed; p.n_zeroed = n_zeroed;
   p.pool = single_tokens ? pool : 0;
   p.pk_pool = pk_pool; p.pv_pool = pv_pool; p.pool_table = pool_table; p.pool_table_width = pool_table_width;
   p.pool_page_size = pool_page_size; p.pool_num_pages = pool_num_pages;

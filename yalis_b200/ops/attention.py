@@ -570,6 +570,21 @@ def prefill_attention_tcgen05(q: torch.Tensor, k_pool: torch.Tensor, v_pool: tor
     return out
 
 
+def general_counters(longest: int, n_requests: int, num_kv_heads: int, device) -> torch.Tensor:
+    """Counters for the general form that a step of portions up to ``longest`` tokens takes: memory of the call, for an earlier
+    kernel of the layer to set to zero.  Nothing is shared between calls, so that steps may run on several streams at once and
+    a recording holds its own."""
+    return torch.empty(n_requests * num_kv_heads if longest == 1 else 2, dtype=torch.int32, device=device)
+
+
+def _own_counters(name: str, q: torch.Tensor, counters: Optional[torch.Tensor], n: int) -> torch.Tensor:
+    if counters is None:
+        return torch.zeros(n, dtype=torch.int32, device=q.device)
+    need(counters.is_cuda and counters.dtype == torch.int32 and counters.is_contiguous() and counters.numel() >= n, name,
+         f"counters must be int32, {n} of them")
+    return counters
+
+
 def prefill_general_applies(q: torch.Tensor, out: torch.Tensor, gate: Optional[torch.Tensor], page_size: int, num_heads: int,
                             num_kv_heads: int, head_dim: int, v_head_dim: int, scale: float) -> bool:
     """Whether ``prefill_attention_general`` takes a step: its head and page sizes, and operands on the 16-byte boundaries
@@ -586,10 +601,12 @@ def prefill_attention_general(q: torch.Tensor, k_pool: torch.Tensor, v_pool: tor
                               window: Optional[int] = None, chunk: Optional[int] = None, softcap: Optional[float] = None,
                               sink: bool = False, sink_logits: Optional[torch.Tensor] = None,
                               slopes: Optional[torch.Tensor] = None, gate: Optional[torch.Tensor] = None,
-                              out_scale: float = 1.0, error_flag: Optional[torch.Tensor] = None) -> torch.Tensor:
+                              out_scale: float = 1.0, error_flag: Optional[torch.Tensor] = None,
+                              counters: Optional[torch.Tensor] = None) -> torch.Tensor:
     """``paged_attention_mma`` with ``exact_weights`` for prompt portions, on the tcgen05 tensor cores: the same arguments,
     head sizes 64 and 128 (keys and values alike).  ``out`` may be a column block of a wider matrix; it, ``q`` and a gate per
-    element start on 16-byte boundaries in every row (see ``prefill_general_applies``)."""
+    element start on 16-byte boundaries in every row (see ``prefill_general_applies``).  ``counters``: int32 of this call
+    alone that a launch before it on the stream has set to zero (see ``general_counters``; made here if missing)."""
     name = "prefill_attention_general"
     LAUNCHED["prefill_tcgen05"] += 1
     n, r = q.shape[0], q_start.numel() - 1
@@ -601,13 +618,14 @@ def prefill_attention_general(q: torch.Tensor, k_pool: torch.Tensor, v_pool: tor
     _check_extras(name, q, num_heads, head_dim, chunk, sink, sink_logits, slopes, gate, None)
     need(prefill_general_applies(q, out, gate, k_pool.shape[2], num_heads, num_kv_heads, head_dim, head_dim, scale), name,
          "head_dim 64 or 128, page_size 8..128 (power of two), at most 128 heads per KV head, rows on 16-byte boundaries")
+    counters = _own_counters(name, q, counters, 2)
     check(lib().yalis_prefill_attention_tcgen05_general(
         ptr(q), i32(q.stride(0)), ptr(out), i32(out.stride(0)), ptr(k_pool), ptr(v_pool), ptr(positions), ptr(q_start),
         ptr(block_table), i32(block_table.shape[1]), i32(k_pool.shape[2]), i32(k_pool.shape[0]), i32(n), i32(r),
         i32(max_q_len), i32(num_heads), i32(num_kv_heads), i32(head_dim), f32(scale), i32(window or 0), i32(chunk or 0),
         f32(softcap or 0.0), i32(int(sink)), ptr(sink_logits), ptr(slopes), ptr(gate),
         i32(gate.stride(0) if gate is not None else 0), i32(_per_head(gate, num_heads, head_dim)), f32(out_scale),
-        ptr(_work_counters(q.device)), ptr(error_flag), stream()), name)
+        ptr(counters), ptr(error_flag), stream()), name)
     return out
 
 
@@ -626,10 +644,11 @@ def decode_attention_general(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torc
                              scale: float, out: torch.Tensor, window: Optional[int] = None, chunk: Optional[int] = None,
                              softcap: Optional[float] = None, sink: bool = False, sink_logits: Optional[torch.Tensor] = None,
                              slopes: Optional[torch.Tensor] = None, gate: Optional[torch.Tensor] = None, out_scale: float = 1.0,
-                             error_flag: Optional[torch.Tensor] = None) -> torch.Tensor:
+                             error_flag: Optional[torch.Tensor] = None, counters: Optional[torch.Tensor] = None) -> torch.Tensor:
     """``paged_attention_mma`` with ``exact_weights`` for steps of one token per request, by the kernel that deals the key tiles
     of all requests evenly to a fixed grid (``decode_attention_lean``): the same arguments.  ``out`` may be a column block of a
-    wider matrix (see ``decode_general_applies``)."""
+    wider matrix (see ``decode_general_applies``).  ``counters`` as for ``prefill_attention_general``, one per request and KV
+    head."""
     name = "decode_attention_general"
     LAUNCHED["decode_lean"] += 1
     n, r = q.shape[0], q_start.numel() - 1
@@ -645,13 +664,14 @@ def decode_attention_general(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torc
     floats = lib().yalis_decode_attention_lean_scratch_floats
     floats.restype = ctypes.c_longlong
     scratch = torch.empty(int(floats(i32(blocks), i32(head_dim))), dtype=torch.float32, device=q.device)
+    counters = _own_counters(name, q, counters, r * num_kv_heads)
     check(lib().yalis_decode_attention_lean_general(
         ptr(q), i32(q.stride(0)), ptr(out), i32(out.stride(0)), ptr(k_pool), ptr(v_pool), ptr(positions), ptr(q_start),
         ptr(block_table), i32(block_table.shape[1]), i32(k_pool.shape[2]), i32(k_pool.shape[0]), i32(n), i32(r),
         i32(num_heads), i32(num_kv_heads), i32(head_dim), f32(scale), i32(window or 0), i32(chunk or 0), f32(softcap or 0.0),
         i32(int(sink)), ptr(sink_logits), ptr(slopes), ptr(gate), i32(gate.stride(0) if gate is not None else 0),
-        i32(_per_head(gate, num_heads, head_dim)), f32(out_scale), i32(blocks), ptr(scratch),
-        ptr(_tickets(q.device, r * num_kv_heads)), ptr(error_flag), stream()), name)
+        i32(_per_head(gate, num_heads, head_dim)), f32(out_scale), i32(blocks), ptr(scratch), ptr(counters), ptr(error_flag),
+        stream()), name)
     return out
 
 

@@ -292,7 +292,7 @@ def qkv_prepare(src: torch.Tensor, offsets, nq: int, nk: int, dim: int, vdim: in
                 bad_flag: Optional[torch.Tensor] = None, interleaved: bool = False, q_temperature=None,
                 rot_scale: float = 1.0, norm_all: bool = False, pool: int = 0, pooled_k: Optional[torch.Tensor] = None,
                 pooled_v: Optional[torch.Tensor] = None, pooled_table: Optional[torch.Tensor] = None,
-                single_tokens: bool = False, maps: int = 1):
+                single_tokens: bool = False, maps: int = 1, zeroed: Optional[torch.Tensor] = None):
     """Prepares the heads of a mixer from its input projection ``src`` [N, ...] (model dtype), whose query,
     key and value heads start at the columns ``offsets`` = (q, k, v):
 
@@ -312,7 +312,8 @@ def qkv_prepare(src: torch.Tensor, offsets, nq: int, nk: int, dim: int, vdim: in
     P the means of every block of P positions that a token of the step completes (keys and values as the pages hold
     them, float32 sums in order) are written to entry position // P of ``pooled_k`` [pages, nk, entries, dim] and
     ``pooled_v`` [.., vdim] by ``pooled_table``; ``single_tokens``: no request brings more than one token.  Without
-    pools (q, k, v) are returned as plain matrices in ``out_dtype``."""
+    pools (q, k, v) are returned as plain matrices in ``out_dtype``.  ``zeroed`` (int32) is set to zero besides: counters
+    of the kernel behind this one."""
     name = "qkv_prepare"
     need_cuda(name, src, positions, req_of_token, q_norm, k_norm, inv_freq, k_pool, v_pool, block_table, bad_flag, *biases)
     need(src.dim() == 2 and src.stride(1) == 1, name, "src must be [N, ...] with unit inner stride")
@@ -327,6 +328,7 @@ def qkv_prepare(src: torch.Tensor, offsets, nq: int, nk: int, dim: int, vdim: in
     for w, heads in ((q_norm, nq), (k_norm, nk * maps)):
         need(w is None or (w.dtype == torch.float32 and w.shape == ((heads * dim if norm_all else dim),) and w.is_contiguous()),
              name, "a norm scale must be float32 [dim], or [heads * dim] when the norm is over all heads")
+    need(zeroed is None or (zeroed.is_cuda and zeroed.dtype == torch.int32 and zeroed.is_contiguous()), name, "counters must be int32")
     rot_dims = 0
     if inv_freq is not None:
         need(inv_freq.dtype == torch.float32 and inv_freq.dim() == 1 and inv_freq.is_contiguous()
@@ -374,5 +376,5 @@ def qkv_prepare(src: torch.Tensor, offsets, nq: int, nk: int, dim: int, vdim: in
         i32(table_width), i32(page_size), i32(num_pages), ptr(positions), ptr(req_of_token), i32(n), i32(nq), i32(nk),
         i32(dim), i32(vdim), ptr(bad_flag), i32(pool), ptr(pooled_k if pool else None), ptr(pooled_v if pool else None),
         ptr(pooled_table if pool else None), i32(pooled_width), i32(pooled_page), i32(pooled_pages), i32(int(single_tokens)),
-        i32(maps), stream()), name)
+        i32(maps), ptr(zeroed), i32(zeroed.numel() if zeroed is not None else 0), stream()), name)
     return q_out if paged else (q_out, k_out, v_out)

@@ -372,6 +372,8 @@ class GeneralAttention(Mixer, Projected):
         q_at = self.spans["q_proj"][0]
         k_at = self.spans["k_proj"][0] if self.own_kv else q_at
         v_at = self.spans["v_proj"][0] if "v_proj" in self.spans else k_at
+        longest, splits = self._launch_shape(ctx.host)
+        counters = attn_ops.general_counters(longest, ctx.n_requests, self.g, z.device) if self._tensor_core_form(z.dtype) else None
         pooling = {} if blocks is None else dict(pool=blocks.size, pooled_k=blocks.k, pooled_v=blocks.v, pooled_table=blocks.table,
                                                  single_tokens=ctx.host.max_q_len == 1)
         q = qkv_prepare(z, (q_at, k_at, v_at), self.nh * self.maps, self.g, self.hs, self.vd, ctx.positions, ctx.req_of_token,
@@ -379,7 +381,7 @@ class GeneralAttention(Mixer, Projected):
                         norm_eps=self.norm_eps or 0.0, inv_freq=freq, k_pool=cache.k, v_pool=cache.v, block_table=table,
                         store=cache.writable, bad_flag=ctx.error_flag, interleaved=interleaved,
                         q_temperature=self.q_temperature, rot_scale=magnitude, norm_all=self.norm_all,
-                        maps=self.maps, **pooling)
+                        maps=self.maps, zeroed=counters, **pooling)
         gate = None
         if self.gated:
             a, b = self.spans["g_proj"]
@@ -388,14 +390,14 @@ class GeneralAttention(Mixer, Projected):
                       v_head_dim=self.vd)
         scale_out = self.out_scale if self.difference is None else 1.0 - self.difference[0]
         if self._tensor_core_form(z.dtype):
-            longest, splits = self._launch_shape(ctx.host)
             if (longest * (self.nh // self.g) > 16 and self.difference is None and self.rel is None and blocks is None
                     and attn_ops.prefill_general_applies(q, y, gate, cache.k.shape[2], self.nh, self.g, self.hs, self.vd, self.scale)):
                 # portions with more rows than a decode tile holds (single tokens of the same step ride along)
                 attn_ops.prefill_attention_general(q, cache.k, cache.v, ctx.positions, ctx.q_start, table, longest, self.nh, self.g,
                                                    self.hs, self.scale, y, window=self.window, chunk=self.chunk,
                                                    softcap=self.softcap, sink=self.sink, sink_logits=self.sink_logits,
-                                                   slopes=self.slopes, gate=gate, out_scale=scale_out, error_flag=ctx.error_flag)
+                                                   slopes=self.slopes, gate=gate, out_scale=scale_out, error_flag=ctx.error_flag,
+                                                   counters=counters)
                 return
             if (longest == 1 and self.difference is None and self.rel is None and blocks is None
                     and attn_ops.decode_general_applies(q, y, gate, ctx.n_requests, cache.k.shape[2], self.nh, self.g, self.hs, self.vd,
@@ -403,7 +405,7 @@ class GeneralAttention(Mixer, Projected):
                 attn_ops.decode_attention_general(q, cache.k, cache.v, ctx.positions, ctx.q_start, table, self.nh, self.g, self.hs,
                                                   self.scale, y, window=self.window, chunk=self.chunk, softcap=self.softcap,
                                                   sink=self.sink, sink_logits=self.sink_logits, slopes=self.slopes, gate=gate,
-                                                  out_scale=scale_out, error_flag=ctx.error_flag)
+                                                  out_scale=scale_out, error_flag=ctx.error_flag, counters=counters)
                 return
             direct = y.data_ptr() % 16 == 0 and y.stride(0) % 2 == 0
             out = attn_ops.paged_attention_mma(q, cache.k, cache.v, ctx.positions, ctx.q_start, ctx.req_of_token, table, longest,
