@@ -40,7 +40,8 @@ gemm_tn_simt_kernel(const TA* A, long long lda, const TW* W, long long ldw, TO* 
   pdl_launch_dependents();
   pdl_wait();
   const int tid = threadIdx.x, group = tid / PER, tx = tid % PER % TX, ty = tid % PER / TX;
-  const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
+  const int m0 = (blockIdx.z * gridDim.y + blockIdx.y) * BM, n0 = blockIdx.x * BN;
+  if (m0 >= M) return;                                     // (the last of several layers of blocks)
   float acc[TM][TN];
 #pragma unroll
   for (int i = 0; i < TM; ++i)
@@ -148,8 +149,9 @@ gemm_tn_simt_kernel(const TA* A, long long lda, const TW* W, long long ldw, TO* 
 template <typename TA, typename TW, typename TO, int BM, int BN, int TM, int TN>
 int launch_tile(const void* A, long long lda, const void* W, long long ldw, void* O, long long ldo, int M, int N, int K,
                 cudaStream_t stream) {
-  const dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM), block(kGroups * (BM / TM) * (BN / TN));
-  if (grid.y > 65535) return YALIS_ERR_SHAPE;
+  // more row tiles than one dimension of a grid holds go on in the next
+  const int row_tiles = (M + BM - 1) / BM, layers = (row_tiles + 65534) / 65535;
+  const dim3 grid((N + BN - 1) / BN, (row_tiles + layers - 1) / layers, layers), block(kGroups * (BM / TM) * (BN / TN));
   const bool vec = K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 && (uintptr_t)A % (4 * sizeof(TA)) == 0 &&
                    (uintptr_t)W % (4 * sizeof(TW)) == 0;
   if (vec)
@@ -168,6 +170,7 @@ int launch_tile(const void* A, long long lda, const void* W, long long ldw, void
 template <typename TA, typename TW, typename TO>
 int launch(const void* A, long long lda, const void* W, long long ldw, void* O, long long ldo, int M, int N, int K,
            cudaStream_t stream) {
+  if (((long long)M + 63) / 64 > 65535) return YALIS_ERR_SHAPE;      // (4,194,240 rows)
   const long long sms = yalis_sm_count();
   const long long blocks = (long long)((N + 127) / 128) * ((M + 31) / 32);
   if (blocks >= sms / 2) return launch_tile<TA, TW, TO, 32, 128, 8, 8>(A, lda, W, ldw, O, ldo, M, N, K, stream);

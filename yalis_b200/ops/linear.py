@@ -31,7 +31,7 @@ FUSED_SILU_MAX_TOKENS = 16
 
 def gemm_simt(x: torch.Tensor, w: torch.Tensor, out_dtype: Optional[torch.dtype] = None,
               out: Optional[torch.Tensor] = None) -> torch.Tensor:
-    """x [M, K] . w [N, K]^T on the CUDA cores, float32 accumulation in k order."""
+    """x [M, K] . w [N, K]^T on the CUDA cores, float32 accumulation in an order that K alone decides."""
     name = "gemm_simt"
     need_cuda(name, x, w, out)
     need(x.dim() == 2 and w.dim() == 2 and x.shape[1] == w.shape[1], name,
