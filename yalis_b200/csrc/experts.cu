@@ -277,7 +277,7 @@ __device__ __forceinline__ void load4(const __nv_bfloat16* p, float& a, float& b
 // the choice.  A block takes TOK tokens: their rows wait in shared memory in their own dtype, the warps share out
 // the experts, and a row of the router read once serves all TOK tokens (each token's sum has the same order whatever
 // TOK is); then warp t chooses for token t.
-template <typename T, int TOK, bool RULES>
+template <typename T, int TOK, int ROWS, bool RULES>
 __global__ void __launch_bounds__(512) route_kernel(const T* x, long x_stride, const float* __restrict__ w, int E, int K, int top,
                              float eps, float factor, const int32_t* req_of_token, int32_t* ids,
                              float* weights, int n_tokens, int sigmoid, const float* __restrict__ side,
@@ -321,10 +321,10 @@ __global__ void __launch_bounds__(512) route_kernel(const T* x, long x_stride, c
       }
     }
   };
-  // Where a block has several tokens, a warp takes two rows of the router at a time: the tokens' values are read from shared
-  // memory once for both, and twice as many loads are under way.  K = 2,048, 16 experts: 2,048 tokens 21.3 -> 18.3 us, 4,096 tokens 40.8 -> 35.1;
-  // 64 experts 55.9 -> 41.1; 128 experts of K = 2,880 136 -> 93.
-  constexpr int ROWS = TOK > 1 ? 2 : 1;
+  // Where a block has several tokens and more rows than warps, a warp takes two rows of the router at a time (ROWS 2): the
+  // tokens' values are read from shared memory once for both, and twice as many loads are under way.  K = 2,048, 16 experts:
+  // 2,048 tokens 21.3 -> 18.3 us, 4,096 tokens 40.8 -> 35.1; 64 experts 55.9 -> 41.1; 128 experts of K = 2,880 136 -> 93.  With 8
+  // experts or fewer the second row of every warp would be its first again: 2,048 tokens 16.1 us with one row, 17.2 with two.
   for (int e = warp; e < rows; e += ROWS * warps) {
     const float* wr[ROWS];
 #pragma unroll
@@ -338,7 +338,7 @@ __global__ void __launch_bounds__(512) route_kernel(const T* x, long x_stride, c
 #pragma unroll
       for (int t = 0; t < TOK; ++t) acc[i][t] = 0.f;
     if (vec) {
-#pragma unroll (TOK == 1 ? 8 : 4)
+#pragma unroll (TOK == 1 ? 8 : 2 * ROWS)
       for (int k = 4 * lane; k < K; k += 128) {
         float4 wv[ROWS];
 #pragma unroll
@@ -397,7 +397,7 @@ __global__ void __launch_bounds__(512) route_kernel(const T* x, long x_stride, c
   }
 }
 
-template <typename T, int TOK, bool RULES>
+template <typename T, int TOK, int ROWS, bool RULES>
 int launch_route(const void* x, long x_stride, const float* w, int n_tokens, int E, int K, int top, float eps, float factor,
                  const int32_t* req_of_token, int32_t* ids, float* weights, int sigmoid, const float* side, float* side_out,
                  const ChoiceRules& rules, cudaStream_t stream) {
@@ -405,13 +405,13 @@ int launch_route(const void* x, long x_stride, const float* w, int n_tokens, int
   if (smem > 200 * 1024) return YALIS_ERR_SHAPE;
   static size_t configured = 0;
   if (smem > 48 * 1024 && smem > configured) {
-    if (cudaFuncSetAttribute(route_kernel<T, TOK, RULES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+    if (cudaFuncSetAttribute(route_kernel<T, TOK, ROWS, RULES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
       return YALIS_ERR_LAUNCH;
     configured = smem;
   }
   // one token a block: blocks are few, so sixteen warps share out the experts
   const int threads = TOK == 1 && n_tokens <= 2 * yalis_sm_count() ? 512 : 256;
-  return yalis_launch(route_kernel<T, TOK, RULES>, dim3((n_tokens + TOK - 1) / TOK), dim3(threads), smem, stream, (const T*)x, x_stride, w, E, K,
+  return yalis_launch(route_kernel<T, TOK, ROWS, RULES>, dim3((n_tokens + TOK - 1) / TOK), dim3(threads), smem, stream, (const T*)x, x_stride, w, E, K,
                       top, eps, factor, req_of_token, ids, weights, n_tokens, sigmoid, side, side_out, rules);
 }
 
@@ -799,8 +799,10 @@ YALIS_API int yalis_route(const void* x, int x_dtype, long x_stride, const float
   const bool many = n_tokens >= 1024 && 8 * ((size_t)K * elt + (size_t)(E + groups) * 4) + 16 <= 96 * 1024;
   const bool ruled = correction || groups > 0 || real < E;
   YALIS_DISPATCH_DTYPE(x_dtype, T, {
-    auto launch = many ? (ruled ? launch_route<T, 8, true> : launch_route<T, 8, false>)
-                       : (ruled ? launch_route<T, 1, true> : launch_route<T, 1, false>);
+    const bool pairs = E + (side ? 1 : 0) > 8;          // more rows than a block of many tokens has warps
+    auto launch = !many ? (ruled ? launch_route<T, 1, 1, true> : launch_route<T, 1, 1, false>)
+                  : pairs ? (ruled ? launch_route<T, 8, 2, true> : launch_route<T, 8, 2, false>)
+                          : (ruled ? launch_route<T, 8, 1, true> : launch_route<T, 8, 1, false>);
     return launch(x, x_stride, w, n_tokens, E, K, top, eps, factor, req_of_token, ids, weights, sigmoid, side, side_out, rules, stream);
   });
   return YALIS_OK;
