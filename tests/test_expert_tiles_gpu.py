@@ -37,6 +37,23 @@ def test_tiles_end_anywhere(bm, act, width, inner, most):
         at += c
 
 
+def test_two_row_blocks_where_the_last_tile_is_half_empty():
+    """Rows of an expert that end in the first block of their last tile: one block a tile for few of them, two for many."""
+    from yalis_b200.ops import experts as X
+    g = torch.Generator().manual_seed(7)
+    ids = (torch.arange(1600) % 4).to(torch.int32)[:, None].cuda()
+    x = torch.randn(1600, 72, generator=g).bfloat16().cuda()
+    for width in (640, 2112):
+        w = (torch.randn(4, width, 72, generator=g) / 72 ** 0.5).bfloat16().cuda()
+        plan = X.expert_plan(ids, 4, 128)
+        rows = X.gather_rows(x, plan, 1)
+        got = X.grouped_gemm_wstream(rows, w, plan).double().view(4, 400, width)
+        want = torch.einsum("esk,enk->esn", rows.double().view(4, 400, 72), w.double())
+        size = torch.einsum("esk,enk->esn", rows.double().view(4, 400, 72).abs(), w.double().abs())
+        # half a step of bfloat16, and float32 sums of 72 terms
+        assert bool(((got - want).abs() <= 2.0 ** -8 * want.abs() + 72 * 2.0 ** -23 * size).all())
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("experts", [1, 8, 9, 16, 17, 31])
 @pytest.mark.parametrize("inner,side", [(256, True), (516, False), (130, True), (131, False)])

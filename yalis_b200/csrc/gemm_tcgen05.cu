@@ -410,7 +410,8 @@ struct GroupedParams {
 // of 128 experts of 768 x 2048:
 //   64: 79 / 99 / 106   128: 105 / 101 / 126   256: 160 / 158 / 171   384: 212 / 203 / 243   512: 270 / 249 / 295   1024: 495 / 459 / 523
 // so two row blocks from kWideSlots slots an expert on, where they never lose (below, fewer and larger tiles fill the last
-// wave worse).  256 slots, one block on an SM, pay for the empty part of an expert's last tile and for an epilogue that nothing
+// wave worse), if an expert's rows fill the second block of its last tile or have tiles enough (eight) for that half to be small:
+// otherwise it fetches and multiplies rows of the next expert, or of none, for nothing.  256 slots, one block on an SM, pay for the empty part of an expert's last tile and for an epilogue that nothing
 // covers; only a plan that asks for them gets them.
 constexpr int kWideSlots = 384;
 
@@ -705,7 +706,7 @@ YALIS_API int yalis_grouped_gemm_wstream(const void* a, long long lda, int rows_
     case 32: return launch_grouped<32, 1>(mw, mx, p, max_tiles, stream);
     case 64: return launch_grouped<64, 1>(mw, mx, p, max_tiles, stream);
     case 128:
-      if (rows_a / n_experts >= kWideSlots) return launch_grouped<128, 2>(mw, mx, p, max_tiles, stream);
+      if (rows_a / n_experts >= kWideSlots && ((N + TILE_N - 1) / TILE_N % 2 == 0 || N >= 8 * 2 * TILE_N)) return launch_grouped<128, 2>(mw, mx, p, max_tiles, stream);
       return launch_grouped<128, 1>(mw, mx, p, max_tiles, stream);
     case 256: return launch_grouped<256, 1>(mw, mx, p, max_tiles, stream);
   }
