@@ -259,8 +259,9 @@ decode_attention_lean_kernel(const __grid_constant__ CUtensorMap map_k, const __
           int page = pi < p.table_width ? bt[pi] : -1;
           int y;
           if constexpr (GEN) {
-            const bool none = page < 0 || page >= p.num_pages || key0 + (i + 1) * p.page_size <= lo_key;
-            y = (none ? p.num_pages * p.g : page * p.g + sg.kvh) * p.page_size;      // past the pool: zeros
+            const bool unseen = key0 + (i + 1) * p.page_size <= lo_key, bad = page < 0 || page >= p.num_pages;
+            if (bad && !unseen && p.error) atomicOr(p.error, YALIS_FLAG_BAD_PAGE);   // a visible key without a page
+            y = (bad || unseen ? p.num_pages * p.g : page * p.g + sg.kvh) * p.page_size;      // past the pool: zeros
           } else {
             if (page < 0 || page >= p.num_pages) { // a visible key without a page: a caller's bug
               if (p.error) atomicOr(p.error, YALIS_FLAG_BAD_PAGE);

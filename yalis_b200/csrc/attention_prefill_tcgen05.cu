@@ -335,14 +335,15 @@ prefill_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
       auto box_row = [&](int j) -> int {
         const int key = ((tile_base + j) << 6) + (my_box << box_shift);
         if (j >= n_tiles || my_box >= boxes_per_tile || key > hi_key) return -1;
-        // general form: rows no query sees (their page may be gone) and rows without a page are zeros (past the pool)
+        // general form: rows no query sees (their page may be gone) are zeros (past the pool), and so is, with the error word
+        // raised, a visible row without a page
         const int none = (p.num_pages * p.g) << page_shift;
         if (GEN && key + box_rows <= lo_key) return none;
         const int pi = key >> page_shift;
         int page = (j == 0 && early_page != -2) ? early_page : (pi < p.table_width ? bt[pi] : -1);
         if (page < 0 || page >= p.num_pages) {
-          if (GEN) return none;
           if (p.error) atomicOr(p.error, YALIS_FLAG_BAD_PAGE);
+          if (GEN) return none;
           page = 0;
         }
         return ((page * p.g + kvh) << page_shift) + (key & (p.page_size - 1));

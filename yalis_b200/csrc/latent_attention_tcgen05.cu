@@ -180,12 +180,14 @@ latent_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map, const L
   const int32_t* bt = a.block_table + (size_t)req * a.table_width;
   auto box_row = [&](int j) -> int {
     // row of the pool at which this lane's box of tile j starts; past the pool (a box of zeros) where the block's queries
-    // see none of its rows or its page is unmapped
+    // see none of its rows, and, with the error word raised, where a visible row has no page
     const int key = ((tile_base + j) << 6) + (lane << box_shift);
     const int none = a.num_pages << page_shift;
     if (lane >= boxes || j >= n_tiles || key > pos_last || key + box_rows <= lo) return none;
     const int pi = key >> page_shift, page = pi < a.table_width ? bt[pi] : -1;
-    return page < 0 || page >= a.num_pages ? none : (page << page_shift) + (key & (a.page_size - 1));
+    if (page >= 0 && page < a.num_pages) return (page << page_shift) + (key & (a.page_size - 1));
+    if (a.error) atomicOr(a.error, YALIS_FLAG_BAD_PAGE);
+    return none;
   };
   auto copy_tile = [&](int j, int y) {                     // the warp: tile j into its buffer, box i from row y of lane i
     const int b = j % a.stages;
