@@ -117,3 +117,35 @@ def test_counters_that_a_recording_may_use_stay_when_a_larger_step_comes(monkeyp
     assert recorded() is not None and attn._tickets("cpu", 1).data_ptr() != recorded().data_ptr()
     # what is kept stays below the size of the buffer in use
     assert sum(t.numel() for t in attn._replaced_tickets) < attn._tickets("cpu", 1).numel()
+
+
+def _host(q_lens, before):
+    from yalis_b200.engine.context import HostStep
+    starts = [0]
+    for q in q_lens:
+        starts.append(starts[-1] + q)
+    return HostStep(slots=list(range(len(q_lens))), q_start=starts, ctx_before=list(before), max_q_len=max(q_lens),
+                    max_kv_len=max(q + b for q, b in zip(q_lens, before)))
+
+
+def test_general_layers_choose_a_form_by_the_step(monkeypatch):
+    from yalis_b200.config.spec import PartSpec
+    from yalis_b200.parts.base import make_part
+    monkeypatch.setattr(attn, "SM_COUNT", 148)
+    base = {"hidden_size": 32, "num_heads": 16, "num_kv_heads": 8, "head_dim": 128, "window": 512}
+    part = make_part("mixer", PartSpec("general_attention", base))
+    form = lambda q, b: part.capture_key(_host(q, b))[1]
+    assert form([1] * 5, [9] * 5) == "decode" and form([8, 1], [0, 3000]) == "mma"
+    assert form([9], [0]) == form([64], [0]) == form([17] * 16, [0] * 16) == "mma"       # one tile of keys, blocks for all at once
+    assert form([65], [0]) == form([17], [48]) == form([9, 1], [0, 64]) == form([64] * 40, [0] * 40) == "prompt"
+    pooled = make_part("mixer", PartSpec("general_attention", {**base, "pool": 4}))
+    assert pooled.capture_key(_host([300], [0]))[1] == pooled.capture_key(_host([1], [0]))[1] == "mma"
+
+
+def test_general_layers_record_one_decode_step_per_bucket(monkeypatch):
+    """The kernel for single tokens launches the same whatever the number of requests: their key splits are another kernel's."""
+    from yalis_b200.config.spec import PartSpec
+    from yalis_b200.parts.base import make_part
+    monkeypatch.setattr(attn, "SM_COUNT", 148)
+    part = make_part("mixer", PartSpec("general_attention", {"hidden_size": 32, "num_heads": 16, "num_kv_heads": 8, "head_dim": 128}))
+    assert len({part.capture_key(_host([1] * n, [100 * n] * n)) for n in (5, 6, 7, 8)}) == 1

@@ -585,6 +585,18 @@ def _own_counters(name: str, q: torch.Tensor, counters: Optional[torch.Tensor], 
     return counters
 
 
+def prefill_general_preferred(host, heads_per_group: int, num_kv_heads: int, head_dim: int) -> bool:
+    """Whether portions of a general layer go to ``prefill_attention_general`` rather than to ``paged_attention_mma``: not where
+    every request's keys fit one tile of 64 and the blocks of 64 rows that the latter makes are all resident at once.  Its
+    blocks are cheap to start, and there is nothing to stream: portions of 5 to 64 tokens without earlier ones, us with
+    either, head size 64: 6.3 to 7.8 / 8.8 to 9.3; head size 128: 8.3 to 10.4 / 9.4 to 10.6; 16 portions of 17, 64 heads of 128
+    over 8: 384 blocks, 18.3 / 13.2.  From one tile more on it loses (17 tokens behind 1,000: 40 / 27 and 66 / 28)."""
+    if host.max_kv_len > 64:
+        return True
+    blocks = sum(-(-(b - a) * heads_per_group // 64) for a, b in zip(host.q_start[:-1], host.q_start[1:])) * num_kv_heads
+    return blocks > 2 * sm_count() * max(1, 128 // head_dim)
+
+
 def prefill_general_applies(q: torch.Tensor, out: torch.Tensor, gate: Optional[torch.Tensor], page_size: int, num_heads: int,
                             num_kv_heads: int, head_dim: int, v_head_dim: int, scale: float) -> bool:
     """Whether ``prefill_attention_general`` takes a step: its head and page sizes, and operands on the 16-byte boundaries

@@ -334,10 +334,23 @@ class GeneralAttention(Mixer, Projected):
         blocks = self.g * (2 if self.difference is not None and rows > 8 else 1)      # two maps: eight rows of each a block
         return host.max_q_len, (attn_ops.decode_splits(len(host.slots), blocks) if rows <= 16 else 1)
 
+    def _form(self, host) -> str:
+        """Which tensor-core kernel a step goes to, where its operands lie as that kernel needs: "decode" (single tokens),
+        "prompt" (portions with more rows than a decode tile holds) or "mma" (the rest)."""
+        if self.difference is not None or self.distance_bias is not None or self.pool is not None or self.vd != self.hs:
+            return "mma"
+        per = self.nh // self.g
+        if host.max_q_len * per > 16:
+            work = lambda: attn_ops.prefill_general_preferred(host, per, self.g, self.hs)
+            return "prompt" if host.once(("prefill_general_preferred", per, self.g, self.hs), work) else "mma"
+        return "decode" if host.max_q_len == 1 else "mma"
+
     def capture_key(self, host):
         # the exact kernel launches the same for every step; the choice among the tensor-core ones and their launch go by the
-        # longest portion
-        return ("general_attention",) + self._launch_shape(host)
+        # longest portion, that of the mma.sync form by the key splits besides
+        form = self._form(host)
+        longest, splits = self._launch_shape(host)
+        return ("general_attention", form, longest, splits if form == "mma" else 1)
 
     def keys_seen(self, position: int) -> int:
         """How many keys the query at ``position`` sees."""
@@ -372,8 +385,10 @@ class GeneralAttention(Mixer, Projected):
         q_at = self.spans["q_proj"][0]
         k_at = self.spans["k_proj"][0] if self.own_kv else q_at
         v_at = self.spans["v_proj"][0] if "v_proj" in self.spans else k_at
-        longest, splits = self._launch_shape(ctx.host)
-        counters = attn_ops.general_counters(longest, ctx.n_requests, self.g, z.device) if self._tensor_core_form(z.dtype) else None
+        (longest, splits), form = self._launch_shape(ctx.host), self._form(ctx.host)
+        counters = None
+        if form != "mma" and self._tensor_core_form(z.dtype):
+            counters = attn_ops.general_counters(longest, ctx.n_requests, self.g, z.device)
         pooling = {} if blocks is None else dict(pool=blocks.size, pooled_k=blocks.k, pooled_v=blocks.v, pooled_table=blocks.table,
                                                  single_tokens=ctx.host.max_q_len == 1)
         q = qkv_prepare(z, (q_at, k_at, v_at), self.nh * self.maps, self.g, self.hs, self.vd, ctx.positions, ctx.req_of_token,
@@ -390,18 +405,17 @@ class GeneralAttention(Mixer, Projected):
                       v_head_dim=self.vd)
         scale_out = self.out_scale if self.difference is None else 1.0 - self.difference[0]
         if self._tensor_core_form(z.dtype):
-            if (longest * (self.nh // self.g) > 16 and self.difference is None and self.rel is None and blocks is None
-                    and attn_ops.prefill_general_applies(q, y, gate, cache.k.shape[2], self.nh, self.g, self.hs, self.vd, self.scale)):
-                # portions with more rows than a decode tile holds (single tokens of the same step ride along)
+            if form == "prompt" and attn_ops.prefill_general_applies(q, y, gate, cache.k.shape[2], self.nh, self.g, self.hs, self.vd,
+                                                                     self.scale):
+                # (single tokens of the same step ride along)
                 attn_ops.prefill_attention_general(q, cache.k, cache.v, ctx.positions, ctx.q_start, table, longest, self.nh, self.g,
                                                    self.hs, self.scale, y, window=self.window, chunk=self.chunk,
                                                    softcap=self.softcap, sink=self.sink, sink_logits=self.sink_logits,
                                                    slopes=self.slopes, gate=gate, out_scale=scale_out, error_flag=ctx.error_flag,
                                                    counters=counters)
                 return
-            if (longest == 1 and self.difference is None and self.rel is None and blocks is None
-                    and attn_ops.decode_general_applies(q, y, gate, ctx.n_requests, cache.k.shape[2], self.nh, self.g, self.hs, self.vd,
-                                                        self.scale)):
+            if form == "decode" and attn_ops.decode_general_applies(q, y, gate, ctx.n_requests, cache.k.shape[2], self.nh, self.g, self.hs,
+                                                                    self.vd, self.scale):
                 attn_ops.decode_attention_general(q, cache.k, cache.v, ctx.positions, ctx.q_start, table, self.nh, self.g, self.hs,
                                                   self.scale, y, window=self.window, chunk=self.chunk, softcap=self.softcap,
                                                   sink=self.sink, sink_logits=self.sink_logits, slopes=self.slopes, gate=gate,
