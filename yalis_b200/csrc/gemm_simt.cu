@@ -173,7 +173,7 @@ int launch(const void* A, long long lda, const void* W, long long ldw, void* O, 
   if (((long long)M + 63) / 64 > 65535) return YALIS_ERR_SHAPE;      // (4,194,240 rows)
   const long long sms = yalis_sm_count();
   const long long blocks = (long long)((N + 127) / 128) * ((M + 31) / 32);
-  if (blocks >= sms / 2) return launch_tile<TA, TW, TO, 32, 128, 8, 8>(A, lda, W, ldw, O, ldo, M, N, K, stream);
+  if (blocks >= sms / 2 && N > 64) return launch_tile<TA, TW, TO, 32, 128, 8, 8>(A, lda, W, ldw, O, ldo, M, N, K, stream);
   return launch_tile<TA, TW, TO, 32, 32, 4, 4>(A, lda, W, ldw, O, ldo, M, N, K, stream);
 }
 
