@@ -20,10 +20,9 @@ namespace {
 // k, added in a fixed order: the same bits whatever M, N and the tile.  Values of the next tile are loaded to registers while
 // the current one is multiplied, 16 bytes at a time where rows are aligned.
 //
-// What bounds it: float32 FMAs (128 a cycle and SM).  8 x 8 outputs a thread read 16 values from shared memory for 64 FMAs,
-// which the two units then spend equally long on.  A warp alone on its scheduler issues an instruction every four cycles
-// whatever their independence, and a step of a few hundred rows has about as many tiles as there are SMs: hence four groups,
-// two warps per scheduler from one block.
+// What bounds it: the FMAs (128 a cycle and SM) and the loads from shared memory beside them, 16 values for the 64 FMAs of
+// 8 x 8 outputs a thread: together 0.43 of the FMA rate for the products of 250 rows.  A step of a few hundred rows has about as
+// many tiles as there are SMs: hence four groups, two warps per scheduler from one block, whose waits cover one another.
 constexpr int kGroups = 4;
 
 template <typename TA, typename TW, typename TO, int BM, int BN, int TM, int TN, bool VEC>
@@ -161,12 +160,14 @@ int launch_tile(const void* A, long long lda, const void* W, long long ldw, void
                       (const TW*)W, ldw, (TO*)O, ldo, M, N, K);
 }
 
-// Which tile: 32 x 128 with 8 x 8 outputs a thread (a warp's lanes lie 2 x 16, which loads from shared memory in fewer passes
-// than 4 x 8) where that makes a block for every other SM at least, else 32 x 32 with 4 x 4: more blocks.
+// Which tile: 32 x 128 with 8 x 8 outputs a thread where that makes a block for every other SM at least and the columns fill it,
+// else 32 x 32 with 4 x 4: more blocks.
 // Measured (us, float32; 64 x 64 tiles with 4 x 4 outputs a thread, as it was -> now), columns x K:
 //   250 rows   3,072 x 2,048  227 -> 147    2,048 x 2,048  158 -> 90     16,384 x 2,048  699 -> 494    2,048 x 8,192  610 -> 331
 //   1,024 rows 3,072 x 2,048  602 -> 424    2,048 x 2,048  411 -> 287    16,384 x 2,048  2,704 -> 1,907  2,048 x 8,192  1,614 -> 1,104
 //   8 rows     3,072 x 2,048  159 -> 71     16,384 x 2,048  221 -> 90    2,048 x 8,192  633 -> 262
+// 1,024 rows were faster still in tiles of 128 x 128 with one chain an output (359, 248 and, for K = 8,192, 956), which 250 rows
+// do not fill the SMs with; an output's bits must not depend on the tile, so one number of chains serves all sizes.
 template <typename TA, typename TW, typename TO>
 int launch(const void* A, long long lda, const void* W, long long ldw, void* O, long long ldo, int M, int N, int K,
            cudaStream_t stream) {

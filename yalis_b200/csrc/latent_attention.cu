@@ -171,8 +171,8 @@ __global__ void head_project_kernel(const TX* x, long xs_n, long xs_h, const T* 
 }
 
 // y[n, h * e + c] = x[n, h, c] * sigmoid(g[n, h * e + c]), four neighbouring values a thread (e a multiple of four, all rows
-// on the boundaries of four values).  Bound by memory: 2,048 tokens of 16 x 128 values, 25 MB: 22 us a value a thread with
-// two divisions each, 10.5 us this way (ncu, cold).
+// on the boundaries of four values).  2,048 tokens of 16 x 128 values, 25 MB: 22 us a value a thread with two divisions each,
+// 10.5 us this way (ncu, cold).  That is 2.4 TB/s, a third of the copy bandwidth: blocks are too short to have much on its way.
 template <typename T, typename TX>
 __global__ void sigmoid_gate_x4_kernel(const TX* x, long xs_n, long xs_h, int e, const T* g, long gs, T* y, long ys, int cols) {
   pdl_launch_dependents();

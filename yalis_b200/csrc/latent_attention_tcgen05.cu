@@ -17,10 +17,11 @@
 // One warp looks up pages and issues the copies (a ring of two or three tiles), one issues the products, whichever are ready:
 // the scores of tile j + 1 run while the softmax of tile j is computed.  Blocks are numbered so that the heaviest tiles of queries start first.
 //
-// What bounds it: the tensor pipe.  A tile of 64 rows costs R + p over 16 products of 128 x 64 x 16 (limited by their
-// operands' way out of shared memory: 48 instead of 32 cycles) and 2 * 64 / 16 of 128 x R x 16.  R = 256, p = 64: 1,984
-// cycles a tile beside about 1,100 of the softmax warps.  The tile is 64 rows wide because O (R columns) and two S fill the
-// tensor memory at R = 384, and because three tiles of 320 columns beside Q are what shared memory holds.
+// What bounds it: the latency of a tile's copies.  At R = 256, p = 64 a tile takes about 3,400 cycles (clock stamps in the
+// kernel): its copies arrive 2,300 to 4,000 cycles after they are asked for, one tile being on its way at a time beside the two
+// in use.  The tensor pipe has work for 1,664 of them (20 products of 128 x 64 x 16, 8 of 128 x 256 x 16), the softmax warps for
+// about 1,100.  The tile is 64 rows wide because O (R columns) and two S fill the tensor memory at R = 384, and because three
+// tiles of 320 columns beside Q are what shared memory holds.
 // Measured: a layer with r = 256, p = 64, 16 heads and 2,048 tokens (products, preparation and gate included) 582 -> 194 us,
 // 523 -> 93 us for this kernel (140 with Q loaded piece by piece and products in a fixed order);
 // 8 single tokens of 16 heads behind 1,024 rows in 16 shares: 37 -> 17 us for this kernel, 22 -> 8 us for the merge.
