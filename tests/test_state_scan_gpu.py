@@ -71,3 +71,28 @@ def test_against_a_walk(rule, dim, vdim):
         assert (got[a:b].double() - want).norm() < 2e-6 * want.norm()
         kept = got_rows[i, :lay.state_floats].cpu().view(heads, vdim, -1)[:, :, :dim].double().transpose(1, 2)
         assert (kept - S).norm() < 2e-6 * S.norm()
+
+
+@pytest.mark.parametrize("dim,vdim", [(16, 40), (64, 128), (200, 33), (256, 128), (512, 6)])
+@pytest.mark.parametrize("rule", ["delta", "general", "selective", "constant"])
+def test_short_portions_have_a_tile_of_their_own(rule, dim, vdim):
+    """Portions of at most four tokens give the bits of the longer tile, which the walk above is compared with."""
+    from yalis_b200.ops.recurrent import StateLayout, state_scan
+    g = torch.Generator(device=DEV).manual_seed(dim + vdim)
+    heads, lens = 3, [2, 4, 1, 0, 3, 4]
+    n, lay = sum(lens), StateLayout(heads, dim, vdim)
+    rnd = lambda *s: torch.randn(*s, generator=g, device=DEV)
+    unit = torch.nn.functional.normalize(rnd(n, heads, dim), dim=-1).flatten(1)
+    more = {"delta": dict(decay=torch.rand(n, heads, generator=g, device=DEV), beta=torch.rand(n, heads, generator=g, device=DEV)),
+            "general": dict(decay=torch.rand(n, heads * dim, generator=g, device=DEV), unit=unit, removal=0.5 * unit),
+            "selective": dict(decay=torch.rand(n, heads, generator=g, device=DEV), beta=torch.rand(n, heads, generator=g, device=DEV),
+                              selective=True, skip=rnd(heads)),
+            "constant": dict(decay=torch.rand(heads, generator=g, device=DEV))}[rule]
+    starts = torch.tensor([0] + lens, device=DEV).cumsum(0).to(torch.int32)
+    slots = torch.arange(len(lens), dtype=torch.int32, device=DEV)
+    rows, q, v = rnd(len(lens) + 1, lay.total), rnd(n, heads * dim) / dim ** 0.5, rnd(n, heads * vdim)
+    got = []
+    for longest in (4, 0):
+        state = rows.clone()
+        got.append((state_scan(q, unit, v, state, lay, starts, slots, kv_heads=heads, max_q_len=longest, **more), state))
+    assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])

@@ -583,8 +583,9 @@ __global__ void head_norm_gate_kernel(const float* o, int o_stride, const float*
 }
 
 // The same for heads of up to 512 values, a multiple of four, on the boundaries of four values: a head stays in registers
-// between the sum and the result, everything is read and written once, four values at a time.  Bound by memory: 2,048 tokens
-// of 16 heads of 128, 34 MB: 19 us a value at a time, 15 us this way (ncu, cold).
+// between the sum and the result, everything is read and written once, four values at a time.  2,048 tokens of 16 heads of 128,
+// 34 MB: 19 us a value at a time, 15 us this way (ncu, cold), 2.3 TB/s: a warp's chain of load, sum and store leaves little on
+// its way.
 template <typename T>
 __global__ void head_norm_gate_x4_kernel(const float* o, int o_stride, const float* weight, const T* gate, int gate_stride,
                                          int gate_kind, T* y, int y_stride, const int32_t* req_of_token, int heads, int vdim,
@@ -820,7 +821,7 @@ YALIS_API int yalis_delta_prepare(const void* x, int dtype, int x_stride, const 
 }
 
 template <int ROWS, int LANES, int COLS, int RULE, int DECAY, int TILE>
-static int launch_scan_tile(const ScanParams& p, int n_requests, cudaStream_t stream) {
+static int launch_scan_tile(const ScanParams& p, int n_requests, bool early, cudaStream_t stream) {
   constexpr int cols = kScanThreads / LANES * COLS, vec_cols = RULE == 2 ? 5 : (DECAY == 2 ? 3 : 2);
   constexpr size_t smem = (2 * (size_t)scan_buffer_floats(vec_cols, TILE, ROWS * LANES, cols) + TILE * cols) * sizeof(float);
   static_assert(smem <= 200 * 1024, "two buffers and the read-outs fit a block");
@@ -828,35 +829,39 @@ static int launch_scan_tile(const ScanParams& p, int n_requests, cudaStream_t st
   if (smem > 48 * 1024 && cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
     return YALIS_ERR_LAUNCH;
   const dim3 grid((p.vdim + cols - 1) / cols, p.heads, n_requests);
-  if (TILE > 1) return yalis_launch_after(kernel, grid, dim3(kScanThreads), smem, stream, p);
+  if (!early) return yalis_launch_after(kernel, grid, dim3(kScanThreads), smem, stream, p);
   return yalis_launch(kernel, grid, dim3(kScanThreads), smem, stream, p);
 }
 
+// The staging tile goes by the longest portion: a tile of 16 tokens for portions of two to four holds shared memory that other
+// blocks of the SM need (64 requests of two tokens, heads of 256, generalized rule: 225 us, 86 in a tile of two).  Portions up
+// to 128 tokens may start before the kernel in front has ended: their blocks do not hold an SM for long.
 template <int ROWS, int LANES, int COLS, int RULE, int DECAY>
-static int launch_scan(const ScanParams& p, int n_requests, int single, cudaStream_t stream) {
-  if (single) return launch_scan_tile<ROWS, LANES, COLS, RULE, DECAY, 1>(p, n_requests, stream);
-  return launch_scan_tile<ROWS, LANES, COLS, RULE, DECAY, (ROWS * LANES > 256 ? 8 : 16)>(p, n_requests, stream);
+static int launch_scan(const ScanParams& p, int n_requests, int longest, cudaStream_t stream) {
+  if (longest == 1) return launch_scan_tile<ROWS, LANES, COLS, RULE, DECAY, 1>(p, n_requests, true, stream);
+  if (longest > 0 && longest <= 4) return launch_scan_tile<ROWS, LANES, COLS, RULE, DECAY, 4>(p, n_requests, true, stream);
+  return launch_scan_tile<ROWS, LANES, COLS, RULE, DECAY, (ROWS * LANES > 256 ? 8 : 16)>(p, n_requests, longest > 0 && longest <= 128, stream);
 }
 
 // The smallest power of two of lanes that covers dim.  Delta rules: 16 rows of one column a thread; the others 8 rows of two
 // neighbouring columns (beyond 256 rows 16 of one).  Sums over a column have one order per rule and dim, whatever the step.
 template <int RULE, int DECAY>
-static int launch_scan_dim(const ScanParams& p, int n_requests, int single, cudaStream_t stream) {
+static int launch_scan_dim(const ScanParams& p, int n_requests, int longest, cudaStream_t stream) {
   if constexpr (RULE == 1) {
-    if (p.dim <= 16) return launch_scan<16, 1, 1, RULE, DECAY>(p, n_requests, single, stream);
-    if (p.dim <= 32) return launch_scan<16, 2, 1, RULE, DECAY>(p, n_requests, single, stream);
-    if (p.dim <= 64) return launch_scan<16, 4, 1, RULE, DECAY>(p, n_requests, single, stream);
-    if (p.dim <= 128) return launch_scan<16, 8, 1, RULE, DECAY>(p, n_requests, single, stream);
-    if (p.dim <= 256) return launch_scan<16, 16, 1, RULE, DECAY>(p, n_requests, single, stream);
+    if (p.dim <= 16) return launch_scan<16, 1, 1, RULE, DECAY>(p, n_requests, longest, stream);
+    if (p.dim <= 32) return launch_scan<16, 2, 1, RULE, DECAY>(p, n_requests, longest, stream);
+    if (p.dim <= 64) return launch_scan<16, 4, 1, RULE, DECAY>(p, n_requests, longest, stream);
+    if (p.dim <= 128) return launch_scan<16, 8, 1, RULE, DECAY>(p, n_requests, longest, stream);
+    if (p.dim <= 256) return launch_scan<16, 16, 1, RULE, DECAY>(p, n_requests, longest, stream);
   } else {
-    if (p.dim <= 8) return launch_scan<8, 1, 2, RULE, DECAY>(p, n_requests, single, stream);
-    if (p.dim <= 16) return launch_scan<8, 2, 2, RULE, DECAY>(p, n_requests, single, stream);
-    if (p.dim <= 32) return launch_scan<8, 4, 2, RULE, DECAY>(p, n_requests, single, stream);
-    if (p.dim <= 64) return launch_scan<8, 8, 2, RULE, DECAY>(p, n_requests, single, stream);
-    if (p.dim <= 128) return launch_scan<8, 16, 2, RULE, DECAY>(p, n_requests, single, stream);
-    if (p.dim <= 256) return launch_scan<8, 32, 2, RULE, DECAY>(p, n_requests, single, stream);
+    if (p.dim <= 8) return launch_scan<8, 1, 2, RULE, DECAY>(p, n_requests, longest, stream);
+    if (p.dim <= 16) return launch_scan<8, 2, 2, RULE, DECAY>(p, n_requests, longest, stream);
+    if (p.dim <= 32) return launch_scan<8, 4, 2, RULE, DECAY>(p, n_requests, longest, stream);
+    if (p.dim <= 64) return launch_scan<8, 8, 2, RULE, DECAY>(p, n_requests, longest, stream);
+    if (p.dim <= 128) return launch_scan<8, 16, 2, RULE, DECAY>(p, n_requests, longest, stream);
+    if (p.dim <= 256) return launch_scan<8, 32, 2, RULE, DECAY>(p, n_requests, longest, stream);
   }
-  return launch_scan<16, 32, 1, RULE, DECAY>(p, n_requests, single, stream);
+  return launch_scan<16, 32, 1, RULE, DECAY>(p, n_requests, longest, stream);
 }
 // decay_kind 0: decay [heads]; 1: decay [N, heads]; 2: decay [N, heads * dim].  delta 1: the delta rule with beta
 // [N, heads]; delta 2: the generalized delta rule with unit keys and removal vectors [N, heads * dim] (contiguous,
@@ -885,15 +890,15 @@ YALIS_API int yalis_state_scan(const float* q, int q_stride, const float* k, int
   p.wide = (dim % 4 == 0 && q_stride % 4 == 0 && k_stride % 4 == 0 && !((uintptr_t)q & 15) && !((uintptr_t)k & 15) &&
             (decay_kind != 2 || !((uintptr_t)decay & 15)) &&
             (delta != 2 || (!((uintptr_t)unit & 15) && !((uintptr_t)removal & 15)))) ? 1 : 0;
-  const int single = max_q_len == 1;
-  if (delta == 2) return launch_scan_dim<2, 2>(p, n_requests, single, stream);
-  if (delta == 3) return launch_scan_dim<3, 1>(p, n_requests, single, stream);
-  if (delta && decay_kind == 1) return launch_scan_dim<1, 1>(p, n_requests, single, stream);
-  if (delta && decay_kind == 2) return launch_scan_dim<1, 2>(p, n_requests, single, stream);
-  if (delta) return launch_scan_dim<1, 0>(p, n_requests, single, stream);
-  if (decay_kind == 0) return launch_scan_dim<0, 0>(p, n_requests, single, stream);
-  if (decay_kind == 1) return launch_scan_dim<0, 1>(p, n_requests, single, stream);
-  return launch_scan_dim<0, 2>(p, n_requests, single, stream);
+  const int longest = max_q_len;
+  if (delta == 2) return launch_scan_dim<2, 2>(p, n_requests, longest, stream);
+  if (delta == 3) return launch_scan_dim<3, 1>(p, n_requests, longest, stream);
+  if (delta && decay_kind == 1) return launch_scan_dim<1, 1>(p, n_requests, longest, stream);
+  if (delta && decay_kind == 2) return launch_scan_dim<1, 2>(p, n_requests, longest, stream);
+  if (delta) return launch_scan_dim<1, 0>(p, n_requests, longest, stream);
+  if (decay_kind == 0) return launch_scan_dim<0, 0>(p, n_requests, longest, stream);
+  if (decay_kind == 1) return launch_scan_dim<0, 1>(p, n_requests, longest, stream);
+  return launch_scan_dim<0, 2>(p, n_requests, longest, stream);
 }
 
 YALIS_API int yalis_head_norm_gate(const float* o, int o_stride, const float* weight, const void* gate, int gate_stride,
