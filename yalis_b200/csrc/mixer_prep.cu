@@ -402,7 +402,7 @@ int launch_qkv_plain(const PrepParams& p, int n_tokens, cudaStream_t stream) {
 // What bounds it: the latency of a token's chain (row, table, loads, norm, store); a row's values through shared memory and
 // one head at a time cost more of it.
 // Measured (16 + 2 x 8 heads of 128 that turn whole, norms, pages; us at 64 / 512 / 2,048 tokens): through shared memory
-// 3.8 / 10.9 / 26.6, here 3.7 / 7.6 / 17.8; 32 + 2 x 8 heads of 64: 4.4 / 15.5 / 38.1 -> 3.7 / 4.6 / 13.8; 16 + 2 x 8 of 256:
+// 3.8 / 10.9 / 26.6, here 3.5 / 7.8 / 17.7; 32 + 2 x 8 heads of 64: 4.4 / 15.5 / 38.1 -> 3.7 / 4.6 / 13.8; 16 + 2 x 8 of 256:
 // 4.4 / 13.7 / 37.6 -> 4.1 / 10.3 / 30.8.  Fetching the rows before the request is known costs registers and gains nothing.
 template <typename T, typename TO, int L, bool INTER>
 __global__ void __launch_bounds__(256) qkv_turn_kernel(const PrepParams p) {
@@ -532,11 +532,13 @@ int launch_qkv_turn(const PrepParams& p, int n_tokens, cudaStream_t stream) {
   const int widest = p.dim < p.vdim ? p.vdim : p.dim, heads = p.nq + (p.maps + 1) * p.nk;
   const int half = p.inv_freq ? p.rot_dims / 2 : 0;
   const size_t smem = 2 * (size_t)((half + 3) & ~3) * sizeof(float);
-  // steps of many tokens: blocks that hold a token's heads in one pass, as far as 256 threads do; few tokens: four warps
+  // steps of many tokens: blocks that hold a token's heads in one pass, as far as 256 threads do; few tokens: four warps.
+  // Up to 64 tokens a group takes one head, so that none waits for a second (8 tokens of 16 + 2 x 8 heads of 128: 3.6 us with
+  // two, 3.15 with one; the general form took 3.3; 256 tokens of 16 + 2 x 8 heads of 256: 7.5 and 8.2).
   auto go = [&](auto kernel, int lanes) {
     const int needed = ((heads + 1) / 2 * lanes + 31) / 32 * 32;
     const bool many = n_tokens >= 2 * yalis_sm_count();
-    const int threads = many ? (needed < 256 ? needed : 256) : 128, pass = 2 * (threads / lanes);
+    const int threads = many ? (needed < 256 ? needed : 256) : 128, pass = (n_tokens > 64 ? 2 : 1) * (threads / lanes);
     return yalis_launch(kernel, dim3(n_tokens, many ? 1 : (heads + pass - 1) / pass), dim3(threads), smem, stream, p);
   };
   if (p.rot_interleaved) {
@@ -769,8 +771,7 @@ YALIS_API int yalis_qkv_prepare(const void* src, int dtype, int src_stride, int 
     return launch_qkv_plain<__nv_bfloat16, __nv_bfloat16>(p, n_tokens, stream);
   if (plain && dtype == YALIS_BF16 && out_dtype == YALIS_F32) return launch_qkv_plain<__nv_bfloat16, float>(p, n_tokens, stream);
   // heads in registers: eight values a lane, four of which turn with four others where pairs are half-split
-  // (one form whatever the number of tokens, so that a row's bits do not depend on the step: from 64 tokens on it is the
-  // faster one, for up to 8 it takes 3.5 us where the general form takes 3.3)
+  // (one form whatever the number of tokens, so that a row's bits do not depend on the step)
   const bool turn = vec && ((dim | vdim) & 7) == 0 && dim <= 256 && vdim <= 256 && !norm_all && pool == 0 &&
                     (rot_interleaved || !inv_freq || (rot_dims & 7) == 0);
   if (turn && dtype == YALIS_F32 && out_dtype == YALIS_F32) return launch_qkv_turn<float, float>(p, n_tokens, stream);
