@@ -26,8 +26,9 @@
 //     decides), and the decoding requests of a step that also holds prompt portions (only_single).
 //
 // Tile handling, masking and the arithmetic are those of decode_attention_tma_kernel; limits are
-// the same (bfloat16, head_dim 64/128/192/256, pages of 8..64 tokens, no window, at most 16 query
-// heads per KV head, one token per request), and at most 4096 requests.  Every mbarrier wait is
+// the same (bfloat16, head_dim 64/128/192/256, pages of 8..64 tokens, at most 16 query heads per KV
+// head, one token per request; a window, chunks and the like in the general form), and at most 4096
+// requests.  Every mbarrier wait is
 // bounded; on a timeout the block raises the error word, drains its copies and returns.
 #include "decode_tiles.cuh"
 
@@ -102,6 +103,38 @@ __device__ __forceinline__ int block_of_tile(long long t, long long total, int b
   return (int)(((t + 1) * blocks + total - 1) / total) - 1;
 }
 
+// The general form deals the tiles in one of three ways, by what the slowest block then has to do, counted in tiles:
+//   * pieces k > 0: every pair to k blocks in equal pieces (one segment a block).  One where no pair has more than five tiles of
+//     64 columns, or fewer wider ones (less than a merge takes: 4 requests of 300 tokens, 8 heads of 64: 7.5 us whole, 8.1 in five
+//     pieces; 4 heads of 256: 13.6 and 10.2), else at most eight or sqrt(2 T) for pairs of T tiles on average: a piece costs its
+//     tiles and about half a tile where the last of them merges;
+//   * pieces -q < 0: q whole pairs to a block, nothing to merge;
+//   * 0: all tiles evenly, whatever pairs they belong to, to as many blocks as pieces of the first kind make.  A block then begins
+//     and ends inside pairs that others share: two segments and two merges, which take about six tiles' time.
+// Measured (us, all tiles evenly to all blocks that are resident -> as many blocks as this makes, and the mma.sync kernel with its
+// key splits; heads over KV heads of a size): 32 requests of 100 tokens, 16 / 8 of 64: 12.3 -> 6.6 (6.5); 64 of 200, 16 / 8 of 64:
+// 17.3 -> 12.9 (16.3); 1 of 1,900, 4 / 4 of 64: 12.4 -> 9.7 (9.9); 1 of 32,000, 16 / 1 of 128: 208 -> 45 (98).
+// (Approximate divisions: every block comes to the same answer, and the step's fixed cost shows in a decode step.)
+struct Deal {
+  int pieces;                  // see above
+  int blocks;                  // that have tiles
+};
+
+__device__ __forceinline__ Deal choose_deal(int grid, int pairs, int most, float total, int size) {
+  float k_max;
+  asm("sqrt.approx.f32 %0, %1;" : "=f"(k_max) : "f"(2.0f * __fdividef(total, (float)pairs)));
+  const int pieces = (long long)most * size <= 5 * 64 ? 1 : max(8, (int)ceilf(k_max));
+  const float blocks = fminf((float)grid, fminf(total, (float)pairs * (float)pieces)), even = __fdividef(total, blocks) + 6.0f;
+  if (pairs <= grid) {
+    const int k = min((int)__fdividef((float)grid + 0.5f, (float)pairs), pieces);
+    if (__fdividef((float)most, (float)k) <= even) return {k, pairs * k};
+  } else {
+    const int q = (pairs + grid - 1) / grid;
+    if ((float)most * (float)q <= even) return {-q, (pairs + q - 1) / q};
+  }
+  return {0, (int)blocks};
+}
+
 // One stretch of a block's range inside one (request, KV head).
 struct Segment {
   int req, kvh;
@@ -147,9 +180,8 @@ struct Walker {
 // GEN: the general form.  A request's tiles start at the first key its query sees (window, chunk), scores may be capped or
 // fall off with the distance, a sink joins the denominator, a gate and a factor multiply the result, and the weights meet V as
 // two bfloat16 halves (16 bits of mantissa).  Rows of V that no query sees or that have no page arrive as zeros.
-// Measured (layers of 16 heads of 128 over 8 KV heads, this kernel / the mma.sync kernel with its key splits, us, L2 flushed, launches
-// included): 1 request of 30 tokens 33 / 43, 1 of 1,900 41 / 45, 8 of 1,000 47 / 47, 32 of 1,000 72 / 78 (window 1,024);
-// 64 of 1,900 131 / 180 (chunk 2,048).  It is no slower anywhere in that range, so it takes every step of single tokens.
+// It takes every step of single tokens that its sizes allow (see Deal for how it splits the work and for times beside the
+// mma.sync kernel's).
 template <int HS, int NST, bool GEN>
 __global__ void __maxnreg__(HS <= 128 ? 168 : 255)
 decode_attention_lean_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
@@ -172,7 +204,8 @@ decode_attention_lean_kernel(const __grid_constant__ CUtensorMap map_k, const __
   uint64_t* empty = full + NST;
   volatile int* abort_flag = reinterpret_cast<volatile int*>(empty + NST);
   int* s_last = const_cast<int*>(abort_flag) + 1;
-  int* cum = s_last + 3;                                                     // [R+1] prefix sum of tile counts
+  int* s_deal = s_last + 3;                                                  // general form: a Deal
+  int* cum = s_deal + 2;                                                     // [R+1] prefix sum of tile counts
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int b = blockIdx.x;
@@ -204,9 +237,15 @@ decode_attention_lean_kernel(const __grid_constant__ CUtensorMap map_k, const __
   __syncthreads();
   if (warp == 0) {
     int carry = 0;
+    int with_tiles = 0, upto = 0, most = 0;              // general form: requests that count, the last of them, its most tiles
     for (int r0 = 0; r0 < p.n_requests; r0 += 32) {
       const int r = r0 + lane;
       int v = r < p.n_requests ? cum[r + 1] : 0;
+      if (GEN && v > 0) {
+        ++with_tiles;
+        upto = r + 1;
+        most = max(most, v);
+      }
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
         const int u = __shfl_up_sync(0xffffffffu, v, o);
@@ -215,12 +254,44 @@ decode_attention_lean_kernel(const __grid_constant__ CUtensorMap map_k, const __
       if (r < p.n_requests) cum[r + 1] = carry + v;
       carry += __shfl_sync(0xffffffffu, v, 31);
     }
+    if constexpr (GEN) {
+      with_tiles = __reduce_add_sync(0xffffffffu, with_tiles);
+      upto = __reduce_max_sync(0xffffffffu, upto);
+      most = __reduce_max_sync(0xffffffffu, most);
+      if (lane == 0) {
+        Deal deal = {0, (int)min((long long)gridDim.x, (long long)carry * p.g)};
+        if (upto == with_tiles && carry > 0)           // pairs can be counted off
+          deal = choose_deal(gridDim.x, with_tiles * p.g, most, (float)carry * (float)p.g, HS);
+        s_deal[0] = deal.pieces;
+        s_deal[1] = deal.blocks;
+      }
+    }
   }
   __syncthreads();
   const long long total = (long long)cum[p.n_requests] * p.g;
-  const int blocks = (int)min((long long)gridDim.x, total);     // every block that works has at least one tile
-  const long long t_lo = b < blocks ? first_tile_of(b, total, blocks) : 0;
-  const long long t_hi = b < blocks ? first_tile_of(b + 1, total, blocks) : 0;
+  const int pieces = GEN ? s_deal[0] : 0;
+  const int blocks = GEN ? s_deal[1] : (int)min((long long)gridDim.x, total);   // (evenly: each has at least one tile)
+  long long t_lo = 0, t_hi = 0;
+  if (b < blocks) {
+    if (GEN && pieces > 0) {
+      const int pair = b / pieces, piece = b - pair * pieces, req = pair / p.g, tiles = cum[req + 1] - cum[req], n = min(pieces, tiles);
+      if (piece < n) {
+        const long long first = (long long)cum[req] * p.g + (long long)(pair - req * p.g) * tiles;
+        t_lo = first + (unsigned)(piece * tiles) / (unsigned)n;
+        t_hi = first + (unsigned)((piece + 1) * tiles) / (unsigned)n;
+      }
+    } else if (GEN && pieces < 0) {
+      auto first_of_pair = [&](int pair) {
+        const int req = pair / p.g;
+        return req >= p.n_requests ? total : (long long)cum[req] * p.g + (long long)(pair - req * p.g) * (cum[req + 1] - cum[req]);
+      };
+      t_lo = first_of_pair(b * -pieces);
+      t_hi = first_of_pair((b + 1) * -pieces);
+    } else {
+      t_lo = first_tile_of(b, total, blocks);
+      t_hi = first_tile_of(b + 1, total, blocks);
+    }
+  }
 
   int armed = 0;                               // tiles this block has asked for (producer) / used (consumers)
   if (warp == CWARPS) {
@@ -497,9 +568,10 @@ decode_attention_lean_kernel(const __grid_constant__ CUtensorMap map_k, const __
       }
       if (!whole) {
         // ---- a pair cut by block borders: the last of its blocks to arrive adds the pieces ----------
-        const int b_first = block_of_tile(sg.first, total, blocks);
-        const int n_parts = block_of_tile(sg.first + sg.tiles - 1, total, blocks) - b_first + 1;
         const int pair = sg.req * p.g + sg.kvh;
+        const bool dealt = !GEN || pieces == 0;
+        const int b_first = dealt ? block_of_tile(sg.first, total, blocks) : pair * pieces;
+        const int n_parts = dealt ? block_of_tile(sg.first + sg.tiles - 1, total, blocks) - b_first + 1 : min(pieces, sg.tiles);
         __threadfence();
         consumer_sync();
         if (threadIdx.x == 0) s_last[0] = (atomicAdd(&p.tickets[pair], 1) == n_parts - 1) ? 1 : 0;
@@ -508,7 +580,7 @@ decode_attention_lean_kernel(const __grid_constant__ CUtensorMap map_k, const __
           __threadfence();
           // Piece j lies in block b_first + j: in its second slot if the pair is not that block's first
           // segment, which can only be so for the first of them.  Read past the L1, four loads in flight.
-          const int slot0 = b_first * 2 + (first_tile_of(b_first, total, blocks) >= sg.first ? 0 : 1);
+          const int slot0 = b_first * 2 + (!dealt || first_tile_of(b_first, total, blocks) >= sg.first ? 0 : 1);
           auto slot_of = [&](int j) { return j == 0 ? slot0 : (b_first + j) * 2; };
           for (int e = threadIdx.x; e < n_rows * VEC; e += CWARPS * 32) {
             const int r = e / VEC, d = (e - r * VEC) * 4;
@@ -565,7 +637,7 @@ decode_attention_lean_kernel(const __grid_constant__ CUtensorMap map_k, const __
 
 size_t lean_smem_bytes(int hs, int stages, int per, int n_requests) {
   return 1024 + (size_t)2 * stages * BN * hs * 2 + (size_t)CWARPS * per * (hs + 2) * 4 + (size_t)16 * (hs + 8) * 2 +
-         2 * stages * 8 + 16 + (size_t)(n_requests + 1) * 4 + 16;
+         2 * stages * 8 + 24 + (size_t)(n_requests + 1) * 4 + 16;
 }
 
 template <int HS, int NST, bool GEN>
