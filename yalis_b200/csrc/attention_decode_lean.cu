@@ -111,9 +111,9 @@ __device__ __forceinline__ int block_of_tile(long long t, long long total, int b
 //   * pieces -q < 0: q whole pairs to a block, nothing to merge;
 //   * 0: all tiles evenly, whatever pairs they belong to, to as many blocks as pieces of the first kind make.  A block then begins
 //     and ends inside pairs that others share: two segments and two merges, which take about six tiles' time.
-// Measured (us, all tiles evenly to all blocks that are resident -> as many blocks as this makes, and the mma.sync kernel with its
-// key splits; heads over KV heads of a size): 32 requests of 100 tokens, 16 / 8 of 64: 12.3 -> 6.6 (6.5); 64 of 200, 16 / 8 of 64:
-// 17.3 -> 12.9 (16.3); 1 of 1,900, 4 / 4 of 64: 12.4 -> 9.7 (9.9); 1 of 32,000, 16 / 1 of 128: 208 -> 45 (98).
+// Measured (us, all tiles evenly to all blocks that are resident -> this, and the mma.sync kernel with its key splits; heads
+// over KV heads of a size): 32 requests of 100 tokens, 16 / 8 of 64: 12.2 -> 7.0 (6.5); 64 of 200, 16 / 8 of 64: 17.2 -> 13.6
+// (16.4); 1 of 1,900, 4 / 4 of 64: 12.2 -> 9.8 (9.6); 1 of 32,000, 16 / 1 of 128: 207 -> 45 (93).  Choosing takes 0.4 us.
 // (Approximate divisions: every block comes to the same answer, and the step's fixed cost shows in a decode step.)
 struct Deal {
   int pieces;                  // see above
