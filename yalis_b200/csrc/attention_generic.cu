@@ -1,6 +1,6 @@
 // Paged causal attention, the exact one: any head size up to 256 (even), any
 // number of heads and KV groups, any page size, float32 or bfloat16 storage,
-// float32 arithmetic throughout.  One block per (token, head); each warp walks
+// float32 arithmetic throughout.  The general form: one block per (token, head); each warp walks
 // every fourth visible key in ascending order with an online softmax and the
 // four partial results are merged in warp order.  For a given (position, head)
 // the order of every sum is therefore fixed, whatever else is in the batch and
@@ -197,6 +197,258 @@ __global__ void paged_attention_generic_kernel(const GenericParams<T> p) {
   }
 }
 
+// ---- the same for float32 heads of 64 and 128, several queries and heads at a time ------------------------------------------
+// The form above spends some sixty instructions a key and head, most of them on the sum over a warp and the two exponentials
+// of every key.  Here a warp takes a tile of 32 keys for up to eight (query, head) pairs that share a key/value head: a lane has a
+// key's scores for all pairs, so there is one maximum, one sum and one exponential a lane for 32 keys, then the lanes
+// share out the head's sizes for the values.  Tiles lie at multiples of 32 positions and warp w walks those whose number is w
+// modulo four, in ascending order; what a query does not see counts as nothing.  So here, too, the order of every sum is fixed for a
+// given position and head.  The keys of the next tile and the values of this one are on their way while a warp computes.
+// A block takes the neighbouring tokens of one request whose positions lie in one aligned group of kPairs / HP: the first
+// of them finds the others, the blocks of the others end at once.
+// What bounds it: reads of shared memory (16 bytes of a pair's query are two passes beside four products a lane) and, for few
+// blocks, the chain of a tile: copy, scores, maximum, exponential, values.  Measured (us, before -> now), 32 heads on 8 of 64 / 128:
+// one token behind 1,000 186 -> 23 / 253 -> 25, 64 such 679 -> 51 / 1,011 -> 144, a prompt of 250 247 -> 48 / 269 -> 61, of 1,024
+// 3,699 -> 417 / 4,096 -> 554, of 16 5.8 -> 4.5 / 6.8 -> 8.3.
+constexpr int kTile = 32;
+
+__device__ __forceinline__ void copy16(float* to, const float* from, bool there) {      // zeros where there is nothing
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((unsigned)__cvta_generic_to_shared(to)), "l"(from), "r"(there ? 16 : 0));
+}
+// The largest of a warp's values; NaN counts for nothing.
+__device__ __forceinline__ float warp_top(float v) {
+  float r;
+  asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+  return r;
+}
+
+template <int D, int PAIRS>
+constexpr size_t tiled_smem() {      // queries; per warp: a tile of keys, the weights
+  return (PAIRS * D + kWarps * kTile * (D + 4) + kWarps * PAIRS * kTile) * sizeof(float);
+}
+
+// D: the head size; HP: heads of a key/value head that a block takes; QT: queries.
+template <int D, int HP, int QT>
+__global__ void __launch_bounds__(kWarps * 32) paged_attention_tiled_kernel(const GenericParams<float> p, int n_tokens) {
+  constexpr int P = HP * QT, LK = D + 4, V = D / 32;           // rows of keys padded: lanes read 16 bytes of rows of their own
+  extern __shared__ __align__(16) float smem[];
+  pdl_launch_dependents();
+  pdl_wait();
+  const int t0 = blockIdx.x, per = p.nh / p.g, parts = per / HP, kvh = blockIdx.y / parts, h0 = kvh * per + (blockIdx.y % parts) * HP;
+  const int req = p.req_of_token[t0], pos0 = p.positions[t0];
+  if (req < 0) return;
+  if (pos0 % QT != 0 && t0 > 0 && p.req_of_token[t0 - 1] == req && p.positions[t0 - 1] == pos0 - 1) return;
+  int nq = 1;
+  while (nq < QT && (pos0 + nq) % QT != 0 && t0 + nq < n_tokens && p.req_of_token[t0 + nq] == req && p.positions[t0 + nq] == pos0 + nq) ++nq;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  float* qs = smem;                                            // [pair][D], a missing query is zeros
+  float* ks = smem + P * D + warp * kTile * LK;
+  float* ws = smem + P * D + kWarps * kTile * LK + warp * P * kTile;
+  for (int e = threadIdx.x; e < P * D; e += kWarps * 32) {
+    const int pair = e / D, i = pair / HP;
+    qs[e] = i < nq ? p.q[(size_t)(t0 + i) * p.q_stride + (size_t)(h0 + pair % HP) * D + e % D] : 0.f;
+  }
+  __syncthreads();
+
+  auto first = [&](int pos) {                                  // the first key that a position sees
+    const int lo = (p.window > 0 && pos - p.window + 1 > 0) ? pos - p.window + 1 : 0;
+    return p.chunk > 0 ? max(lo, (pos / p.chunk) * p.chunk) : lo;
+  };
+  const int lo = first(pos0), hi = pos0 + nq - 1;              // (a later position's first key is no earlier)
+  const int32_t* bt = p.block_table + (size_t)req * p.table_width;
+  // the row in the pools of a lane's key, or -1
+  auto find = [&](int tile) {
+    const int j = tile * kTile + lane, pi = j / p.page_size;
+    if (j < lo || j > hi || pi >= p.table_width) return -1;
+    const int page = bt[pi];
+    return page < 0 || page >= p.num_pages ? -1 : (page * p.g + kvh) * p.page_size + (j - pi * p.page_size);
+  };
+  auto fetch_keys = [&](int row) {
+#pragma unroll
+    for (int e = 0; e < kTile * D / 4; e += 32) {
+      const int r = (e + lane) / (D / 4), d = (e + lane) % (D / 4) * 4, at = __shfl_sync(0xffffffffu, row, r);
+      copy16(ks + r * LK + d, p.k_pool + (at < 0 ? 0 : (size_t)at * D + d), at >= 0);
+    }
+    asm volatile("cp.async.commit_group;" ::);
+  };
+  // a lane's sizes (V neighbouring ones) of the values of rows r .. r + 3 of the tile
+  auto fetch_values = [&](int row, int r, float (&v)[4][V]) {
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int at = __shfl_sync(0xffffffffu, row, r + u);
+      const float* from = p.v_pool + (size_t)max(at, 0) * D + lane * V;
+      if constexpr (V == 4) {
+        const float4 x = at >= 0 ? *reinterpret_cast<const float4*>(from) : make_float4(0.f, 0.f, 0.f, 0.f);
+        v[u][0] = x.x; v[u][1] = x.y; v[u][2] = x.z; v[u][3] = x.w;
+      } else {
+        const float2 x = at >= 0 ? *reinterpret_cast<const float2*>(from) : make_float2(0.f, 0.f);
+        v[u][0] = x.x; v[u][1] = x.y;
+      }
+    }
+  };
+
+  float acc[P][V], m[P], l[P];
+#pragma unroll
+  for (int a = 0; a < P; ++a) {
+    m[a] = -INFINITY;
+    l[a] = 0.f;
+#pragma unroll
+    for (int i = 0; i < V; ++i) acc[a][i] = 0.f;
+  }
+  const int last = hi / kTile;
+  int tile = lo / kTile + ((warp - lo / kTile) & (kWarps - 1));
+  int row = tile <= last ? find(tile) : -1;
+  if (tile <= last) fetch_keys(row);
+  for (; tile <= last; tile += kWarps) {
+    const int j = tile * kTile + lane, here = row, next = tile + kWarps;
+    float v[2][4][V];
+    fetch_values(here, 0, v[0]);
+    row = next <= last ? find(next) : -1;
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncwarp();
+    float s[P][4];
+#pragma unroll
+    for (int a = 0; a < P; ++a) s[a][0] = s[a][1] = s[a][2] = s[a][3] = 0.f;
+#pragma unroll 4
+    for (int d = 0; d < D; d += 4) {
+      const float4 k = *reinterpret_cast<const float4*>(ks + lane * LK + d);
+#pragma unroll
+      for (int a = 0; a < P; ++a) {
+        const float4 q = *reinterpret_cast<const float4*>(qs + a * D + d);
+        s[a][0] = __fmaf_rn(q.x, k.x, s[a][0]); s[a][1] = __fmaf_rn(q.y, k.y, s[a][1]);
+        s[a][2] = __fmaf_rn(q.z, k.z, s[a][2]); s[a][3] = __fmaf_rn(q.w, k.w, s[a][3]);
+      }
+    }
+    __syncwarp();
+    if (next <= last) fetch_keys(row);
+    uint32_t seen[QT];
+    bool whole = true;
+#pragma unroll
+    for (int i = 0; i < QT; ++i) {
+      seen[i] = __ballot_sync(0xffffffffu, i < nq && here >= 0 && j <= pos0 + i && j >= first(pos0 + i));
+      whole = whole && seen[i] == 0xffffffffu;
+    }
+#pragma unroll
+    for (int a = 0; a < P; ++a) {
+      const int i = a / HP, h = h0 + a % HP;
+      float x = ((s[a][0] + s[a][1]) + (s[a][2] + s[a][3])) * p.scale;
+      if (p.slopes) x -= p.slopes[h] * (float)(pos0 + i - j);
+      if (p.rel) x += p.rel[(size_t)h * p.rel_len + max(0, min(pos0 + i - j, p.rel_len - 1))];
+      if (p.softcap > 0.f) x = p.softcap * tanhf(x / p.softcap);
+      const bool see = (seen[i] >> lane) & 1;
+      const float top = fmaxf(m[a], warp_top(see ? x : -INFINITY));
+      const float e = see ? expf(x - top) : 0.f, corr = seen[i] != 0 ? expf(m[a] - top) : 1.f;
+      l[a] = l[a] * corr + e;                                  // this lane's keys; the lanes meet at the end
+      m[a] = top;
+      ws[a * kTile + lane] = e;
+#pragma unroll
+      for (int u = 0; u < V; ++u) acc[a][u] *= corr;
+    }
+    __syncwarp();
+#pragma unroll
+    for (int r = 0; r < kTile; r += 4) {
+      float (&now)[4][V] = v[(r / 4) & 1];
+      if (r + 4 < kTile) fetch_values(here, r + 4, v[(r / 4 + 1) & 1]);
+#pragma unroll
+      for (int i = 0; i < QT; ++i) {
+        float mine[4][V];
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+#pragma unroll
+          for (int e = 0; e < V; ++e) mine[u][e] = now[u][e];
+        if (!whole) {                                          // what a query does not see must not reach it, be it infinite
+#pragma unroll
+          for (int u = 0; u < 4; ++u)
+#pragma unroll
+            for (int e = 0; e < V; ++e) mine[u][e] = (seen[i] >> (r + u) & 1) ? mine[u][e] : 0.f;
+        }
+#pragma unroll
+        for (int a = i * HP; a < (i + 1) * HP; ++a) {
+          const float4 w = *reinterpret_cast<const float4*>(ws + a * kTile + r);
+#pragma unroll
+          for (int e = 0; e < V; ++e)
+            acc[a][e] = __fmaf_rn(w.w, mine[3][e], __fmaf_rn(w.z, mine[2][e], __fmaf_rn(w.y, mine[1][e], __fmaf_rn(w.x, mine[0][e], acc[a][e]))));
+        }
+      }
+    }
+    __syncwarp();
+  }
+  // the warps' shares, added in warp order
+  __syncthreads();
+  float* share = smem + P * D;                                 // [warp][pair][D], then maxima and sums [warp][pair]
+  float* ms = share + kWarps * P * D;
+  float* ls = ms + kWarps * P;
+#pragma unroll
+  for (int a = 0; a < P; ++a) {
+    const float sum = warp_sum(l[a]);
+#pragma unroll
+    for (int e = 0; e < V; ++e) share[(warp * P + a) * D + lane * V + e] = acc[a][e];
+    if (lane == 0) {
+      ms[warp * P + a] = m[a];
+      ls[warp * P + a] = sum;
+    }
+  }
+  __syncthreads();
+  for (int a = warp; a < nq * HP; a += kWarps) {
+    const int t = t0 + a / HP, h = h0 + a % HP;
+    const float z = (p.sink && p.sink_logits) ? p.sink_logits[h] : 0.f;
+    float top = p.sink ? z : -INFINITY;
+#pragma unroll
+    for (int w = 0; w < kWarps; ++w) top = fmaxf(top, ms[w * P + a]);
+    float sum = p.sink ? expf(z - top) : 0.f, wgt[kWarps];
+#pragma unroll
+    for (int w = 0; w < kWarps; ++w) {
+      wgt[w] = ms[w * P + a] == -INFINITY ? 0.f : expf(ms[w * P + a] - top);
+      sum += ls[w * P + a] * wgt[w];
+    }
+#pragma unroll
+    for (int e = 0; e < V; ++e) {
+      const int d = lane + 32 * e;
+      float o = 0.f;
+#pragma unroll
+      for (int w = 0; w < kWarps; ++w) o += share[(w * P + a) * D + d] * wgt[w];
+      float res = sum > 0.f ? o / sum * p.out_scale : 0.f;
+      if (p.gate) res *= 1.0f / (1.0f + expf(-p.gate[(size_t)t * p.gate_stride + (p.gate_per_head ? (size_t)h : (size_t)h * D + d)]));
+      p.out[(size_t)t * p.out_stride + (size_t)h * D + d] = res;
+    }
+  }
+}
+
+template <int D, int HP, int QT>
+int launch_tiled(const GenericParams<float>& p, int n_tokens, cudaStream_t stream) {
+  constexpr int P = HP * QT;
+  constexpr size_t smem = tiled_smem<D, P>();
+  static_assert(kWarps * P * D + 2 * kWarps * P <= kWarps * kTile * (D + 4) + kWarps * P * kTile, "the shares fit where the tiles were");
+  if (cudaFuncSetAttribute(paged_attention_tiled_kernel<D, HP, QT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+    return YALIS_ERR_LAUNCH;
+  return yalis_launch(paged_attention_tiled_kernel<D, HP, QT>, dim3(n_tokens, p.nh / HP), dim3(kWarps * 32), smem, stream, p, n_tokens);
+}
+// Which form (the bits are the same): as many heads a block, up to four, as leave two blocks an SM, since a block's walk over
+// the keys is what a step of few tokens waits for (a token behind 8,000, 32 heads of 128 on 8: 180 us with one head a block, 282 with
+// four); several queries a block where one makes more than eight blocks an SM (64 tokens behind 1,000 with 16 heads of 64 on
+// 16, all of requests of their own: 346 us with eight queries a block).
+template <int D>
+int launch_tiled_heads(const GenericParams<float>& p, int n_tokens, cudaStream_t stream) {
+  const int per = p.nh / p.g;
+  const long long pairs = (long long)n_tokens * p.nh, sms = yalis_sm_count();
+  const int hp = per % 4 == 0 && pairs / 4 >= 2 * sms ? 4 : per % 2 == 0 && pairs / 2 >= 2 * sms ? 2 : 1;
+  const bool single = pairs / hp <= 8 * sms;
+  if (hp == 4) return single ? launch_tiled<D, 4, 1>(p, n_tokens, stream) : launch_tiled<D, 4, 2>(p, n_tokens, stream);
+  if (hp == 2) return single ? launch_tiled<D, 2, 1>(p, n_tokens, stream) : launch_tiled<D, 2, 4>(p, n_tokens, stream);
+  return single ? launch_tiled<D, 1, 1>(p, n_tokens, stream) : launch_tiled<D, 1, 4>(p, n_tokens, stream);
+}
+
+// Rows of the pools in 16-byte pieces whose numbers fit 32 bits, one map, no pooled blocks.
+template <typename T>
+bool takes_tiles(const GenericParams<T>& p, int maps) {
+  return sizeof(T) == 4 && maps == 1 && p.pool == 0 && p.hs == p.hsv && (p.hs == 64 || p.hs == 128) &&
+         ((uintptr_t)p.k_pool | (uintptr_t)p.v_pool) % 16 == 0 && (long long)p.num_pages * p.g * p.page_size < (1ll << 31);
+}
+int launch_tiles(const GenericParams<float>& p, int n_tokens, cudaStream_t stream) {
+  return p.hs == 64 ? launch_tiled_heads<64>(p, n_tokens, stream) : launch_tiled_heads<128>(p, n_tokens, stream);
+}
+int launch_tiles(const GenericParams<__nv_bfloat16>&, int, cudaStream_t) { return YALIS_ERR_DTYPE; }
+
 }  // namespace
 
 // maps 2: two maps, hs the size of one map's queries and keys; no sink, gate or pooled blocks.
@@ -233,6 +485,7 @@ YALIS_API int yalis_paged_attention_generic(const void* q, int q_stride, void* o
     p.pool = pool; p.pk_pool = (const T*)pk_pool; p.pv_pool = (const T*)pv_pool; p.pool_table = pool_table;
     p.pool_table_width = pool_table_width; p.pool_page_size = pool_page_size; p.pool_num_pages = pool_num_pages;
     p.lambda = lambda; p.diff_eps = diff_eps;
+    if (takes_tiles(p, maps)) return launch_tiles(p, n_tokens, stream);
     return maps == 2 ? yalis_launch(paged_attention_generic_kernel<T, 2>, grid, dim3(kWarps * 32), smem, stream, p)
                      : yalis_launch(paged_attention_generic_kernel<T, 1>, grid, dim3(kWarps * 32), smem, stream, p);
   });
