@@ -1,4 +1,5 @@
-// y = x W^T on the CUDA cores: the matrix product of the float32 path.
+// y = x W^T on the CUDA cores: the float32 path's product with small and unaligned weights
+// (the others: gemm_f32_mma.cu), and the twin of the tensor-core products in tests.
 //
 // x [M, K] and W [N, K] are both K-contiguous (a Linear layer's weight as it
 // is stored).  Products and sums are float32 FMAs; there is no tensor-core

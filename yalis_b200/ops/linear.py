@@ -2,8 +2,11 @@
 
 Two precisions, chosen by the operands' dtype:
 
-* float32 operands: the SIMT kernel of csrc/gemm_simt.cu.  True 32-bit FMAs in
-  a fixed order, no tensor cores, no TF32.
+* float32 weights: true 32-bit products, no TF32.  Larger ones part each operand
+  into three bfloat16 values without loss and form the products on the tensor cores
+  (csrc/gemm_f32_mma.cu); small and unaligned ones are FMAs on the CUDA cores
+  (csrc/gemm_simt.cu).  Which of the two depends on the weight alone and either sums in
+  an order that the weight's shape fixes, so a row's bits do not depend on the others.
 * bfloat16 operands: float32 accumulation on the tensor cores.  Steps of up
   to 32 tokens (decode) go to the engine's own tcgen05 weight-streaming kernel,
   which takes up to 256 tokens but is the faster one only for few; larger
@@ -49,12 +52,40 @@ def gemm_simt(x: torch.Tensor, w: torch.Tensor, out_dtype: Optional[torch.dtype]
     return out
 
 
+F32_SPLIT_MIN = 128             # the fewest rows and columns of a weight
+
+
+def gemm_f32_takes(w: torch.Tensor) -> bool:
+    """float32, at least 128 x 128, rows of whole 16-byte pieces.  Below that a tile of 128 rows, or a sum of 32 values of
+    k, is mostly padding."""
+    return (w.dtype == torch.float32 and w.dim() == 2 and min(w.shape) >= F32_SPLIT_MIN and w.shape[1] % 4 == 0
+            and w.stride(1) == 1 and w.stride(0) % 4 == 0 and w.data_ptr() % 16 == 0)
+
+
+def gemm_f32(x: torch.Tensor, w: torch.Tensor, out_dtype: Optional[torch.dtype] = None) -> torch.Tensor:
+    """x [M, K] (float32 or bfloat16) . w [N, K]^T (float32) in 32 bits on the tensor cores; a row's bits depend on the row and w."""
+    name = "gemm_f32"
+    need_cuda(name, x, w)
+    need(gemm_f32_takes(w), name, "needs a float32 weight of at least 128 x 128, rows of whole 16-byte pieces")
+    need(x.dim() == 2 and x.shape[1] == w.shape[1], name, f"shapes {tuple(x.shape)} and {tuple(w.shape)} do not agree in K")
+    need(x.stride(1) == 1, name, "operands must be K-contiguous")
+    m, k = x.shape
+    n = w.shape[0]
+    out_dtype = out_dtype or x.dtype
+    out = torch.empty((m, n), dtype=out_dtype, device=x.device)
+    check(lib().yalis_gemm_f32_parts(ptr(x), i32(dtype_code(x.dtype)), i64(x.stride(0)), ptr(w), i64(w.stride(0)), ptr(out),
+                                     i32(dtype_code(out_dtype)), i64(n), i32(m), i32(n), i32(k), stream()), name)
+    return out
+
+
 def linear(x: torch.Tensor, w: torch.Tensor, out_dtype: Optional[torch.dtype] = None) -> torch.Tensor:
     """The projection used by the parts: picks the kernel by dtype and size (see module docstring)."""
     need_cuda("linear", x, w)
     out_dtype = out_dtype or x.dtype
     if x.dtype == torch.float32 or w.dtype == torch.float32:
         # the true 32-bit path, and a weight that its checkpoint stored in float32 (it stays so) under bfloat16 rows
+        if gemm_f32_takes(w):
+            return gemm_f32(x, w, out_dtype)
         return gemm_simt(x, w, out_dtype)
     need(x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16, "linear", "operands must be bfloat16 or float32")
     if wstream_preferred(x, w):
