@@ -1,0 +1,111 @@
+"""The recurrences by chunks of sixteen tokens: portions around a chunk's end beside short ones, every rule that goes this way, column
+tiles that are not full, against a float64 walk and beside the walk token by token."""
+
+import pytest
+import torch
+
+from test_state_scan_gpu import walk
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+RULES = ["constant", "token", "delta constant", "delta", "selective"]
+
+
+def inputs(rule, heads, kv_heads, vdim, lens, g, keep=0.5):
+    n, dim = sum(lens), 128
+    rnd = lambda *s: torch.randn(*s, generator=g)
+    q, k, v = rnd(n, kv_heads, dim) / dim ** 0.5, rnd(n, kv_heads, dim) / dim ** 0.5, rnd(n, heads, vdim)
+    if "delta" in rule:
+        k = torch.nn.functional.normalize(k, dim=-1)
+    rate = lambda *s: keep + (1 - keep) * torch.rand(*s, generator=g)
+    decay = rate(heads) if "constant" in rule else rate(n, heads)
+    beta = torch.rand(n, heads, generator=g) if "delta" in rule or rule == "selective" else None
+    skip = rnd(heads) if rule == "selective" else None
+    return q, k, v, decay, beta, skip
+
+
+def run(rule, lay, kv_heads, data, rows, lens, slots, chunks):
+    from yalis_b200.ops.recurrent import state_scan
+    q, k, v, decay, beta, skip = (None if t is None else t.to(DEV) for t in data)
+    starts = torch.tensor([0] + lens).cumsum(0).to(torch.int32).to(DEV)
+    return state_scan(q.flatten(1), k.flatten(1), v.flatten(1), rows, lay, starts, torch.tensor(slots, dtype=torch.int32, device=DEV),
+                      kv_heads=kv_heads, decay=decay, beta=beta, max_q_len=max(lens), selective=rule == "selective", skip=skip,
+                      chunks=chunks).view(-1, lay.heads, lay.vdim)
+
+
+def exact(rule, data, first, a, b, heads, kv_heads):
+    q, k, v, decay, beta, skip = (None if t is None else t.double() for t in data)
+    cut = lambda t: None if t is None else t[a:b]
+    d = decay.view(1, heads, 1).expand(b - a, heads, 1) if decay.dim() == 1 else decay[a:b, :, None]
+    wide = lambda t: t[a:b].repeat_interleave(heads // kv_heads, 1)
+    return walk(first, wide(q), wide(k), cut(v), d, cut(beta), None, None, rule == "selective", skip)
+
+
+@pytest.mark.parametrize("rule", RULES)
+@pytest.mark.parametrize("heads,kv_heads,vdim,keep", [(3, 3, 128, 0.5), (4, 2, 20, 0.9), (2, 1, 64, 0.999), (6, 1, 4, 0.0)])
+def test_against_a_walk(rule, heads, kv_heads, vdim, keep):
+    from yalis_b200.ops.recurrent import StateLayout
+    g = torch.Generator().manual_seed(heads * vdim)
+    from yalis_b200.ops.recurrent import CHUNKS_FROM
+    f = CHUNKS_FROM[{"selective": 3}.get(rule, int("delta" in rule))]
+    lens, slots = [1, f, f + 1, f - 1, 0, f + 72, f + 15, 17], [3, 0, 7, 1, 5, 2, 4, 6]
+    lay = StateLayout(heads, 128, vdim, conv_channels=3, taps=3)
+    data = inputs(rule, heads, kv_heads, vdim, lens, g, keep)
+    rows = torch.randn(9, lay.total, generator=g)
+    got_rows, plain_rows = rows.to(DEV), rows.to(DEV)
+    got = run(rule, lay, kv_heads, data, got_rows, lens, slots, True)
+    plain = run(rule, lay, kv_heads, data, plain_rows, lens, slots, False)
+    state = lambda r, i: r[slots[i], :lay.state_floats].cpu().view(heads, vdim, 128).double().transpose(1, 2)
+    a = 0
+    for i, l in enumerate(lens):
+        b = a + l
+        if l < f:                                  # left to the walk token by token
+            assert torch.equal(got[a:b], plain[a:b]) and torch.equal(got_rows[slots[i]], plain_rows[slots[i]])
+        else:
+            want, last = exact(rule, data, state(rows, i), a, b, heads, kv_heads)
+            err, err0 = (got[a:b].cpu().double() - want).norm() / want.norm(), (plain[a:b].cpu().double() - want).norm() / want.norm()
+            # 32-bit sums of 128 terms carried over up to 600 tokens
+            assert err < 1e-6, (i, err, err0)
+            assert (state(got_rows, i) - last).norm() < 1e-6 * last.norm(), i
+            alone_rows = rows.to(DEV)
+            alone = run(rule, lay, kv_heads, [None if t is None else t if t.dim() == 1 else t[a:b] for t in data], alone_rows, [l], [slots[i]], True)
+            assert torch.equal(alone, got[a:b]) and torch.equal(alone_rows[slots[i]], got_rows[slots[i]])
+        a = b
+    assert torch.equal(got_rows[8], rows[8].to(DEV))
+    tail = got_rows[:, lay.state_floats:].cpu()
+    assert torch.equal(tail, rows[:, lay.state_floats:])
+
+
+@pytest.mark.parametrize("rule", RULES)
+def test_a_long_portion_is_no_further_off_than_the_walk(rule):
+    """2,048 tokens with slow decays: what a rounded decay per chunk would add up to."""
+    from yalis_b200.ops.recurrent import StateLayout
+    g = torch.Generator().manual_seed(5)
+    heads, vdim, n = 4, 32, 2048
+    lay = StateLayout(heads, 128, vdim)
+    data = inputs(rule, heads, heads, vdim, [n], g, 0.995)
+    if "constant" in rule:
+        data = data[:3] + (torch.tensor([0.9993, 0.99, 0.9999, 1.0]),) + data[4:]
+    want, last = exact(rule, data, torch.zeros(heads, 128, vdim, dtype=torch.float64), 0, n, heads, heads)
+    errors = []
+    for chunks in (True, False):
+        rows = torch.zeros(1, lay.total, device=DEV)
+        got = run(rule, lay, heads, data, rows, [n], [0], chunks).cpu().double()
+        kept = rows[0, :lay.state_floats].cpu().view(heads, vdim, 128).double().transpose(1, 2)
+        errors.append((float((got - want).norm() / want.norm()), float((kept - last).norm() / last.norm())))
+    print(rule, errors)
+    assert errors[0][0] < max(1.1 * errors[1][0], 3e-7) and errors[0][1] < max(1.1 * errors[1][1], 3e-7), errors
+
+
+def test_what_is_not_finite_reaches_later_tokens_only():
+    from yalis_b200.ops.recurrent import StateLayout
+    g = torch.Generator().manual_seed(1)
+    lay, n = StateLayout(2, 128, 32), 528
+    for rule in RULES:
+        data = inputs(rule, 2, 2, 32, [n], g)
+        plain = run(rule, lay, 2, data, torch.zeros(1, lay.total, device=DEV), [n], [0], True)
+        v = data[2].clone()
+        v[70, 1, 5] = float("inf")
+        got = run(rule, lay, 2, data[:2] + (v,) + data[3:], torch.zeros(1, lay.total, device=DEV), [n], [0], True)
+        assert torch.equal(got[:70], plain[:70]) and torch.equal(got[:, 0], plain[:, 0])
+        assert torch.equal(got[:, 1, :5], plain[:, 1, :5]) and not bool(got[70:, 1, 5].isfinite().any())

@@ -129,7 +129,7 @@ class Retention(_ProjectedMixer):
         else:
             q, k, v = self._rotated(z, ctx)
         o = rec_ops.state_scan(q, k, v, cache.state, self.layout, ctx.q_start, ctx.slots, kv_heads=self.h, decay=self.decay,
-                               max_q_len=ctx.host.max_q_len)
+                               max_q_len=ctx.host.max_q_len, chunks=z.dtype == torch.bfloat16)
         if self.norm_kind == "all":
             rec_ops.gate_norm(o, gate, 1, self.norm_w, self.eps, ctx.req_of_token, y, out_scale=self.out_scale,
                               gate_kind=self.gate_kind, after=True)
@@ -226,7 +226,8 @@ class GatedDelta(_ProjectedMixer):
             dt_bias=self.dt_bias, b_raw=self._block(z, "b"),
             single_tokens=ctx.host.max_q_len == 1)
         o = rec_ops.state_scan(conv[:, :gd], conv[:, gd:2 * gd], conv[:, 2 * gd:], cache.state, self.layout, ctx.q_start,
-                               ctx.slots, kv_heads=self.g, decay=decay, beta=beta, max_q_len=ctx.host.max_q_len)
+                               ctx.slots, kv_heads=self.g, decay=decay, beta=beta, max_q_len=ctx.host.max_q_len,
+                               chunks=z.dtype == torch.bfloat16)
         if self.gate_kind == "silu":
             gate, kind = self._block(z, "g"), rec_ops.GATE_SILU
         else:
@@ -357,7 +358,7 @@ class StateSpace(_ProjectedMixer):
         b, c = self.inner, self.inner + self.g * self.n
         o = rec_ops.state_scan(conv[:, c:], conv[:, b:c], conv[:, :b], cache.state, self.layout, ctx.q_start, ctx.slots,
                                kv_heads=self.g, decay=decay, beta=step, selective=True, skip=self.skip,
-                               max_q_len=ctx.host.max_q_len)
+                               max_q_len=ctx.host.max_q_len, chunks=z.dtype == torch.bfloat16)
         rec_ops.gate_norm(o, blk("z"), self.parts, self.norm_w, self.eps, ctx.req_of_token, y, out_scale=self.out_scale)
 
 
