@@ -109,3 +109,18 @@ def test_what_is_not_finite_reaches_later_tokens_only():
         got = run(rule, lay, 2, data[:2] + (v,) + data[3:], torch.zeros(1, lay.total, device=DEV), [n], [0], True)
         assert torch.equal(got[:70], plain[:70]) and torch.equal(got[:, 0], plain[:, 0])
         assert torch.equal(got[:, 1, :5], plain[:, 1, :5]) and not bool(got[70:, 1, 5].isfinite().any())
+
+
+def test_a_query_that_is_not_finite_reaches_its_own_token_only():
+    """The dot products of a chunk's tokens are formed from parts, which an infinity does not have."""
+    from yalis_b200.ops.recurrent import StateLayout
+    g = torch.Generator().manual_seed(2)
+    lay, n = StateLayout(2, 128, 32), 203
+    for rule in RULES:
+        data = inputs(rule, 2, 2, 32, [n], g)
+        plain = run(rule, lay, 2, data, torch.zeros(1, lay.total, device=DEV), [n], [0], True)
+        q = data[0].clone()
+        q[70, 1, 5] = float("inf")
+        got = run(rule, lay, 2, (q,) + data[1:], torch.zeros(1, lay.total, device=DEV), [n], [0], True)
+        assert torch.equal(got[:70], plain[:70]) and torch.equal(got[71:], plain[71:]) and torch.equal(got[:, 0], plain[:, 0])
+        assert not bool(got[70, 1].isfinite().any())

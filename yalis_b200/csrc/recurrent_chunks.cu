@@ -17,13 +17,18 @@
 // A chunk starts where its request's portion starts: a long portion's results depend on how the request was cut, by rounding.
 // Errors against float64 beside the walk's (2,048 tokens, slow decays, read-outs / state): constant decay 1.9e-7 / 7.7e-7 (2.0e-7 /
 // 9.4e-7), delta rule 1.4e-7 / 3.6e-7 (1.1e-7 / 3.6e-7), selective 0.7e-7 / 2.2e-7 (1.1e-7 / 5.0e-7).
-// What bounds it: for one request the chain of a chunk, some 2,000 cycles: parts of the state, two products, two small sums, the
-// state's products; for several the copies of k and q, which the blocks of a head's columns all ask for (3 TB/s).
-// Measured (us, walk token by token -> both kernels), 16 heads of 128 x 128 (selective: 32 of 128 x 64): delta rule 1 x 2,048
-// 382 -> 186, 1 x 128 26 -> 24, 4 x 901 357 -> 246, 32 x 128 346 -> 270; plain 1 x 2,048 251 -> 145, 4 x 901 217 -> 194,
-// 8 x 512 214 -> 225, 32 x 128 195 -> 224; selective 1 x 2,048 256 -> 135, 32 x 128 211 -> 207.
-// Not taken: eight row warps (1 x 2,048: 179, 4 x 901: 321), 32 columns a block (304 and 294), two chunks in shared memory (253 and 304),
-// four (no gain), k and q copied in pieces whose order differs from block to block (236).
+// What bounds it: for one request the instructions of a chunk's chain, some 1,600 cycles by the delta rule: a warp alone on its
+// scheduler issues one in about four cycles (clock counts between the chain's stages), so sums start from no cleared
+// registers, the six products of parts are one chain, pairs of float32 operations go in one instruction, and what the chain does not
+// need is left to other warps: waiting for copies, by the delta rule the products with q.  For several requests the copies of k and q,
+// which the blocks of a head's columns all ask for.
+// Measured (us, walk token by token -> both kernels; before copies ran up to four chunks ahead and the chain was shortened), 16
+// heads of 128 x 128 (delta rule: 8 key heads; selective: 32 of 128 x 64), L2 flushed: delta rule 1 x 2,048 387 -> 155 (196),
+// 1 x 128 31 -> 26 to 33 (28), 4 x 901 363 -> 244 (259), 32 x 128 352 -> 259 (282); plain 1 x 2,048 257 -> 108 (155), 4 x 901 224 -> 171 (208),
+// 8 x 512 221 -> 196 (237), 32 x 128 202 -> 200 (234); selective 1 x 2,048 261 -> 99 (144), 4 x 901 237 -> 153 (187), 32 x 128 217 -> 172 (206).
+// Not taken: eight row warps and 32 columns a block (for several requests no gain: 282 and 218 for 4 x 901), two chunks in
+// shared memory, k and q copied in pieces whose order differs from block to block, the products with q by the reading warps in the
+// other rules too (1 x 2,048 plain 175, 4 x 901 214: those warps become the chain).
 #include "common.cuh"
 
 namespace {
@@ -58,17 +63,6 @@ __device__ __forceinline__ uint32_t two_bf16(float lo, float hi) {
   __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
   return *reinterpret_cast<uint32_t*>(&v);
 }
-// Two values as three pairs of bfloat16 values whose sums they are.
-__device__ __forceinline__ void part2(float a, float b, uint32_t (&o)[3]) {
-#pragma unroll
-  for (int i = 0; i < 3; ++i) {
-    o[i] = two_bf16(a, b);
-    if (i < 2) {
-      a -= __uint_as_float(o[i] << 16);
-      b -= __uint_as_float(o[i] & 0xffff0000u);
-    }
-  }
-}
 __device__ __forceinline__ void ldmatrix4(uint32_t (&r)[4], uint32_t addr) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
 }
@@ -78,6 +72,29 @@ __device__ __forceinline__ void ldmatrix4_trans(uint32_t (&r)[4], uint32_t addr)
 __device__ __forceinline__ void mma(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
   asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+// The same from zero: no registers are cleared first.
+__device__ __forceinline__ void mma0(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+               : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.f));
+}
+// The parts of a product's operands, small products first: (2, 0), (0, 2), (1, 1), (1, 0), (0, 1), (0, 0).
+__device__ __forceinline__ constexpr int first_part(int o) { return o == 0 ? 2 : o == 2 || o == 3 ? 1 : 0; }
+__device__ __forceinline__ constexpr int second_part(int o) { return o == 1 ? 2 : o == 2 || o == 4 ? 1 : 0; }
+// Two float32 operations in one instruction, each rounded as the single one is.
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  uint64_t d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(*reinterpret_cast<uint64_t*>(&a)), "l"(*reinterpret_cast<uint64_t*>(&b)), "l"(*reinterpret_cast<uint64_t*>(&c)));
+  return *reinterpret_cast<float2*>(&d);
+}
+// Two values as three pairs of bfloat16 values whose sums they are.
+__device__ __forceinline__ void part2(float a, float b, uint32_t (&o)[3]) {
+  float2 x = make_float2(a, b);
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    o[i] = two_bf16(x.x, x.y);
+    if (i < 2) x = fma2(make_float2(__uint_as_float(o[i] << 16), __uint_as_float(o[i] & 0xffff0000u)), make_float2(-1.f, -1.f), x);
+  }
 }
 constexpr uint32_t kSpinLimit = 1u << 22;      // polls of a wait before the block gives up
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -101,9 +118,7 @@ __device__ __forceinline__ void copy16(void* to, const void* from, bool there) {
 // A block per chunk, key head and request: parts of k and q, the dot products, then a warp per head of the group.
 template <int RULE>
 __global__ void __launch_bounds__(kWarps * 32) chunk_prepare_kernel(const ChunkParams p) {
-  constexpr int LD = kD + 4;
-  __shared__ __align__(16) float ks[kC * LD];
-  __shared__ __align__(16) float qs[kC * LD];
+  __shared__ __align__(128) __nv_bfloat16 ps_s[6 * kPart];                     // parts of k, then of q, as they go to memory
   __shared__ float kk[kC * kC], qk[kC * kC], ratio[kWarps][kC * kC];
   pdl_launch_dependents();
   pdl_wait();
@@ -121,33 +136,58 @@ __global__ void __launch_bounds__(kWarps * 32) chunk_prepare_kernel(const ChunkP
       x[0] = load4_f32(from);
       x[1] = load4_f32(from + 4);
     }
-    float* to = (which ? qs : ks) + t * LD + c * 8;
-    store4(to, x[0]);
-    store4(to + 4, x[1]);
     uint32_t o[4][3];
     part2(x[0].x, x[0].y, o[0]); part2(x[0].z, x[0].w, o[1]); part2(x[1].x, x[1].y, o[2]); part2(x[1].z, x[1].w, o[3]);
 #pragma unroll
-    for (int i = 0; i < 3; ++i)
-      *reinterpret_cast<uint4*>(parts + (which * 3 + i) * kPart + t * kD + ((c ^ (t & 7)) * 8)) = make_uint4(o[0][i], o[1][i], o[2][i], o[3][i]);
+    for (int i = 0; i < 3; ++i) {
+      const int at = (which * 3 + i) * kPart + t * kD + ((c ^ (t & 7)) * 8);
+      const uint4 piece = make_uint4(o[0][i], o[1][i], o[2][i], o[3][i]);
+      *reinterpret_cast<uint4*>(parts + at) = piece;
+      *reinterpret_cast<uint4*>(ps_s + at) = piece;
+    }
   }
   __syncthreads();
-  {
-    // two tokens by two, four sums of 32 products each: half of the threads for q k, the others for k k
-    const int t = tid % 64 / 8 * 2, s = tid % 8 * 2;
-    const float* xs = tid < 64 ? qs : ks;
-    if (s <= t + 1 && (RULE == 1 || tid < 64)) {
-      float4 a[4] = {};
-      auto add = [](float4& c, const float4& x, const float4& y) {
-        c.x = __fmaf_rn(x.x, y.x, c.x); c.y = __fmaf_rn(x.y, y.y, c.y); c.z = __fmaf_rn(x.z, y.z, c.z); c.w = __fmaf_rn(x.w, y.w, c.w);
-      };
-#pragma unroll 4
-      for (int d = 0; d < kD; d += 4) {
-        const float4 x0 = load4_f32(xs + t * LD + d), x1 = load4_f32(xs + (t + 1) * LD + d);
-        const float4 y0 = load4_f32(ks + s * LD + d), y1 = load4_f32(ks + (s + 1) * LD + d);
-        add(a[0], x0, y0); add(a[1], x0, y1); add(a[2], x1, y0); add(a[3], x1, y1);
-      }
+  if (RULE == 1 || warp < 2) {
+    // q k by two warps, k k by two, eight of the second operand's tokens each: sums of 16 products, small ones first, added in order
+    const bool qk_here = warp < 2;
+    const int s0 = (warp & 1) * 8;
+    const uint32_t as = smem_u32(ps_s) + (qk_here ? 3 * kPart * 2 : 0) + (lane & 15) * (kD * 2);
+    const uint32_t bs = smem_u32(ps_s) + (s0 + (lane & 7)) * (kD * 2);
+    float sum[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-      for (int i = 0; i < 4; ++i) (tid < 64 ? qk : kk)[(t + i / 2) * kC + s + i % 2] = (a[i].x + a[i].y) + (a[i].z + a[i].w);
+    for (int j = 0; j < kD / 32; ++j) {                            // 32 values
+      uint32_t fa[3][2][4], fb[3][4];
+#pragma unroll
+      for (int i = 0; i < 3; ++i) {
+        ldmatrix4(fb[i], bs + i * kPart * 2 + (((4 * j + (lane >> 3)) ^ (lane & 7)) << 4));
+#pragma unroll
+        for (int n = 0; n < 2; ++n) ldmatrix4(fa[i][n], as + i * kPart * 2 + (((4 * j + 2 * n + (lane >> 4)) ^ (lane & 7)) << 4));
+      }
+      float more[2][4];
+#pragma unroll
+      for (int o = 0; o < 6; ++o)
+#pragma unroll
+        for (int n = 0; n < 2; ++n) {
+          const uint32_t(&b)[4] = fb[second_part(o)];
+          if (o == 0) mma0(more[n], fa[first_part(o)][n], b[2 * n], b[2 * n + 1]);
+          else mma(more[n], fa[first_part(o)][n], b[2 * n], b[2 * n + 1]);
+        }
+#pragma unroll
+      for (int n = 0; n < 2; ++n)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) sum[e] += more[n][e];
+    }
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int t = (lane >> 2) + 8 * (e >> 1), s = s0 + 2 * (lane & 3) + (e & 1);
+      if (!(fabsf(sum[e]) <= 3.402823466e38f) && t < valid && s < valid) {      // what parts cannot hold: infinities, the largest values
+        const float* x = (qk_here ? p.q + (size_t)(t0 + t) * p.q_stride : p.k + (size_t)(t0 + t) * p.k_stride) + kvh * kD;
+        const float* y = p.k + (size_t)(t0 + s) * p.k_stride + kvh * kD;
+        float z = 0.f;
+        for (int d = 0; d < kD; ++d) z = __fmaf_rn(x[d], y[d], z);
+        sum[e] = z;
+      }
+      (qk_here ? qk : kk)[t * kC + s] = sum[e];
     }
   }
   __syncthreads();
@@ -201,70 +241,117 @@ __global__ void __launch_bounds__(kWarps * 32) chunk_prepare_kernel(const ChunkP
 }
 
 // A block per 16 columns of a head and request.  Four warps walk: each has 32 rows of the state.  Four
-// more form the read-outs of a chunk while those are at the next, one fetches.  All meet once per chunk, when its u are there;
-// everything that the read-outs need lies in two buffers.  Shared memory: stages of (k and q in parts, coefficients, v
-// [t][column]), the row warps' shares of S^T q [buffer][row warp][t][column] and of S^T k, u [buffer][column][t], v - G S^T k
-// [column][t], u P_16 in parts [buffer][part][t][column].
-constexpr int kV = 16, kRowWarps = 4, kStages = 3;                      // columns of a block, row warps, chunks in shared memory
-constexpr int kReaders = 4, kWalk = kRowWarps * 32, kAll = kWalk + (kReaders + 1) * 32;
-constexpr int kLdV = kV + 4, kLdT = kC + 4, kShares = kC * kLdV;
+// more form the read-outs of a chunk while those are at the next, from the state's parts that the walking warps leave
+// them, one fetches.  All meet once per chunk, when its u are there.  Shared memory: stages of (k and q in parts, coefficients, v
+// [t][column]), the state in parts as operands [row warp][part][tile][lane], the row warps' shares of S^T q [row warp][t][column] and of S^T k,
+// u [buffer][column][t], v - G S^T k [column][t], u P_16 in parts [buffer][part][t][column].
+constexpr int kV = 16, kRowWarps = 4;                                   // columns of a block, row warps
+constexpr int kWalk = kRowWarps * 32, kAll = 2 * kWalk + 32;            // threads that walk (as many form read-outs), of the block
+constexpr int kRowTiles = kD / (16 * kRowWarps), kStateParts = kRowWarps * 3 * kRowTiles * 32;      // a warp's rows, sixteen at a time; 16-byte pieces
+constexpr int kLdT = kC + 4, kShares = kV * kLdT;                       // floats between a column's tokens and the next one's
 constexpr int kStage = (6 * kPart * 2 + kCoef * 4 + kC * kV * 4 + 127) / 128 * 128;
-template <int RULE>
+template <int RULE, int STAGES>
 constexpr size_t walk_smem() {
-  return kStages * kStage + (kRowWarps * (RULE == 1 ? 3 : 2) * kShares + (RULE == 1 ? 3 : 2) * kV * kLdT) * sizeof(float) + 2 * 3 * kC * kV * 2 + kStages * 8 + 16;
+  return STAGES * kStage + (RULE == 1 ? kStateParts * 16 : 0) + (2 * kRowWarps * kShares + (RULE == 1 ? 3 : 2) * kV * kLdT) * sizeof(float) + 2 * 3 * kC * kV * 2 + STAGES * 8 + 16;
 }
 template <int ID, int N>
 __device__ __forceinline__ void meet() { asm volatile("bar.sync %0, %1;" ::"n"(ID), "n"(N) : "memory"); }
+constexpr int kMeetAll = 0, kMeetWalk = 1, kMeetRead = 2, kMeetTaken = 3;
 
 // Sums over the tokens up to t of a coefficient times a column's value: later ones take no part, be they infinite.
-__device__ __forceinline__ float upto(const float* m, const float* y, int t) {
-  float a = 0.f, b = 0.f;
+__device__ __forceinline__ void load_row(const float* m, float (&c)[kC]) {
 #pragma unroll
   for (int s = 0; s < kC; s += 4) {
-    const float4 c = load4_f32(m + s), x = load4_f32(y + s);
-    a = __fmaf_rn(c.x, s > t ? 0.f : x.x, a); b = __fmaf_rn(c.y, s + 1 > t ? 0.f : x.y, b);
-    a = __fmaf_rn(c.z, s + 2 > t ? 0.f : x.z, a); b = __fmaf_rn(c.w, s + 3 > t ? 0.f : x.w, b);
+    const float4 x = load4_f32(m + s);
+    c[s] = x.x; c[s + 1] = x.y; c[s + 2] = x.z; c[s + 3] = x.w;
+  }
+}
+__device__ __forceinline__ float upto(const float (&c)[kC], const float (&y)[kC], int t) {
+  float a = 0.f, b = 0.f;
+#pragma unroll
+  for (int s = 0; s < kC; s += 2) {
+    if (s <= t) a = __fmaf_rn(c[s], y[s], a);
+    if (s + 1 <= t) b = __fmaf_rn(c[s + 1], y[s + 1], b);
   }
   return a + b;
 }
 
-template <int RULE>
-__global__ void __launch_bounds__(kAll) chunk_walk_kernel(const ChunkParams p) {
-  constexpr int NJ = kD / (16 * kRowWarps);                           // a warp's rows, sixteen at a time
+// A warp's rows of the state, transposed and in parts, times 16 tokens' vectors in parts at `from`: its share of S^T k or S^T q.
+__device__ __forceinline__ void read_state(const uint32_t (&fs)[3][kRowTiles][4], uint32_t from, float* to, int warp, int lane) {
+  constexpr int NJ = kRowTiles;
+  const int lt = (lane & 7) + (lane >> 4) * 8;                 // ldmatrix: tokens 0-7 by two pieces, tokens 8-15 by two
+  uint32_t f[3][NJ][4];
+#pragma unroll
+  for (int i = 0; i < 3; ++i)
+#pragma unroll
+    for (int j = 0; j < NJ; ++j)
+      ldmatrix4(f[i][j], from + i * kPart * 2 + lt * (kD * 2) + (((2 * NJ * warp + 2 * j + ((lane >> 3) & 1)) ^ (lt & 7)) << 4));
+  float sum[NJ][2][4];
+#pragma unroll
+  for (int o = 0; o < 6; ++o)
+#pragma unroll
+    for (int j = 0; j < NJ; ++j)
+#pragma unroll
+      for (int n = 0; n < 2; ++n) {
+        const uint32_t(&b)[4] = f[second_part(o)][j];
+        if (o == 0) mma0(sum[j][n], fs[first_part(o)][j], b[2 * n], b[2 * n + 1]);
+        else mma(sum[j][n], fs[first_part(o)][j], b[2 * n], b[2 * n + 1]);
+      }
+#pragma unroll
+  for (int n = 0; n < 2; ++n)
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {                              // columns lane / 4 and 8 further; two tokens
+      float2 y = make_float2(sum[0][n][2 * e], sum[0][n][2 * e + 1]);
+#pragma unroll
+      for (int j = 1; j < NJ; ++j) {
+        y.x += sum[j][n][2 * e];
+        y.y += sum[j][n][2 * e + 1];
+      }
+      *reinterpret_cast<float2*>(to + ((lane >> 2) + 8 * e) * kLdT + 8 * n + 2 * (lane & 3)) = y;
+    }
+}
+
+template <int RULE, int STAGES>
+__global__ void __launch_bounds__(kAll, STAGES == 3 ? 2 : 1) chunk_walk_kernel(const ChunkParams p) {
+  constexpr int NJ = kRowTiles;
+  constexpr bool EARLY = STAGES > 3;                                  // who waits for a chunk's copies: the warp that fetches, or the walking ones
   extern __shared__ __align__(128) unsigned char smem[];
   pdl_launch_dependents();
   pdl_wait();
   const int req = blockIdx.z, h = blockIdx.y, j0 = blockIdx.x * kV, start = p.q_start[req], len = p.q_start[req + 1] - start;
   if (len < p.shortest) return;
-  const int tid = threadIdx.x, lane = tid & 31, kvh = h / (p.heads / p.kv_heads);
+  const int role = threadIdx.x / kWalk, tid = threadIdx.x % kWalk;      // role 0 walks, 1 reads, 2 fetches
+  const int lane = tid & 31, kvh = h / (p.heads / p.kv_heads);
   const int chunks = (len + kC - 1) / kC;
   const size_t first = first_chunk(start, req);
-  float* shares_q = reinterpret_cast<float*>(smem + kStages * kStage);
-  float* shares_k = shares_q + 2 * kRowWarps * kShares;
-  float* us = shares_k + (RULE == 1 ? kRowWarps * kShares : 0);
+  uint4* state_parts = reinterpret_cast<uint4*>(smem + STAGES * kStage);
+  float* shares_q = reinterpret_cast<float*>(state_parts + (RULE == 1 ? kStateParts : 0));      // RULE 1: one buffer
+  float* shares_k = shares_q + kRowWarps * kShares;                                             // RULE 1
+  float* us = shares_q + 2 * kRowWarps * kShares;
   float* rest = us + 2 * kV * kLdT;
   __nv_bfloat16* ups = reinterpret_cast<__nv_bfloat16*>(rest + (RULE == 1 ? kV * kLdT : 0));
   uint64_t* there = reinterpret_cast<uint64_t*>(ups + 2 * 3 * kC * kV);
-  volatile int* lost = reinterpret_cast<volatile int*>(there + kStages);      // a wait for chunk c ran out: [c & 1]
-  if (tid == 0) {
-    for (int s = 0; s < kStages; ++s) asm volatile("mbarrier.init.shared::cta.b64 [%0], 33;" ::"r"(smem_u32(&there[s])));      // lane 0 and every lane's copies
+  volatile int* lost = reinterpret_cast<volatile int*>(there + STAGES);      // a wait ran out
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < STAGES; ++s) asm volatile("mbarrier.init.shared::cta.b64 [%0], 33;" ::"r"(smem_u32(&there[s])));      // lane 0 and every lane's copies
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    lost[0] = lost[1] = 0;
+    *lost = 0;
   }
   __syncthreads();
-  auto coef_of = [&](int c) { return reinterpret_cast<const float*>(smem + c % kStages * kStage + 6 * kPart * 2); };
-  auto await = [&](int c) {                                    // a whole warp
-    if (lane == 0 && !copies_there(&there[c % kStages], (c / kStages) & 1)) lost[c & 1] = 1;
+  auto coef_of = [&](int c) { return reinterpret_cast<const float*>(smem + c % STAGES * kStage + 6 * kPart * 2); };
+  // A wait that runs out ends neither the copies nor the meetings; what is formed then is dropped at the end.
+  auto await = [&](int c) {
+    if (c < chunks && !copies_there(&there[c % STAGES], (c / STAGES) & 1)) *lost = 1;
     __syncwarp();
   };
 
-  if (tid >= kWalk + kReaders * 32) {
+  if (role == 2) {
     // One copy each for the parts and the coefficients; the values 16 bytes at a time, zeros behind the portion's end and the last
     // column (a bulk copy for every row of 64 bytes took longer than all else).
     auto fetch = [&](int c) {
       if (c >= chunks) return;
-      unsigned char* to = smem + c % kStages * kStage;
-      uint64_t* bar = &there[c % kStages];
+      unsigned char* to = smem + c % STAGES * kStage;
+      uint64_t* bar = &there[c % STAGES];
       if (lane == 0) {
         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(6 * kPart * 2 + kCoef * 4) : "memory");
         copy_bulk(to, p.parts + ((first + c) * p.kv_heads + kvh) * (6 * kPart), 6 * kPart * 2, bar);
@@ -279,38 +366,57 @@ __global__ void __launch_bounds__(kAll) chunk_walk_kernel(const ChunkParams p) {
       }
       asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
     };
-    for (int c = 0; c < kStages - 1; ++c) fetch(c);
+    for (int c = 0; c < STAGES - 1; ++c) fetch(c);
+    // EARLY: it waits for a chunk's copies before it joins the meeting of the chunk before: past that they are there for all.
+    if constexpr (EARLY) await(0);
+    meet<kMeetAll, kAll>();
     for (int c = 0; c < chunks; ++c) {
-      meet<0, kAll>();                                          // everyone is done with the chunk before
-      if (lost[c & 1]) {
-        // (what was asked for and not waited for ends before the block does)
-        for (int n = c; n < min(c + kStages - 1, chunks); ++n) copies_there(&there[n % kStages], (n / kStages) & 1);
-        if (lane == 0) atomicOr(p.error, YALIS_FLAG_WAIT_PRODUCT);
-        break;
-      }
-      fetch(c + kStages - 1);
+      if constexpr (EARLY) await(c + 1);
+      meet<kMeetAll, kAll>();                                   // everyone is done with the chunk before
+      fetch(c + STAGES - 1);
     }
+    // (all copies end before the block does, also those that a wait gave up on)
+    for (int c = max(0, chunks - STAGES); c < chunks; ++c) copies_there(&there[c % STAGES], (c / STAGES) & 1);
+    __syncwarp();
+    if (lane == 0 && *lost) atomicOr(p.error, YALIS_FLAG_WAIT_PRODUCT);
     return;
   }
 
-  if (tid >= kWalk) {
+  if (role == 1) {
     // read-outs: a thread has CPT columns of a token
-    constexpr int CPT = kC * kV / (kReaders * 32);
-    const int rt = tid - kWalk, t = rt / (kV / CPT), v0 = rt % (kV / CPT) * CPT;
+    constexpr int CPT = kC * kV / kWalk;
+    const int rt = tid, t = rt / (kV / CPT), v0 = rt % (kV / CPT) * CPT;
     const float skip = (RULE == 3 && p.skip) ? p.skip[h] : 0.f;
+    meet<kMeetAll, kAll>();
     for (int c = 0; c < chunks; ++c) {
-      await(c);
-      meet<0, kAll>();
-      if (lost[c & 1]) break;
+      meet<kMeetAll, kAll>();
+      const float* shares = shares_q + (RULE == 1 ? 0 : (c & 1) * kRowWarps * kShares);
+      if constexpr (RULE == 1) {
+        const int rw = rt / 32;
+        uint32_t fs[3][kRowTiles][4];
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+#pragma unroll
+          for (int j = 0; j < kRowTiles; ++j) {
+            const uint4 x = state_parts[((rw * 3 + i) * kRowTiles + j) * 32 + lane];
+            fs[i][j][0] = x.x; fs[i][j][1] = x.y; fs[i][j][2] = x.z; fs[i][j][3] = x.w;
+          }
+        if (c + 1 < chunks) asm volatile("bar.arrive %0, %1;" ::"n"(kMeetTaken), "n"(2 * kWalk) : "memory");
+        read_state(fs, smem_u32(smem + c % STAGES * kStage) + 3 * kPart * 2, shares_q + rw * kShares, rw, lane);
+        meet<kMeetRead, kWalk>();
+      }
       const float* coef = coef_of(c);
       const float g = coef[kCoefG + t];
-      float o[CPT];
+      float o[CPT], row_t[kC];
+      load_row(coef + kCoefM + t * kC, row_t);
 #pragma unroll
       for (int i = 0; i < CPT; ++i) {
         float read = 0.f;
 #pragma unroll
-        for (int w = 0; w < kRowWarps; ++w) read += shares_q[((c & 1) * kRowWarps + w) * kShares + t * kLdV + v0 + i];
-        o[i] = __fmaf_rn(g, read, upto(coef + kCoefM + t * kC, us + ((c & 1) * kV + v0 + i) * kLdT, t));
+        for (int w = 0; w < kRowWarps; ++w) read += shares[w * kShares + (v0 + i) * kLdT + t];
+        float y[kC];
+        load_row(us + ((c & 1) * kV + v0 + i) * kLdT, y);
+        o[i] = __fmaf_rn(g, read, upto(row_t, y, t));
         if constexpr (RULE == 3) o[i] = __fmaf_rn(skip, coef[kCoef + t * kV + v0 + i], o[i]);
       }
       if (c * kC + t < len && j0 + v0 < p.vdim) {
@@ -326,144 +432,138 @@ __global__ void __launch_bounds__(kAll) chunk_walk_kernel(const ChunkParams p) {
   // the state, transposed: a lane's columns are col and col + 8, its rows row + 8 n and the one after
   const int col = lane >> 2, row = 16 * NJ * warp + 2 * (lane & 3);
   float* sp = p.state + (size_t)p.slots[req] * p.slot_stride + ((size_t)h * p.vdim + j0 + col) * kD + row;
-  float S[2 * NJ][4];
+  float2 S[2 * NJ][2];
 #pragma unroll
   for (int n = 0; n < 2 * NJ; ++n)
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
-      const float2 x = j0 + col + 8 * e < p.vdim ? *reinterpret_cast<const float2*>(sp + (size_t)e * 8 * kD + 8 * n) : make_float2(0.f, 0.f);
-      S[n][2 * e] = x.x; S[n][2 * e + 1] = x.y;
+      S[n][e] = j0 + col + 8 * e < p.vdim ? *reinterpret_cast<const float2*>(sp + (size_t)e * 8 * kD + 8 * n) : make_float2(0.f, 0.f);
     }
-  // parts (of the first operand, of the second), small products first, in two chains that are added: (2, 0), (1, 1), (1, 0) and
-  // (0, 2), (0, 1), (0, 0)
-  constexpr int order[2][3][2] = {{{2, 0}, {1, 1}, {1, 0}}, {{0, 2}, {0, 1}, {0, 0}}};
-  constexpr int CPT = kC * kV / kWalk;                           // a thread's columns of a token in the small sums
-  const int t = tid / (kV / CPT), v0 = tid % (kV / CPT) * CPT;
-  const int lt = (lane & 7) + (lane >> 4) * 8;                 // ldmatrix: tokens 0-7 by two pieces, tokens 8-15 by two
+  static_assert(kC * kV == 2 * kWalk, "two tokens of a column a thread");
+  const int v = tid % kV, t = tid / kV * 2;                     // a thread's column, and its first token, in the small sums
   const int tt = (lane & 7) + ((lane >> 3) & 1) * 8;           // ldmatrix: two halves of the tokens by a piece, then by the next
 
-  bool whole = true;
+  meet<kMeetAll, kAll>();                                             // the first chunk is there
   for (int c = 0; c < chunks; ++c) {
-    // S^T k and S^T q over this warp's rows
+    // the state in parts: for S^T k here and S^T q by the reading warps, or for S^T q
     uint32_t fs[3][NJ][4];
 #pragma unroll
     for (int j = 0; j < NJ; ++j)
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         uint32_t o[3];
-        part2(S[2 * j + (i >> 1)][2 * (i & 1)], S[2 * j + (i >> 1)][2 * (i & 1) + 1], o);
+        part2(S[2 * j + (i >> 1)][i & 1].x, S[2 * j + (i >> 1)][i & 1].y, o);
         fs[0][j][i] = o[0]; fs[1][j][i] = o[1]; fs[2][j][i] = o[2];
       }
-    await(c);
-    const uint32_t ks = smem_u32(smem + c % kStages * kStage), qs = ks + 3 * kPart * 2;
+    const uint32_t ks = smem_u32(smem + c % STAGES * kStage), qs = ks + 3 * kPart * 2;
     const float* coef = coef_of(c);
     const float* vs = coef + kCoef;
-    auto read = [&](uint32_t from, float* to) {
-      uint32_t f[3][NJ][4];
+    if constexpr (RULE == 1) {
+      if (c > 0) meet<kMeetTaken, 2 * kWalk>();                 // the reading warps have the last chunk's
 #pragma unroll
       for (int i = 0; i < 3; ++i)
 #pragma unroll
         for (int j = 0; j < NJ; ++j)
-          ldmatrix4(f[i][j], from + i * kPart * 2 + lt * (kD * 2) + (((2 * NJ * warp + 2 * j + ((lane >> 3) & 1)) ^ (lt & 7)) << 4));
-      float sum[NJ][2][2][4] = {};
+          state_parts[((warp * 3 + i) * NJ + j) * 32 + lane] = make_uint4(fs[i][j][0], fs[i][j][1], fs[i][j][2], fs[i][j][3]);
+      if constexpr (!EARLY) await(c);
+      read_state(fs, ks, shares_k + warp * kShares, warp, lane);
+    } else {
+      if constexpr (!EARLY) await(c);
+      read_state(fs, qs, shares_q + ((c & 1) * kRowWarps + warp) * kShares, warp, lane);
+    }
+    // the state's products' operands that do not wait for the others
+    uint32_t fk[3][NJ][4];
+    auto load_k = [&]() {
 #pragma unroll
-      for (int o = 0; o < 3; ++o)
+      for (int i = 0; i < 3; ++i)
 #pragma unroll
         for (int j = 0; j < NJ; ++j)
-#pragma unroll
-          for (int a = 0; a < 2; ++a)
-#pragma unroll
-            for (int n = 0; n < 2; ++n) mma(sum[j][a][n], fs[order[a][o][0]][j], f[order[a][o][1]][j][2 * n], f[order[a][o][1]][j][2 * n + 1]);
-#pragma unroll
-      for (int n = 0; n < 2; ++n)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          float y = sum[0][0][n][e] + sum[0][1][n][e];
-#pragma unroll
-          for (int j = 1; j < NJ; ++j) y += sum[j][0][n][e] + sum[j][1][n][e];
-          to[(8 * n + 2 * (lane & 3) + (e & 1)) * kLdV + col + 8 * (e >> 1)] = y;
-        }
+          ldmatrix4_trans(fk[i][j], ks + i * kPart * 2 + tt * (kD * 2) + (((2 * NJ * warp + 2 * j + (lane >> 4)) ^ (tt & 7)) << 4));
     };
-    if constexpr (RULE == 1) read(ks, shares_k + warp * kShares);
-    read(qs, shares_q + ((c & 1) * kRowWarps + warp) * kShares);
-    const float w = coef[kCoefW + t];
-    float u[CPT];
+    const float2 w = *reinterpret_cast<const float2*>(coef + kCoefW + t), x = make_float2(vs[t * kV + v], vs[(t + 1) * kV + v]);
+    float2 u;
     if constexpr (RULE == 1) {
-      meet<1, kWalk>();
-      const float g = coef[kCoefG + t];
+      const float2 g = *reinterpret_cast<const float2*>(coef + kCoefG + t);
+      float row[2][kC];
+      load_row(coef + kCoefT + t * kC, row[0]);
+      load_row(coef + kCoefT + (t + 1) * kC, row[1]);
+      meet<kMeetWalk, kWalk>();
+      float2 a = make_float2(0.f, 0.f);
 #pragma unroll
-      for (int i = 0; i < CPT; ++i) {
-        float a = 0.f;
-#pragma unroll
-        for (int r = 0; r < kRowWarps; ++r) a += shares_k[r * kShares + t * kLdV + v0 + i];
-        rest[(v0 + i) * kLdT + t] = __fmaf_rn(-g, a, vs[t * kV + v0 + i]);
+      for (int r = 0; r < kRowWarps; ++r) {
+        const float2 y = *reinterpret_cast<const float2*>(shares_k + r * kShares + v * kLdT + t);
+        a.x += y.x;
+        a.y += y.y;
       }
-      meet<1, kWalk>();
-#pragma unroll
-      for (int i = 0; i < CPT; ++i) u[i] = upto(coef + kCoefT + t * kC, rest + (v0 + i) * kLdT, t);
+      *reinterpret_cast<float2*>(rest + v * kLdT + t) = make_float2(__fmaf_rn(-g.x, a.x, x.x), __fmaf_rn(-g.y, a.y, x.y));
+      meet<kMeetWalk, kWalk>();
+      load_k();
+      float y[kC];
+      load_row(rest + v * kLdT, y);
+      u = make_float2(upto(row[0], y, t), upto(row[1], y, t + 1));
     } else {                                                   // u is known at once
-      const float b = coef[kCoefB + t];
-#pragma unroll
-      for (int i = 0; i < CPT; ++i) u[i] = b * vs[t * kV + v0 + i];
+      load_k();
+      const float2 b = *reinterpret_cast<const float2*>(coef + kCoefB + t);
+      u = make_float2(b.x * x.x, b.y * x.y);
     }
     {                                                          // u, and u times the decays after it in parts
       uint32_t o[3];
-      part2(w * u[0], w * u[CPT - 1], o);
+      part2(w.x * u.x, w.y * u.y, o);
+      *reinterpret_cast<float2*>(us + ((c & 1) * kV + v) * kLdT + t) = u;
 #pragma unroll
-      for (int i = 0; i < CPT; ++i) us[((c & 1) * kV + v0 + i) * kLdT + t] = u[i];
-#pragma unroll
-      for (int i = 0; i < 3; ++i) {
-        __nv_bfloat16* to = ups + (((c & 1) * 3 + i) * kC + t) * kV + v0;
-        if constexpr (CPT == 2) *reinterpret_cast<uint32_t*>(to) = o[i];
-        else *reinterpret_cast<uint16_t*>(to) = (uint16_t)o[i];
-      }
+      for (int i = 0; i < 3; ++i) *reinterpret_cast<uint32_t*>(ups + (((c & 1) * 3 + i) * kV + v) * kC + t) = o[i];
     }
-    meet<0, kAll>();
-    if (lost[c & 1]) {
-      whole = false;
-      break;
-    }
+    const float hi = coef[kCoefL], lo = coef[kCoefL + 1];
+    meet<kMeetAll, kAll>();
     // the state: u times the decays after its token, times k
     uint32_t fu[3][4];
 #pragma unroll
-    for (int i = 0; i < 3; ++i)                                // ldmatrix: tokens 0-7 by two pieces of columns, tokens 8-15 by two
-      ldmatrix4_trans(fu[i], smem_u32(ups + (((c & 1) * 3 + i) * kC + lt) * kV + ((lane >> 3) & 1) * 8));
-    const float hi = coef[kCoefL], lo = coef[kCoefL + 1];
+    for (int i = 0; i < 3; ++i)                                // ldmatrix: two halves of the columns by eight tokens, then by the next
+      ldmatrix4(fu[i], smem_u32(ups + (((c & 1) * 3 + i) * kV + tt) * kC + (lane >> 4) * 8));
+    float more[NJ][2][4];
 #pragma unroll
-    for (int j = 0; j < NJ; ++j) {
-      uint32_t f[3][4];
+    for (int o = 0; o < 6; ++o)
 #pragma unroll
-      for (int i = 0; i < 3; ++i)
-        ldmatrix4_trans(f[i], ks + i * kPart * 2 + tt * (kD * 2) + (((2 * NJ * warp + 2 * j + (lane >> 4)) ^ (tt & 7)) << 4));
-      float more[2][2][4] = {};
+      for (int j = 0; j < NJ; ++j)
 #pragma unroll
-      for (int o = 0; o < 3; ++o)
+        for (int n = 0; n < 2; ++n) {
+          const uint32_t(&b)[4] = fk[second_part(o)][j];
+          if (o == 0) mma0(more[j][n], fu[first_part(o)], b[2 * n], b[2 * n + 1]);
+          else mma(more[j][n], fu[first_part(o)], b[2 * n], b[2 * n + 1]);
+        }
 #pragma unroll
-        for (int a = 0; a < 2; ++a)
-#pragma unroll
-          for (int n = 0; n < 2; ++n) mma(more[a][n], fu[order[a][o][0]], f[order[a][o][1]][2 * n], f[order[a][o][1]][2 * n + 1]);
+    for (int j = 0; j < NJ; ++j)
 #pragma unroll
       for (int n = 0; n < 2; ++n)
 #pragma unroll
-        for (int e = 0; e < 4; ++e)
-          S[2 * j + n][e] = __fmaf_rn(hi, S[2 * j + n][e], __fmaf_rn(lo, S[2 * j + n][e], more[0][n][e] + more[1][n][e]));
-    }
+        for (int e = 0; e < 2; ++e) {
+          float2& x = S[2 * j + n][e];
+          x = fma2(make_float2(hi, hi), x, fma2(make_float2(lo, lo), x, make_float2(more[j][n][2 * e], more[j][n][2 * e + 1])));
+        }
   }
-  if (!whole) return;
+  if (*lost) return;
 #pragma unroll
   for (int n = 0; n < 2 * NJ; ++n)
 #pragma unroll
     for (int e = 0; e < 2; ++e)
-      if (j0 + col + 8 * e < p.vdim) *reinterpret_cast<float2*>(sp + (size_t)e * 8 * kD + 8 * n) = make_float2(S[n][2 * e], S[n][2 * e + 1]);
+      if (j0 + col + 8 * e < p.vdim) *reinterpret_cast<float2*>(sp + (size_t)e * 8 * kD + 8 * n) = S[n][e];
 }
 
+template <int RULE, int STAGES>
+int launch_walk(const ChunkParams& p, int n_requests, cudaStream_t stream) {
+  constexpr size_t smem = walk_smem<RULE, STAGES>();
+  if (cudaFuncSetAttribute(chunk_walk_kernel<RULE, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return YALIS_ERR_LAUNCH;
+  return yalis_launch_after(chunk_walk_kernel<RULE, STAGES>, dim3((p.vdim + kV - 1) / kV, p.heads, n_requests), dim3(kAll), smem, stream, p);
+}
+
+// Chunks in shared memory: three leave room for two blocks on an SM, which cover each other's copies; where there is a block an SM at
+// most, five.
 template <int RULE>
 int launch_chunks(const ChunkParams& p, int n_requests, int longest, cudaStream_t stream) {
-  constexpr size_t smem = walk_smem<RULE>();
-  if (cudaFuncSetAttribute(chunk_walk_kernel<RULE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return YALIS_ERR_LAUNCH;
   const int st = yalis_launch(chunk_prepare_kernel<RULE>, dim3((longest + kC - 1) / kC, p.kv_heads, n_requests), dim3(kWarps * 32), 0, stream, p);
   if (st != YALIS_OK) return st;
-  return yalis_launch_after(chunk_walk_kernel<RULE>, dim3((p.vdim + kV - 1) / kV, p.heads, n_requests), dim3(kAll), smem, stream, p);
+  const long long blocks = (long long)((p.vdim + kV - 1) / kV) * p.heads * n_requests;
+  return blocks <= yalis_sm_count() ? launch_walk<RULE, 5>(p, n_requests, stream) : launch_walk<RULE, 3>(p, n_requests, stream);
 }
 
 }  // namespace

@@ -119,10 +119,10 @@ def short_conv_silu(x: torch.Tensor, weight: torch.Tensor, slot_rows: torch.Tens
 
 
 # Portions of so many tokens, by rule, may go by chunks of sixteen (a portion's length alone decides, so that a request's result
-# does not depend on what runs beside it).  Where the lines lie: one portion of 128 tokens gains a tenth by the delta rule (26 -> 24 us,
-# 32 of them 346 -> 270) and by the selective form (18.5 -> 17.7, 32 of them 211 -> 207); the plain rule, which walks with no
-# sum between its tokens, loses 15 % with 32 portions of 128 and 5 % with 8 of 512, but gains 36 % with one of 512, 11 % with 4 of 901.
-CHUNKS_FROM = {0: 512, 1: 128, 3: 128}
+# does not depend on what runs beside it).  Where the lines lie (us, walk -> chunks): delta rule 1 x 128 31 -> 26 to 33, 32 x 128
+# 352 -> 259; plain 1 x 128 23 -> 21.5, 32 x 128 202 -> 200; selective 1 x 128 23 -> 30 (its one key head makes few blocks of the
+# first kernel), 1 x 192 32 -> 32, 16 x 192 169 -> 132.
+CHUNKS_FROM = {0: 128, 1: 128, 3: 192}
 CHUNK = 16
 
 
