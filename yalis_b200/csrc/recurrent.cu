@@ -75,6 +75,28 @@ __device__ __forceinline__ void load_inputs(const T* p, float (&o)[V]) {
   }
 }
 
+// Decays and write strengths of the tokens n0 .. n1 - 1, shared out among the blocks of a tile.
+template <typename T>
+__device__ __forceinline__ void rates_and_strengths(const DeltaPrepareParams& p, int n0, int n1) {
+  if (p.a_raw != nullptr) {
+    const T* a_raw = reinterpret_cast<const T*>(p.a_raw);
+    const T* b_raw = reinterpret_cast<const T*>(p.b_raw);
+    const int per = p.a_cols / p.heads;           // 1, or dim
+    const int first = blockIdx.y * blockDim.x + threadIdx.x, step = gridDim.y * blockDim.x;
+    for (int e = first; e < (n1 - n0) * p.a_cols; e += step) {
+      const int n = n0 + e / p.a_cols, c = e % p.a_cols;
+      if (p.req_of_token[n] < 0) continue;
+      const float s = softplus_f(to_f32<T>(a_raw[(size_t)n * p.a_stride + c]) + p.dt_bias[c]);
+      p.g_out[(size_t)n * p.a_cols + c] = expf(-expf(p.a_log[c / per]) * s);
+      if (b_raw == nullptr) p.beta_out[(size_t)n * p.heads + c] = s;
+    }
+    for (int e = first; b_raw != nullptr && e < (n1 - n0) * p.heads; e += step) {
+      const int n = n0 + e / p.heads, h = e % p.heads;
+      if (p.req_of_token[n] >= 0) p.beta_out[(size_t)n * p.heads + h] = sigmoid_f(to_f32<T>(b_raw[(size_t)n * p.b_stride + h]));
+    }
+  }
+}
+
 // KMAX: the most taps (a bound known at compile time keeps the history in registers); V: channels a thread takes.
 template <typename T, int KMAX, int V>
 __global__ void delta_prepare_kernel(const DeltaPrepareParams p) {
@@ -147,23 +169,7 @@ __global__ void delta_prepare_kernel(const DeltaPrepareParams p) {
       }
     }
   }
-  if (p.a_raw != nullptr) {
-    const T* a_raw = reinterpret_cast<const T*>(p.a_raw);
-    const T* b_raw = reinterpret_cast<const T*>(p.b_raw);
-    const int per = p.a_cols / p.heads;           // 1, or dim
-    const int first = blockIdx.y * blockDim.x + threadIdx.x, step = gridDim.y * blockDim.x;
-    for (int e = first; e < (n1 - n0) * p.a_cols; e += step) {
-      const int n = n0 + e / p.a_cols, c = e % p.a_cols;
-      if (p.req_of_token[n] < 0) continue;
-      const float s = softplus_f(to_f32<T>(a_raw[(size_t)n * p.a_stride + c]) + p.dt_bias[c]);
-      p.g_out[(size_t)n * p.a_cols + c] = expf(-expf(p.a_log[c / per]) * s);
-      if (b_raw == nullptr) p.beta_out[(size_t)n * p.heads + c] = s;
-    }
-    for (int e = first; b_raw != nullptr && e < (n1 - n0) * p.heads; e += step) {
-      const int n = n0 + e / p.heads, h = e % p.heads;
-      if (p.req_of_token[n] >= 0) p.beta_out[(size_t)n * p.heads + h] = sigmoid_f(to_f32<T>(b_raw[(size_t)n * p.b_stride + h]));
-    }
-  }
+  rates_and_strengths<T>(p, n0, n1);
   if (p.kv_heads > 0) {
     __syncthreads();                              // the block reads back what it wrote itself
     const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
@@ -180,6 +186,95 @@ __global__ void delta_prepare_kernel(const DeltaPrepareParams p) {
       for (int d = lane; d < p.dim; d += 32) v[d] *= r;
     }
   }
+}
+
+// The same over portions, for up to four taps and pieces of 128 channels (where heads are brought to unit length, a head each): a warp
+// has a piece of two tokens, all of whose inputs it asks for before it needs the first, and holds a head's results until its
+// length is known.  Sums in the order of the form above: the same bits.
+// What bounds it: expf and the division of silu, some 30 instructions a value, and a block's wait for its rows.  The form above
+// waits for a token's index, slot and row before it asks for the next one's, and reads its results back for their length.
+// Measured (us with the tails' kernel, L2 flushed, above -> here): 4,096 channels, 16 heads to unit length, a rate per head: 64 tokens
+// 13.3 -> 13.3, 256 17.4 -> 15.4, 512 23.6 -> 17.4, 1,024 31.7 -> 23.6, 2,048 46 -> 38; 6,144, 32 heads, a rate per channel: 128 tokens
+// 19.5 -> 17.4, 2,048 89 -> 77; 2,304, none: 128 tokens 13.3 -> 15.3, 256 13.3 -> 13.3, 512 17.4 -> 15.4, 3,000 38 -> 36: so from 256 tokens on.
+// Four tokens a warp 38, 83 and 38 for the longest, eight 46, 112 and 46: fewer warps.
+constexpr int kConvTile = 2, kConvTileFrom = 256;
+
+template <typename T>
+__global__ void __launch_bounds__(256) conv_tile_kernel(const DeltaPrepareParams p) {
+  constexpr int LAGS = 3, NJ = 4, TILE = kConvTile;
+  pdl_launch_dependents();
+  pdl_wait();
+  const int lane = threadIdx.x & 31, piece = blockIdx.y * 8 + (threadIdx.x >> 5);
+  const int n0 = blockIdx.x * TILE, n1 = min(n0 + TILE, p.n_tokens), keep = p.taps - 1;
+  if (piece * 128 < p.channels) {
+    float x[NJ][TILE + LAGS], w[NJ][LAGS + 1], bias[NJ], y[NJ][TILE];
+    const bool quads = p.taps == 4 && ((uintptr_t)p.w & 15) == 0;
+#pragma unroll
+    for (int j = 0; j < NJ; ++j) {
+      const int c = piece * 128 + j * 32 + lane;
+      const T* xc = reinterpret_cast<const T*>(p.x) + c;
+#pragma unroll
+      for (int m = 0; m < TILE + LAGS; ++m) {
+        const int n = n0 - LAGS + m;
+        x[j][m] = n >= 0 && n < n1 ? to_f32<T>(xc[(size_t)n * p.x_stride]) : 0.f;
+      }
+      if (quads) {
+        const float4 v = load4_f32(p.w + (size_t)c * 4);
+        w[j][0] = v.x; w[j][1] = v.y; w[j][2] = v.z; w[j][3] = v.w;
+      } else {
+#pragma unroll
+        for (int lag = 0; lag <= LAGS; ++lag) w[j][LAGS - lag] = lag <= keep ? p.w[(size_t)c * p.taps + keep - lag] : 0.f;
+      }
+      bias[j] = p.conv_bias ? p.conv_bias[c] : 0.f;
+    }
+    int index = -1, slot = 0;                       // lane t: of token n0 + t within its request's portion
+    if (n0 + lane < n1 && lane < TILE) {
+      const int req = p.req_of_token[n0 + lane];
+      if (req >= 0) {
+        index = n0 + lane - p.q_start[req];
+        slot = p.slots[req];
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < NJ; ++j) {
+      const int c = piece * 128 + j * 32 + lane;
+#pragma unroll
+      for (int t = 0; t < TILE; ++t) {
+        const int i = __shfl_sync(0xffffffffu, index, t), at = __shfl_sync(0xffffffffu, slot, t);
+        float h[LAGS + 1];
+#pragma unroll
+        for (int m = 0; m <= LAGS; ++m) h[m] = x[j][t + m];
+        if (i >= 0 && i < keep) {                   // the portion begins here: what is before it waits in the slot
+#pragma unroll
+          for (int lag = 1; lag <= LAGS; ++lag)
+            if (lag > i && lag <= keep) h[LAGS - lag] = p.tail[(size_t)at * p.slot_stride + (size_t)c * keep + (keep + i - lag)];
+        }
+        float acc = 0.f;
+#pragma unroll
+        for (int m = 0; m <= LAGS; ++m)
+          if (LAGS - m <= keep) acc = __fmaf_rn(w[j][m], h[m], acc);     // oldest input first
+        y[j][t] = silu_exact(acc + bias[j]);
+      }
+    }
+    const bool unit = piece < 2 * p.kv_heads;
+#pragma unroll
+    for (int t = 0; t < TILE; ++t) {
+      if (unit) {
+        float ss = 0.f;
+#pragma unroll
+        for (int j = 0; j < NJ; ++j) ss = __fmaf_rn(y[j][t], y[j][t], ss);
+        ss = warp_sum(ss);
+        const float r = (piece < p.kv_heads ? p.q_scale : 1.0f) / sqrtf(ss + p.unit_eps);
+#pragma unroll
+        for (int j = 0; j < NJ; ++j) y[j][t] *= r;
+      }
+      if (__shfl_sync(0xffffffffu, index, t) >= 0) {
+#pragma unroll
+        for (int j = 0; j < NJ; ++j) p.out[(size_t)(n0 + t) * p.out_stride + piece * 128 + j * 32 + lane] = y[j][t];
+      }
+    }
+  }
+  rates_and_strengths<T>(p, n0, n1);
 }
 
 // After the step: the tail becomes the last K-1 inputs the request has seen.
@@ -808,9 +903,12 @@ YALIS_API int yalis_delta_prepare(const void* x, int dtype, int x_stride, const 
   p.tile = n_tokens >= 1024 ? 8 : (n_tokens >= 256 ? 2 : 1);
   const dim3 grid((n_tokens + p.tile - 1) / p.tile, (channels + p.piece - 1) / p.piece);
   if (grid.y > 65535) return YALIS_ERR_SHAPE;
+  const int pieces = (channels / 128 + 7) / 8;
+  const bool by_tiles = !single_tokens && n_tokens >= kConvTileFrom && taps <= 4 && channels % 128 == 0 && (kv_heads == 0 || dim == 128) && pieces <= 65535;
   YALIS_DISPATCH_DTYPE(dtype, T, {
     int st;
-    if (taps <= 4)
+    if (by_tiles) st = yalis_launch(conv_tile_kernel<T>, dim3((n_tokens + kConvTile - 1) / kConvTile, pieces), dim3(256), 0, stream, p);
+    else if (taps <= 4)
       st = pairs ? yalis_launch(delta_prepare_kernel<T, 4, 2>, grid, dim3(threads), 0, stream, p)
                  : yalis_launch(delta_prepare_kernel<T, 4, 1>, grid, dim3(threads), 0, stream, p);
     else
