@@ -621,22 +621,32 @@ __global__ void activation_bf16x8_kernel(const __nv_bfloat16* x, int x_stride, _
 // Four elements a thread with float32 results (bfloat16 rows on 8-byte boundaries, float32 rows on 16-byte ones).  Its
 // reader may be a kernel of few, long blocks (a recurrence over the rows it makes): those are let in only once this one
 // has begun, so that they do not crowd onto the SMs that come free first.
+// A block has a row's next 256 x kActQuads groups of four; a thread asks for all of its own before it needs the first.
+// 2,926 rows of bfloat16 values, silu: 27.9 us with a 64-bit division for the row of every group, 20.2 here; the rest is expf and a division a
+// value.
+constexpr int kActQuads = 3;
 template <typename T>
-__global__ void activation_f32x4_kernel(const T* x, int x_stride, float* y, int y_stride, int rows,
+__global__ void __launch_bounds__(256) activation_f32x4_kernel(const T* x, int x_stride, float* y, int y_stride, int rows,
                                         int cols, int act, const float* __restrict__ bias) {
   pdl_wait();
   pdl_launch_dependents();
-  const int quads = cols >> 2;
-  const size_t total = (size_t)rows * quads;
-  for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (size_t)gridDim.x * blockDim.x) {
-    const size_t r = e / quads;
-    const int c = (int)(e - r * quads) << 2;
-    float4 z = load4_f32(x + r * x_stride + c);
+  const size_t r = blockIdx.x;
+  const int quads = cols >> 2, first = blockIdx.y * (kActQuads * blockDim.x) + threadIdx.x;
+  float4 z[kActQuads];
+#pragma unroll
+  for (int i = 0; i < kActQuads; ++i) {
+    const int c = first + i * blockDim.x;
+    if (c < quads) z[i] = load4_f32(x + r * x_stride + 4 * c);
+  }
+#pragma unroll
+  for (int i = 0; i < kActQuads; ++i) {
+    const int c = first + i * blockDim.x;
+    if (c >= quads) return;
     if (bias) {
-      const float4 b = load4_f32(bias + c);
-      z.x += b.x; z.y += b.y; z.z += b.z; z.w += b.w;
+      const float4 b = load4_f32(bias + 4 * c);
+      z[i].x += b.x; z[i].y += b.y; z[i].z += b.z; z[i].w += b.w;
     }
-    store4(y + r * y_stride + c, make_float4(act_value(z.x, act), act_value(z.y, act), act_value(z.z, act), act_value(z.w, act)));
+    store4(y + r * y_stride + 4 * c, make_float4(act_value(z[i].x, act), act_value(z[i].y, act), act_value(z[i].z, act), act_value(z[i].w, act)));
   }
 }
 
@@ -800,10 +810,9 @@ YALIS_API int yalis_activation(const void* x, int x_stride, void* y, int y_strid
   const size_t total = (size_t)rows * cols;
   const int blocks = (int)((total + 255) / 256 < 148 * 16 ? (total + 255) / 256 : 148 * 16);
   if (y_f32 && cols % 4 == 0 && x_stride % 4 == 0 && y_stride % 4 == 0 && !((uintptr_t)x & (dtype == YALIS_BF16 ? 7 : 15)) &&
-      !(((uintptr_t)y | (uintptr_t)bias) & 15)) {
-    const size_t quads = (total / 4 + 255) / 256;
-    const dim3 grid((unsigned)(quads < 148 * 16 ? quads : 148 * 16));
-    YALIS_DISPATCH_DTYPE(dtype, T, return yalis_launch(activation_f32x4_kernel<T>, grid, dim3(256), 0, stream, (const T*)x,
+      !(((uintptr_t)y | (uintptr_t)bias) & 15) && cols <= 65535 * 1024) {
+    const int groups = (cols / 4 + 256 * kActQuads - 1) / (256 * kActQuads);
+    YALIS_DISPATCH_DTYPE(dtype, T, return yalis_launch(activation_f32x4_kernel<T>, dim3(rows, groups), dim3(256), 0, stream, (const T*)x,
                                                        x_stride, (float*)y, y_stride, rows, cols, act, bias));
   }
   if (y_f32 && dtype == YALIS_BF16)
