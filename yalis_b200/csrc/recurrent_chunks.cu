@@ -17,7 +17,7 @@
 // A chunk starts where its request's portion starts: a long portion's results depend on how the request was cut, by rounding.
 // Errors against float64 beside the walk's (2,048 tokens, slow decays, read-outs / state): constant decay 1.9e-7 / 7.7e-7 (2.0e-7 /
 // 9.4e-7), delta rule 1.4e-7 / 3.6e-7 (1.1e-7 / 3.6e-7), selective 0.7e-7 / 2.2e-7 (1.1e-7 / 5.0e-7).
-// What bounds it: for one request the instructions of a chunk's chain, some 1,600 cycles by the delta rule: a warp alone on its
+// What bounds it: for one request the instructions of a chunk's chain, some 1,900 cycles by the delta rule: a warp alone on its
 // scheduler issues one in about four cycles (clock counts between the chain's stages), so sums start from no cleared
 // registers, the six products of parts are one chain, pairs of float32 operations go in one instruction, and what the chain does not
 // need is left to other warps: waiting for copies, by the delta rule the products with q.  For several requests the copies of k and q,
