@@ -124,3 +124,75 @@ def test_a_query_that_is_not_finite_reaches_its_own_token_only():
         got = run(rule, lay, 2, (q,) + data[1:], torch.zeros(1, lay.total, device=DEV), [n], [0], True)
         assert torch.equal(got[:70], plain[:70]) and torch.equal(got[71:], plain[71:]) and torch.equal(got[:, 0], plain[:, 0])
         assert not bool(got[70, 1].isfinite().any())
+
+
+@pytest.mark.parametrize("rule,lens,bound", [("constant", [100], 128), ("delta", [100], 128), ("selective", [150], 256), ("token", [100, 1, 128], 128),
+                                             ("delta", [127, 128, 33], 256), ("selective", [191, 192], 256), ("delta constant", [300], 128)])
+def test_a_bound_above_or_below_the_portions_leaves_nobody_out(rule, lens, bound):
+    """What a recording gives instead of the longest portion: what each length gives alone, in the form that its own length chooses (a
+    portion that is longer than the bound walks)."""
+    from yalis_b200.ops.recurrent import StateLayout, state_scan
+    g = torch.Generator().manual_seed(sum(lens))
+    heads, kv_heads, vdim = 4, 2, 36
+    lay, n, slots = StateLayout(heads, 128, vdim), sum(lens), list(range(len(lens)))[::-1]
+    q, k, v, decay, beta, skip = (None if t is None else t.to(DEV) for t in inputs(rule, heads, kv_heads, vdim, lens, g))
+    first = torch.randn(len(lens), lay.total, generator=g).to(DEV)
+    starts = torch.tensor([0] + lens).cumsum(0)
+
+    def run_with(a, b, lens, slots, rows, **how):
+        cut = lambda t: None if t is None else t if t.dim() == 1 else t[a:b]
+        return state_scan(cut(q).flatten(1), cut(k).flatten(1), cut(v).flatten(1), rows, lay, torch.tensor([0] + lens).cumsum(0).to(torch.int32).to(DEV),
+                          torch.tensor(slots, dtype=torch.int32, device=DEV), kv_heads=kv_heads, decay=cut(decay), beta=cut(beta),
+                          selective=rule == "selective", skip=skip, **how)
+
+    rows = first.clone()
+    got = run_with(0, n, lens, slots, rows, max_q_len=bound, chunks=True)
+    want_rows = first.clone()
+    for l, a, slot in zip(lens, starts.tolist(), slots):
+        want = run_with(a, a + l, [l], [slot], want_rows, max_q_len=l, chunks=l <= bound)
+        assert torch.equal(got[a:a + l], want)
+    assert torch.equal(rows, want_rows) and not bool((rows == first).all(1).any())
+
+
+MODELS = [("tirezen_models", {"architecture": "Tirezen", "width": 256, "vocab": 320, "norm": {"eps": 1e-5}, "layers": [
+              {"type": "delta", "mixer": {"heads": 2, "kv_heads": 1, "dim": 128, "vdim": 128, "conv": 4}, "mlp": {"kind": "dense", "ff": 256}},
+              {"type": "retention", "mixer": {"heads": 2, "dim": 128, "vdim": 128, "decay": [0.96, 0.99], "rot": {"dims": 128, "base": 10000.0}},
+               "mlp": {"kind": "dense", "ff": 256}}]}, [100, 128, 127, 65]),
+          ("ludelorn_models", {"architecture": "Ludelorn", "embedding": {"scale": 8.0}, "norm": {"eps": 1e-6}, "width": 256, "vocab": 320, "layers": [
+              {"type": "parallel", "mixer": {
+                  "left": {"heads": 2, "kv_heads": 1, "dim": 64, "vdim": 64, "scale": 0.125, "mask": {"size": 64},
+                           "rot": {"dims": 64, "base": 500000.0, "scaling": {"factor": 8.0, "original": 4096, "fast": 32.0, "slow": 1.0}}},
+                  "right": {"heads": 4, "vdim": 64, "state": 128, "groups": 1, "norm_groups": 1, "conv": 4}}, "mlp": {"kind": "dense", "ff": 256}}]},
+           [150, 192, 191, 140])]
+
+
+@pytest.mark.parametrize("order", [1, -1])
+@pytest.mark.parametrize("module,config,lengths", MODELS, ids=lambda x: x if isinstance(x, str) else "")
+def test_a_prompt_from_a_recording_is_the_launched_one(module, config, lengths, order, tmp_path):
+    """One request a step, its portion shorter than the recording's bound, at and around the length from which chunks are taken; ten more
+    tokens read the state that the prompt left.  All lengths share one recording."""
+    import importlib
+
+    from yalis_b200.engine.engine import Engine, StepEntry
+    folder = importlib.import_module(module).write_model(config, str(tmp_path), 3)
+    eng = Engine(folder, dtype="bfloat16", page_size=16, cache_tokens=1024, max_slots=2)
+    g = torch.Generator().manual_seed(4)
+    prompt, more = (torch.randint(0, 320, (m,), generator=g).tolist() for m in (max(lengths), 10))
+
+    def logits(length, graphs):
+        eng.add_request("r")
+        out = eng.run([StepEntry("r", prompt[:length], [length * i // 8 - 1 for i in range(1, 9)])], graphs=graphs)
+        rows, replayed = [out.logits.clone()], out.captured
+        rows += [eng.run([StepEntry("r", [t], [0])], graphs=False).logits.clone() for t in more]
+        eng.finish_request("r")
+        return torch.cat(rows), replayed
+
+    for length in lengths[::order]:
+        want = logits(length, False)[0]
+        replays = 0
+        for _ in range(3):
+            got, replayed = logits(length, True)
+            replays += replayed
+            # the recording's padded rows may take the library's products to another kernel: bfloat16 roundings
+            assert float((got - want).norm() / want.norm()) < 1e-2, length
+        assert replays >= 2

@@ -323,7 +323,7 @@ struct ScanParams {
   const int32_t* q_start; const int32_t* slots;
   int heads, kv_heads, dim, dim_padded, vdim;
   int wide;                          // 1: rows of q, k and the decay may be copied 16 bytes at a time
-  int limit;                         // > 0: portions of so many tokens and more are left to the form by chunks
+  int limit, upto;                   // limit > 0: portions of limit to upto tokens are left to the form by chunks
 };
 
 __device__ __forceinline__ void copy_async4(float* smem, const float* gmem) {
@@ -451,7 +451,7 @@ __global__ void __launch_bounds__(kScanThreads) state_scan_kernel(const ScanPara
   pdl_wait();
   const int req = blockIdx.z, h = blockIdx.y;
   const int t_begin = p.q_start[req], q_len = p.q_start[req + 1] - t_begin;
-  if (q_len <= 0 || (p.limit > 0 && q_len >= p.limit)) return;
+  if (q_len <= 0 || (p.limit > 0 && q_len >= p.limit && q_len <= p.upto)) return;
   const int tid = threadIdx.x, l = tid % L, c = tid / L;
   const int j = blockIdx.x * cols + c * C;               // the thread's first column
   const int kvh = h / (p.heads / p.kv_heads);
@@ -968,12 +968,12 @@ static int launch_scan_dim(const ScanParams& p, int n_requests, int longest, cud
 // kv_heads = heads, decay_kind 2); delta 3: the selective form, beta [N, heads] the step sizes and skip [heads] (or null)
 // the token's own value in the read-out (decay_kind 1).
 // max_q_len: the longest portion of the step if the caller knows it (0: not known); it only chooses the staging tile.
-// limit > 0: portions of so many tokens and more are left alone.
+// limit > 0: portions of limit to upto tokens are left alone.
 YALIS_API int yalis_state_scan(const float* q, int q_stride, const float* k, int k_stride, const float* v, int v_stride,
                                const float* decay, int decay_kind, const float* beta, const float* skip, const float* unit,
                                const float* removal, float* state, int64_t slot_stride,
                                float* out, int out_stride, const int32_t* q_start, const int32_t* slots, int n_requests,
-                               int heads, int kv_heads, int dim, int vdim, int delta, int max_q_len, int limit, cudaStream_t stream) {
+                               int heads, int kv_heads, int dim, int vdim, int delta, int max_q_len, int limit, int upto, cudaStream_t stream) {
   if (n_requests <= 0) return YALIS_OK;
   if (dim <= 0 || vdim <= 0 || heads <= 0 || kv_heads <= 0 || heads % kv_heads || heads > 65535 || n_requests > 65535)
     return YALIS_ERR_SHAPE;
@@ -987,7 +987,7 @@ YALIS_API int yalis_state_scan(const float* q, int q_stride, const float* k, int
   p.q = q; p.q_stride = q_stride; p.k = k; p.k_stride = k_stride; p.v = v; p.v_stride = v_stride;
   p.decay = decay; p.beta = beta; p.skip = skip; p.unit = unit; p.removal = removal; p.state = state; p.slot_stride = (size_t)slot_stride; p.out = out;
   p.out_stride = out_stride; p.q_start = q_start; p.slots = slots; p.heads = heads; p.kv_heads = kv_heads;
-  p.dim = dim; p.dim_padded = dim_padded; p.vdim = vdim; p.limit = limit;
+  p.dim = dim; p.dim_padded = dim_padded; p.vdim = vdim; p.limit = limit; p.upto = upto;
   p.wide = (dim % 4 == 0 && q_stride % 4 == 0 && k_stride % 4 == 0 && !((uintptr_t)q & 15) && !((uintptr_t)k & 15) &&
             (decay_kind != 2 || !((uintptr_t)decay & 15)) &&
             (delta != 2 || (!((uintptr_t)unit & 15) && !((uintptr_t)removal & 15)))) ? 1 : 0;

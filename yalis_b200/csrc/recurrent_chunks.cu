@@ -50,7 +50,7 @@ struct ChunkParams {
   float* state; size_t slot_stride;
   float* out; int out_stride;
   const int32_t* q_start; const int32_t* slots;
-  int heads, kv_heads, vdim, shortest;          // portions below `shortest` tokens are left out
+  int heads, kv_heads, vdim, shortest, longest; // portions of other lengths are left out
   __nv_bfloat16* parts;                         // [chunk][kv_head][k, q][3][16][128], 16-byte pieces swapped within rows
   float* coef;                                  // [chunk][head][kCoef]
   int32_t* error;
@@ -124,7 +124,7 @@ __global__ void __launch_bounds__(kWarps * 32) chunk_prepare_kernel(const ChunkP
   pdl_wait();
   const int req = blockIdx.z, kvh = blockIdx.y, start = p.q_start[req], len = p.q_start[req + 1] - start;
   const int t0 = start + blockIdx.x * kC, valid = min(kC, start + len - t0);
-  if (len < p.shortest || valid <= 0) return;
+  if (len < p.shortest || len > p.longest || valid <= 0) return;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const size_t chunk = first_chunk(start, req) + blockIdx.x;
   __nv_bfloat16* parts = p.parts + (chunk * p.kv_heads + kvh) * (6 * kPart);
@@ -319,7 +319,7 @@ __global__ void __launch_bounds__(kAll, STAGES == 3 ? 2 : 1) chunk_walk_kernel(c
   pdl_launch_dependents();
   pdl_wait();
   const int req = blockIdx.z, h = blockIdx.y, j0 = blockIdx.x * kV, start = p.q_start[req], len = p.q_start[req + 1] - start;
-  if (len < p.shortest) return;
+  if (len < p.shortest || len > p.longest) return;
   const int role = threadIdx.x / kWalk, tid = threadIdx.x % kWalk;      // role 0 walks, 1 reads, 2 fetches
   const int lane = tid & 31, kvh = h / (p.heads / p.kv_heads);
   const int chunks = (len + kC - 1) / kC;
@@ -572,8 +572,8 @@ int launch_chunks(const ChunkParams& p, int n_requests, int longest, cudaStream_
 // bfloat16 values per key head in `parts`.
 YALIS_API int yalis_state_chunks_coefficients() { return kCoef; }
 
-// The portions of `shortest` tokens and more of a step, the others are left alone.  dim 128, vdim a multiple of four, rows on
-// 16-byte boundaries; rule 0: plain, 1: delta, 3: selective; decay_kind 0 or 1 as in yalis_state_scan.  longest: the longest portion.
+// The portions of `shortest` to `longest` tokens of a step, the others are left alone.  dim 128, vdim a multiple of four, rows on
+// 16-byte boundaries; rule 0: plain, 1: delta, 3: selective; decay_kind 0 or 1 as in yalis_state_scan.
 YALIS_API int yalis_state_chunks(const float* q, int q_stride, const float* k, int k_stride, const float* v, int v_stride,
                                  const float* decay, int decay_kind, const float* beta, const float* skip, float* state,
                                  int64_t slot_stride, float* out, int out_stride, const int32_t* q_start, const int32_t* slots,
@@ -587,7 +587,7 @@ YALIS_API int yalis_state_chunks(const float* q, int q_stride, const float* k, i
       (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)state | (uintptr_t)out | (uintptr_t)parts | (uintptr_t)coef) & 15))
     return YALIS_ERR_ALIGN;
   const ChunkParams p = {q, q_stride, k, k_stride, v, v_stride, decay, decay_kind, beta, skip, state, (size_t)slot_stride, out, out_stride,
-                         q_start, slots, heads, kv_heads, vdim, shortest, (__nv_bfloat16*)parts, (float*)coef, error};
+                         q_start, slots, heads, kv_heads, vdim, shortest, longest, (__nv_bfloat16*)parts, (float*)coef, error};
   if (rule == 0) return launch_chunks<0>(p, n_requests, longest, stream);
   if (rule == 1) return launch_chunks<1>(p, n_requests, longest, stream);
   return launch_chunks<3>(p, n_requests, longest, stream);

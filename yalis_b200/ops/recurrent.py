@@ -145,8 +145,8 @@ def state_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, slot_rows: tor
     channel too); ``beta`` float32 [N, heads].  With ``unit`` and ``removal`` (float32 [N, heads * dim]) the rule is the generalized delta rule instead:
     S <- diag(g) S - removal (unit^T S) + k v^T, both terms reading the old state; it needs a decay per key channel
     and kv_heads = heads, and ``decay``, ``unit``, ``removal`` contiguous.  ``selective``: S <- g S + k (beta v)^T and
-    o = S^T q + skip v with the step sizes ``beta``, a decay per token and ``skip`` float32 [heads] (None: 0).  ``max_q_len``: the longest portion of the step if known (it bounds
-    the tile of tokens staged in shared memory, nothing else).  ``chunks``: long portions of the rules with one decay per head may be
+    o = S^T q + skip v with the step sizes ``beta``, a decay per token and ``skip`` float32 [heads] (None: 0).  ``max_q_len``: a bound on the step's portions if one is known
+    (0: none); the tile of tokens staged in shared memory and the launch by chunks are sized by it.  ``chunks``: long portions of the rules with one decay per head may be
     taken sixteen tokens at a time (``CHUNKS_FROM``, heads of 128 rows): float32 sums in another order, so that a
     token's bits depend on where its portion began.  Returns float32 [N, heads * vdim]."""
     name = "state_scan"
@@ -186,9 +186,15 @@ def state_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, slot_rows: tor
                  f"{what} must be contiguous float32 [N, heads * dim]")
         rule = 2
     out = torch.empty((n, h * vd), dtype=torch.float32, device=q.device)
-    limit = 0
-    if chunks and _takes_chunks(q, k, v, slot_rows, d, vd, kind, rule, max_q_len):
-        limit = CHUNKS_FROM[rule]
+    limit = CHUNKS_FROM[rule] if chunks and _takes_chunks(q, k, v, slot_rows, d, vd, kind, rule, max_q_len) else 0
+    # Both forms are launched, and each leaves the other's portions alone by their length on the device: max_q_len is the caller's
+    # bound (a recording's above all), behind which every portion may be a short one.  The walk takes what is longer, too.
+    check(lib().yalis_state_scan(
+        ptr(q), i32(q.stride(0)), ptr(k), i32(k.stride(0)), ptr(v), i32(v.stride(0)), ptr(decay), i32(kind), ptr(beta), ptr(skip),
+        ptr(unit), ptr(removal), ptr(slot_rows), i64(slot_rows.stride(0)), ptr(out), i32(out.stride(0)), ptr(q_start), ptr(slots),
+        i32(slots.numel()), i32(h), i32(kv_heads), i32(d), i32(vd), i32(rule), i32(min(max_q_len, limit - 1) if limit else max_q_len),
+        i32(limit), i32(max_q_len), stream()), name)
+    if limit:
         at_most = n // CHUNK + slots.numel() + 1                  # chunks of the step
         parts = torch.empty((at_most, kv_heads, 2, 3, CHUNK, d), dtype=torch.bfloat16, device=q.device)
         coef = torch.empty((at_most, h, int(lib().yalis_state_chunks_coefficients())), dtype=torch.float32, device=q.device)
@@ -197,12 +203,6 @@ def state_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, slot_rows: tor
             ptr(slot_rows), i64(slot_rows.stride(0)), ptr(out), i32(out.stride(0)), ptr(q_start), ptr(slots), i32(slots.numel()), i32(h),
             i32(kv_heads), i32(d), i32(vd), i32(rule), i32(max_q_len), i32(limit), ptr(parts), ptr(coef), ptr(error_word(q.device)),
             stream()), name)
-        if slots.numel() == 1:
-            return out
-    check(lib().yalis_state_scan(
-        ptr(q), i32(q.stride(0)), ptr(k), i32(k.stride(0)), ptr(v), i32(v.stride(0)), ptr(decay), i32(kind), ptr(beta), ptr(skip),
-        ptr(unit), ptr(removal), ptr(slot_rows), i64(slot_rows.stride(0)), ptr(out), i32(out.stride(0)), ptr(q_start), ptr(slots),
-        i32(slots.numel()), i32(h), i32(kv_heads), i32(d), i32(vd), i32(rule), i32(max_q_len), i32(limit), stream()), name)
     return out
 
 

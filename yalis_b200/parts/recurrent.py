@@ -65,8 +65,8 @@ class _ProjectedMixer(Mixer, Projected):
         return self.project_and_mix(x, ctx, cache)
 
     def capture_key(self, host):
-        # the kernels read the step's arrays on the device and their grids follow the shapes alone; only the tile of
-        # tokens that the recurrence stages at a time follows the longest portion, up to 16
+        # the kernels read the step's arrays on the device and their grids follow the shapes and the longest portion, of which a
+        # recording of portions has a bound of its own; that a step has single tokens alone, or up to 4 or 16, is in the key
         return min(host.max_q_len, 16)
 
 
