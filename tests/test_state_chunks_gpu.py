@@ -126,8 +126,8 @@ def test_a_query_that_is_not_finite_reaches_its_own_token_only():
         assert not bool(got[70, 1].isfinite().any())
 
 
-@pytest.mark.parametrize("rule,lens,bound", [("constant", [100], 128), ("delta", [100], 128), ("selective", [150], 256), ("token", [100, 1, 128], 128),
-                                             ("delta", [127, 128, 33], 256), ("selective", [191, 192], 256), ("delta constant", [300], 128)])
+@pytest.mark.parametrize("rule,lens,bound", [("constant", [200], 256), ("delta", [100], 128), ("selective", [150], 256), ("token", [255, 1, 256], 256),
+                                             ("delta", [127, 128, 33], 256), ("selective", [207, 208], 256), ("delta constant", [300], 128)])
 def test_a_bound_above_or_below_the_portions_leaves_nobody_out(rule, lens, bound):
     """What a recording gives instead of the longest portion: what each length gives alone, in the form that its own length chooses (a
     portion that is longer than the bound walks)."""
@@ -154,16 +154,17 @@ def test_a_bound_above_or_below_the_portions_leaves_nobody_out(rule, lens, bound
     assert torch.equal(rows, want_rows) and not bool((rows == first).all(1).any())
 
 
-MODELS = [("tirezen_models", {"architecture": "Tirezen", "width": 256, "vocab": 320, "norm": {"eps": 1e-5}, "layers": [
+MODELS = [
+          ("tirezen_models", {"architecture": "Tirezen", "width": 256, "vocab": 320, "norm": {"eps": 1e-5}, "layers": [
               {"type": "delta", "mixer": {"heads": 2, "kv_heads": 1, "dim": 128, "vdim": 128, "conv": 4}, "mlp": {"kind": "dense", "ff": 256}},
               {"type": "retention", "mixer": {"heads": 2, "dim": 128, "vdim": 128, "decay": [0.96, 0.99], "rot": {"dims": 128, "base": 10000.0}},
-               "mlp": {"kind": "dense", "ff": 256}}]}, [100, 128, 127, 65]),
+               "mlp": {"kind": "dense", "ff": 256}}]}, lengths) for lengths in ([100, 128, 127, 65], [200, 256, 255, 193])] + [
           ("ludelorn_models", {"architecture": "Ludelorn", "embedding": {"scale": 8.0}, "norm": {"eps": 1e-6}, "width": 256, "vocab": 320, "layers": [
               {"type": "parallel", "mixer": {
                   "left": {"heads": 2, "kv_heads": 1, "dim": 64, "vdim": 64, "scale": 0.125, "mask": {"size": 64},
                            "rot": {"dims": 64, "base": 500000.0, "scaling": {"factor": 8.0, "original": 4096, "fast": 32.0, "slow": 1.0}}},
                   "right": {"heads": 4, "vdim": 64, "state": 128, "groups": 1, "norm_groups": 1, "conv": 4}}, "mlp": {"kind": "dense", "ff": 256}}]},
-           [150, 192, 191, 140])]
+           [200, 208, 207, 193])]
 
 
 @pytest.mark.parametrize("order", [1, -1])
@@ -196,3 +197,25 @@ def test_a_prompt_from_a_recording_is_the_launched_one(module, config, lengths, 
             # the recording's padded rows may take the library's products to another kernel: bfloat16 roundings
             assert float((got - want).norm() / want.norm()) < 1e-2, length
         assert replays >= 2
+
+
+@pytest.mark.parametrize("keep", [0.0, 0.5, 0.9, 0.995])
+@pytest.mark.parametrize("rule", RULES)
+def test_errors_are_no_larger_than_the_walks(rule, keep):
+    """Decays from ``keep`` up to 1, fast ones above all: there the walk rounds little and what the tensor cores cut off shows."""
+    from yalis_b200.ops.recurrent import StateLayout
+    heads, vdim, n = 16, 64, 256
+    lay, squares = StateLayout(heads, 128, vdim), torch.zeros(2, 2, dtype=torch.float64)
+    for seed in range(4):
+        g = torch.Generator().manual_seed(seed)
+        data = inputs(rule, heads, heads, vdim, [n], g, keep)
+        on = [None if t is None else t.to(DEV) for t in data]
+        want, last = exact(rule, on, torch.zeros(heads, 128, vdim, dtype=torch.float64, device=DEV), 0, n, heads, heads)
+        for i, chunks in enumerate((True, False)):
+            rows = torch.zeros(1, lay.total, device=DEV)
+            got = run(rule, lay, heads, data, rows, [n], [0], chunks).double()
+            kept = rows[0, :lay.state_floats].view(heads, vdim, 128).double().transpose(1, 2)
+            squares[i] += torch.stack([((got - want).norm() / want.norm()) ** 2, ((kept - last).norm() / last.norm()) ** 2]).cpu()
+    errors = squares.sqrt()
+    # (five per cent: the spread of such sums over the seeds)
+    assert bool((errors[0] <= 1.05 * errors[1]).all()), errors / 2

@@ -12,20 +12,23 @@
 // gemm_f32_mma.cu), T, P (q . k) and the decays, whose products are taken in 64 bits.  The second walks the chunks: a block has 16
 // columns of a head's state, a warp 32 of its rows, as accumulators of the tensor cores in float32 (transposed, so that
 // they are also the operand of the products with k and q).  All sums are float32: products of parts are summed on the tensor cores
-// over 16 values at most, small ones first, and added in registers; the state is scaled in registers, by a decay of two floats (one
-// rounded factor per chunk would add up over a prompt).
+// over 16 values at most, small ones first, and added in registers; dot products of a chunk's tokens are added in 64 bits; the state is
+// scaled in registers, by a decay of two floats (one rounded factor per chunk would add up over a prompt).
 // A chunk starts where its request's portion starts: a long portion's results depend on how the request was cut, by rounding.
-// Errors against float64 beside the walk's (2,048 tokens, slow decays, read-outs / state): constant decay 1.9e-7 / 7.7e-7 (2.0e-7 /
-// 9.4e-7), delta rule 1.4e-7 / 3.6e-7 (1.1e-7 / 3.6e-7), selective 0.7e-7 / 2.2e-7 (1.1e-7 / 5.0e-7).
-// What bounds it: for one request the instructions of a chunk's chain, some 1,900 cycles by the delta rule: a warp alone on its
+// Errors against float64 beside the walk's, read-outs / state in 1e-8 (256 tokens of 16 heads, decays drawn from the named value up to 1,
+// twelve seeds): delta rule from 0: 6.4 / 4.6 (8.9 / 5.1), 0.5: 7.3 / 5.1 (9.5 / 6.1), 0.995: 12 / 10 (28 / 32); selective from 0: 2.6 / 4.3
+// (5.7 / 4.4), 0.5: 2.6 / 4.5 (5.7 / 5.6); a decay a token from 0: 5.4 / 3.4 (8.2 / 3.6); constant decays from 0.5: 8.0 / 5.2 (13.8 / 13).  With
+// single sums on the tensor cores and the chunk's own products first: delta rule from 0: 9.8 / 6.9, from 0.5 10.2 / 7.3.
+// What bounds it: for one request the instructions of a chunk's chain, some 2,150 cycles by the delta rule: a warp alone on its
 // scheduler issues one in about four cycles (clock counts between the chain's stages), so sums start from no cleared
 // registers, the six products of parts are one chain, pairs of float32 operations go in one instruction, and what the chain does not
 // need is left to other warps: waiting for copies, by the delta rule the products with q.  For several requests the copies of k and q,
 // which the blocks of a head's columns all ask for.
 // Measured (us, walk token by token -> both kernels; before copies ran up to four chunks ahead and the chain was shortened), 16
-// heads of 128 x 128 (delta rule: 8 key heads; selective: 32 of 128 x 64), L2 flushed: delta rule 1 x 2,048 387 -> 155 (196),
-// 1 x 128 31 -> 26 to 33 (28), 4 x 901 363 -> 244 (259), 32 x 128 352 -> 259 (282); plain 1 x 2,048 257 -> 108 (155), 4 x 901 224 -> 171 (208),
-// 8 x 512 221 -> 196 (237), 32 x 128 202 -> 200 (234); selective 1 x 2,048 261 -> 99 (144), 4 x 901 237 -> 153 (187), 32 x 128 217 -> 172 (206).
+// heads of 128 x 128 (delta rule: 8 key heads; selective: 32 of 128 x 64, one), L2 flushed: delta rule 1 x 2,048 388 -> 172 (196),
+// 1 x 128 31.7 -> 29.7 (28), 4 x 901 364 -> 253 (259), 32 x 128 352 -> 273 (282); plain 1 x 2,048 257 -> 120 (155), 4 x 901 224 -> 185 (208),
+// 8 x 512 220 -> 212 (237); selective 1 x 2,048 261 -> 110 (144), 4 x 901 237 -> 161 (187), 16 x 256 219 -> 169.  What keeps the errors where
+// the walk has them (the last products of a chunk twice, the own token last, 64-bit sums) is 14 us of the delta rule's 1 x 2,048, 10 of the plain rule's.
 // Not taken: eight row warps and 32 columns a block (for several requests no gain: 282 and 218 for 4 x 901), two chunks in
 // shared memory, k and q copied in pieces whose order differs from block to block, the products with q by the reading warps in the
 // other rules too (1 x 2,048 plain 175, 4 x 901 214: those warps become the chain).
@@ -77,6 +80,16 @@ __device__ __forceinline__ void mma(float (&c)[4], const uint32_t (&a)[4], uint3
 __device__ __forceinline__ void mma0(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
   asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
                : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.f));
+}
+// Eight tokens' products: from zero, and on top of another sum, which stays.
+__device__ __forceinline__ void half0(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t b) {
+  asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%7,%7,%7,%7};"
+               : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3]) : "r"(a0), "r"(a1), "r"(b), "f"(0.f));
+}
+__device__ __forceinline__ void half_on(float (&d)[4], const float (&c)[4], uint32_t a0, uint32_t a1, uint32_t b) {
+  asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%7,%8,%9,%10};"
+               : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+               : "r"(a0), "r"(a1), "r"(b), "f"(c[0]), "f"(c[1]), "f"(c[2]), "f"(c[3]));
 }
 // The parts of a product's operands, small products first: (2, 0), (0, 2), (1, 1), (1, 0), (0, 1), (0, 0).
 __device__ __forceinline__ constexpr int first_part(int o) { return o == 0 ? 2 : o == 2 || o == 3 ? 1 : 0; }
@@ -148,12 +161,13 @@ __global__ void __launch_bounds__(kWarps * 32) chunk_prepare_kernel(const ChunkP
   }
   __syncthreads();
   if (RULE == 1 || warp < 2) {
-    // q k by two warps, k k by two, eight of the second operand's tokens each: sums of 16 products, small ones first, added in order
+    // q k by two warps, k k by two, eight of the second operand's tokens each: per 16 values the products of the first parts and the
+    // five small ones apart, and all sums in 64 bits (a decay of a half leaves of a read-out little but these products)
     const bool qk_here = warp < 2;
     const int s0 = (warp & 1) * 8;
     const uint32_t as = smem_u32(ps_s) + (qk_here ? 3 * kPart * 2 : 0) + (lane & 15) * (kD * 2);
     const uint32_t bs = smem_u32(ps_s) + (s0 + (lane & 7)) * (kD * 2);
-    float sum[4] = {0.f, 0.f, 0.f, 0.f};
+    double sum[4] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll
     for (int j = 0; j < kD / 32; ++j) {                            // 32 values
       uint32_t fa[3][2][4], fb[3][4];
@@ -163,31 +177,33 @@ __global__ void __launch_bounds__(kWarps * 32) chunk_prepare_kernel(const ChunkP
 #pragma unroll
         for (int n = 0; n < 2; ++n) ldmatrix4(fa[i][n], as + i * kPart * 2 + (((4 * j + 2 * n + (lane >> 4)) ^ (lane & 7)) << 4));
       }
-      float more[2][4];
+      float large[2][4], small[2][4];
 #pragma unroll
       for (int o = 0; o < 6; ++o)
 #pragma unroll
         for (int n = 0; n < 2; ++n) {
           const uint32_t(&b)[4] = fb[second_part(o)];
-          if (o == 0) mma0(more[n], fa[first_part(o)][n], b[2 * n], b[2 * n + 1]);
-          else mma(more[n], fa[first_part(o)][n], b[2 * n], b[2 * n + 1]);
+          if (o == 0) mma0(small[n], fa[first_part(o)][n], b[2 * n], b[2 * n + 1]);
+          else if (o < 5) mma(small[n], fa[first_part(o)][n], b[2 * n], b[2 * n + 1]);
+          else mma0(large[n], fa[first_part(o)][n], b[2 * n], b[2 * n + 1]);
         }
 #pragma unroll
       for (int n = 0; n < 2; ++n)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) sum[e] += more[n][e];
+        for (int e = 0; e < 4; ++e) sum[e] += (double)small[n][e] + (double)large[n][e];
     }
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
       const int t = (lane >> 2) + 8 * (e >> 1), s = s0 + 2 * (lane & 3) + (e & 1);
-      if (!(fabsf(sum[e]) <= 3.402823466e38f) && t < valid && s < valid) {      // what parts cannot hold: infinities, the largest values
+      float dot = (float)sum[e];
+      if (!(fabsf(dot) <= 3.402823466e38f) && t < valid && s < valid) {      // what parts cannot hold: infinities, the largest values
         const float* x = (qk_here ? p.q + (size_t)(t0 + t) * p.q_stride : p.k + (size_t)(t0 + t) * p.k_stride) + kvh * kD;
         const float* y = p.k + (size_t)(t0 + s) * p.k_stride + kvh * kD;
         float z = 0.f;
         for (int d = 0; d < kD; ++d) z = __fmaf_rn(x[d], y[d], z);
-        sum[e] = z;
+        dot = z;
       }
-      (qk_here ? qk : kk)[t * kC + s] = sum[e];
+      (qk_here ? qk : kk)[t * kC + s] = dot;
     }
   }
   __syncthreads();
@@ -258,7 +274,7 @@ template <int ID, int N>
 __device__ __forceinline__ void meet() { asm volatile("bar.sync %0, %1;" ::"n"(ID), "n"(N) : "memory"); }
 constexpr int kMeetAll = 0, kMeetWalk = 1, kMeetRead = 2, kMeetTaken = 3;
 
-// Sums over the tokens up to t of a coefficient times a column's value: later ones take no part, be they infinite.
+// A row of a chunk's coefficients.
 __device__ __forceinline__ void load_row(const float* m, float (&c)[kC]) {
 #pragma unroll
   for (int s = 0; s < kC; s += 4) {
@@ -266,12 +282,14 @@ __device__ __forceinline__ void load_row(const float* m, float (&c)[kC]) {
     c[s] = x.x; c[s + 1] = x.y; c[s + 2] = x.z; c[s + 3] = x.w;
   }
 }
-__device__ __forceinline__ float upto(const float (&c)[kC], const float (&y)[kC], int t) {
+// Sum over the tokens before t of a coefficient times a column's value: later ones take no part, be they infinite.  (The token's own
+// product, the largest where decays are fast, is added last.)
+__device__ __forceinline__ float before(const float (&c)[kC], const float (&y)[kC], int t) {
   float a = 0.f, b = 0.f;
 #pragma unroll
   for (int s = 0; s < kC; s += 2) {
-    if (s <= t) a = __fmaf_rn(c[s], y[s], a);
-    if (s + 1 <= t) b = __fmaf_rn(c[s + 1], y[s + 1], b);
+    if (s < t) a = __fmaf_rn(c[s], y[s], a);
+    if (s + 1 < t) b = __fmaf_rn(c[s + 1], y[s + 1], b);
   }
   return a + b;
 }
@@ -406,7 +424,7 @@ __global__ void __launch_bounds__(kAll, STAGES == 3 ? 2 : 1) chunk_walk_kernel(c
         meet<kMeetRead, kWalk>();
       }
       const float* coef = coef_of(c);
-      const float g = coef[kCoefG + t];
+      const float g = coef[kCoefG + t], own = coef[kCoefM + t * kC + t];
       float o[CPT], row_t[kC];
       load_row(coef + kCoefM + t * kC, row_t);
 #pragma unroll
@@ -416,7 +434,7 @@ __global__ void __launch_bounds__(kAll, STAGES == 3 ? 2 : 1) chunk_walk_kernel(c
         for (int w = 0; w < kRowWarps; ++w) read += shares[w * kShares + (v0 + i) * kLdT + t];
         float y[kC];
         load_row(us + ((c & 1) * kV + v0 + i) * kLdT, y);
-        o[i] = __fmaf_rn(g, read, upto(row_t, y, t));
+        o[i] = __fmaf_rn(own, us[((c & 1) * kV + v0 + i) * kLdT + t], __fmaf_rn(g, read, before(row_t, y, t)));
         if constexpr (RULE == 3) o[i] = __fmaf_rn(skip, coef[kCoef + t * kV + v0 + i], o[i]);
       }
       if (c * kC + t < len && j0 + v0 < p.vdim) {
@@ -495,12 +513,14 @@ __global__ void __launch_bounds__(kAll, STAGES == 3 ? 2 : 1) chunk_walk_kernel(c
         a.x += y.x;
         a.y += y.y;
       }
-      *reinterpret_cast<float2*>(rest + v * kLdT + t) = make_float2(__fmaf_rn(-g.x, a.x, x.x), __fmaf_rn(-g.y, a.y, x.y));
+      const float2 own = make_float2(coef[kCoefT + t * kC + t], coef[kCoefT + (t + 1) * kC + t + 1]);
+      const float2 left = make_float2(__fmaf_rn(-g.x, a.x, x.x), __fmaf_rn(-g.y, a.y, x.y));
+      *reinterpret_cast<float2*>(rest + v * kLdT + t) = left;
       meet<kMeetWalk, kWalk>();
       load_k();
       float y[kC];
       load_row(rest + v * kLdT, y);
-      u = make_float2(upto(row[0], y, t), upto(row[1], y, t + 1));
+      u = make_float2(__fmaf_rn(own.x, left.x, before(row[0], y, t)), __fmaf_rn(own.y, left.y, before(row[1], y, t + 1)));
     } else {                                                   // u is known at once
       load_k();
       const float2 b = *reinterpret_cast<const float2*>(coef + kCoefB + t);
@@ -520,16 +540,22 @@ __global__ void __launch_bounds__(kAll, STAGES == 3 ? 2 : 1) chunk_walk_kernel(c
 #pragma unroll
     for (int i = 0; i < 3; ++i)                                // ldmatrix: two halves of the columns by eight tokens, then by the next
       ldmatrix4(fu[i], smem_u32(ups + (((c & 1) * 3 + i) * kV + tt) * kC + (lane >> 4) * 8));
-    float more[NJ][2][4];
+    // The tensor cores cut off the last bits of a sum and of every small term beside a large one.  The first parts' products of the later
+    // eight tokens, the largest where decays are fast, are formed twice: negative, and positive on top of that, which leaves what was
+    // cut off.  The small products join that, then the earlier tokens' first parts; all this joins the old state before the negative sum is
+    // taken off it.
+    float less[NJ][2][4], more[NJ][2][4];
 #pragma unroll
-    for (int o = 0; o < 6; ++o)
+    for (int o = -2; o < 6; ++o)
 #pragma unroll
       for (int j = 0; j < NJ; ++j)
 #pragma unroll
         for (int n = 0; n < 2; ++n) {
-          const uint32_t(&b)[4] = fk[second_part(o)][j];
-          if (o == 0) mma0(more[j][n], fu[first_part(o)], b[2 * n], b[2 * n + 1]);
-          else mma(more[j][n], fu[first_part(o)], b[2 * n], b[2 * n + 1]);
+          const uint32_t(&b)[4] = fk[o < 0 ? 0 : second_part(o)][j];
+          if (o == -2) half0(less[j][n], fu[0][2] ^ 0x80008000u, fu[0][3] ^ 0x80008000u, b[2 * n + 1]);
+          else if (o == -1) half_on(more[j][n], less[j][n], fu[0][2], fu[0][3], b[2 * n + 1]);
+          else if (o < 5) mma(more[j][n], fu[first_part(o)], b[2 * n], b[2 * n + 1]);
+          else half_on(more[j][n], more[j][n], fu[0][0], fu[0][1], b[2 * n]);
         }
 #pragma unroll
     for (int j = 0; j < NJ; ++j)
@@ -538,7 +564,8 @@ __global__ void __launch_bounds__(kAll, STAGES == 3 ? 2 : 1) chunk_walk_kernel(c
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
           float2& x = S[2 * j + n][e];
-          x = fma2(make_float2(hi, hi), x, fma2(make_float2(lo, lo), x, make_float2(more[j][n][2 * e], more[j][n][2 * e + 1])));
+          const float2 y = fma2(make_float2(hi, hi), x, fma2(make_float2(lo, lo), x, make_float2(more[j][n][2 * e], more[j][n][2 * e + 1])));
+          x = fma2(make_float2(less[j][n][2 * e], less[j][n][2 * e + 1]), make_float2(-1.f, -1.f), y);
         }
   }
   if (*lost) return;

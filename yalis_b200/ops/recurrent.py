@@ -119,10 +119,10 @@ def short_conv_silu(x: torch.Tensor, weight: torch.Tensor, slot_rows: torch.Tens
 
 
 # Portions of so many tokens, by rule, may go by chunks of sixteen (a portion's length alone decides, so that a request's result
-# does not depend on what runs beside it).  Where the lines lie (us, walk -> chunks): delta rule 1 x 128 31 -> 26 to 33, 32 x 128
-# 352 -> 259; plain 1 x 128 23 -> 21.5, 32 x 128 202 -> 200; selective 1 x 128 23 -> 30 (its one key head makes few blocks of the
-# first kernel), 1 x 192 32 -> 32, 16 x 192 169 -> 132.
-CHUNKS_FROM = {0: 128, 1: 128, 3: 192}
+# does not depend on what runs beside it).  Where the lines lie (us, walk -> chunks): delta rule 1 x 128 31.7 -> 29.7, 32 x 128
+# 352 -> 273; plain 16 x 192 157 -> 163, 1 x 256 39.8 -> 27.7, 32 x 256 387 -> 384; selective with one key head (few blocks of the
+# first kernel) 1 x 192 31.7 -> 33.8, 1 x 256 39.9 -> 35.8, 16 x 192 168 -> 138, with eight 1 x 192 31.7 -> 25.6.
+CHUNKS_FROM = {0: 256, 1: 128, 3: 208}
 CHUNK = 16
 
 
