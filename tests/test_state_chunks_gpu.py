@@ -219,3 +219,44 @@ def test_errors_are_no_larger_than_the_walks(rule, keep):
     errors = squares.sqrt()
     # (five per cent: the spread of such sums over the seeds)
     assert bool((errors[0] <= 1.05 * errors[1]).all()), errors / 2
+
+
+@pytest.mark.parametrize("what", ["state", "key", "largest", "tiny", "least"])
+@pytest.mark.parametrize("rule", RULES)
+def test_values_that_parts_cannot_hold(rule, what):
+    """Infinities, values that round to one and very small ones: what the walk gives, and the columns beside them as they were."""
+    from yalis_b200.ops.recurrent import StateLayout
+    g = torch.Generator().manual_seed(7)
+    heads, vdim, n = 2, 32, 300
+    lay = StateLayout(heads, 128, vdim)
+    q, k, v, decay, beta, skip = inputs(rule, heads, heads, vdim, [n], g, 0.8)
+    first = torch.randn(1, lay.total, generator=g)
+    plain_rows = first.to(DEV)
+    plain = run(rule, lay, heads, (q, k, v, decay, beta, skip), plain_rows, [n], [0], True)
+    k, v, untouched = k.clone(), v.clone(), torch.ones(heads, vdim, dtype=torch.bool)
+    state = first[0, :lay.state_floats].view(heads, vdim, 128)
+    if what == "state":
+        state[1, 5, 77], untouched[1, 5] = float("inf"), False
+    elif what == "key":
+        k[250, 1, 9], untouched[1] = float("inf"), False
+    elif what == "largest":
+        v[100, 1, 5], untouched[1, 5] = 3.4e38, False
+    else:                                          # a whole head: about 2^-120, or below the normal numbers
+        size = 1e-36 if what == "tiny" else 1e-41
+        v[:, 1] *= size
+        state[1] *= size
+        untouched[1] = False
+    data = (q, k, v, decay, beta, skip)
+    rows, walk_rows = first.to(DEV), first.to(DEV)
+    got, want = run(rule, lay, heads, data, rows, [n], [0], True), run(rule, lay, heads, data, walk_rows, [n], [0], False)
+    cut = lambda r: r[0, :lay.state_floats].view(heads, vdim, 128)
+    assert torch.equal(got[:, untouched], plain[:, untouched]) and torch.equal(cut(rows)[untouched], cut(plain_rows)[untouched])
+    for a, b in ((got, want), (cut(rows), cut(walk_rows))):
+        assert torch.equal(a.isnan(), b.isnan()) and torch.equal(a[b.isinf()], b[b.isinf()])
+        a, b = (x.double().masked_fill(~b.isfinite(), 0) for x in (a, b))
+        if what in ("tiny", "least"):
+            # float32 sums in two orders; below the normal numbers a rounding is half of 1.4e-45 at each of some hundred terms
+            error = (a - b)[..., 1, :] if a.shape[0] == n else (a - b)[1]
+            assert float(error.norm()) <= 1e-6 * float((b[:, 1] if b.shape[0] == n else b[1]).norm()) + 1e-43 * error.numel() ** 0.5
+        else:
+            assert float((a - b).norm()) <= 1e-5 * float(b.norm())

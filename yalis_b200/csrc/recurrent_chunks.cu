@@ -14,6 +14,10 @@
 // they are also the operand of the products with k and q).  All sums are float32: products of parts are summed on the tensor cores
 // over 16 values at most, small ones first, and added in registers; dot products of a chunk's tokens are added in 64 bits; the state is
 // scaled in registers, by a decay of two floats (one rounded factor per chunk would add up over a prompt).
+// Parts do not hold everything: an infinity has no difference to its rounded self, the largest values round to one, and of values below 2^-110
+// the last parts fall below bfloat16's range.  So the tokens of a block are walked again, one by one, where a read-out or a value of the new
+// state is not finite or a read-out lies below 2^-80, and such values are taken from there.  (A portion whose read-outs all lie above that or are zero
+// has errors of up to 2^-134 times the other operand besides: nothing beside a read-out for q and k up to 2^20.)
 // A chunk starts where its request's portion starts: a long portion's results depend on how the request was cut, by rounding.
 // Errors against float64 beside the walk's, read-outs / state in 1e-8 (256 tokens of 16 heads, decays drawn from the named value up to 1,
 // twelve seeds): delta rule from 0: 6.4 / 4.6 (8.9 / 5.1), 0.5: 7.3 / 5.1 (9.5 / 6.1), 0.995: 12 / 10 (28 / 32); selective from 0: 2.6 / 4.3
@@ -195,15 +199,7 @@ __global__ void __launch_bounds__(kWarps * 32) chunk_prepare_kernel(const ChunkP
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
       const int t = (lane >> 2) + 8 * (e >> 1), s = s0 + 2 * (lane & 3) + (e & 1);
-      float dot = (float)sum[e];
-      if (!(fabsf(dot) <= 3.402823466e38f) && t < valid && s < valid) {      // what parts cannot hold: infinities, the largest values
-        const float* x = (qk_here ? p.q + (size_t)(t0 + t) * p.q_stride : p.k + (size_t)(t0 + t) * p.k_stride) + kvh * kD;
-        const float* y = p.k + (size_t)(t0 + s) * p.k_stride + kvh * kD;
-        float z = 0.f;
-        for (int d = 0; d < kD; ++d) z = __fmaf_rn(x[d], y[d], z);
-        dot = z;
-      }
-      (qk_here ? qk : kk)[t * kC + s] = dot;
+      (qk_here ? qk : kk)[t * kC + s] = (float)sum[e];
     }
   }
   __syncthreads();
@@ -272,7 +268,9 @@ constexpr size_t walk_smem() {
 }
 template <int ID, int N>
 __device__ __forceinline__ void meet() { asm volatile("bar.sync %0, %1;" ::"n"(ID), "n"(N) : "memory"); }
-constexpr int kMeetAll = 0, kMeetWalk = 1, kMeetRead = 2, kMeetTaken = 3;
+constexpr int kMeetAll = 0, kMeetWalk = 1, kMeetRead = 2, kMeetTaken = 3, kMeetEnd = 4;
+__device__ __forceinline__ bool finite(float x) { return fabsf(x) <= 3.402823466e38f; }
+__device__ __forceinline__ bool sure(float x) { return finite(x) && fabsf(x) >= 8.3e-25f; }
 
 // A row of a chunk's coefficients.
 __device__ __forceinline__ void load_row(const float* m, float (&c)[kC]) {
@@ -329,8 +327,49 @@ __device__ __forceinline__ void read_state(const uint32_t (&fs)[3][kRowTiles][4]
     }
 }
 
+// The tokens of a portion one by one, for a column c whose state before it is W, eight lanes a column and sixteen rows a lane: takes the place of
+// what the chunks' form did not hold.
+template <int RULE>
+__device__ __noinline__ void walk_again(const ChunkParams& p, float (&W)[kD / 8], float* column, int start, int len, int h, int kvh, int c) {
+  const int lane = threadIdx.x % 8;
+  const bool mine = c < p.vdim;
+  const float skip = (RULE == 3 && p.skip) ? p.skip[h] : 0.f;
+#pragma unroll 1
+  for (int n = start; n < start + len; ++n) {
+    const float* k = p.k + (size_t)n * p.k_stride + kvh * kD + lane * 4;
+    const float* q = p.q + (size_t)n * p.q_stride + kvh * kD + lane * 4;
+    const float g = p.decay_kind == 0 ? p.decay[h] : p.decay[(size_t)n * p.heads + h];
+    const float v = mine ? p.v[(size_t)n * p.v_stride + (size_t)h * p.vdim + c] : 0.f;
+    float u = v, dot = 0.f, read = 0.f;
+#pragma unroll
+    for (int i = 0; i < kD / 8; ++i) {
+      W[i] *= g;
+      dot = __fmaf_rn(k[i / 4 * 32 + i % 4], W[i], dot);
+    }
+    if constexpr (RULE == 1) {
+      for (int o = 1; o < 8; o <<= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
+      u = v - dot;
+    }
+    if constexpr (RULE != 0) u *= p.beta[(size_t)n * p.heads + h];
+#pragma unroll
+    for (int i = 0; i < kD / 8; ++i) {
+      W[i] = __fmaf_rn(k[i / 4 * 32 + i % 4], u, W[i]);
+      read = __fmaf_rn(q[i / 4 * 32 + i % 4], W[i], read);
+    }
+    for (int o = 1; o < 8; o <<= 1) read += __shfl_xor_sync(0xffffffffu, read, o);
+    if constexpr (RULE == 3) read = __fmaf_rn(skip, v, read);
+    if (mine && lane == 0) {
+      float* to = p.out + (size_t)n * p.out_stride + (size_t)h * p.vdim + c;
+      if (!sure(*to)) *to = read;
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < kD / 8; ++i)
+    if (mine && !sure(column[i / 4 * 32 + i % 4])) column[i / 4 * 32 + i % 4] = W[i];
+}
+
 template <int RULE, int STAGES>
-__global__ void __launch_bounds__(kAll, STAGES == 3 ? 2 : 1) chunk_walk_kernel(const ChunkParams p) {
+__global__ void __launch_bounds__(kAll, STAGES == 3 ? 2 : 1) chunk_walk_kernel(const __grid_constant__ ChunkParams p) {
   constexpr int NJ = kRowTiles;
   constexpr bool EARLY = STAGES > 3;                                  // who waits for a chunk's copies: the warp that fetches, or the walking ones
   extern __shared__ __align__(128) unsigned char smem[];
@@ -350,10 +389,12 @@ __global__ void __launch_bounds__(kAll, STAGES == 3 ? 2 : 1) chunk_walk_kernel(c
   __nv_bfloat16* ups = reinterpret_cast<__nv_bfloat16*>(rest + (RULE == 1 ? kV * kLdT : 0));
   uint64_t* there = reinterpret_cast<uint64_t*>(ups + 2 * 3 * kC * kV);
   volatile int* lost = reinterpret_cast<volatile int*>(there + STAGES);      // a wait ran out
+  volatile int* again = lost + 1;                                            // something was not held
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) asm volatile("mbarrier.init.shared::cta.b64 [%0], 33;" ::"r"(smem_u32(&there[s])));      // lane 0 and every lane's copies
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     *lost = 0;
+    *again = 0;
   }
   __syncthreads();
   auto coef_of = [&](int c) { return reinterpret_cast<const float*>(smem + c % STAGES * kStage + 6 * kPart * 2); };
@@ -405,6 +446,7 @@ __global__ void __launch_bounds__(kAll, STAGES == 3 ? 2 : 1) chunk_walk_kernel(c
     constexpr int CPT = kC * kV / kWalk;
     const int rt = tid, t = rt / (kV / CPT), v0 = rt % (kV / CPT) * CPT;
     const float skip = (RULE == 3 && p.skip) ? p.skip[h] : 0.f;
+    bool all = true;                                          // held by the parts
     meet<kMeetAll, kAll>();
     for (int c = 0; c < chunks; ++c) {
       meet<kMeetAll, kAll>();
@@ -440,9 +482,14 @@ __global__ void __launch_bounds__(kAll, STAGES == 3 ? 2 : 1) chunk_walk_kernel(c
       if (c * kC + t < len && j0 + v0 < p.vdim) {
         float* to = p.out + (size_t)(start + c * kC + t) * p.out_stride + (size_t)h * p.vdim + j0 + v0;
 #pragma unroll
-        for (int i = 0; i < CPT; i += 2) *reinterpret_cast<float2*>(to + i) = make_float2(o[i], o[i + 1]);
+        for (int i = 0; i < CPT; i += 2) {
+          *reinterpret_cast<float2*>(to + i) = make_float2(o[i], o[i + 1]);
+          all = all && (sure(o[i]) || o[i] == 0.f) && (sure(o[i + 1]) || o[i + 1] == 0.f);
+        }
       }
     }
+    if (!all) *again = 1;
+    meet<kMeetEnd, 2 * kWalk>();
     return;
   }
 
@@ -568,12 +615,34 @@ __global__ void __launch_bounds__(kAll, STAGES == 3 ? 2 : 1) chunk_walk_kernel(c
           x = fma2(make_float2(less[j][n][2 * e], less[j][n][2 * e + 1]), make_float2(-1.f, -1.f), y);
         }
   }
-  if (*lost) return;
+  bool whole = true;
 #pragma unroll
   for (int n = 0; n < 2 * NJ; ++n)
 #pragma unroll
-    for (int e = 0; e < 2; ++e)
-      if (j0 + col + 8 * e < p.vdim) *reinterpret_cast<float2*>(sp + (size_t)e * 8 * kD + 8 * n) = S[n][e];
+    for (int e = 0; e < 2; ++e) whole = whole && finite(S[n][e].x) && finite(S[n][e].y);
+  if (!whole) *again = 1;
+  meet<kMeetEnd, 2 * kWalk>();
+  if (*lost) return;
+  auto store = [&]() {
+#pragma unroll
+    for (int n = 0; n < 2 * NJ; ++n)
+#pragma unroll
+      for (int e = 0; e < 2; ++e)
+        if (j0 + col + 8 * e < p.vdim) *reinterpret_cast<float2*>(sp + (size_t)e * 8 * kD + 8 * n) = S[n][e];
+  };
+  if (!*again) {
+    store();
+    return;
+  }
+  float W[kD / 8];                                             // the state before the portion, eight lanes a column
+  const int c = j0 + tid / 8;
+  float* column = p.state + (size_t)p.slots[req] * p.slot_stride + ((size_t)h * p.vdim + c) * kD + tid % 8 * 4;
+#pragma unroll
+  for (int i = 0; i < kD / 8; ++i) W[i] = c < p.vdim ? column[i / 4 * 32 + i % 4] : 0.f;
+  meet<kMeetWalk, kWalk>();
+  store();
+  meet<kMeetWalk, kWalk>();
+  walk_again<RULE>(p, W, column, start, len, h, kvh, c);
 }
 
 template <int RULE, int STAGES>
