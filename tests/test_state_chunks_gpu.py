@@ -260,3 +260,19 @@ def test_values_that_parts_cannot_hold(rule, what):
             assert float(error.norm()) <= 1e-6 * float((b[:, 1] if b.shape[0] == n else b[1]).norm()) + 1e-43 * error.numel() ** 0.5
         else:
             assert float((a - b).norm()) <= 1e-5 * float(b.norm())
+
+
+@pytest.mark.parametrize("rule", ["constant", "delta", "selective"])
+@pytest.mark.parametrize("room", [1, 7, 20, 64])
+def test_a_step_in_several_launches_has_the_same_bits(rule, room, monkeypatch):
+    """Fewer chunks than the step has, or even a portion: what is left goes in further launches, from the state that the last one left."""
+    from yalis_b200.ops import recurrent
+    g = torch.Generator().manual_seed(room)
+    heads, kv_heads, vdim, lens, slots = 4, 2, 36, [300, 3, 0, 256, 513, 209, 1], [2, 0, 3, 6, 1, 5, 4]
+    lay = recurrent.StateLayout(heads, 128, vdim)
+    data, first = inputs(rule, heads, kv_heads, vdim, lens, g), torch.randn(7, lay.total, generator=g).to(DEV)
+    rows, few_rows = first.clone(), first.clone()
+    whole = run(rule, lay, kv_heads, data, rows, lens, slots, True)
+    monkeypatch.setattr(recurrent, "CHUNK_BYTES", (room - 1) * kv_heads * 2 * 3 * 16 * 128 * 2)
+    few = run(rule, lay, kv_heads, data, few_rows, lens, slots, True)
+    assert torch.equal(few, whole) and torch.equal(few_rows, rows)

@@ -23,16 +23,16 @@
 // twelve seeds): delta rule from 0: 6.4 / 4.6 (8.9 / 5.1), 0.5: 7.3 / 5.1 (9.5 / 6.1), 0.995: 12 / 10 (28 / 32); selective from 0: 2.6 / 4.3
 // (5.7 / 4.4), 0.5: 2.6 / 4.5 (5.7 / 5.6); a decay a token from 0: 5.4 / 3.4 (8.2 / 3.6); constant decays from 0.5: 8.0 / 5.2 (13.8 / 13).  With
 // single sums on the tensor cores and the chunk's own products first: delta rule from 0: 9.8 / 6.9, from 0.5 10.2 / 7.3.
-// What bounds it: for one request the instructions of a chunk's chain, some 2,150 cycles by the delta rule: a warp alone on its
+// What bounds it: for one request the instructions of a chunk's chain, some 2,100 cycles by the delta rule: a warp alone on its
 // scheduler issues one in about four cycles (clock counts between the chain's stages), so sums start from no cleared
 // registers, the six products of parts are one chain, pairs of float32 operations go in one instruction, and what the chain does not
 // need is left to other warps: waiting for copies, by the delta rule the products with q.  For several requests the copies of k and q,
 // which the blocks of a head's columns all ask for.
 // Measured (us, walk token by token -> both kernels; before copies ran up to four chunks ahead and the chain was shortened), 16
-// heads of 128 x 128 (delta rule: 8 key heads; selective: 32 of 128 x 64, one), L2 flushed: delta rule 1 x 2,048 388 -> 172 (196),
-// 1 x 128 31.7 -> 29.7 (28), 4 x 901 364 -> 253 (259), 32 x 128 352 -> 273 (282); plain 1 x 2,048 257 -> 120 (155), 4 x 901 224 -> 185 (208),
-// 8 x 512 220 -> 212 (237); selective 1 x 2,048 261 -> 110 (144), 4 x 901 237 -> 161 (187), 16 x 256 219 -> 169.  What keeps the errors where
-// the walk has them (the last products of a chunk twice, the own token last, 64-bit sums) is 14 us of the delta rule's 1 x 2,048, 10 of the plain rule's.
+// heads of 128 x 128 (delta rule: 8 key heads; selective: 32 of 128 x 64, one), L2 flushed: delta rule 1 x 2,048 387 -> 168 (196),
+// 1 x 128 30.7 -> 30.7 (28), 4 x 901 363 -> 254 (259), 32 x 128 351 -> 275 (282); plain 1 x 2,048 257 -> 120 (155), 4 x 901 223 -> 185 (208),
+// 8 x 512 219 -> 196 (237); selective 1 x 2,048 260 -> 110 (144), 4 x 901 236 -> 163 (187), 16 x 256 219 -> 169.  What keeps the errors where
+// the walk has them (the last products of a chunk twice, the own token last, 64-bit sums) is 10 us of each rule's 1 x 2,048.
 // Not taken: eight row warps and 32 columns a block (for several requests no gain: 282 and 218 for 4 x 901), two chunks in
 // shared memory, k and q copied in pieces whose order differs from block to block, the products with q by the reading warps in the
 // other rules too (1 x 2,048 plain 175, 4 x 901 214: those warps become the chain).
@@ -58,13 +58,24 @@ struct ChunkParams {
   float* out; int out_stride;
   const int32_t* q_start; const int32_t* slots;
   int heads, kv_heads, vdim, shortest, longest; // portions of other lengths are left out
+  int from, room;                               // the places of chunks that this launch takes: from ... from + room - 1
   __nv_bfloat16* parts;                         // [chunk][kv_head][k, q][3][16][128], 16-byte pieces swapped within rows
   float* coef;                                  // [chunk][head][kCoef]
   int32_t* error;
 };
 
-// The chunks of request r begin here: no two requests' chunks share a place.
-__device__ __forceinline__ int first_chunk(int start, int r) { return start / kC + r; }
+// The tokens of request r that this launch takes, and where its chunks lie: no two requests' chunks share a place.
+struct Portion {
+  int start, len;                               // len 0: none
+  int first;
+};
+__device__ __forceinline__ Portion portion_of(const ChunkParams& p, int r) {
+  const int start = p.q_start[r], len = p.q_start[r + 1] - start, place = start / kC + r - p.from;      // of its first chunk
+  const int skip = max(0, -place) * kC;                                                                // taken before
+  Portion o = {start + skip, min(len - skip, (p.room - max(0, place)) * kC), max(0, place)};
+  if (len < p.shortest || len > p.longest || o.len < 0) o.len = 0;
+  return o;
+}
 
 __device__ __forceinline__ uint32_t two_bf16(float lo, float hi) {
   __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
@@ -139,11 +150,12 @@ __global__ void __launch_bounds__(kWarps * 32) chunk_prepare_kernel(const ChunkP
   __shared__ float kk[kC * kC], qk[kC * kC], ratio[kWarps][kC * kC];
   pdl_launch_dependents();
   pdl_wait();
-  const int req = blockIdx.z, kvh = blockIdx.y, start = p.q_start[req], len = p.q_start[req + 1] - start;
-  const int t0 = start + blockIdx.x * kC, valid = min(kC, start + len - t0);
-  if (len < p.shortest || len > p.longest || valid <= 0) return;
+  const int req = blockIdx.z, kvh = blockIdx.y;
+  const Portion portion = portion_of(p, req);
+  const int t0 = portion.start + blockIdx.x * kC, valid = min(kC, portion.len - (int)blockIdx.x * kC);
+  if (valid <= 0) return;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const size_t chunk = first_chunk(start, req) + blockIdx.x;
+  const size_t chunk = portion.first + (int)blockIdx.x;
   __nv_bfloat16* parts = p.parts + (chunk * p.kv_heads + kvh) * (6 * kPart);
   for (int e = tid; e < 2 * kC * (kD / 8); e += kWarps * 32) {
     const int which = e / (kC * (kD / 8)), t = e / (kD / 8) % kC, c = e % (kD / 8);       // k, then q; a piece of eight values
@@ -375,12 +387,17 @@ __global__ void __launch_bounds__(kAll, STAGES == 3 ? 2 : 1) chunk_walk_kernel(c
   extern __shared__ __align__(128) unsigned char smem[];
   pdl_launch_dependents();
   pdl_wait();
-  const int req = blockIdx.z, h = blockIdx.y, j0 = blockIdx.x * kV, start = p.q_start[req], len = p.q_start[req + 1] - start;
-  if (len < p.shortest || len > p.longest) return;
+  const int req = blockIdx.z, h = blockIdx.y, j0 = blockIdx.x * kV;
+  Portion portion = portion_of(p, req);
+  if (portion.len <= 0) return;
+  // (that there is a first chunk is kept from the compiler: without the check in front of its loops it orders a chunk's instructions
+  // otherwise, 179 us in place of 165 for the delta rule's 1 x 2,048)
+  asm volatile("" : "+r"(portion.start), "+r"(portion.len), "+r"(portion.first));
+  const int start = portion.start, len = portion.len;
   const int role = threadIdx.x / kWalk, tid = threadIdx.x % kWalk;      // role 0 walks, 1 reads, 2 fetches
   const int lane = tid & 31, kvh = h / (p.heads / p.kv_heads);
   const int chunks = (len + kC - 1) / kC;
-  const size_t first = first_chunk(start, req);
+  const size_t first = portion.first;
   uint4* state_parts = reinterpret_cast<uint4*>(smem + STAGES * kStage);
   float* shares_q = reinterpret_cast<float*>(state_parts + (RULE == 1 ? kStateParts : 0));      // RULE 1: one buffer
   float* shares_k = shares_q + kRowWarps * kShares;                                             // RULE 1
@@ -655,17 +672,22 @@ int launch_walk(const ChunkParams& p, int n_requests, cudaStream_t stream) {
 // Chunks in shared memory: three leave room for two blocks on an SM, which cover each other's copies; where there is a block an SM at
 // most, five.
 template <int RULE>
-int launch_chunks(const ChunkParams& p, int n_requests, int longest, cudaStream_t stream) {
-  const int st = yalis_launch(chunk_prepare_kernel<RULE>, dim3((longest + kC - 1) / kC, p.kv_heads, n_requests), dim3(kWarps * 32), 0, stream, p);
-  if (st != YALIS_OK) return st;
+int launch_chunks(ChunkParams p, int n_requests, int places, cudaStream_t stream) {
   const long long blocks = (long long)((p.vdim + kV - 1) / kV) * p.heads * n_requests;
-  return blocks <= yalis_sm_count() ? launch_walk<RULE, 5>(p, n_requests, stream) : launch_walk<RULE, 3>(p, n_requests, stream);
+  const dim3 grid(min((p.longest + kC - 1) / kC, p.room), p.kv_heads, n_requests);
+  for (p.from = 0; p.from < places; p.from += p.room) {
+    int st = yalis_launch(chunk_prepare_kernel<RULE>, grid, dim3(kWarps * 32), 0, stream, p);
+    if (st == YALIS_OK) st = blocks <= yalis_sm_count() ? launch_walk<RULE, 5>(p, n_requests, stream) : launch_walk<RULE, 3>(p, n_requests, stream);
+    if (st != YALIS_OK) return st;
+  }
+  return YALIS_OK;
 }
 
 }  // namespace
 
-// float32 values per (chunk, head) of `coef`; a step has n_tokens / 16 + n_requests + 1 chunks at most, each with 6 x 16 x 128
-// bfloat16 values per key head in `parts`.
+// float32 values per (chunk, head) of `coef`; a chunk has 6 x 16 x 128 bfloat16 values per key head in `parts`.  places: of chunks in the
+// step, n_tokens / 16 + n_requests + 1; room: chunks that parts and coef hold.  Where there are more places the step is taken in
+// several launches, to the same bits: between two of them the state is the slots'.
 YALIS_API int yalis_state_chunks_coefficients() { return kCoef; }
 
 // The portions of `shortest` to `longest` tokens of a step, the others are left alone.  dim 128, vdim a multiple of four, rows on
@@ -674,8 +696,9 @@ YALIS_API int yalis_state_chunks(const float* q, int q_stride, const float* k, i
                                  const float* decay, int decay_kind, const float* beta, const float* skip, float* state,
                                  int64_t slot_stride, float* out, int out_stride, const int32_t* q_start, const int32_t* slots,
                                  int n_requests, int heads, int kv_heads, int dim, int vdim, int rule, int longest, int shortest,
-                                 void* parts, void* coef, int32_t* error, cudaStream_t stream) {
+                                 int places, int room, void* parts, void* coef, int32_t* error, cudaStream_t stream) {
   if (n_requests <= 0 || longest <= 0) return YALIS_OK;
+  if (places <= 0 || places > (1 << 30) || room <= 0) return YALIS_ERR_SHAPE;
   if (dim != kD || vdim <= 0 || vdim % 4 || heads <= 0 || kv_heads <= 0 || heads % kv_heads || heads > 65535 || n_requests > 65535)
     return YALIS_ERR_SHAPE;
   if (decay_kind < 0 || decay_kind > 1 || !decay || (rule != 0 && rule != 1 && rule != 3) || (rule && !beta)) return YALIS_ERR_SHAPE;
@@ -683,8 +706,8 @@ YALIS_API int yalis_state_chunks(const float* q, int q_stride, const float* k, i
       (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)state | (uintptr_t)out | (uintptr_t)parts | (uintptr_t)coef) & 15))
     return YALIS_ERR_ALIGN;
   const ChunkParams p = {q, q_stride, k, k_stride, v, v_stride, decay, decay_kind, beta, skip, state, (size_t)slot_stride, out, out_stride,
-                         q_start, slots, heads, kv_heads, vdim, shortest, longest, (__nv_bfloat16*)parts, (float*)coef, error};
-  if (rule == 0) return launch_chunks<0>(p, n_requests, longest, stream);
-  if (rule == 1) return launch_chunks<1>(p, n_requests, longest, stream);
-  return launch_chunks<3>(p, n_requests, longest, stream);
+                         q_start, slots, heads, kv_heads, vdim, shortest, longest, 0, room < places ? room : places, (__nv_bfloat16*)parts, (float*)coef, error};
+  if (rule == 0) return launch_chunks<0>(p, n_requests, places, stream);
+  if (rule == 1) return launch_chunks<1>(p, n_requests, places, stream);
+  return launch_chunks<3>(p, n_requests, places, stream);
 }

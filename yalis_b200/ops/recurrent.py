@@ -119,11 +119,15 @@ def short_conv_silu(x: torch.Tensor, weight: torch.Tensor, slot_rows: torch.Tens
 
 
 # Portions of so many tokens, by rule, may go by chunks of sixteen (a portion's length alone decides, so that a request's result
-# does not depend on what runs beside it).  Where the lines lie (us, walk -> chunks): delta rule 1 x 128 31.7 -> 29.7, 32 x 128
-# 352 -> 273; plain 16 x 192 157 -> 163, 1 x 256 39.8 -> 27.7, 32 x 256 387 -> 384; selective with one key head (few blocks of the
-# first kernel) 1 x 192 31.7 -> 33.8, 1 x 256 39.9 -> 35.8, 16 x 192 168 -> 138, with eight 1 x 192 31.7 -> 25.6.
+# does not depend on what runs beside it).  Where the lines lie (us, walk -> chunks): delta rule 1 x 128 30.7 -> 30.7, 32 x 128
+# 351 -> 275; plain 16 x 192 157 -> 163, 1 x 256 38.9 -> 29.7, 32 x 256 386 -> 376; selective with one key head (few blocks of the
+# first kernel) 1 x 192 31.7 -> 33.8, 16 x 192 167 -> 138, with eight 1 x 192 30.7 -> 25.6.
 CHUNKS_FROM = {0: 256, 1: 128, 3: 208}
 CHUNK = 16
+# The most that the parts of k and q of one launch take (24 KB a chunk and key head): longer steps are taken in several launches, to the same
+# bits.  A step of 2,048 tokens with 16 key heads has 51 MB, one of 32,768 would have 806.  (32 x 256 tokens by the plain rule in
+# two launches instead of one: 384 -> 419 us.)
+CHUNK_BYTES = 256 << 20
 
 
 def _takes_chunks(q, k, v, slot_rows, dim, vdim, kind, rule, longest) -> bool:
@@ -195,13 +199,14 @@ def state_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, slot_rows: tor
         i32(slots.numel()), i32(h), i32(kv_heads), i32(d), i32(vd), i32(rule), i32(min(max_q_len, limit - 1) if limit else max_q_len),
         i32(limit), i32(max_q_len), stream()), name)
     if limit:
-        at_most = n // CHUNK + slots.numel() + 1                  # chunks of the step
-        parts = torch.empty((at_most, kv_heads, 2, 3, CHUNK, d), dtype=torch.bfloat16, device=q.device)
-        coef = torch.empty((at_most, h, int(lib().yalis_state_chunks_coefficients())), dtype=torch.float32, device=q.device)
+        places = n // CHUNK + slots.numel() + 1                   # of chunks in the step
+        room = min(places, CHUNK_BYTES // (kv_heads * 2 * 3 * CHUNK * d * 2) + 1)
+        parts = torch.empty((room, kv_heads, 2, 3, CHUNK, d), dtype=torch.bfloat16, device=q.device)
+        coef = torch.empty((room, h, int(lib().yalis_state_chunks_coefficients())), dtype=torch.float32, device=q.device)
         check(lib().yalis_state_chunks(
             ptr(q), i32(q.stride(0)), ptr(k), i32(k.stride(0)), ptr(v), i32(v.stride(0)), ptr(decay), i32(kind), ptr(beta), ptr(skip),
             ptr(slot_rows), i64(slot_rows.stride(0)), ptr(out), i32(out.stride(0)), ptr(q_start), ptr(slots), i32(slots.numel()), i32(h),
-            i32(kv_heads), i32(d), i32(vd), i32(rule), i32(max_q_len), i32(limit), ptr(parts), ptr(coef), ptr(error_word(q.device)),
+            i32(kv_heads), i32(d), i32(vd), i32(rule), i32(max_q_len), i32(limit), i32(places), i32(room), ptr(parts), ptr(coef), ptr(error_word(q.device)),
             stream()), name)
     return out
 
