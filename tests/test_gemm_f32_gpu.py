@@ -44,3 +44,33 @@ def test_values_that_parts_cannot_hold():
     # rows of tiny values: float32 FMAs in another order (the smallest products fall below the normal range)
     torch.testing.assert_close(got[4, :9], want[4, :9], rtol=1e-5, atol=1e-41)
     assert torch.equal(got[7:, :9], plain[7:, :9]) and torch.equal(got[0, 11:], plain[0, 11:])
+
+
+@pytest.mark.parametrize("small,large", [(1e-37, 1e34), (1e-41, 1e20), (1e-42, 1e38), (1e-36, 1e30), (1e-30, 1e-14)])
+@pytest.mark.parametrize("m", [5, 70, 300])
+def test_small_values_beside_large_ones(small, large, m):
+    """Values whose last parts bfloat16 does not hold, against values large enough to bring the product back: in rows of x, in rows of W, in
+    single places; the rows beside them keep their bits."""
+    from yalis_b200.ops.linear import gemm_f32
+    g = torch.Generator().manual_seed(m)
+    n, k = 140, 260
+    x, w = torch.randn(m, k, generator=g).to(DEV), torch.randn(n, k, generator=g).to(DEV)
+    plain = gemm_f32(x, w)
+    y, v = x.clone(), w.clone()
+    y[1] *= small
+    v[7] *= large
+    y[2] *= large
+    v[9] *= small
+    y[3], v[11] = 0.0, 0.0
+    y[3, 5], v[11, 5], v[12, 5] = small, large, small
+    y[4] = 0.0
+    got = gemm_f32(y, v)
+    want, size = y.double() @ v.double().t(), y.double().abs() @ v.double().abs().t()
+    # float32 sums; below the normal numbers (products of two small values) a rounding is half of 1.4e-45
+    bound = (k + 1) * (2.0 ** -24 * size + 1.4e-45)
+    finite = size < 3e38                                       # (partial sums of FMAs may leave the range beyond)
+    assert bool(((got.double() - want).abs() <= bound)[finite].all()), float(((got.double() - want).abs() / bound)[finite].max())
+    assert not bool(got[4].any())
+    others = torch.ones(n, dtype=torch.bool)
+    others[[7, 9, 11, 12]] = False
+    assert torch.equal(got[5:, others], plain[5:, others]) and torch.equal(got[0, others], plain[0, others])

@@ -11,8 +11,9 @@
 // its rows as float32, some steps ahead by asynchronous copies that each reads back itself, part them and lay the parts out in
 // shared memory (two stages, pieces of 16 bytes swapped within rows of 64: neither the stores nor ldmatrix meet in a bank).
 //
-// An output that is not finite or is tiny is computed again in float32 FMAs: an infinity has no difference to its rounded
-// self, the rounding of the largest values overflows, and the parts of the smallest ones fall below bfloat16's range.
+// The parts are those of the values times 2^16: so even the last bit of the smallest float32 value lies in bfloat16's range.  An output is computed again
+// in float32 FMAs where its sum is not finite (an infinity has no difference to its rounded self, and values from 2^112 and
+// outputs from 2^96 on leave the range at its other end) or below 2^-80 (an output below 2^-112: the small parts' products leave it).
 //
 // What bounds it: mma.sync, which gives 2,048 products a two cycles and SM (973 a cycle measured alone; 0.64 of that here: the
 // warps load and multiply in step with one another), and in small steps the chain of a step: copy, part, barrier, load, twelve
@@ -36,15 +37,28 @@ __device__ __forceinline__ uint32_t two_bf16(float lo, float hi) {
   __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
   return *reinterpret_cast<uint32_t*>(&v);
 }
-// Four values as three groups of four bfloat16 values whose sums they are.
+constexpr float kScale = 65536.f;
+// Two float32 operations in one instruction, each rounded as the single one is.
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  uint64_t d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(*reinterpret_cast<uint64_t*>(&a)), "l"(*reinterpret_cast<uint64_t*>(&b)), "l"(*reinterpret_cast<uint64_t*>(&c)));
+  return *reinterpret_cast<float2*>(&d);
+}
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+  uint64_t d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(*reinterpret_cast<uint64_t*>(&a)), "l"(*reinterpret_cast<uint64_t*>(&b)));
+  return *reinterpret_cast<float2*>(&d);
+}
+// Four values times kScale as three groups of four bfloat16 values whose sums they are.
 __device__ __forceinline__ void part(const float4 v, uint2 (&o)[3]) {
-  float a[4] = {v.x, v.y, v.z, v.w};
+  const float2 scale = make_float2(kScale, kScale), minus = make_float2(-1.f, -1.f);
+  float2 a = mul2(make_float2(v.x, v.y), scale), b = mul2(make_float2(v.z, v.w), scale);
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
-    o[i] = make_uint2(two_bf16(a[0], a[1]), two_bf16(a[2], a[3]));
+    o[i] = make_uint2(two_bf16(a.x, a.y), two_bf16(b.x, b.y));
     if (i < 2) {
-      a[0] -= __uint_as_float(o[i].x << 16); a[1] -= __uint_as_float(o[i].x & 0xffff0000u);
-      a[2] -= __uint_as_float(o[i].y << 16); a[3] -= __uint_as_float(o[i].y & 0xffff0000u);
+      a = fma2(make_float2(__uint_as_float(o[i].x << 16), __uint_as_float(o[i].x & 0xffff0000u)), minus, a);
+      b = fma2(make_float2(__uint_as_float(o[i].y << 16), __uint_as_float(o[i].y & 0xffff0000u)), minus, b);
     }
   }
 }
@@ -211,6 +225,7 @@ __global__ void __launch_bounds__((WR * WT + FW) * 32) gemm_f32_parts_kernel(con
     const int t = e / ROWS, r = e % ROWS, m = m0 + t, n = n0 + r;
     float y = sums[e];
     const float size = fabsf(y);
+    y *= 1.f / kScale / kScale;
     const bool mine = m < p.M && n < p.N, again = mine && !(size <= 3.402823466e38f && (size >= 8.3e-25f || size == 0.f));
     for (uint32_t todo = __ballot_sync(0xffffffffu, again); todo != 0; todo &= todo - 1) {
       const int who = __ffs(todo) - 1;

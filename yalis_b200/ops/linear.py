@@ -7,6 +7,8 @@ Two precisions, chosen by the operands' dtype:
   (csrc/gemm_f32_mma.cu); small and unaligned ones are FMAs on the CUDA cores
   (csrc/gemm_simt.cu).  Which of the two depends on the weight alone and either sums in
   an order that the weight's shape fixes, so a row's bits do not depend on the others.
+  As in the bfloat16 kernels a weight is fetched while the kernel in front still runs:
+  no kernel of a step may write it.
 * bfloat16 operands: float32 accumulation on the tensor cores.  Steps of up
   to 32 tokens (decode) go to the engine's own tcgen05 weight-streaming kernel,
   which takes up to 256 tokens but is the faster one only for few; larger
