@@ -118,3 +118,93 @@ def test_later_values_and_missing_pages_do_not_reach_a_query():
     s = s.masked_fill((j[None] > j[:, None]) | ((j[None] // 16 == 2) | (j[None] >= 64)), -math.inf)
     want = s.softmax(-1) @ v.double()
     assert (got.double() - want).norm() < 1e-6 * want.norm()
+
+
+# heads and key/value heads that make a block take four heads and two queries, two and four, one and four in steps of these many tokens
+FORMS = [(32, 8), (16, 8), (27, 9)]
+LENS, BEFORE = [61, 1, 2, 47, 30, 3, 16], [0, 9, 30, 3, 101, 62, 32]
+
+
+def step(heads, kv, dim, g, page=16):
+    rnd = lambda *s: torch.randn(*s, generator=g)
+    held = [a + b for a, b in zip(LENS, BEFORE)]
+    ks, vs, q = [rnd(h, kv, dim) for h in held], [rnd(h, kv, dim) for h in held], rnd(sum(LENS), heads * dim)
+    counts = [-(-h // page) for h in held]
+    order, table, at = torch.randperm(sum(counts), generator=g) + 1, torch.full((len(held), max(counts)), -1, dtype=torch.int32), 0
+    pools = [torch.full((sum(counts) + 1, kv, page, dim), math.nan) for _ in range(2)]
+    for r, h in enumerate(held):
+        for i in range(counts[r]):
+            table[r, i] = int(order[at])
+            rows = slice(i * page, min(h, (i + 1) * page))
+            for pool, x in zip(pools, (ks, vs)):
+                pool[order[at], :, :rows.stop - rows.start] = x[r][rows].transpose(0, 1)
+            at += 1
+    tokens = [(r, b + i) for r, (l, b) in enumerate(zip(LENS, BEFORE)) for i in range(l)]
+    return q, ks, vs, pools, table, tokens
+
+
+def attend(q, pools, table, tokens, heads, kv, dim, which, gate=None, **o):
+    from yalis_b200.ops.attention import paged_attention_generic
+    at = torch.tensor(which)
+    ints = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    dev = lambda t: t.to(DEV) if torch.is_tensor(t) else t
+    return paged_attention_generic(q[at].to(DEV), pools[0].to(DEV), pools[1].to(DEV), ints([tokens[i][1] for i in which]), ints([tokens[i][0] for i in which]),
+                                   table.to(DEV), heads, kv, dim, gate=None if gate is None else gate[at].to(DEV), **{k: dev(v) for k, v in o.items()}).cpu()
+
+
+@pytest.mark.parametrize("options", OPTIONS, ids=lambda o: "-".join(o) or "plain")
+@pytest.mark.parametrize("heads,kv", FORMS)
+@pytest.mark.parametrize("dim", [64, 128])
+def test_several_queries_a_block(heads, kv, dim, options):
+    """Steps large enough for every form with several queries: portions that begin and end within a group of positions, single tokens beside
+    them, against float64; the tokens one at a time, thus a query and a head a block, have the same bits."""
+    g = torch.Generator().manual_seed(heads + dim)
+    q, ks, vs, pools, table, tokens = step(heads, kv, dim, g)
+    n = len(tokens)
+    o = {k: v for k, v in options.items() if k in ("window", "chunk", "softcap", "out_scale")}
+    gate = None if "gate" not in options else torch.randn(n, heads * dim if options["gate"] == "value" else heads, generator=g)
+    if options.get("sink"):
+        o["sink"] = True
+        if options["sink"] == "logits":
+            o["sink_logits"] = torch.randn(heads, generator=g)
+    if "slopes" in options:
+        o["slopes"] = torch.rand(heads, generator=g) * 0.1
+    if "rel" in options:
+        o["rel"] = torch.randn(heads, 20, generator=g)
+    got, a = attend(q, pools, table, tokens, heads, kv, dim, list(range(n)), gate, **o), 0
+    for r, l in enumerate(LENS):
+        mine = {**o, **({} if gate is None else {"gate": gate[a:a + l]})}
+        want = plain(q[a:a + l].double().view(l, heads, dim), ks[r].double(), vs[r].double(), torch.arange(BEFORE[r], BEFORE[r] + l), mine, dim ** -0.5)
+        # as above
+        assert (got[a:a + l].view_as(want).double() - want).norm() < 1e-6 * want.norm(), r
+        a += l
+    some = list(range(0, n, 9)) + [60, 61, 62, 63, 64, n - 1]
+    alone = torch.cat([attend(q, pools, table, tokens, heads, kv, dim, [i], gate, **o) for i in some])
+    assert torch.equal(alone, got[torch.tensor(some)])
+    assert torch.equal(attend(q, pools, table, tokens, heads, kv, dim, list(range(n))[::-1], gate, **o), got.flip(0))
+
+
+@pytest.mark.parametrize("heads,kv", FORMS)
+@pytest.mark.parametrize("dim", [64, 128])
+def test_several_queries_later_values_and_missing_pages(heads, kv, dim):
+    g = torch.Generator().manual_seed(dim)
+    q, ks, vs, pools, table, tokens = step(heads, kv, dim, g)
+    every = list(range(len(tokens)))
+    whole = attend(q, pools, table, tokens, heads, kv, dim, every)
+    bad, place = [pools[0], pools[1].clone()], 37
+    bad[1][table[0, place // 16], :, place % 16] = math.inf
+    got = attend(q, bad, table, tokens, heads, kv, dim, every)
+    reached = torch.tensor([r == 0 and p >= place for r, p in tokens])
+    assert torch.equal(got[~reached], whole[~reached]) and bool(got[reached].isinf().all())
+    gaps = table.clone()
+    gaps[4, 2], gaps[0, 1] = -1, 10 ** 6                       # keys without a page count as masked
+    got, a = attend(q, pools, gaps, tokens, heads, kv, dim, every), 0
+    for r, l in enumerate(LENS):
+        pos, j = torch.arange(BEFORE[r], BEFORE[r] + l), torch.arange(BEFORE[r] + l)
+        k, v = (x[r].double().repeat_interleave(heads // kv, 1) for x in (ks, vs))
+        s = torch.einsum("thd,lhd->thl", q[a:a + l].double().view(l, heads, dim), k) * dim ** -0.5
+        gone = {4: 2, 0: 1}.get(r, -1)
+        s = s.masked_fill(((j[None] > pos[:, None]) | (j[None] // 16 == gone))[:, None], -math.inf)
+        want = torch.einsum("thl,lhd->thd", s.softmax(-1), v)
+        assert (got[a:a + l].view_as(want).double() - want).norm() < 1e-6 * want.norm(), r
+        a += l
