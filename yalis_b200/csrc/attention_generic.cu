@@ -207,9 +207,12 @@ __global__ void paged_attention_generic_kernel(const GenericParams<T> p) {
 // A block takes the neighbouring tokens of one request whose positions lie in one aligned group of kPairs / HP: the first
 // of them finds the others, the blocks of the others end at once.
 // What bounds it: reads of shared memory (16 bytes of a pair's query are two passes beside four products a lane) and, for few
-// blocks, the chain of a tile: copy, scores, maximum, exponential, values.  Measured (us, before -> now), 32 heads on 8 of 64 / 128:
-// one token behind 1,000 186 -> 23 / 253 -> 25, 64 such 679 -> 51 / 1,011 -> 144, a prompt of 250 247 -> 48 / 269 -> 61, of 1,024
-// 3,699 -> 417 / 4,096 -> 554, of 16 5.8 -> 4.5 / 6.8 -> 8.3.
+// blocks, the chain of a tile: copy, scores, maximum, exponential, values (as many as registers leave room for are asked for ahead; behind a
+// context's end none is waited for).  Measured (us, general form -> now; with half as many registers and every value of the last tile waited for), 32
+// heads on 8 of 64 / 128: one token behind 200 40 -> 5.8 (7.0) / 53 -> 7.1 (7.9), 16 tokens behind 8,000 2,132 -> 262 (259) / 2,400 -> 291 (505), 64
+// tokens of their own behind 1,000 679 -> 50 / 1,011 -> 140 (143), a prompt of 250 247 -> 42 (48) / 269 -> 60, of 1,024 3,699 -> 352 (418) / 4,096 -> 552,
+// of 16 6.0 -> 4.1 (4.5) / 6.9 -> 5.4 (8.3), of 8 3.8 -> 3.6 (4.2) / 4.4 -> 4.2 (4.9), of 4 3.0 -> 3.5 (4.0) / 3.3 -> 4.1 (4.5): contexts of a few
+// keys are the general form's, but which form a token takes must not depend on what runs beside it.
 constexpr int kTile = 32;
 
 __device__ __forceinline__ void copy16(float* to, const float* from, bool there) {      // zeros where there is nothing
@@ -228,8 +231,11 @@ constexpr size_t tiled_smem() {      // queries; per warp: a tile of keys, the w
 }
 
 // D: the head size; HP: heads of a key/value head that a block takes; QT: queries.
+// Blocks an SM for a query a block: what shared memory holds (three for a size of 128) or what leaves registers for the values ahead.  Several
+// queries: left to the compiler (0; three or two blocks: prompts of 250 to 1,024 3 to 10 % slower).
+constexpr int tiled_blocks(int d, int hp, int qt) { return qt > 1 ? 0 : d == 128 ? 3 : hp == 1 ? 6 : hp == 2 ? 5 : 4; }
 template <int D, int HP, int QT>
-__global__ void __launch_bounds__(kWarps * 32) paged_attention_tiled_kernel(const GenericParams<float> p, int n_tokens) {
+__global__ void __launch_bounds__(kWarps * 32, tiled_blocks(D, HP, QT)) paged_attention_tiled_kernel(const GenericParams<float> p, int n_tokens) {
   constexpr int P = HP * QT, LK = D + 4, V = D / 32;           // rows of keys padded: lanes read 16 bytes of rows of their own
   extern __shared__ __align__(16) float smem[];
   pdl_launch_dependents();
@@ -321,12 +327,13 @@ __global__ void __launch_bounds__(kWarps * 32) paged_attention_tiled_kernel(cons
     }
     __syncwarp();
     if (next <= last) fetch_keys(row);
-    uint32_t seen[QT];
+    uint32_t seen[QT], any = 0;
     bool whole = true;
 #pragma unroll
     for (int i = 0; i < QT; ++i) {
       seen[i] = __ballot_sync(0xffffffffu, i < nq && here >= 0 && j <= pos0 + i && j >= first(pos0 + i));
       whole = whole && seen[i] == 0xffffffffu;
+      any |= seen[i];
     }
 #pragma unroll
     for (int a = 0; a < P; ++a) {
@@ -345,10 +352,8 @@ __global__ void __launch_bounds__(kWarps * 32) paged_attention_tiled_kernel(cons
       for (int u = 0; u < V; ++u) acc[a][u] *= corr;
     }
     __syncwarp();
-#pragma unroll
-    for (int r = 0; r < kTile; r += 4) {
-      float (&now)[4][V] = v[(r / 4) & 1];
-      if (r + 4 < kTile) fetch_values(here, r + 4, v[(r / 4 + 1) & 1]);
+    auto add_values = [&](int r, float (&now)[4][V], float (&next)[4][V]) {
+      if (r + 4 < kTile) fetch_values(here, r + 4, next);
 #pragma unroll
       for (int i = 0; i < QT; ++i) {
         float mine[4][V];
@@ -369,6 +374,16 @@ __global__ void __launch_bounds__(kWarps * 32) paged_attention_tiled_kernel(cons
           for (int e = 0; e < V; ++e)
             acc[a][e] = __fmaf_rn(w.w, mine[3][e], __fmaf_rn(w.z, mine[2][e], __fmaf_rn(w.y, mine[1][e], __fmaf_rn(w.x, mine[0][e], acc[a][e]))));
         }
+      }
+    };
+    if (QT > 1 || HP == 4 || any >> (kTile - 4) != 0) {
+#pragma unroll
+      for (int r = 0; r < kTile; r += 4) add_values(r, v[(r / 4) & 1], v[(r / 4 + 1) & 1]);
+    } else {                                                   // a context's end: the values behind it are not waited for
+#pragma unroll 1
+      for (int r = 0; r < kTile && any >> r != 0; r += 8) {
+        add_values(r, v[0], v[1]);
+        add_values(r + 4, v[1], v[0]);
       }
     }
     __syncwarp();
@@ -423,7 +438,8 @@ int launch_tiled(const GenericParams<float>& p, int n_tokens, cudaStream_t strea
     return YALIS_ERR_LAUNCH;
   return yalis_launch(paged_attention_tiled_kernel<D, HP, QT>, dim3(n_tokens, p.nh / HP), dim3(kWarps * 32), smem, stream, p, n_tokens);
 }
-// Which form (the bits are the same): as many heads a block, up to four, as leave two blocks an SM, since a block's walk over
+// Which form (the bits are the same): as many heads a block, up to four, as leave two blocks an SM (for a size of 128, of whose blocks an SM has three
+// places, one and a half: 16 tokens of 32 heads are then one round of blocks, 8.3 -> 5.4 us), since a block's walk over
 // the keys is what a step of few tokens waits for (a token behind 8,000, 32 heads of 128 on 8: 180 us with one head a block, 282 with
 // four); several queries a block where one makes more than eight blocks an SM (64 tokens behind 1,000 with 16 heads of 64 on
 // 16, all of requests of their own: 346 us with eight queries a block).
@@ -431,7 +447,8 @@ template <int D>
 int launch_tiled_heads(const GenericParams<float>& p, int n_tokens, cudaStream_t stream) {
   const int per = p.nh / p.g;
   const long long pairs = (long long)n_tokens * p.nh, sms = yalis_sm_count();
-  const int hp = per % 4 == 0 && pairs / 4 >= 2 * sms ? 4 : per % 2 == 0 && pairs / 2 >= 2 * sms ? 2 : 1;
+  const long long many = D == 128 ? 3 * sms / 2 : 2 * sms;
+  const int hp = per % 4 == 0 && pairs / 4 > many ? 4 : per % 2 == 0 && pairs / 2 > many ? 2 : 1;
   const bool single = pairs / hp <= 8 * sms;
   if (hp == 4) return single ? launch_tiled<D, 4, 1>(p, n_tokens, stream) : launch_tiled<D, 4, 2>(p, n_tokens, stream);
   if (hp == 2) return single ? launch_tiled<D, 2, 1>(p, n_tokens, stream) : launch_tiled<D, 2, 4>(p, n_tokens, stream);
