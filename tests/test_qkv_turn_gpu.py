@@ -62,3 +62,25 @@ def test_heads_turn(dim, vdim, rot, interleaved, normed, dtypes):
         assert bool(((y - x).abs() <= slack).all()), (i, ((y - x).abs() / slack).max().item())
     few = run(5)
     assert all(torch.equal(a[:5], b) for a, b in zip(got, few))
+
+
+@pytest.mark.parametrize("dim", [64, 128, 256])
+@pytest.mark.parametrize("interleaved", [False, True])
+@pytest.mark.parametrize("dtypes", [(torch.bfloat16, torch.bfloat16), (torch.bfloat16, torch.float32), (torch.float32, torch.float32)])
+def test_steps_of_more_blocks_than_places_have_the_same_bits(dim, interleaved, dtypes):
+    """The form in fewer registers, for many blocks, beside the other one."""
+    from yalis_b200.ops.elementwise import qkv_prepare
+    nq, nk, n, few = 7, 2, 2300, 310
+    g = torch.Generator().manual_seed(dim)
+    src = torch.randn(n, (nq + 2 * nk) * dim, generator=g).to(dtypes[0]).cuda()
+    norm, freq = torch.rand(dim, generator=g).cuda(), torch.rand(dim // 2, generator=g).cuda()
+    positions, req = torch.arange(n, dtype=torch.int32).cuda(), torch.zeros(n, dtype=torch.int32).cuda()
+
+    def run(a, b):
+        return qkv_prepare(src[a:b], (0, nq * dim, (nq + nk) * dim), nq, nk, dim, dim, positions[a:b].contiguous(), req[a:b].contiguous(),
+                           out_dtype=dtypes[1], q_norm=norm, k_norm=norm, norm_eps=1e-6, inv_freq=freq, interleaved=interleaved)
+
+    whole = run(0, n)
+    for a in (0, 1100, n - few):
+        for x, y in zip(run(a, a + few), whole):
+            assert torch.equal(x, y[a:a + few])

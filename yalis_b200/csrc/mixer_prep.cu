@@ -404,10 +404,12 @@ int launch_qkv_plain(const PrepParams& p, int n_tokens, cudaStream_t stream) {
 // Measured (16 + 2 x 8 heads of 128 that turn whole, norms, pages; us at 64 / 512 / 2,048 tokens): through shared memory
 // 3.8 / 10.9 / 26.6, here 3.5 / 7.8 / 17.7; 32 + 2 x 8 heads of 64: 4.4 / 15.5 / 38.1 -> 3.7 / 4.6 / 13.8; 16 + 2 x 8 of 256:
 // 4.4 / 13.7 / 37.6 -> 4.1 / 10.3 / 30.8.  Fetching the rows before the request is known costs registers and gains nothing.
-// Four blocks an SM (64 registers): 2,048 tokens of 32 heads of 128, interleaved pairs, as a prompt's layer meets it, 22.0 -> 18.7 us (66 registers, three
-// blocks); five spill.
-template <typename T, typename TO, int L, bool INTER>
-__global__ void __launch_bounds__(256, 4) qkv_turn_kernel(const PrepParams p) {
+// BLOCKS 4: four blocks of 256 threads on an SM, in 64 registers; 0: as many registers as it takes (66 to 77, three such blocks).  Four where the
+// step's blocks have no room in one round otherwise (us, 0 -> 4: 2,048 tokens of 32 + 2 x 8 heads of 128, interleaved pairs, 21.2 -> 18.4, of 16 + 2 x 8 of
+// 256 23.4 -> 21.9, 512 tokens of 16 + 2 x 8 of 128 7.1 -> 4.8); the others would have the registers' shortage alone, heads of 256 (8 to 16 bytes
+// spilled) above all (64 tokens of 16 + 2 x 8 of 256 3.8 -> 4.2, 512 of 8 + 2 x 2 4.3 -> 4.8, of 32 + 2 x 8 of 64 4.4 -> 4.6).  Five blocks spill more.
+template <typename T, typename TO, int L, bool INTER, int BLOCKS>
+__global__ void __launch_bounds__(256, BLOCKS) qkv_turn_kernel(const PrepParams p) {
   extern __shared__ __align__(16) float table_s[];  // cosines, then sines
   pdl_launch_dependents();
   pdl_wait();
@@ -537,20 +539,22 @@ int launch_qkv_turn(const PrepParams& p, int n_tokens, cudaStream_t stream) {
   // steps of many tokens: blocks that hold a token's heads in one pass, as far as 256 threads do; few tokens: four warps.
   // Up to 64 tokens a group takes one head, so that none waits for a second (8 tokens of 16 + 2 x 8 heads of 128: 3.6 us with
   // two, 3.15 with one; the general form took 3.3; 256 tokens of 16 + 2 x 8 heads of 256: 7.5 and 8.2).
-  auto go = [&](auto kernel, int lanes) {
+  auto go = [&](auto lean, auto full, int lanes) {
     const int needed = ((heads + 1) / 2 * lanes + 31) / 32 * 32;
     const bool many = n_tokens >= 2 * yalis_sm_count();
     const int threads = many ? (needed < 256 ? needed : 256) : 128, pass = (n_tokens > 64 ? 2 : 1) * (threads / lanes);
-    return yalis_launch(kernel, dim3(n_tokens, many ? 1 : (heads + pass - 1) / pass), dim3(threads), smem, stream, p);
+    const dim3 grid(n_tokens, many ? 1 : (heads + pass - 1) / pass);
+    const int places = yalis_sm_count() * (65536 / ((lanes == 32 ? 80 : 72) * threads));      // of the form with all its registers
+    return yalis_launch((long long)grid.x * grid.y > places ? lean : full, grid, dim3(threads), smem, stream, p);
   };
   if (p.rot_interleaved) {
-    if (widest <= 64) return go(qkv_turn_kernel<T, TO, 8, true>, 8);
-    if (widest <= 128) return go(qkv_turn_kernel<T, TO, 16, true>, 16);
-    return go(qkv_turn_kernel<T, TO, 32, true>, 32);
+    if (widest <= 64) return go(qkv_turn_kernel<T, TO, 8, true, 4>, qkv_turn_kernel<T, TO, 8, true, 0>, 8);
+    if (widest <= 128) return go(qkv_turn_kernel<T, TO, 16, true, 4>, qkv_turn_kernel<T, TO, 16, true, 0>, 16);
+    return go(qkv_turn_kernel<T, TO, 32, true, 4>, qkv_turn_kernel<T, TO, 32, true, 0>, 32);
   }
-  if (widest <= 64) return go(qkv_turn_kernel<T, TO, 8, false>, 8);
-  if (widest <= 128) return go(qkv_turn_kernel<T, TO, 16, false>, 16);
-  return go(qkv_turn_kernel<T, TO, 32, false>, 32);
+  if (widest <= 64) return go(qkv_turn_kernel<T, TO, 8, false, 4>, qkv_turn_kernel<T, TO, 8, false, 0>, 8);
+  if (widest <= 128) return go(qkv_turn_kernel<T, TO, 16, false, 4>, qkv_turn_kernel<T, TO, 16, false, 0>, 16);
+  return go(qkv_turn_kernel<T, TO, 32, false, 4>, qkv_turn_kernel<T, TO, 32, false, 0>, 32);
 }
 
 template <typename T, typename TO>
