@@ -81,3 +81,20 @@ def test_what_another_kernel_writes_is_not_read_through_restrict(path):
     assert "__ldg" not in text
     for kind, name in re.findall(r"([\w ]+)\*\s*__restrict__\s+(\w+)", text):
         assert "const " in kind and name in CONSTANTS, (kind, name)
+
+
+def test_every_bit_of_the_error_word_says_which_kernels_raise_it():
+    """The bits that a source raises have a text, and a source that raises a wait's bit is of the kind that the text names."""
+    import pathlib
+    import re
+
+    from yalis_b200.ops import _lib
+    root = pathlib.Path(_lib.__file__).parent.parent / "csrc"
+    bits = {n: int(v) for n, v in re.findall(r"YALIS_FLAG_(\w+) = (\d+)", (root / "common.cuh").read_text())}
+    assert bits == {n[5:]: v for n, v in vars(_lib).items() if re.fullmatch(r"FLAG_[A-Z_]+", n)}
+    kinds = {"WAIT_ATTENTION": "attention", "WAIT_PRODUCT": "gemm", "WAIT_RECURRENCE": "recurrent"}
+    for source in root.glob("*.cu"):
+        for name in set(re.findall(r"YALIS_FLAG_(WAIT_\w+)", source.read_text())):
+            assert kinds[name] in source.name, (source.name, name)
+    texts = [_lib.describe_error_word(v) for v in bits.values()]
+    assert len(set(texts)) == len(bits) and not any("unknown" in t for t in texts)

@@ -26,6 +26,7 @@ enum : int {
   YALIS_FLAG_BAD_PAGE = 2,        // a block-table entry outside the pool (the token was skipped)
   YALIS_FLAG_WAIT_ATTENTION = 4,  // a bounded wait of an attention kernel ran out (its block gave up)
   YALIS_FLAG_WAIT_PRODUCT = 8,    // a bounded wait of the weight-streaming product ran out
+  YALIS_FLAG_WAIT_RECURRENCE = 16, // a bounded wait of a recurrence by chunks ran out (its block gave up)
 };
 
 inline int yalis_launch_status() {

@@ -454,7 +454,7 @@ __global__ void __launch_bounds__(kAll, STAGES == 3 ? 2 : 1) chunk_walk_kernel(c
     // (all copies end before the block does, also those that a wait gave up on)
     for (int c = max(0, chunks - STAGES); c < chunks; ++c) copies_there(&there[c % STAGES], (c / STAGES) & 1);
     __syncwarp();
-    if (lane == 0 && *lost) atomicOr(p.error, YALIS_FLAG_WAIT_PRODUCT);
+    if (lane == 0 && *lost) atomicOr(p.error, YALIS_FLAG_WAIT_RECURRENCE);
     return;
   }
 

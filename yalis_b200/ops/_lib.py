@@ -71,12 +71,13 @@ def stream() -> ctypes.c_void_p:
 # ---- the device error word -----------------------------------------------------------------------
 # One int32 per device that every kernel of the library may raise bits in (csrc/common.cuh) instead of trapping;
 # the host reads it where it synchronises anyway.
-FLAG_BAD_ID, FLAG_BAD_PAGE, FLAG_WAIT_ATTENTION, FLAG_WAIT_PRODUCT = 1, 2, 4, 8
+FLAG_BAD_ID, FLAG_BAD_PAGE, FLAG_WAIT_ATTENTION, FLAG_WAIT_PRODUCT, FLAG_WAIT_RECURRENCE = 1, 2, 4, 8, 16
 _FLAG_TEXT = {
     FLAG_BAD_ID: "a token id outside the vocabulary",
     FLAG_BAD_PAGE: "a block-table entry outside the page pool (a visible token without a page)",
     FLAG_WAIT_ATTENTION: "a bounded wait inside an attention kernel ran out (its block gave up)",
     FLAG_WAIT_PRODUCT: "a bounded wait inside the weight-streaming product ran out (its block gave up)",
+    FLAG_WAIT_RECURRENCE: "a bounded wait inside a recurrence by chunks ran out (its block gave up)",
 }
 _error_words = {}
 
