@@ -276,3 +276,34 @@ def test_a_step_in_several_launches_has_the_same_bits(rule, room, monkeypatch):
     monkeypatch.setattr(recurrent, "CHUNK_BYTES", (room - 1) * kv_heads * 2 * 3 * 16 * 128 * 2)
     few = run(rule, lay, kv_heads, data, few_rows, lens, slots, True)
     assert torch.equal(few, whole) and torch.equal(few_rows, rows)
+
+
+@pytest.mark.parametrize("kind,params", [
+    ("retention", {"hidden_size": 64, "heads": 2, "dim": 128, "vdim": 128, "decay": [0.9, 0.99], "rotary": None, "eps": 1e-5}),
+    ("gated_delta", {"hidden_size": 64, "heads": 2, "kv_heads": 1, "dim": 128, "vdim": 128, "conv": 4, "eps": 1e-5, "decay": "head"}),
+    ("state_space", {"hidden_size": 64, "heads": 4, "vdim": 64, "state": 128, "groups": 1, "conv": 4, "norm_groups": 1, "eps": 1e-5})])
+def test_a_part_can_be_told_to_walk(kind, params):
+    """Then a position's result has the same bits however a request is cut; the chunks agree with it to a rounding."""
+    from ctx_helper import make_context
+    from yalis_b200.config.spec import PartSpec
+    from yalis_b200.parts.base import SlotStateCache, make_part
+    n, results = 500, {}
+    for by_chunks in (False, True):
+        part = make_part("mixer", PartSpec(kind, {**params, "by_chunks": by_chunks}))
+        g = torch.Generator().manual_seed(2)
+        part.load({name: (0.3 * torch.randn(ps.shape, generator=g)).to(DEV, torch.float32 if ps.keep_float32 else torch.bfloat16)
+                   for name, ps in part.param_specs().items()})
+        z = torch.randn(n, part.in_weight().shape[0], generator=g).to(DEV, torch.bfloat16)
+        for cut in ([n], [300, 200], [1, 299, 2, 198]):
+            cache = SlotStateCache(torch.zeros(1, part.layout.total, device=DEV))
+            y, a = torch.empty(n, part.hidden_width, dtype=torch.bfloat16, device=DEV), 0
+            for c in cut:
+                ctx, _ = make_context([c], [a], 16)
+                part.mix(z[a:a + c], ctx, cache, y[a:a + c])
+                a += c
+            results.setdefault(by_chunks, []).append((y, cache.state))
+    for y, state in results[False]:
+        assert torch.equal(y, results[False][0][0]) and torch.equal(state, results[False][0][1])
+    assert not torch.equal(results[True][0][1], results[False][0][1])
+    for (y, state), (want, last) in zip(results[True], results[False]):
+        assert float((y.double() - want.double()).norm()) < 1e-3 * float(want.double().norm()) and float((state - last).norm()) < 1e-6 * float(last.norm())

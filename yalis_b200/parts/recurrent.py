@@ -18,7 +18,10 @@
 All of them are ``Projected``: an arrangement may run their input and output products together with those of its
 other parts.  What the recurrences keep (state matrices in float32, the convolution's last inputs) is one row
 of slot memory per request; the kernels walk a request's tokens in order, so the result at a position does not
-depend on how the request was cut into steps.
+depend on how the request was cut into steps.  But for one case: bfloat16 models take long portions (``CHUNKS_FROM``) of
+heads of 128 rows with one decay by chunks of sixteen tokens from the portion's start on (``retention``, ``gated_delta``
+with a decay per head, ``state_space``), so that float32 roundings depend on where a long portion began; a part with the parameter
+``by_chunks`` False walks them, too.
 """
 
 from __future__ import annotations
@@ -51,6 +54,7 @@ class _ProjectedMixer(Mixer, Projected):
         self.w_in: Optional[torch.Tensor] = None
         self.w_out: Optional[torch.Tensor] = None
         self.out_scale = float(spec.params.get("out_scale", 1.0))
+        self.by_chunks = bool(spec.params.get("by_chunks", True))
 
     def in_weight(self) -> torch.Tensor:
         return self.w_in
@@ -129,7 +133,7 @@ class Retention(_ProjectedMixer):
         else:
             q, k, v = self._rotated(z, ctx)
         o = rec_ops.state_scan(q, k, v, cache.state, self.layout, ctx.q_start, ctx.slots, kv_heads=self.h, decay=self.decay,
-                               max_q_len=ctx.host.max_q_len, chunks=z.dtype == torch.bfloat16)
+                               max_q_len=ctx.host.max_q_len, chunks=self.by_chunks and z.dtype == torch.bfloat16)
         if self.norm_kind == "all":
             rec_ops.gate_norm(o, gate, 1, self.norm_w, self.eps, ctx.req_of_token, y, out_scale=self.out_scale,
                               gate_kind=self.gate_kind, after=True)
@@ -227,7 +231,7 @@ class GatedDelta(_ProjectedMixer):
             single_tokens=ctx.host.max_q_len == 1)
         o = rec_ops.state_scan(conv[:, :gd], conv[:, gd:2 * gd], conv[:, 2 * gd:], cache.state, self.layout, ctx.q_start,
                                ctx.slots, kv_heads=self.g, decay=decay, beta=beta, max_q_len=ctx.host.max_q_len,
-                               chunks=z.dtype == torch.bfloat16)
+                               chunks=self.by_chunks and z.dtype == torch.bfloat16)
         if self.gate_kind == "silu":
             gate, kind = self._block(z, "g"), rec_ops.GATE_SILU
         else:
@@ -358,7 +362,7 @@ class StateSpace(_ProjectedMixer):
         b, c = self.inner, self.inner + self.g * self.n
         o = rec_ops.state_scan(conv[:, c:], conv[:, b:c], conv[:, :b], cache.state, self.layout, ctx.q_start, ctx.slots,
                                kv_heads=self.g, decay=decay, beta=step, selective=True, skip=self.skip,
-                               max_q_len=ctx.host.max_q_len, chunks=z.dtype == torch.bfloat16)
+                               max_q_len=ctx.host.max_q_len, chunks=self.by_chunks and z.dtype == torch.bfloat16)
         rec_ops.gate_norm(o, blk("z"), self.parts, self.norm_w, self.eps, ctx.req_of_token, y, out_scale=self.out_scale)
 
 
