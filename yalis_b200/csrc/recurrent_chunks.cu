@@ -177,13 +177,14 @@ __global__ void __launch_bounds__(kWarps * 32) chunk_prepare_kernel(const ChunkP
   }
   __syncthreads();
   if (RULE == 1 || warp < 2) {
-    // q k by two warps, k k by two, eight of the second operand's tokens each: per 16 values the products of the first parts and the
-    // five small ones apart, and all sums in 64 bits (a decay of a half leaves of a read-out little but these products)
+    // q k by two warps, k k by two, eight of the second operand's tokens each: the products of the first parts, 16 values at a time, are added in
+    // 64 bits (a decay of a half leaves of a read-out little but these products), the five small ones in one chain on the tensor cores
     const bool qk_here = warp < 2;
     const int s0 = (warp & 1) * 8;
     const uint32_t as = smem_u32(ps_s) + (qk_here ? 3 * kPart * 2 : 0) + (lane & 15) * (kD * 2);
     const uint32_t bs = smem_u32(ps_s) + (s0 + (lane & 7)) * (kD * 2);
     double sum[4] = {0.0, 0.0, 0.0, 0.0};
+    float small[2][4];
 #pragma unroll
     for (int j = 0; j < kD / 32; ++j) {                            // 32 values
       uint32_t fa[3][2][4], fb[3][4];
@@ -193,25 +194,25 @@ __global__ void __launch_bounds__(kWarps * 32) chunk_prepare_kernel(const ChunkP
 #pragma unroll
         for (int n = 0; n < 2; ++n) ldmatrix4(fa[i][n], as + i * kPart * 2 + (((4 * j + 2 * n + (lane >> 4)) ^ (lane & 7)) << 4));
       }
-      float large[2][4], small[2][4];
+      float large[2][4];
 #pragma unroll
       for (int o = 0; o < 6; ++o)
 #pragma unroll
         for (int n = 0; n < 2; ++n) {
           const uint32_t(&b)[4] = fb[second_part(o)];
-          if (o == 0) mma0(small[n], fa[first_part(o)][n], b[2 * n], b[2 * n + 1]);
+          if (o == 0 && j == 0) mma0(small[n], fa[first_part(o)][n], b[2 * n], b[2 * n + 1]);
           else if (o < 5) mma(small[n], fa[first_part(o)][n], b[2 * n], b[2 * n + 1]);
           else mma0(large[n], fa[first_part(o)][n], b[2 * n], b[2 * n + 1]);
         }
 #pragma unroll
       for (int n = 0; n < 2; ++n)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) sum[e] += (double)small[n][e] + (double)large[n][e];
+        for (int e = 0; e < 4; ++e) sum[e] += (double)large[n][e];
     }
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
       const int t = (lane >> 2) + 8 * (e >> 1), s = s0 + 2 * (lane & 3) + (e & 1);
-      (qk_here ? qk : kk)[t * kC + s] = (float)sum[e];
+      (qk_here ? qk : kk)[t * kC + s] = (float)(sum[e] + (double)(small[0][e] + small[1][e]));
     }
   }
   __syncthreads();
