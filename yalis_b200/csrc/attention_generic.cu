@@ -204,7 +204,7 @@ __global__ void paged_attention_generic_kernel(const GenericParams<T> p) {
 // share out the head's sizes for the values.  Tiles lie at multiples of 32 positions and warp w walks those whose number is w
 // modulo four, in ascending order; what a query does not see counts as nothing.  So here, too, the order of every sum is fixed for a
 // given position and head.  The keys of the next tile and the values of this one are on their way while a warp computes.
-// A block takes the neighbouring tokens of one request whose positions lie in one aligned group of kPairs / HP: the first
+// A block takes the neighbouring tokens of one request whose positions lie in one aligned group of QT (one, two or four): the first
 // of them finds the others, the blocks of the others end at once.
 // What bounds it: reads of shared memory (16 bytes of a pair's query are two passes beside four products a lane) and, for few
 // blocks, the chain of a tile: copy, scores, maximum, exponential, values (as many as registers leave room for are asked for ahead; behind a

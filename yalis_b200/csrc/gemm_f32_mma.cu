@@ -260,8 +260,8 @@ int launch_parts(const F32Params& p, cudaStream_t stream) {
 // Measured (us, FMAs on the CUDA cores as it was -> now), columns x K:
 //   1 token     3,072 x 2,048  39 -> 26    16,384 x 2,048  116 -> 49    2,048 x 8,192  171 -> 105
 //   64 tokens   3,072 x 2,048  62 -> 47    16,384 x 2,048  141 -> 91    2,048 x 8,192  238 -> 172
-//   250 tokens  3,072 x 2,048  142 -> 91   16,384 x 2,048  486 -> 312   2,048 x 8,192  461 -> 198    2,048 x 2,048  119 -> 51
-//   1,024       3,072 x 2,048  416 -> 266  16,384 x 2,048  1,893 -> 1,223
+//   250 tokens  3,072 x 2,048  142 -> 91   16,384 x 2,048  486 -> 315   2,048 x 8,192  461 -> 198    2,048 x 2,048  119 -> 52
+//   1,024       3,072 x 2,048  416 -> 269  16,384 x 2,048  1,893 -> 1,238
 // (1,024 tokens in tiles of 128 x 128: 1,166 for 16,384 columns, 333 for 3,072: not taken.)
 template <typename TX, bool VECX>
 int launch_sizes(const F32Params& p, cudaStream_t stream) {

@@ -8,8 +8,8 @@
 //   o_t = G_t S^T q_t + sum_(s<=t) P_ts (q_t . k_s) u_s,     S <- G_16 S + sum_s P_16,s k_s u_s^T
 //
 // (the plain rule: u = v; the selective form: u = beta v, and skip v beside o).  What does not depend on the state is computed
-// for all chunks side by side by the first kernel: k and q in three bfloat16 parts each (nothing of a float32 value is lost; see
-// gemm_f32_mma.cu), T, P (q . k) and the decays, whose products are taken in 64 bits.  The second walks the chunks: a block has 16
+// for all chunks side by side by the first kernel: k and q in three bfloat16 parts each (as in gemm_f32_mma.cu, but unscaled:
+// see below), T, P (q . k) and the decays, whose products are taken in 64 bits.  The second walks the chunks: a block has 16
 // columns of a head's state, a warp 32 of its rows, as accumulators of the tensor cores in float32 (transposed, so that
 // they are also the operand of the products with k and q).  All sums are float32: products of parts are summed on the tensor cores
 // over 16 values at most, small ones first, and added in registers; dot products of a chunk's tokens are added in 64 bits; the state is
@@ -29,10 +29,10 @@
 // need is left to other warps: waiting for copies, by the delta rule the products with q.  For several requests the copies of k and q,
 // which the blocks of a head's columns all ask for.
 // Measured (us, walk token by token -> both kernels; before copies ran up to four chunks ahead and the chain was shortened), 16
-// heads of 128 x 128 (delta rule: 8 key heads; selective: 32 of 128 x 64, one), L2 flushed: delta rule 1 x 2,048 387 -> 168 (196),
-// 1 x 128 30.7 -> 30.7 (28), 4 x 901 363 -> 254 (259), 32 x 128 351 -> 275 (282); plain 1 x 2,048 257 -> 120 (155), 4 x 901 223 -> 185 (208),
-// 8 x 512 219 -> 196 (237); selective 1 x 2,048 260 -> 110 (144), 4 x 901 236 -> 163 (187), 16 x 256 219 -> 169.  What keeps the errors where
-// the walk has them (the last products of a chunk twice, the own token last, 64-bit sums) is 10 us of each rule's 1 x 2,048.
+// heads of 128 x 128 (delta rule: 8 key heads; selective: 32 of 128 x 64, one), L2 flushed: delta rule 1 x 2,048 387 -> 169 (196),
+// 1 x 128 30.7 -> 29.7 (28), 4 x 901 363 -> 253 (259), 32 x 128 351 -> 275 (282); plain 1 x 2,048 256 -> 116 (155), 4 x 901 223 -> 185 (208),
+// 8 x 512 219 -> 192 (237); selective 1 x 2,048 260 -> 110 (144), 4 x 901 236 -> 163 (187), 16 x 256 219 -> 169.  What keeps the errors where
+// the walk has them (the last products of a chunk twice, the own token last, 64-bit sums) is 6 to 12 us of 1 x 2,048.
 // Not taken: eight row warps and 32 columns a block (for several requests no gain: 282 and 218 for 4 x 901), two chunks in
 // shared memory, k and q copied in pieces whose order differs from block to block, the products with q by the reading warps in the
 // other rules too (1 x 2,048 plain 175, 4 x 901 214: those warps become the chain).

@@ -119,10 +119,10 @@ def short_conv_silu(x: torch.Tensor, weight: torch.Tensor, slot_rows: torch.Tens
 
 
 # Portions of so many tokens, by rule, may go by chunks of sixteen (a portion's length alone decides, so that a request's result
-# does not depend on what runs beside it).  Where the lines lie (us, walk -> chunks): delta rule 1 x 128 30.7 -> 30.7, 32 x 128
-# 351 -> 275; plain 16 x 192 157 -> 163, 1 x 256 38.9 -> 29.7, 32 x 256 386 -> 376; selective with one key head (few blocks of the
-# first kernel) 1 x 192 31.7 -> 33.8, 16 x 192 167 -> 138, with eight 1 x 192 30.7 -> 25.6.
-CHUNKS_FROM = {0: 256, 1: 128, 3: 208}
+# does not depend on what runs beside it).  Where the lines lie (us, walk -> chunks): delta rule 1 x 128 30.7 -> 29.7, 32 x 128
+# 351 -> 275; plain 32 x 128 200 -> 212, 1 x 192 30.7 -> 25.6, 16 x 192 156 -> 157; selective with one key head (few blocks of the
+# first kernel) 1 x 192 30.7 -> 33.8, 1 x 256 38.9 -> 35.9, 16 x 192 166 -> 138, with eight 1 x 192 30.7 -> 25.6.
+CHUNKS_FROM = {0: 192, 1: 128, 3: 208}
 CHUNK = 16
 # The most that the parts of k and q of one launch take (24 KB a chunk and key head): longer steps are taken in several launches, to the same
 # bits.  A step of 2,048 tokens with 16 key heads has 51 MB, one of 32,768 would have 806.  (32 x 256 tokens by the plain rule in
