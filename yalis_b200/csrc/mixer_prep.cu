@@ -627,13 +627,34 @@ __global__ void activation_bf16x8_kernel(const __nv_bfloat16* x, int x_stride, _
 // Four elements a thread with float32 results (bfloat16 rows on 8-byte boundaries, float32 rows on 16-byte ones).  Its
 // reader may be a kernel of few, long blocks (a recurrence over the rows it makes): those are let in only once this one
 // has begun, so that they do not crowd onto the SMs that come free first.
-// A block has a row's next 256 x kActQuads groups of four; a thread asks for all of its own before it needs the first.
-// 2,926 rows of bfloat16 values, silu: 27.9 us with a 64-bit division for the row of every group, 20.2 here; the rest is expf and a division a
-// value.
+template <typename T>
+__global__ void activation_f32x4_kernel(const T* x, int x_stride, float* y, int y_stride, int rows,
+                                        int cols, int act, const float* __restrict__ bias) {
+  pdl_wait();
+  pdl_launch_dependents();
+  const int quads = cols >> 2;
+  const size_t total = (size_t)rows * quads;
+  for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (size_t)gridDim.x * blockDim.x) {
+    const size_t r = e / quads;
+    const int c = (int)(e - r * quads) << 2;
+    float4 z = load4_f32(x + r * x_stride + c);
+    if (bias) {
+      const float4 b = load4_f32(bias + c);
+      z.x += b.x; z.y += b.y; z.z += b.z; z.w += b.w;
+    }
+    store4(y + r * y_stride + c, make_float4(act_value(z.x, act), act_value(z.y, act), act_value(z.z, act), act_value(z.w, act)));
+  }
+}
+
+// The same for many wide rows, without a 64-bit division for the row of every group: a block has a row's next 256 x kActQuads groups of
+// four; a thread asks for all of its own before it needs the first.
+// Measured (us, above -> here, silu of bfloat16 values): 2,926 x 6,144 27.3 -> 19.5, x 1,024 5.8 -> 5.4, 512 x 6,144 6.0 -> 5.2; the rest is expf and
+// a division a value.  Narrow rows leave the block's threads idle and few rows the SMs: 16,384 x 256 7.2 -> 18.0, 2,926 x 512 3.7 -> 4.5,
+// 64 x 6,144 2.1 -> 2.5.  So for rows of 1,024 values and more, from 131,072 groups on (512 x 1,024: 2.3 either way).
 constexpr int kActQuads = 3;
 template <typename T>
-__global__ void __launch_bounds__(256) activation_f32x4_kernel(const T* x, int x_stride, float* y, int y_stride, int rows,
-                                        int cols, int act, const float* __restrict__ bias) {
+__global__ void __launch_bounds__(256) activation_f32_rows_kernel(const T* x, int x_stride, float* y, int y_stride, int cols, int act,
+                                                                   const float* __restrict__ bias) {
   pdl_wait();
   pdl_launch_dependents();
   const size_t r = blockIdx.x;
@@ -816,9 +837,14 @@ YALIS_API int yalis_activation(const void* x, int x_stride, void* y, int y_strid
   const size_t total = (size_t)rows * cols;
   const int blocks = (int)((total + 255) / 256 < 148 * 16 ? (total + 255) / 256 : 148 * 16);
   if (y_f32 && cols % 4 == 0 && x_stride % 4 == 0 && y_stride % 4 == 0 && !((uintptr_t)x & (dtype == YALIS_BF16 ? 7 : 15)) &&
-      !(((uintptr_t)y | (uintptr_t)bias) & 15) && cols <= 65535 * 1024) {
+      !(((uintptr_t)y | (uintptr_t)bias) & 15)) {
     const int groups = (cols / 4 + 256 * kActQuads - 1) / (256 * kActQuads);
-    YALIS_DISPATCH_DTYPE(dtype, T, return yalis_launch(activation_f32x4_kernel<T>, dim3(rows, groups), dim3(256), 0, stream, (const T*)x,
+    if (cols >= 1024 && total >= 4 * 131072 && groups <= 65535)
+      YALIS_DISPATCH_DTYPE(dtype, T, return yalis_launch(activation_f32_rows_kernel<T>, dim3(rows, groups), dim3(256), 0, stream, (const T*)x,
+                                                         x_stride, (float*)y, y_stride, cols, act, bias));
+    const size_t quads = (total / 4 + 255) / 256;
+    const dim3 grid((unsigned)(quads < 148 * 16 ? quads : 148 * 16));
+    YALIS_DISPATCH_DTYPE(dtype, T, return yalis_launch(activation_f32x4_kernel<T>, grid, dim3(256), 0, stream, (const T*)x,
                                                        x_stride, (float*)y, y_stride, rows, cols, act, bias));
   }
   if (y_f32 && dtype == YALIS_BF16)
