@@ -39,3 +39,11 @@ def test_same_bits_as_token_by_token(dtype, channels, kv_heads, taps, per_channe
             for u, v in zip(got, want):
                 assert torch.equal(u[i:i + 1], v), (r, t)
     assert torch.equal(rows, kept)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("channels,kv_heads,taps,per_channel,bias", [(4096, 16, 4, False, False), (3968, 3, 3, True, True), (4224, 0, 4, False, True),
+                                                                    (3968, 0, 2, False, False), (4096, 1, 1, True, False)])
+def test_as_many_values_as_take_tiles(dtype, channels, kv_heads, taps, per_channel, bias):
+    """Steps of 271 tokens with 2^20 values and more."""
+    test_same_bits_as_token_by_token(dtype, channels, kv_heads, taps, per_channel, bias)

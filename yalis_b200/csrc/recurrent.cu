@@ -195,7 +195,10 @@ __global__ void delta_prepare_kernel(const DeltaPrepareParams p) {
 // waits for a token's index, slot and row before it asks for the next one's, and reads its results back for their length.
 // Measured (us with the tails' kernel, L2 flushed, above -> here): 4,096 channels, 16 heads to unit length, a rate per head: 64 tokens
 // 13.3 -> 13.3, 256 17.4 -> 15.4, 512 23.6 -> 17.4, 1,024 31.7 -> 23.6, 2,048 46 -> 38; 6,144, 32 heads, a rate per channel: 128 tokens
-// 19.5 -> 17.4, 2,048 89 -> 77; 2,304, none: 128 tokens 13.3 -> 15.3, 256 13.3 -> 13.3, 512 17.4 -> 15.4, 3,000 38 -> 36: so from 256 tokens on.
+// 19.5 -> 17.4, 2,048 89 -> 77; 2,304, none: 128 tokens 13.3 -> 15.3, 256 13.3 -> 13.3, 512 17.4 -> 15.4, 3,000 38 -> 36.
+// Few values leave it with too few warps in flight, and portions of a few tokens wait for their slots' inputs at every tile (replayed, without a
+// flush: 512 channels with two heads, 512 tokens 7.2 -> 7.7, 128 channels 5.0 -> 5.8; 2,304 channels, 256 tokens 6.4 -> 6.8, 512 tokens 9.5 -> 7.6, but of
+// 128 requests 11.3 -> 13.0; 4,096 channels, 256 tokens 10.3 -> 8.1): so from 256 tokens and 2^20 values on, eight tokens a request on average.
 // Four tokens a warp 38, 83 and 38 for the longest, eight 46, 112 and 46: fewer warps.
 constexpr int kConvTile = 2, kConvTileFrom = 256;
 
@@ -904,7 +907,8 @@ YALIS_API int yalis_delta_prepare(const void* x, int dtype, int x_stride, const 
   const dim3 grid((n_tokens + p.tile - 1) / p.tile, (channels + p.piece - 1) / p.piece);
   if (grid.y > 65535) return YALIS_ERR_SHAPE;
   const int pieces = (channels / 128 + 7) / 8;
-  const bool by_tiles = !single_tokens && n_tokens >= kConvTileFrom && taps <= 4 && channels % 128 == 0 && (kv_heads == 0 || dim == 128) && pieces <= 65535;
+  const bool by_tiles = !single_tokens && n_tokens >= kConvTileFrom && n_tokens >= 8ll * n_requests && (long long)n_tokens * channels >= (1 << 20) &&
+                        taps <= 4 && channels % 128 == 0 && (kv_heads == 0 || dim == 128) && pieces <= 65535;
   YALIS_DISPATCH_DTYPE(dtype, T, {
     int st;
     if (by_tiles) st = yalis_launch(conv_tile_kernel<T>, dim3((n_tokens + kConvTile - 1) / kConvTile, pieces), dim3(256), 0, stream, p);
