@@ -426,15 +426,16 @@ int launch_route(const void* x, long x_stride, const float* w, int n_tokens, int
 
 // One block.  entries = n_tokens * top.  tiles: (expert, first slot) per row tile of `bm` slots, ended by n_tiles.
 // What bounds it: the latency of one block's steps.  The first kPlanKeep * 1,024 entries stay in registers with their place among
-// their expert's, which a warp takes for all its entries of an expert in one addition; the experts' first slots come from a scan.
-// 4,096 entries of 16 experts: 9.6 us behind the router with every entry read and added twice and a scan by one thread, 6.7 here.
+// their expert's, from one addition an entry; the experts' first slots come from a scan.
+// Measured (us, every entry read and added twice and a scan by one thread -> here, replayed): 4,096 entries of 16 experts 4.7 -> 4.1, 12,288 of 64
+// 14.4 -> 10.9, 16 of 16 2.9 -> 2.4, 64 of 256 16.4 -> 4.0; one addition for all of a warp's entries of an expert (by __match_any_sync): 5.7, 17.3, 2.5, 4.2.
 constexpr int kPlanKeep = 8;
 
 __global__ void __launch_bounds__(1024) expert_plan_kernel(const int32_t* ids, int entries, int E, int bm, int32_t* offsets,
                                    int32_t* perm, int32_t* inv, int32_t* tile_expert,
                                    int32_t* tile_slot, int32_t* n_tiles) {
   __shared__ int count[kMaxExperts], start[kMaxExperts + 1], tile0[kMaxExperts + 1], cursor[kMaxExperts];
-  const int lane = threadIdx.x & 31, kept = min(entries, kPlanKeep * (int)blockDim.x);
+  const int kept = min(entries, kPlanKeep * (int)blockDim.x);
   for (int e = threadIdx.x; e < E; e += blockDim.x) count[e] = 0;
   __syncthreads();
   pdl_launch_dependents();
@@ -448,12 +449,7 @@ __global__ void __launch_bounds__(1024) expert_plan_kernel(const int32_t* ids, i
 #pragma unroll
   for (int k = 0; k < kPlanKeep; ++k) {
     if (k * (int)blockDim.x >= kept) break;                       // the same for all
-    const int e = mine[k] >= 0 && mine[k] < E ? mine[k] : -1;
-    const uint32_t same = __match_any_sync(0xffffffffu, e);
-    const int leader = __ffs(same) - 1;
-    int base = 0;
-    if (lane == leader && e >= 0) base = atomicAdd(&count[e], __popc(same));
-    place[k] = __shfl_sync(0xffffffffu, base, leader) + __popc(same & ((1u << lane) - 1));
+    place[k] = mine[k] >= 0 && mine[k] < E ? atomicAdd(&count[mine[k]], 1) : 0;
   }
   if (kept < entries) {
     __syncthreads();
@@ -466,6 +462,7 @@ __global__ void __launch_bounds__(1024) expert_plan_kernel(const int32_t* ids, i
   }
   __syncthreads();
   if (threadIdx.x < 32) {
+    const int lane = threadIdx.x;
     int at = 0, tiles = 0;                                        // slots and tiles of the experts before these 32
     for (int e0 = 0; e0 < E; e0 += 32) {
       const int c = e0 + lane < E ? count[e0 + lane] : 0, nt = (c + bm - 1) / bm;
